@@ -59,23 +59,12 @@ template <typename TA, typename TB, typename TC> struct GemmProblem {
 // Bytes of the per-class tile index a launch_gemm_batch of nprobs problems needs.
 inline size_t gemm_index_bytes(size_t nprobs) { return (nprobs + 16) * sizeof(int); }
 
-__device__ __forceinline__ void mac(double& c, double a, double b) { c = fma(a, b, c); }
-__device__ __forceinline__ void mac(cd& c, cd a, double b) {
-    c.x = fma(a.x, b, c.x);
-    c.y = fma(a.y, b, c.y);
+__device__ __forceinline__ cd dress(double x, double ea, double eb, cd z) {
+    const double dx = z.x - (eb - ea), t = x * recip_pos(fma(dx, dx, z.y * z.y));
+    return cd{dx * t, -(z.y * t)};
 }
-__device__ __forceinline__ void mac(cd& c, double a, cd b) {
-    c.x = fma(a, b.x, c.x);
-    c.y = fma(a, b.y, c.y);
-}
-__device__ __forceinline__ void mac(cd& c, cd a, cd b) {
-    c.x = fma(a.x, b.x, c.x);
-    c.x = fma(-a.y, b.y, c.x);
-    c.y = fma(a.x, b.y, c.y);
-    c.y = fma(a.y, b.x, c.y);
-}
-template <typename T> __device__ __forceinline__ cd dress(T x, double ea, double eb, cd z) {
-    return tocd(x) * inv_fast(cd{z.x - (eb - ea), z.y});
+__device__ __forceinline__ cd dress(cd x, double ea, double eb, cd z) {
+    return x * inv_fast(cd{z.x - (eb - ea), z.y});
 }
 __device__ __forceinline__ double scale_by(double a, double s) { return a * s; }
 __device__ __forceinline__ cd scale_by(cd a, double s) { return cd{a.x * s, a.y * s}; }
@@ -92,29 +81,86 @@ template <> __device__ __forceinline__ cd zero_of<cd>() { return cd{0.0, 0.0}; }
 
 constexpr int GEMM_BM = 64, GEMM_BN = 64, GEMM_THREADS = 256;
 
-// Tile shapes (BM x BN, outputs per thread): 64x64 (4x4); 16x128, 128x16
-// (1x8, 8x1); 64x32, 64x48, 32x64, 48x64 (4x2, 4x3, 2x4, 3x4); 4x128, 128x4
-// (1x2, 2x1) for products with at most 4 rows or columns, so the skinny
-// products of the anchored G2 do not run in a wide tile.
-// Shared memory is double-buffered: the next k-tile's global loads are issued
-// into registers before the current tile's products, so their latency
-// overlaps the arithmetic, and one barrier per k-tile suffices.
+// ---- FP64 tensor-core step (mma.sync m8n8k4): D += A B for an 8 x 4 A and a
+// 4 x 8 B.  Lane l holds A(l / 4, l % 4), B(l % 4, l / 4) and D(l / 4,
+// 2 (l % 4) + {0, 1}).
+__device__ __forceinline__ void mma_f64(double2& d, double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(d.x), "+d"(d.y)
+        : "d"(a), "d"(b));
+}
+// Accumulator of one 8 x 8 tile: re (and im where an operand is complex).
+struct AccR {
+    double2 re;
+};
+struct AccC {
+    double2 re, im;
+};
+__device__ __forceinline__ void mma_tile(AccR& c, double a, double b) { mma_f64(c.re, a, b); }
+__device__ __forceinline__ void mma_tile(AccC& c, cd a, double b) {
+    mma_f64(c.re, a.x, b);
+    mma_f64(c.im, a.y, b);
+}
+__device__ __forceinline__ void mma_tile(AccC& c, double a, cd b) {
+    mma_f64(c.re, a, b.x);
+    mma_f64(c.im, a, b.y);
+}
+__device__ __forceinline__ void mma_tile(AccC& c, cd a, cd b) {
+    mma_f64(c.re, a.x, b.x);
+    mma_f64(c.im, a.x, b.y);
+    mma_f64(c.re, -a.y, b.y);
+    mma_f64(c.im, a.y, b.x);
+}
+__device__ __forceinline__ void acc_zero(AccR& c) { c.re = double2{0.0, 0.0}; }
+__device__ __forceinline__ void acc_zero(AccC& c) { c.re = c.im = double2{0.0, 0.0}; }
+__device__ __forceinline__ double acc_at(const AccR& c, int u) { return u ? c.re.y : c.re.x; }
+__device__ __forceinline__ cd acc_at(const AccC& c, int u) { return u ? cd{c.re.y, c.im.y} : cd{c.re.x, c.im.x}; }
+
+// Element copies global -> shared without a register in between; the bytes of
+// an element outside the problem are zero-filled (nothing is read).
+__device__ __forceinline__ void cp_elem(double* dst, const double* src, bool in) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(in ? 8 : 0));
+}
+__device__ __forceinline__ void cp_elem(cd* dst, const cd* src, bool in) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(in ? 16 : 0));
+}
+
+// Tile shapes (BM x BN) and the rows of warps that share one (8 warps; a warp
+// has BM / WR rows and BN / (8 / WR) columns, in 8 x 8 tiles of the FP64
+// tensor cores).  Skinny shapes keep the products of a few anchors out of
+// 64-row tiles.
+__host__ __device__ constexpr int gemm_wr(int bm) { return bm <= 16 ? 1 : bm <= 48 ? 2 : bm <= 64 ? 4 : 8; }
+
+// What bounds it: the FP64 pipe (a 64 x 64 complex tile has 16384 fused
+// multiply-adds per k for 128 operand elements).  Shared memory is
+// double-buffered: undressed operands go there by cp.async and dressed ones
+// through registers, both issued before the current k-tile's products.  The
+// leading dimensions (BM + 2 complex, BM + 4 real) put the 4 k x 4 (8) rows
+// that a fragment load touches together in different banks.  Complex x complex
+// 2048^3: 27.4 TFLOP/s (peak of the FP64 tensor path 37); the chi3 of Anderson
+// 1+5 on 32 x 32 duplets, whose products these are: 23.3 ms with scalar FMAs
+// on 4 x 4 register tiles, 17.6 ms so.  Dressed operands in a large product
+// leave the tensor path 60% busy (75% undressed): the rest is the barrier per
+// k-tile between the dressing and the products.
 template <typename TA, typename TB, typename TC, int BM, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 2)
     gemm_tiles_kernel(const GemmProblem<TA, TB, TC>* __restrict__ probs, const int* __restrict__ tile0, int nprobs) {
     using VA = typename val_t<TA>::type;  // operand values as they enter the product
     using VB = typename val_t<TB>::type;
-    using TAcc = typename std::conditional<is_cd<VA>::value || is_cd<VB>::value, cd, double>::type;
-    constexpr int BK = (is_cd<VA>::value || is_cd<VB>::value) ? 8 : 16;
-    // thread grid NY x NX (256 threads), each thread an TM x TN sub-tile
-    constexpr int NX = (BM == 4) ? 64 : (BN == 4) ? 4 : 16;
-    constexpr int NY = GEMM_THREADS / NX;
-    constexpr int TM = BM / NY, TN = BN / NX;
-    static_assert(TM * NY == BM && TN * NX == BN, "tile shape does not fit the thread grid");
+    constexpr bool CX = is_cd<VA>::value || is_cd<VB>::value;
+    using Acc = typename std::conditional<CX, AccC, AccR>::type;
+    constexpr bool DA = is_dressed<TA>::value, DB = is_dressed<TB>::value;
+    constexpr int BK = CX ? 8 : 16;
+    constexpr int WR = gemm_wr(BM), WC = GEMM_THREADS / 32 / WR;
+    constexpr int WM = BM / WR, WN = BN / WC, FM = WM / 8, FN = WN / 8;
+    static_assert(FM * 8 * WR == BM && FN * 8 * WC == BN, "tile shape does not fit the warp grid");
     constexpr int LA = (BM * BK + GEMM_THREADS - 1) / GEMM_THREADS;
     constexpr int LB = (BN * BK + GEMM_THREADS - 1) / GEMM_THREADS;
-    __shared__ VA As[2][BK][BM + 1];
-    __shared__ VB Bs[2][BK][BN + 1];
+    constexpr int LDA = BM + (is_cd<VA>::value ? 2 : 4), LDB = BN + (is_cd<VB>::value ? 2 : 4);
+    __shared__ __align__(16) VA As[2][BK][LDA];
+    __shared__ __align__(16) VB Bs[2][BK][LDB];
 
     // tile0[q] = first tile of problem q (prefix sum); find this CTA's problem
     const int tile = blockIdx.x;
@@ -124,29 +170,28 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2)
         if (tile0[mid] <= tile) lo = mid;
         else hi = mid - 1;
     }
-    GemmProblem<TA, TB, TC> p = probs[lo];
+    const GemmProblem<TA, TB, TC>& p = probs[lo];
     const int tn_count = (p.N + BN - 1) / BN, per_item = ((p.M + BM - 1) / BM) * tn_count;
     const int local = tile - tile0[lo];
     const int item = local / per_item, rem = local % per_item;
     const int i0 = (rem / tn_count) * BM, j0 = (rem % tn_count) * BN;
-    if (item > 0) {
-        p.A += item * p.ba;
-        p.B += item * p.bb;
-        p.C += item * p.bc;
-    }
-    if (p.dzs) p.dz = p.dzs[item];
-    const int tid = threadIdx.x, tx = tid % NX, ty = tid / NX;
+    const auto* pA = p.A + item * p.ba;
+    const auto* pB = p.B + item * p.bb;
+    const int M = p.M, N = p.N, K = p.K;
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    const int wr = warp / WC, wc = warp % WC;
+    cd dz{0.0, 0.0};
+    if constexpr (DA || DB) dz = p.dzs ? p.dzs[item] : p.dz;
 
-    TAcc acc[TM][TN];
+    Acc acc[FM][FN];
 #pragma unroll
-    for (int a = 0; a < TM; ++a)
+    for (int a = 0; a < FM; ++a)
 #pragma unroll
-        for (int b = 0; b < TN; ++b) acc[a][b] = zero_of<TAcc>();
+        for (int b = 0; b < FN; ++b) acc_zero(acc[a][b]);
 
     const bool a_i_fast = (p.sa_i == 1);
     const bool b_j_fast = (p.sb_j == 1);
-    VA ra[LA];
-    VB rb[LB];
+    const bool a_reg = DA || p.conj_a, b_reg = DB || p.kscale != nullptr;
     // position (row or column, k) inside the tile of element l of a k-tile
     auto a_pos = [&](int l, int& ii, int& kk) {
         if (a_i_fast) {
@@ -166,103 +211,130 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2)
             kk = l % BK;
         }
     };
-    auto load = [&](int k0) {
+    using SA = typename src_t<TA>::type;
+    using SB = typename src_t<TB>::type;
+    SA ra[LA];
+    SB rb[LB];
+    double ea[DA || DB ? (DA ? LA : LB) : 1], eb[DA || DB ? (DA ? LA : LB) : 1];
+    // issues the loads of the k-tile at k0 (buffer buf)
+    auto load = [&](int k0, int buf) {
 #pragma unroll
         for (int q = 0; q < LA; ++q) {
             const int l = tid + q * GEMM_THREADS;
-            VA v = zero_of<VA>();
-            if (l < BM * BK) {
+            if (BM * BK % GEMM_THREADS == 0 || l < BM * BK) {
                 int ii, kk;
                 a_pos(l, ii, kk);
                 const int gi = i0 + ii, gk = k0 + kk;
-                if (gi < p.M && gk < p.K) {
-                    const long kq = p.a_kidx ? p.a_kidx[gk] : gk;
-                    const long iq = p.a_iidx ? p.a_iidx[gi] : gi;
-                    if constexpr (is_dressed<TA>::value)
-                        v = dress(p.A[iq * p.sa_i + kq * p.sa_k], p.dEa[iq], p.dEb[kq], p.dz);
-                    else
-                        v = maybe_conj(p.A[iq * p.sa_i + kq * p.sa_k], p.conj_a);
+                const bool in = gi < M && gk < K;
+                long kq = 0, iq = 0;
+                if (in) {
+                    kq = p.a_kidx ? p.a_kidx[gk] : gk;
+                    iq = p.a_iidx ? p.a_iidx[gi] : gi;
+                }
+                const SA* src = pA + iq * p.sa_i + kq * p.sa_k;
+                if constexpr (DA) {
+                    ra[q] = in ? *src : zero_of<SA>();
+                    ea[q] = in ? p.dEa[iq] : 0.0;
+                    eb[q] = in ? p.dEb[kq] : 0.0;
+                } else {
+                    if (a_reg) ra[q] = in ? maybe_conj(*src, 1) : zero_of<SA>();
+                    else cp_elem(&As[buf][kk][ii], src, in);
                 }
             }
-            ra[q] = v;
         }
 #pragma unroll
         for (int q = 0; q < LB; ++q) {
             const int l = tid + q * GEMM_THREADS;
-            VB v = zero_of<VB>();
-            if (l < BN * BK) {
+            if (BN * BK % GEMM_THREADS == 0 || l < BN * BK) {
                 int jj, kk;
                 b_pos(l, jj, kk);
                 const int gj = j0 + jj, gk = k0 + kk;
-                if (gj < p.N && gk < p.K) {
-                    const long kq = p.b_kidx ? p.b_kidx[gk] : gk;
-                    const long jq = p.b_jidx ? p.b_jidx[gj] : gj;
-                    if constexpr (is_dressed<TB>::value) {
-                        v = dress(p.B[kq * p.sb_k + jq * p.sb_j], p.dEa[kq], p.dEb[jq], p.dz);
-                    } else {
-                        v = p.B[kq * p.sb_k + jq * p.sb_j];
-                        if (p.kscale) v = scale_by(v, p.kscale[gk]);
-                    }
+                const bool in = gj < N && gk < K;
+                long kq = 0, jq = 0;
+                if (in) {
+                    kq = p.b_kidx ? p.b_kidx[gk] : gk;
+                    jq = p.b_jidx ? p.b_jidx[gj] : gj;
+                }
+                const SB* src = pB + kq * p.sb_k + jq * p.sb_j;
+                if constexpr (DB) {
+                    rb[q] = in ? *src : zero_of<SB>();
+                    ea[q] = in ? p.dEa[kq] : 0.0;
+                    eb[q] = in ? p.dEb[jq] : 0.0;
+                } else {
+                    if (b_reg) rb[q] = in ? scale_by(*src, p.kscale[gk]) : zero_of<SB>();
+                    else cp_elem(&Bs[buf][kk][jj], src, in);
                 }
             }
-            rb[q] = v;
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto store = [&](int buf) {
+    // stores the register operands of that k-tile (dressed), then waits for its copies
+    auto store = [&](int k0, int buf) {
+        if (a_reg) {
 #pragma unroll
-        for (int q = 0; q < LA; ++q) {
-            const int l = tid + q * GEMM_THREADS;
-            if (l < BM * BK) {
-                int ii, kk;
-                a_pos(l, ii, kk);
-                As[buf][kk][ii] = ra[q];
+            for (int q = 0; q < LA; ++q) {
+                const int l = tid + q * GEMM_THREADS;
+                if (BM * BK % GEMM_THREADS == 0 || l < BM * BK) {
+                    int ii, kk;
+                    a_pos(l, ii, kk);
+                    if constexpr (DA)
+                        As[buf][kk][ii] = i0 + ii < M && k0 + kk < K ? dress(ra[q], ea[q], eb[q], dz) : cd{0.0, 0.0};
+                    else As[buf][kk][ii] = ra[q];
+                }
             }
         }
+        if (b_reg) {
 #pragma unroll
-        for (int q = 0; q < LB; ++q) {
-            const int l = tid + q * GEMM_THREADS;
-            if (l < BN * BK) {
-                int jj, kk;
-                b_pos(l, jj, kk);
-                Bs[buf][kk][jj] = rb[q];
+            for (int q = 0; q < LB; ++q) {
+                const int l = tid + q * GEMM_THREADS;
+                if (BN * BK % GEMM_THREADS == 0 || l < BN * BK) {
+                    int jj, kk;
+                    b_pos(l, jj, kk);
+                    if constexpr (DB)
+                        Bs[buf][kk][jj] = j0 + jj < N && k0 + kk < K ? dress(rb[q], ea[q], eb[q], dz) : cd{0.0, 0.0};
+                    else Bs[buf][kk][jj] = rb[q];
+                }
             }
         }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
     };
 
-    load(0);
-    store(0);
+    load(0, 0);
+    store(0, 0);
     __syncthreads();
     int buf = 0;
-    for (int k0 = 0; k0 < p.K; k0 += BK) {
-        const bool more = k0 + BK < p.K;
-        if (more) load(k0 + BK);
+    for (int k0 = 0; k0 < K; k0 += BK) {
+        const bool more = k0 + BK < K;
+        if (more) load(k0 + BK, buf ^ 1);
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            VA a[TM];
-            VB b[TN];
+        for (int k4 = 0; k4 < BK; k4 += 4) {
+            VA a[FM];
+            VB b[FN];
 #pragma unroll
-            for (int q = 0; q < TM; ++q) a[q] = As[buf][kk][ty + NY * q];
+            for (int q = 0; q < FM; ++q) a[q] = As[buf][k4 + lane % 4][wr * WM + 8 * q + lane / 4];
 #pragma unroll
-            for (int q = 0; q < TN; ++q) b[q] = Bs[buf][kk][tx + NX * q];
+            for (int q = 0; q < FN; ++q) b[q] = Bs[buf][k4 + lane % 4][wc * WN + 8 * q + lane / 4];
 #pragma unroll
-            for (int qa = 0; qa < TM; ++qa)
+            for (int qa = 0; qa < FM; ++qa)
 #pragma unroll
-                for (int qb = 0; qb < TN; ++qb) mac(acc[qa][qb], a[qa], b[qb]);
+                for (int qb = 0; qb < FN; ++qb) mma_tile(acc[qa][qb], a[qa], b[qb]);
         }
-        if (more) store(buf ^ 1);
+        if (more) store(k0 + BK, buf ^ 1);
         __syncthreads();
         buf ^= 1;
     }
+    TC* pC = p.C + item * p.bc;
 #pragma unroll
-    for (int qa = 0; qa < TM; ++qa) {
-        const int gi = i0 + ty + NY * qa;
-        if (gi >= p.M) continue;
+    for (int qa = 0; qa < FM; ++qa) {
+        const int gi = i0 + wr * WM + 8 * qa + lane / 4;
+        if (gi >= M) continue;
 #pragma unroll
-        for (int qb = 0; qb < TN; ++qb) {
-            const int gj = j0 + tx + NX * qb;
-            if (gj >= p.N) continue;
-            store_c(p.C[gi * p.sc_i + gj * p.sc_j], acc[qa][qb], p.accumulate);
-        }
+        for (int qb = 0; qb < FN; ++qb)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int gj = j0 + wc * WN + 8 * qb + 2 * (lane % 4) + u;
+                if (gj < N) store_c(pC[gi * p.sc_i + gj * p.sc_j], acc_at(acc[qa][qb], u), p.accumulate);
+            }
     }
 }
 
@@ -283,8 +355,8 @@ template <typename TA, typename TB, typename TC> const char* gemm_name() {
 // (ties: the larger tile); the classes other than 64x64 are used only when
 // their short side covers the problem's M or N in one tile.
 constexpr int GEMM_NCLS = 9;
-constexpr int GEMM_CLS_M[GEMM_NCLS] = {64, 16, 128, 64, 64, 32, 48, 4, 128};
-constexpr int GEMM_CLS_N[GEMM_NCLS] = {64, 128, 16, 32, 48, 64, 64, 128, 4};
+constexpr int GEMM_CLS_M[GEMM_NCLS] = {64, 16, 128, 64, 64, 32, 48, 8, 128};
+constexpr int GEMM_CLS_N[GEMM_NCLS] = {64, 128, 16, 32, 48, 64, 64, 128, 8};
 
 template <typename P> inline int gemm_class(const P& p) {
     int best = 0;
@@ -305,11 +377,11 @@ template <typename P> inline int gemm_class(const P& p) {
 // ------------------------------------------------------------ tuned class choice
 // A context's table of measured-fastest tile classes (pgx_autotune), keyed by
 // the operand types and the (M, N) size buckets; -1 keeps the padding rule.
-// The bucket bounds are the narrow classes' limits (4, 16, 32, 48), so a class
+// The bucket bounds are the narrow classes' limits (8, 16, 32, 48), so a class
 // measured at a bucket's upper bound is valid for every size in the bucket.
-constexpr int GEMM_BUCKET_REP[GEMM_NBUCKET] = {4, 16, 32, 48, 64, 128, 256};
+constexpr int GEMM_BUCKET_REP[GEMM_NBUCKET] = {8, 16, 32, 48, 64, 128, 256};
 inline int gemm_bucket(int x) {
-    return x <= 4 ? 0 : x <= 16 ? 1 : x <= 32 ? 2 : x <= 48 ? 3 : x <= 64 ? 4 : x <= 128 ? 5 : 6;
+    return x <= 8 ? 0 : x <= 16 ? 1 : x <= 32 ? 2 : x <= 48 ? 3 : x <= 64 ? 4 : x <= 128 ? 5 : 6;
 }
 template <typename T> struct type_code { static constexpr int v = is_cd<T>::value ? 1 : 0; };
 template <typename T> struct type_code<Dressed<T>> { static constexpr int v = 2 + (is_cd<T>::value ? 1 : 0); };
@@ -444,8 +516,8 @@ void launch_gemm_batch(const std::vector<GemmProblem<TA, TB, TC>>& probs, void* 
     launch_gemm_class<TA, TB, TC, 64, 48>(dp, di + istart[4], pstart[4], pstart[5], ntiles[4], st);
     launch_gemm_class<TA, TB, TC, 32, 64>(dp, di + istart[5], pstart[5], pstart[6], ntiles[5], st);
     launch_gemm_class<TA, TB, TC, 48, 64>(dp, di + istart[6], pstart[6], pstart[7], ntiles[6], st);
-    launch_gemm_class<TA, TB, TC, 4, 128>(dp, di + istart[7], pstart[7], pstart[8], ntiles[7], st);
-    launch_gemm_class<TA, TB, TC, 128, 4>(dp, di + istart[8], pstart[8], pstart[9], ntiles[8], st);
+    launch_gemm_class<TA, TB, TC, 8, 128>(dp, di + istart[7], pstart[7], pstart[8], ntiles[7], st);
+    launch_gemm_class<TA, TB, TC, 128, 8>(dp, di + istart[8], pstart[8], pstart[9], ntiles[8], st);
 }
 
 // C = A B through the int8 split scheme (pgx_ozaki.cu): S slices, plain
