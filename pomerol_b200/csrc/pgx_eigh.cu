@@ -9,8 +9,8 @@
 //      with the matrix in distributed shared memory (blocks up to 464 states);
 //      larger blocks: a blocked reduction (panels of 32 columns, trailing
 //      updates and Q by GEMMs) over the whole GPU.  Q is stored column-major.
-//   2. bisect_kernel, one thread per eigenvalue: bisection with Sturm counts
-//      on the unreduced pieces of T (8.4.1).
+//   2. bisect_kernel: multisection with Sturm counts on the unreduced pieces
+//      of T (8.4.1).
 //   3. vector_kernel, one thread per eigenvalue: inverse iteration with a
 //      partial-pivoting tridiagonal LU; ortho_kernel: modified Gram-Schmidt
 //      inside chains of close eigenvalues; eigenvalues are ranked so that the
@@ -474,8 +474,7 @@ __global__ void __launch_bounds__(CL_THREADS) eigh_cluster_kernel(ClusterArgs g)
 // perturbation of T of the size of the Householder stage's own backward
 // error).  Exact degeneracies of H show up as such splits, so eigenvectors of
 // different pieces are orthogonal by support.
-//   * eigenvalues: bisection with Sturm counts, one thread per eigenvalue
-//     (Golub & Van Loan, 8.4.1), as 32-point multisection by one warp;
+//   * eigenvalues: multisection with Sturm counts (Golub & Van Loan, 8.4.1);
 //   * eigenvectors: two steps of inverse iteration, one thread per
 //     eigenvalue (Golub & Van Loan, 8.2.2).  Each solve factors T - lambda I
 //     by Gaussian elimination with partial pivoting.  In a chain of
@@ -535,74 +534,151 @@ __device__ double load_tri(const double* tri, long eo, int n, double* d, double*
     return tn;
 }
 
-__device__ void piece_of(const double* e, int n, int j, int& a, int& b) {
-    a = j;
-    b = j;
-    while (a > 0 && e[a - 1] != 0.0) --a;
-    while (b < n - 1 && e[b] != 0.0) ++b;
+// Eigenvalues by multisection with Sturm counts: `lp` lanes (a power of two)
+// take the counts at lp equally spaced interior points of their eigenvalue's
+// bracketing interval, narrowing it lp + 1-fold a round.  One lane (bisection)
+// needs the fewest counts, 53 sweeps of T per eigenvalue; 32 lanes need
+// 32 x 11 but only 11 in a row.  bisect_lanes() takes as many lanes as keep
+// the GPU's threads busy and no more.
+//
+// A count is the number of sign changes of the leading principal minors
+//   p_i = (d_i - x) p_i-1 - e_i-1^2 p_i-2
+// (Golub & Van Loan, 8.4.1), T scaled by a power of two to norm about one and
+// the pair (p_i, p_i-1) rescaled by a power of two every eight steps: a step
+// grows it at most fivefold and shrinks it at most by the smallest kept e^2,
+// so eight steps stay far inside the double range.  An exact zero counts as
+// positive; the sum over it and its neighbour is that of either sign.  One
+// step is three FP64 operations with one FMA in the dependent chain, where the
+// quotient form has a division there.  64 models of 3 to 6 bath sites
+// (312 832 eigenvalues): 86 -> 4.6 ms; Anderson 1+5 (4096
+// eigenvalues): 0.57 -> 0.18 ms.
+constexpr int BIS_THREADS = 256;
+
+// lanes per eigenvalue for `total` eigenvalues: 148 SMs x 1024 threads
+__host__ inline int bisect_lanes(long total) {
+    int lp = 32;
+    while (lp > 1 && total * lp > 148L * 1024) lp /= 2;
+    return lp;
 }
 
-// Multisection with one warp per eigenvalue: each round the 32 lanes take the
-// Sturm counts at 32 equally spaced interior points of the bracketing
-// interval, narrowing it 33-fold (about 11 rounds to full precision).
-constexpr int BIS_WARPS = 8;  // eigenvalues per CTA
-constexpr int BIS_THREADS = 32 * BIS_WARPS;
-
-// number of eigenvalues of T[a..b] below x
-__device__ int sturm(const double* d, const double* e, int a, int b, double x, double pivmin) {
-    double q = d[a] - x;
-    if (fabs(q) < pivmin) q = -pivmin;
-    int cnt = q < 0.0;
-    for (int i = a + 1; i <= b; ++i) {
-        q = (d[i] - x) - e[i - 1] * (e[i - 1] / q);
-        if (fabs(q) < pivmin) q = -pivmin;
-        cnt += q < 0.0;
+// number of eigenvalues of T[a..b] below x (e2: squared sub-diagonal)
+__device__ int sturm(const double* d, const double* e2, int a, int b, double x) {
+    double p0 = 1.0, p1 = d[a] - x;
+    int h1 = __double2hiint(p1);
+    unsigned cnt = (unsigned)h1 >> 31;
+    auto step = [&](int i) {
+        const double pn = fma(d[i] - x, p1, -(e2[i - 1] * p0));
+        const int hn = __double2hiint(pn);
+        cnt += (unsigned)(hn ^ h1) >> 31;
+        p0 = p1;
+        p1 = pn;
+        h1 = hn;
+    };
+    int i = a + 1;
+    for (; i + 7 <= b; i += 8) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) step(i + u);
+        const int ex = max(h1 & 0x7ff00000, __double2hiint(p0) & 0x7ff00000);
+        const double sc = __hiloint2double(0x7fe00000 - min(ex, 0x7fd00000), 0);
+        p0 *= sc;
+        p1 *= sc;
     }
-    return cnt;
+    for (; i <= b; ++i) step(i);
+    return (int)cnt;
 }
 
-__global__ void __launch_bounds__(BIS_THREADS) bisect_kernel(TriArgs g, const TriItem* bitems) {
+__global__ void __launch_bounds__(BIS_THREADS) bisect_kernel(TriArgs g, const TriItem* bitems, int lp) {
     extern __shared__ double sh[];
+    __shared__ int s_first[BIS_THREADS], s_last[BIS_THREADS];  // split points around each thread's share of the rows
     const TriItem it = bitems[blockIdx.x];
     const int n = g.dims[it.block];
     const long eo = g.eoff[it.block];
     double* d = sh;
     double* e = sh + n;
-    load_tri(g.tri, eo, n, d, e);
-    const int lane = threadIdx.x & 31;
-    const int j = it.j0 + (int)(threadIdx.x >> 5);
-    if (j >= it.j1) return;
-    int a, b;
-    piece_of(e, n, j, a, b);
-    double lo = 1e300, hi = -1e300, em = 0.0;
-    for (int i = a; i <= b; ++i) {
-        const double r = (i > a ? fabs(e[i - 1]) : 0.0) + (i < b ? fabs(e[i]) : 0.0);
-        lo = fmin(lo, d[i] - r);
-        hi = fmax(hi, d[i] + r);
-        if (i < b) em = fmax(em, e[i] * e[i]);
+    const double tn = load_tri(g.tri, eo, n, d, e);
+    const int tid = threadIdx.x, lane = tid & 31;
+    // piece of a row: the nearest split at or before it, and at or after it
+    const int per = (n + BIS_THREADS - 1) / BIS_THREADS;
+    const int c0 = tid * per, c1 = min(n, c0 + per);
+    int fs = -1, ls = n;
+    for (int i = c0; i < c1; ++i)
+        if (i == 0 || e[i - 1] == 0.0) fs = i;
+    for (int i = c1 - 1; i >= c0; --i)
+        if (i == n - 1 || e[i] == 0.0) ls = i;
+    s_first[tid] = fs;
+    s_last[tid] = ls;
+    __syncthreads();
+    for (int o = 1; o < BIS_THREADS; o *= 2) {
+        const int x = tid >= o ? max(s_first[tid], s_first[tid - o]) : s_first[tid];
+        const int y = tid + o < BIS_THREADS ? min(s_last[tid], s_last[tid + o]) : s_last[tid];
+        __syncthreads();
+        s_first[tid] = x;
+        s_last[tid] = y;
+        __syncthreads();
     }
-    const double pivmin = SAFE_MIN * fmax(1.0, em);
+    const int j = it.j0 + tid / lp, gl = tid % lp;
+    const bool active = j < it.j1;
+    int a = 0, b = 0;
+    if (active) {
+        const int t = j / per;
+        for (a = j; a >= t * per && !(a == 0 || e[a - 1] == 0.0); --a) {}
+        if (a < t * per) a = s_first[t - 1];
+        const int end = min(n, (t + 1) * per);
+        for (b = j; b < end && !(b == n - 1 || e[b] == 0.0); ++b) {}
+        if (b == end) b = s_last[t + 1];
+    }
+    // Gershgorin interval of the piece
+    double lo = 1e300, hi = -1e300;
+    if (active)
+        for (int i = a + gl; i <= b; i += lp) {
+            const double r = (i > a ? fabs(e[i - 1]) : 0.0) + (i < b ? fabs(e[i]) : 0.0);
+            lo = fmin(lo, d[i] - r);
+            hi = fmax(hi, d[i] + r);
+        }
+    for (int o = lp / 2; o > 0; o >>= 1) {
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    // scale T to norm [1, 2) and square the sub-diagonal
+    const int te = tn > 0.0 ? max(-1000, min(1000, ilogb(tn))) : 0;
+    const double sc = scalbn(1.0, -te);
+    __syncthreads();
+    for (int i = tid; i < n; i += BIS_THREADS) {
+        const double ei = e[i] * sc;
+        d[i] *= sc;
+        e[i] = ei * ei;
+    }
+    __syncthreads();
+    lo *= sc;
+    hi *= sc;
     const double gn = fmax(fabs(lo), fabs(hi));
-    const double w = 2.0 * EPS * gn + pivmin;
+    const double w = 2.0 * EPS * gn + SAFE_MIN;
     lo -= w;
     hi += w;
-    const double atol = 0.25 * EPS * gn + pivmin;
+    const double atol = 0.25 * EPS * gn + SAFE_MIN;
     const int k = j - a;
-    // every lane holds the same lo, hi: the loop and its exits are warp-uniform
-    for (int round = 0; round < 64; ++round) {
-        if (hi - lo <= atol + 2.0 * EPS * fmin(fabs(lo), fabs(hi))) break;
-        const double step = (hi - lo) / 33.0;
-        if (!(lo + step > lo && lo + step * 32.0 < hi)) break;  // interval at the resolution of doubles
-        const int cnt = sturm(d, e, a, b, lo + step * (lane + 1), pivmin);
+    const unsigned shift = lane / lp * lp, mask = lp == 32 ? 0xffffffffu : (1u << lp) - 1u;
+    const double part = 1.0 / (lp + 1);
+    // the lanes of an eigenvalue hold the same lo, hi; those of a warp leave together
+    for (int round = 0; round < 128; ++round) {
+        const double step = (hi - lo) * part;
+        const bool go = active && hi - lo > atol + 2.0 * EPS * fmin(fabs(lo), fabs(hi)) && lo + step > lo &&
+                        lo + step * lp < hi;  // else converged, or at the resolution of doubles
+        if (!__any_sync(0xffffffffu, go)) break;
+        int cnt = 0;
+        if (go) cnt = sturm(d, e, a, b, lo + step * (gl + 1));
         // counts grow with x: the eigenvalue lies between point `below` and `below + 1`
-        const int below = __popc(__ballot_sync(0xffffffffu, cnt <= k));
-        const double nlo = (below > 0) ? lo + step * below : lo;
-        const double nhi = (below < 32) ? lo + step * (below + 1) : hi;
-        lo = nlo;
-        hi = nhi;
+        const unsigned vote = __ballot_sync(0xffffffffu, go && cnt <= k);
+        if (go) {
+            const int below = __popc((vote >> shift) & mask);
+            const double nlo = (below > 0) ? lo + step * below : lo;
+            const double nhi = (below < lp) ? lo + step * (below + 1) : hi;
+            lo = nlo;
+            hi = nhi;
+        }
     }
-    if (lane == 0) {
-        g.lam[eo + j] = 0.5 * (lo + hi);
+    if (active && gl == 0) {
+        g.lam[eo + j] = scalbn(0.5 * (lo + hi), te);
         g.sb[2 * eo + j] = a;
         g.sb[2 * eo + n + j] = b;
     }
@@ -896,9 +972,15 @@ __global__ void cx_extract_kernel(const int* dims, const long* moff, const long*
 
 }  // namespace
 
+static long total_dim(const std::vector<int>& dims) {
+    long s = 0;
+    for (int n : dims) s += n;
+    return s;
+}
+
 // Work items, largest blocks first: vector_kernel takes TRI_THREADS
-// eigen-indices per CTA, bisect_kernel BIS_WARPS; both lists go into one
-// descriptor upload (vector items, then bisection items).
+// eigen-indices per CTA, bisect_kernel BIS_THREADS / bisect_lanes; both lists
+// go into one descriptor upload (vector items, then bisection items).
 static void tri_plan(const std::vector<int>& dims, std::vector<TriItem>& items, size_t* n_vec = nullptr) {
     std::vector<int> order(dims.size());
     for (size_t b = 0; b < dims.size(); ++b) order[b] = (int)b;
@@ -910,9 +992,9 @@ static void tri_plan(const std::vector<int>& dims, std::vector<TriItem>& items, 
             soff += 4L * dims[b] * TRI_THREADS;
         }
     if (n_vec) *n_vec = items.size();
+    const int per = BIS_THREADS / bisect_lanes(total_dim(dims));
     for (int b : order)
-        for (int j0 = 0; j0 < dims[b]; j0 += BIS_WARPS)
-            items.push_back(TriItem{b, j0, std::min(dims[b], j0 + BIS_WARPS), 0, 0});
+        for (int j0 = 0; j0 < dims[b]; j0 += per) items.push_back(TriItem{b, j0, std::min(dims[b], j0 + per), 0, 0});
 }
 
 constexpr int CL_NCLS = 5;
@@ -1377,7 +1459,7 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
     }
     {
         ProfRange pr("bisect_kernel", st, 0.0, 16.0 * esum + 8.0 * esum + 8.0 * esum);
-        bisect_kernel<<<(unsigned)n_bis, BIS_THREADS, smem_b, st>>>(t, bis_items);
+        bisect_kernel<<<(unsigned)n_bis, BIS_THREADS, smem_b, st>>>(t, bis_items, bisect_lanes(total_dim(dims)));
         check_launch("bisect_kernel");
     }
     {
