@@ -2,20 +2,20 @@
 //
 // Replaces Eigen::SelfAdjointEigenSolver as called by HamiltonianPart::computeImpl
 // (HamiltonianPart.cpp:90-102).  Stages:
-//   1. Householder reduction to tridiagonal form T and explicit accumulation
-//      of the orthogonal factor Q (Golub & Van Loan, "Matrix Computations",
-//      4th ed., 8.3.1):
-//      eigh_cluster_kernel, one thread-block cluster of 1-8 CTAs per block
-//      with the matrix in distributed shared memory (blocks up to 464 states);
+//   1. Householder reduction to tridiagonal form T (Golub & Van Loan, "Matrix
+//      Computations", 4th ed., 8.3.1):
+//      eigh_cluster_kernel, one thread-block cluster of 1-16 CTAs per block
+//      with the matrix in distributed shared memory (blocks up to 513 states);
 //      larger blocks: a blocked reduction (panels of 32 columns, trailing
-//      updates and Q by GEMMs) over the whole GPU.  Q is stored column-major.
+//      updates by GEMMs) over the whole GPU.
 //   2. bisect_kernel: multisection with Sturm counts on the unreduced pieces
 //      of T (8.4.1).
 //   3. vector_kernel, one thread per eigenvalue: inverse iteration with a
 //      partial-pivoting tridiagonal LU; ortho_kernel: modified Gram-Schmidt
 //      inside chains of close eigenvalues; eigenvalues are ranked so that the
 //      output is ascending.
-//   4. U = Q Z as one batched FP64 GEMM over all blocks.
+//   4. the reflectors applied to Z panel by panel (bt_apply_kernel); blocks
+//      beyond 2165 states form Q and U = Q Z by GEMMs.
 // A non-finite eigenvector sets a device status word instead of trapping.
 
 #include <cooperative_groups.h>
@@ -60,12 +60,13 @@ __device__ double block_sum(double v, double* red) {
 // with A the matrix as it was at the start of the panel: the trailing matrix
 // is only read per column (bhh_symv_kernel) and written once per panel,
 // A(k+p:, k+p:) -= V W^T + W V^T, by one GEMM of inner size 2p.
-// The reflectors stay in the columns of A below the diagonal (zeros above),
-// and Q = H_0 ... H_{n-3} is formed panel by panel, from the last one, as
+// The reflectors stay, scaled to tau = 1, in the columns of A below the
+// diagonal (zeros above).  Up to 2165 states the eigenvectors are formed from
+// them directly (bt_apply_kernel); beyond, Q = H_0 ... H_{n-3} is formed panel
+// by panel, from the last one, as
 // Q(k+1:, k+1:) += V (-T) (V^T Q(k+1:, k+1:)), where T is the upper
 // triangular factor of the panel's block reflector I - V T V^T (LAPACK
 // dlarft).  Every such block of a problem advances in the same launches.
-// The outputs (tridiagonal, column-major Q) are those of the cluster kernel.
 constexpr int BHH_NB = 32;  // panel width
 constexpr int BHH_COL_THREADS = 1024;
 constexpr int BHH_SYMV_THREADS = 256;
@@ -181,11 +182,11 @@ __global__ void __launch_bounds__(BHH_COL_THREADS) bhh_col_kernel(BigArgs g) {
             tau[j] = tj;
         }
         __syncthreads();
-        const double tj = hh[0], v0 = hh[1];
+        const double tj = hh[0], v0 = hh[1], st = sqrt(tj);
         for (int r = tid; r < n; r += nt) {
             const double vr = (tj != 0.0 && r > j) ? ((r == j + 1) ? v0 : a[r]) : 0.0;
             a[r] = vr;
-            A[(long)r * n + j] = vr;  // column j of A: zeros down to the diagonal, then v
+            A[(long)r * n + j] = vr * st;  // column j of A: zeros down to the diagonal, then sqrt(tau) v
         }
     }
 }
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(BHH_SYMV_THREADS) bhh_symv_kernel(BigArgs g) {
     }
 }
 
-// the last 2 x 2 of the tridiagonal, and Q = I, per large block
+// the last 2 x 2 of the tridiagonal, and Q = I for the first nact blocks (those that form Q)
 __global__ void bhh_finish_kernel(BigArgs g) {
     const int b = g.big[blockIdx.x];
     const int n = g.dims[b];
@@ -241,11 +242,12 @@ __global__ void bhh_finish_kernel(BigArgs g) {
         g.tri[2 * eo + n - 1] = A[(long)(n - 1) * n + (n - 1)];
         g.tri[2 * eo + n + n - 1] = 0.0;
     }
-    for (long i = threadIdx.x; i < (long)n * n; i += blockDim.x) Z[i] = ((i / n) == (i % n)) ? 1.0 : 0.0;
+    if ((int)blockIdx.x < g.nact)
+        for (long i = threadIdx.x; i < (long)n * n; i += blockDim.x) Z[i] = ((i / n) == (i % n)) ? 1.0 : 0.0;
 }
 
 // -T of every panel's block reflector from its Gram matrix G = V^T V (LAPACK
-// dlarft, forward, columnwise): T_ii = tau_i, T(0:i, i) = -tau_i T(0:i, 0:i) G(0:i, i).
+// dlarft, forward, columnwise; tau = 1): T_ii = 1, T(0:i, i) = -T(0:i, 0:i) G(0:i, i).
 // One warp per (block, panel); lane t owns row t of T.
 __global__ void bhh_tfactor_kernel(BigArgs g) {
     int q = blockIdx.x, bi = 0;
@@ -258,7 +260,6 @@ __global__ void bhh_tfactor_kernel(BigArgs g) {
     const int n = g.dims[g.big[bi]];
     const int k = q * BHH_NB, p = min(BHH_NB, n - 2 - k);
     double* base = g.S + g.boff[bi];
-    const double* tau = base + 2L * BHH_NB * n + n + k;
     const double* G = base + 2L * BHH_NB * n + 2L * n + (long)q * BHH_NB * BHH_NB;
     double* nT = base + 2L * BHH_NB * n + 2L * n + (bhh_panels(n) + q) * BHH_NB * BHH_NB;
     const int t = threadIdx.x;
@@ -268,13 +269,13 @@ __global__ void bhh_tfactor_kernel(BigArgs g) {
 #pragma unroll
     for (int i = 0; i < BHH_NB; ++i) {
         if (i < p) {
-            if (t == i) row[i] = tau[i];
+            if (t == i) row[i] = 1.0;
             if (t < i) {
                 double acc = 0.0;
 #pragma unroll
                 for (int s2 = 0; s2 < BHH_NB; ++s2)
                     if (s2 >= t && s2 < i) acc = fma(row[s2], G[s2 * BHH_NB + i], acc);
-                row[i] = -tau[i] * acc;
+                row[i] = -acc;
             }
         }
     }
@@ -301,13 +302,10 @@ __global__ void bhh_tfactor_kernel(BigArgs g) {
 //   into its copy, and applies B -= v w^T + w v^T to its own rows r >= k+2.
 // A CTA one step ahead writes the other parity's buffers, and cannot get two
 // steps ahead before the others pass the barrier, so no reader is overrun.
-// CTA 0 stores d_k, e_k and sqrt(tau) v (row k of V in global memory).
-// Q = H_0 ... H_{n-3} is then formed from V with the CTAs owning columns
-// j = c (mod C) of Q: a column's update needs only that column, so this
-// phase has no cross-CTA traffic.  The outputs (tridiagonal, column-major Q)
-// are those of the blocked large-block path.
+// CTA 0 stores d_k, e_k and sqrt(tau) v (row k of V in global memory), from
+// which the eigenvectors are formed (bt_apply_kernel).
 constexpr int CL_THREADS = 512;
-constexpr int CL_MAX_DIM = CL_THREADS + 1;  // the prefetch of a reflector uses one element per thread
+constexpr int CL_MAX_DIM = CL_THREADS + 1;
 
 struct ClusterArgs {
     const int* blocks;  // cluster -> block
@@ -316,7 +314,6 @@ struct ClusterArgs {
     const long* eoff;
     const double* H;
     double* V;          // per block n x n: row k holds sqrt(tau_k) v_k in columns k+1..n-1
-    double* Zc;         // per block: Q column-major
     double* tri;
 };
 
@@ -336,8 +333,8 @@ __global__ void __launch_bounds__(CL_THREADS) eigh_cluster_kernel(ClusterArgs g)
     const int n = g.dims[b];
     const long mo = g.moff[b], eo = g.eoff[b];
     const int R = (n + C - 1) / C;
-    const int nrows = (n - c + C - 1) / C;  // rows (and later columns) c, c + C, ...
-    double* slab = sh;                      // R x n rows | later R x n columns of Q
+    const int nrows = (n - c + C - 1) / C;  // rows c, c + C, ...
+    double* slab = sh;                      // R x n rows
     double* v = sh + (size_t)R * n;         // n
     double* w = v + n;                      // n
     double* cur = w + n;                    // n: row k, up to date (this CTA's copy)
@@ -434,37 +431,243 @@ __global__ void __launch_bounds__(CL_THREADS) eigh_cluster_kernel(ClusterArgs g)
         g.tri[2 * eo + n - 1] = elem(n - 1, n - 1);
         g.tri[2 * eo + n + n - 1] = 0.0;
     }
-    __threadfence();
-    cl.sync();  // V is visible to every CTA; no CTA reads another's shared memory after this point
+    cl.sync();  // no CTA reads another's shared memory after this point
+}
 
-    // ---- Q = H_0 ... H_{n-3}, columns j = c + C t of Q in shared memory (column-major)
-    double* Qs = slab;
-    double* u = v;
-    for (long idx = tid; idx < (long)nrows * n; idx += nt) {
-        const int t = (int)(idx / n), i = (int)(idx % n);
-        Qs[idx] = (i == c + C * t) ? 1.0 : 0.0;
+// ----------------------------------------------------------------------------
+// Back-transformation U = H_0 ... H_{n-3} Z without forming Q: panels of
+// BT_NB reflectors as block reflectors I - V T V^T (LAPACK dlarft, reflectors
+// scaled to tau = 1, so T_ii = 1), applied from the last panel to the first.
+// bt_tfactor_kernel forms -T of every panel from its Gram matrix; then each
+// CTA of bt_apply_kernel keeps BT columns of Z in shared memory through all
+// panels (columns of Z are independent), reading the panels from L2:
+//   W = V^T Z,  W <- -T W,  Z += V W, all on the FP64 tensor cores.
+// 2 n^3 operations and two launches for all blocks, against 4/3 n^3 + 2 n^3
+// in 2 n steps of a cluster, or three GEMM launches per panel, and a product
+// Q Z.  What bounds it: the FP64 pipe for the wide classes; reading V (twice
+// per panel) from L2 for the narrow ones.  Anderson 1+5
+// (blocks to 400 states): 0.16 ms, against 0.74 ms of the clusters' time and
+// 0.09 ms of products; 7-site ring (blocks to 1225): 3.6 ms against 11.
+// The reflectors: element (r, k) of V at V[k ks + r rs], zero for r <= k.
+constexpr int BT_NB = 32, BT_THREADS = 256, BT_ROWS = 32;  // reflectors a panel, threads, rows of V a tile
+constexpr int BT_LDV = BT_NB + 4;                          // 4 mod 16 doubles: conflict-free fragment loads
+// Columns of Z per CTA and the largest n whose slab fits 227 KB beside the
+// tiles of V and W: 32 up to 679 states, 16 to 1273, 8 to 2165; larger blocks
+// form Q by GEMMs (launch_big).
+constexpr int BT_NCLS = 3;
+constexpr int BT_COLS[BT_NCLS] = {32, 16, 8};
+constexpr size_t BT_SMEM_MAX = 227 * 1024;
+__host__ __device__ constexpr size_t bt_smem_doubles(int n, int C) {
+    return (size_t)n * (C + 4) + 2 * BT_ROWS * BT_LDV + 2 * BT_NB * (C + 4);
+}
+// the largest n of the last class
+constexpr int BT_MAX_DIM =
+    (int)((BT_SMEM_MAX / sizeof(double) - bt_smem_doubles(0, BT_COLS[BT_NCLS - 1])) / (BT_COLS[BT_NCLS - 1] + 4));
+static int bt_class(int n) {
+    for (int q = 0; q < BT_NCLS; ++q)
+        if (bt_smem_doubles(n, BT_COLS[q]) * sizeof(double) <= BT_SMEM_MAX) return q;
+    return -1;
+}
+__host__ __device__ inline int bt_panels(int n) { return n > 2 ? (n - 2 + BT_NB - 1) / BT_NB : 0; }
+
+struct BtItem {
+    int block, at;    // block; its panel (T factors) or first column (application)
+    int n, by_col;    // size; reflector k is column k (1) or row k (0) of V
+    long moff, toff;  // matrix offset; offset of the block's T factors in T
+};
+
+// tile of BT_ROWS rows of the panel's V from row r0, zero outside it
+__device__ __forceinline__ void bt_load_v(double* dst, const double* V, int by_col, int n, int k0, int r0) {
+    for (int l = threadIdx.x; l < BT_ROWS * BT_NB; l += BT_THREADS) {
+        int r, k;
+        if (by_col) {
+            r = l / BT_NB;
+            k = l % BT_NB;
+        } else {
+            r = l % BT_ROWS;
+            k = l / BT_ROWS;
+        }
+        const int gr = r0 + r, gk = k0 + k;
+        const bool in = gr < n && gk < n - 2 && gr > gk;
+        const double* src = V + (in ? (by_col ? (long)gr * n + gk : (long)gk * n + gr) : 0L);
+        cp_elem(dst + r * BT_LDV + k, src, in);
     }
-    double pre = 0.0;
-    if (n >= 3 && tid < 2) pre = V[(size_t)(n - 3) * n + (n - 2) + tid];
-    for (int k = n - 3; k >= 0; --k) {
-        const int m = n - k - 1;
-        __syncthreads();  // the previous reflector is no longer read
-        if (tid < m) u[tid] = pre;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(BT_THREADS) bt_tfactor_kernel(const BtItem* items, const double* Vall, double* T) {
+    __shared__ __align__(16) double vt[2][BT_ROWS * BT_LDV];
+    __shared__ double G[BT_NB][BT_NB + 1];
+    const BtItem it = items[blockIdx.x];
+    const int n = it.n, k0 = it.at * BT_NB;
+    const double* V = Vall + it.moff;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // G = V^T V: warp -> rows 8 (warp % 4), columns 16 (warp / 4)
+    const int gi = 8 * (warp % 4), gj = 16 * (warp / 4);
+    double2 acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
+    bt_load_v(vt[0], V, it.by_col, n, k0, k0 + 1);
+    int buf = 0;
+    for (int r0 = k0 + 1; r0 < n; r0 += BT_ROWS) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        if (k >= 1 && tid < m + 1) pre = V[(size_t)(k - 1) * n + k + tid];
-        const int t0 = (k + 1 - c + C - 1) / C;
-        for (int t = t0 + wid; t < nrows; t += nw) {
-            double* col = Qs + (size_t)t * n + (k + 1);
-            double s = 0.0;
-            for (int i = lane; i < m; i += 32) s = fma(u[i], col[i], s);
-            s = warp_sum(s);
-            for (int i = lane; i < m; i += 32) col[i] -= u[i] * s;
+        if (r0 + BT_ROWS < n) bt_load_v(vt[buf ^ 1], V, it.by_col, n, k0, r0 + BT_ROWS);
+        const double* v = vt[buf];
+#pragma unroll
+        for (int r = 0; r < BT_ROWS; r += 4) {
+            const double a = v[(r + lane % 4) * BT_LDV + gi + lane / 4];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) mma_f64(acc[u], a, v[(r + lane % 4) * BT_LDV + gj + 8 * u + lane / 4]);
+        }
+        buf ^= 1;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        G[gi + lane / 4][gj + 8 * u + 2 * (lane % 4)] = acc[u].x;
+        G[gi + lane / 4][gj + 8 * u + 2 * (lane % 4) + 1] = acc[u].y;
+    }
+    __syncthreads();
+    if (warp > 0) return;
+    // T(0:i, i) = -T(0:i, 0:i) G(0:i, i), lane t owning row t of T; stored as -T
+    double row[BT_NB];
+#pragma unroll
+    for (int i = 0; i < BT_NB; ++i) row[i] = 0.0;
+#pragma unroll
+    for (int i = 0; i < BT_NB; ++i) {
+        double acc2 = 0.0;
+#pragma unroll
+        for (int s = 0; s < i; ++s) acc2 = fma(row[s], G[s][i], acc2);  // row[s] = 0 for s < lane
+        row[i] = lane == i ? 1.0 : lane < i ? -acc2 : 0.0;
+    }
+    double* out = T + it.toff + (long)it.at * BT_NB * BT_NB;
+#pragma unroll
+    for (int i = 0; i < BT_NB; ++i) out[lane * BT_NB + i] = -row[i];
+}
+
+// Warps: MG groups of 8 MF rows of W, NG of 8 NF columns and two halves of the
+// rows of Z for W = V^T Z; one 8-row strip at a time for Z += V W.
+template <int C>
+__global__ void __launch_bounds__(BT_THREADS) bt_apply_kernel(const BtItem* items, const double* Vall, const double* T,
+                                                               const double* Zall, double* Uall) {
+    constexpr int LDZ = C + 4, NF = C >= 16 ? 2 : 1, NG = C / (8 * NF), MG = 4 / NG, MF = 4 / MG;
+    extern __shared__ __align__(16) double sh[];
+    const BtItem it = items[blockIdx.x];
+    const int n = it.n, c0 = it.at, nc = min(C, n - c0);
+    const double* V = Vall + it.moff;
+    const double* Z = Zall + it.moff;  // column-major
+    double* vt = sh;                            // 2 tiles of V
+    double* W = vt + 2 * BT_ROWS * BT_LDV;      // 2 partial W; the first then holds -T W
+    double* zs = W + 2 * BT_NB * LDZ;           // n x C slab of Z
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int l4 = lane % 4, l8 = lane / 4;
+    for (long l = tid; l < (long)n * C; l += BT_THREADS) {
+        const int c = (int)(l / n), r = (int)(l % n);
+        zs[(long)r * LDZ + c] = c < nc ? Z[(long)(c0 + c) * n + r] : 0.0;
+    }
+    const int half = warp / 4, wm = (warp % 4) / NG * 8 * MF, wn = (warp % 4) % NG * 8 * NF;
+    for (int q = bt_panels(n) - 1; q >= 0; --q) {
+        const int k0 = q * BT_NB, rb = k0 + 1, nt = (n - rb + BT_ROWS - 1) / BT_ROWS;
+        // ---- W = V^T Z
+        double2 w[MF][NF];
+#pragma unroll
+        for (int a = 0; a < MF; ++a)
+#pragma unroll
+            for (int b = 0; b < NF; ++b) w[a][b] = double2{0.0, 0.0};
+        __syncthreads();  // the tiles of V and W are free, the slab is up to date
+        bt_load_v(vt, V, it.by_col, n, k0, rb);
+        for (int t = 0; t < nt; ++t) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            const double* v = vt + (t & 1) * BT_ROWS * BT_LDV;
+            // the last tile of V stays in shared memory for the second sweep
+            if (t + 1 < nt) bt_load_v(vt + ((t + 1) & 1) * BT_ROWS * BT_LDV, V, it.by_col, n, k0, rb + (t + 1) * BT_ROWS);
+#pragma unroll
+            for (int r = 0; r < BT_ROWS / 2; r += 4) {
+                const int rr = half * (BT_ROWS / 2) + r + l4, gr = min(rb + t * BT_ROWS + rr, n - 1);  // V is 0 beyond
+                double a[MF], b[NF];
+#pragma unroll
+                for (int u = 0; u < MF; ++u) a[u] = v[rr * BT_LDV + wm + 8 * u + l8];
+#pragma unroll
+                for (int u = 0; u < NF; ++u) b[u] = zs[(long)gr * LDZ + wn + 8 * u + l8];
+#pragma unroll
+                for (int x = 0; x < MF; ++x)
+#pragma unroll
+                    for (int y = 0; y < NF; ++y) mma_f64(w[x][y], a[x], b[y]);
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < MF; ++x)
+#pragma unroll
+            for (int y = 0; y < NF; ++y)
+                *reinterpret_cast<double2*>(&W[half * BT_NB * LDZ + (wm + 8 * x + l8) * LDZ + wn + 8 * y + 2 * l4]) = w[x][y];
+        __syncthreads();
+        // ---- W <- -T (W_0 + W_1), by the first four warps
+        const double* nT = T + it.toff + (long)q * BT_NB * BT_NB;
+#pragma unroll
+        for (int x = 0; x < MF; ++x)
+#pragma unroll
+            for (int y = 0; y < NF; ++y) w[x][y] = double2{0.0, 0.0};
+        if (half == 0) {
+#pragma unroll
+            for (int k = 0; k < BT_NB; k += 4) {
+                double a[MF], b[NF];
+#pragma unroll
+                for (int u = 0; u < MF; ++u) a[u] = nT[(wm + 8 * u + l8) * BT_NB + k + l4];
+#pragma unroll
+                for (int u = 0; u < NF; ++u) {
+                    const int o = (k + l4) * LDZ + wn + 8 * u + l8;
+                    b[u] = W[o] + W[BT_NB * LDZ + o];
+                }
+#pragma unroll
+                for (int x = 0; x < MF; ++x)
+#pragma unroll
+                    for (int y = 0; y < NF; ++y) mma_f64(w[x][y], a[x], b[y]);
+            }
+        }
+        __syncthreads();
+        if (half == 0)
+#pragma unroll
+            for (int x = 0; x < MF; ++x)
+#pragma unroll
+                for (int y = 0; y < NF; ++y)
+                    *reinterpret_cast<double2*>(&W[(wm + 8 * x + l8) * LDZ + wn + 8 * y + 2 * l4]) = w[x][y];
+        __syncthreads();
+        // ---- Z += V W, tiles of V in reverse, strips of 8 rows: four warps a tile, C / 2 columns each
+        constexpr int HC = C >= 16 ? C / 16 : 1;  // 8-column tiles a warp takes
+        const int strip = 8 * (warp % 4), hc = C >= 16 ? warp / 4 * (C / 2) : 0;
+        const bool mine = C >= 16 || warp < 4;
+        double wb[BT_NB / 4][HC];
+#pragma unroll
+        for (int k = 0; k < BT_NB / 4; ++k)
+#pragma unroll
+            for (int y = 0; y < HC; ++y) wb[k][y] = W[(4 * k + l4) * LDZ + hc + 8 * y + l8];
+        for (int t = nt - 1; t >= 0; --t) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            const double* v = vt + (t & 1) * BT_ROWS * BT_LDV;
+            if (t > 0) bt_load_v(vt + ((t - 1) & 1) * BT_ROWS * BT_LDV, V, it.by_col, n, k0, rb + (t - 1) * BT_ROWS);
+            const int gr = rb + t * BT_ROWS + strip + l8;
+            if (mine) {
+                double2 z[HC];
+#pragma unroll
+                for (int y = 0; y < HC; ++y)
+                    z[y] = gr < n ? *reinterpret_cast<double2*>(&zs[(long)gr * LDZ + hc + 8 * y + 2 * l4]) : double2{0.0, 0.0};
+#pragma unroll
+                for (int k = 0; k < BT_NB / 4; ++k) {
+                    const double a = v[(strip + l8) * BT_LDV + 4 * k + l4];
+#pragma unroll
+                    for (int y = 0; y < HC; ++y) mma_f64(z[y], a, wb[k][y]);
+                }
+                if (gr < n)
+#pragma unroll
+                    for (int y = 0; y < HC; ++y) *reinterpret_cast<double2*>(&zs[(long)gr * LDZ + hc + 8 * y + 2 * l4]) = z[y];
+            }
         }
     }
     __syncthreads();
-    for (long idx = tid; idx < (long)nrows * n; idx += nt) {
-        const int t = (int)(idx / n), i = (int)(idx % n);
-        g.Zc[mo + (long)(c + C * t) * n + i] = Qs[idx];
+    double* U = Uall + it.moff;
+    for (long l = tid; l < (long)n * C; l += BT_THREADS) {
+        const int r = (int)(l / C), c = (int)(l % C);
+        if (c < nc) U[(long)r * n + c0 + c] = zs[(long)r * LDZ + c];
     }
 }
 
@@ -498,7 +701,7 @@ struct TriArgs {
     double* lam;        // per block: eigenvalues, ascending inside each piece
     int* sb;            // per block: 2 n ints (first and last row of the piece)
     int* rank;          // per block: n ints (position in the ascending order)
-    double* Z;          // per block: n x n column-major eigenvectors of T, sorted
+    double *Z, *Zq;     // per block: n x n column-major eigenvectors of T, sorted: Z, or Zq where Q was formed
     double* S;          // per vector_kernel CTA: 4 arrays of n x TRI_THREADS, thread-interleaved
     double* E;          // eigenvalues, ascending
     int* status;
@@ -533,6 +736,7 @@ __device__ double load_tri(const double* tri, long eo, int n, double* d, double*
     __syncthreads();
     return tn;
 }
+
 
 // Eigenvalues by multisection with Sturm counts: `lp` lanes (a power of two)
 // take the counts at lp equally spaced interior points of their eigenvalue's
@@ -802,7 +1006,7 @@ __global__ void __launch_bounds__(TRI_THREADS) vector_kernel(TriArgs g) {
     const double pfloor = (tn > 0.0) ? EPS * tn : 1.0;
     const int* sa = g.sb + 2 * eo;
     const int* sbe = sa + n;
-    double* Zb = g.Z + mo;
+    double* Zb = (n > BT_MAX_DIM ? g.Zq : g.Z) + mo;
     // this thread's working vector and LU diagonals, interleaved with the CTA's other threads
     const int st = blockDim.x;
     double* zt = g.S + it.soff + threadIdx.x;
@@ -861,7 +1065,7 @@ __global__ void __launch_bounds__(TRI_THREADS) ortho_kernel(TriArgs g) {
     const int* sa = g.sb + 2 * eo;
     const int* sbe = sa + n;
     const int* rank = g.rank + eo;
-    double* Zb = g.Z + mo;
+    double* Zb = (n > BT_MAX_DIM ? g.Zq : g.Z) + mo;
     for (int j = it.j0; j < it.j1; ++j) {
         const int a = sa[j], b = sbe[j];
         if (j > a && lam[j] - lam[j - 1] <= ortol) continue;  // not the head of a chain
@@ -1013,13 +1217,65 @@ static int cluster_class(int n) {
     return -1;
 }
 
+// Back-transformation plan: the T factors' items (one per panel), then the
+// column slabs of each class, largest blocks first.  first[q] is where list q
+// starts (0: T factors, 1 + c: class c), first[BT_NCLS + 1] the total; nmax[c]
+// the largest block of class c.
+struct BtPlan {
+    std::vector<BtItem> items;
+    size_t first[BT_NCLS + 2];
+    int nmax[BT_NCLS];
+};
+static BtPlan bt_plan(const std::vector<int>& dims) {
+    std::vector<int> order(dims.size());
+    std::vector<long> moff(dims.size()), toff(dims.size());
+    long m = 0, t = 0;
+    for (size_t b = 0; b < dims.size(); ++b) {
+        order[b] = (int)b;
+        moff[b] = m;
+        toff[b] = t;
+        m += (long)dims[b] * dims[b];
+        if (bt_class(dims[b]) >= 0) t += (long)bt_panels(dims[b]) * BT_NB * BT_NB;
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return dims[x] > dims[y]; });
+    BtPlan p;
+    auto add = [&](int b, int at) {
+        p.items.push_back(BtItem{b, at, dims[b], cluster_class(dims[b]) < 0 ? 1 : 0, moff[b], toff[b]});
+    };
+    p.first[0] = 0;
+    for (int b : order)
+        if (bt_class(dims[b]) >= 0)
+            for (int q = 0; q < bt_panels(dims[b]); ++q) add(b, q);
+    for (int c = 0; c < BT_NCLS; ++c) {
+        p.first[c + 1] = p.items.size();
+        p.nmax[c] = 0;
+        for (int b : order) {
+            if (bt_class(dims[b]) != c) continue;
+            p.nmax[c] = std::max(p.nmax[c], dims[b]);
+            for (int j = 0; j < dims[b]; j += BT_COLS[c]) add(b, j);
+        }
+    }
+    p.first[BT_NCLS + 1] = p.items.size();
+    return p;
+}
+template <int C>
+static void launch_bt_apply(const BtItem* items, size_t n, int nmax, const double* V, const double* T, const double* Z,
+                            double* U, cudaStream_t st) {
+    const size_t smem = bt_smem_doubles(nmax, C) * sizeof(double);
+    PGX_CUDA(cudaFuncSetAttribute(bt_apply_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BT_SMEM_MAX));
+    bt_apply_kernel<C><<<(unsigned)n, BT_THREADS, smem, st>>>(items, V, T, Z, U);
+    check_launch("bt_apply_kernel");
+}
+
 // doubles of vector_kernel scratch (EighDev::S); the large-block path uses
 // the same buffer before the vector stage (a -1 scale vector, then one
 // scratch per large block)
 size_t eigh_vec_scratch_doubles(const std::vector<int>& dims) {
     size_t s = 0, big = 2 * BHH_NB;
     for (int n : dims) {
-        s += 4 * (size_t)n * TRI_THREADS * ((n + TRI_THREADS - 1) / TRI_THREADS);
+        // the vectors' scratch, later the T factors
+        s += std::max(4 * (size_t)n * TRI_THREADS * ((n + TRI_THREADS - 1) / TRI_THREADS),
+                      (size_t)bt_panels(n) * BT_NB * BT_NB);
         if (cluster_class(n) < 0) big += (size_t)bhh_scratch_doubles(n);
     }
     return std::max<size_t>(std::max(s, big), 1);
@@ -1066,7 +1322,8 @@ static size_t big_desc_bytes(const std::vector<int>& dims) {
 size_t eigh_item_bytes(const std::vector<int>& dims) {
     std::vector<TriItem> items;
     tri_plan(dims, items);
-    return items.size() * sizeof(TriItem) + dims.size() * sizeof(int) + big_desc_bytes(dims);
+    return items.size() * sizeof(TriItem) + bt_plan(dims).items.size() * sizeof(BtItem) + dims.size() * sizeof(int) +
+           big_desc_bytes(dims);
 }
 
 size_t eigh_gemm_bytes(const std::vector<int>& dims, size_t* tiles_bytes) {
@@ -1190,14 +1447,18 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
         }
         launch_gemm_batch(probs, d.gemm_probs, probs_cap, d.gemm_tiles, tiles_cap, st);
     }
-    a.nact = nbig;
+    // blocks beyond the direct back-transformation, a prefix of the list
+    int nwide = 0;
+    while (nwide < nbig && bt_class(dims[big[nwide]]) < 0) ++nwide;
+    a.nact = nwide;
     bhh_finish_kernel<<<(unsigned)nbig, 256, 0, st>>>(a);
     check_launch("bhh_finish_kernel");
+    if (nwide == 0) return;
     // ---- Q: Gram matrices and -T of every panel, then the panels from the last
     probs.clear();
     long npan_total = 0;
     long npan_max = 0;
-    for (int i = 0; i < nbig; ++i) {
+    for (int i = 0; i < nwide; ++i) {
         const int n = dims[big[i]];
         const long np = bhh_panels(n);
         npan_max = std::max(npan_max, np);
@@ -1222,13 +1483,12 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
         }
     }
     launch_gemm_batch(probs, d.gemm_probs, probs_cap, d.gemm_tiles, tiles_cap, st);
-    a.nact = nbig;
     bhh_tfactor_kernel<<<(unsigned)npan_total, 32, 0, st>>>(a);
     check_launch("bhh_tfactor_kernel");
     for (long q = npan_max - 1; q >= 0; --q) {
         const int k = (int)q * BHH_NB;
         std::vector<GemmProblem<double, double, double>> py, pt, pu;
-        for (int i = 0; i < nact(k); ++i) {
+        for (int i = 0; i < std::min(nwide, nact(k)); ++i) {
             const int n = dims[big[i]];
             const int p = std::min(BHH_NB, n - 2 - k), m = n - k - 1;
             const double* Vp = d.A + moff[big[i]] + (long)(k + 1) * n + k;
@@ -1305,7 +1565,6 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
     ca.eoff = d.eoff;
     ca.H = d.H;
     ca.V = d.A;
-    ca.Zc = d.Zc;
     ca.tri = d.tri;
     size_t cl_smem[CL_NCLS] = {0, 0, 0, 0, 0};
     PGX_CUDA(cudaFuncSetAttribute(eigh_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CL_SMEM_MAX));
@@ -1344,10 +1603,12 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
         cl_off[q] = lists.size();
         lists.insert(lists.end(), hp.cls[q].begin(), hp.cls[q].end());
     }
+    const BtPlan bt = bt_plan(dims);
+    const size_t lists_at = items.size() * sizeof(TriItem) + bt.items.size() * sizeof(BtItem);
     // large blocks: scratch offsets (doubles into S) and, per panel width p, the
     // column gathers of the panel update [V_0..V_p-1 W_0..W_p-1] and [W.. V..]
     const std::vector<int>& big = hp.global;
-    const size_t lists_end = items.size() * sizeof(TriItem) + lists.size() * sizeof(int);
+    const size_t lists_end = lists_at + lists.size() * sizeof(int);
     const size_t boff_at = (lists_end + 7) & ~size_t(7);
     size_t host_bytes = lists_end;
     std::vector<long> boff;
@@ -1374,13 +1635,16 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
     }
     std::vector<char> host(host_bytes);
     std::memcpy(host.data(), items.data(), items.size() * sizeof(TriItem));
-    std::memcpy(host.data() + items.size() * sizeof(TriItem), lists.data(), lists.size() * sizeof(int));
+    if (!bt.items.empty())
+        std::memcpy(host.data() + items.size() * sizeof(TriItem), bt.items.data(), bt.items.size() * sizeof(BtItem));
+    std::memcpy(host.data() + lists_at, lists.data(), lists.size() * sizeof(int));
     if (!big.empty()) {
         std::memcpy(host.data() + boff_at, boff.data(), boff.size() * sizeof(long));
         std::memcpy(host.data() + boff_at + boff.size() * sizeof(long), kidx.data(), kidx.size() * sizeof(int));
     }
     h2d(d.items, host.data(), host.size(), st);
-    const int* d_lists = reinterpret_cast<const int*>(static_cast<const char*>(d.items) + items.size() * sizeof(TriItem));
+    const BtItem* d_bt = reinterpret_cast<const BtItem*>(static_cast<const TriItem*>(d.items) + items.size());
+    const int* d_lists = reinterpret_cast<const int*>(static_cast<const char*>(d.items) + lists_at);
     const long* d_boff = reinterpret_cast<const long*>(static_cast<const char*>(d.items) + boff_at);
     const int* d_kidx = reinterpret_cast<const int*>(static_cast<const char*>(d.items) + boff_at +
                                                      boff.size() * sizeof(long));
@@ -1443,7 +1707,8 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
     t.lam = d.lam;
     t.sb = d.sb;
     t.rank = d.rank;
-    t.Z = d.A;   // the Householder workspace is free again
+    t.Z = d.Zc;
+    t.Zq = d.A;  // the reflectors are in Q
     t.S = d.S;
     t.E = d.E;
     t.status = d.status;
@@ -1473,10 +1738,32 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
         check_launch("ortho_kernel");
     }
 
-    // U = Q Z: Q column-major (Zc), Z column-major (A), U row-major
+    // the reflectors (A) applied to Z (Zc); the T factors take the vector stage's scratch
+    if (bt.first[1] > 0) {
+        ProfRange pr("bt_tfactor_kernel", st, 0.0, 0.0);
+        bt_tfactor_kernel<<<(unsigned)bt.first[1], BT_THREADS, 0, st>>>(d_bt, d.A, d.S);
+        check_launch("bt_tfactor_kernel");
+    }
+    for (int c = 0; c < BT_NCLS; ++c) {
+        const size_t nit = bt.first[c + 2] - bt.first[c + 1];
+        if (nit == 0) continue;
+        double fl = 0.0, by = 0.0;
+        for (int n : dims)
+            if (bt_class(n) == c) {
+                fl += 2.0 * n * (double)n * n;
+                by += 24.0 * n * (double)n;
+            }
+        ProfRange pr("bt_apply_kernel", st, fl, by);
+        const BtItem* q = d_bt + bt.first[c + 1];
+        if (BT_COLS[c] == 32) launch_bt_apply<32>(q, nit, bt.nmax[c], d.A, d.S, d.Zc, d.U, st);
+        else if (BT_COLS[c] == 16) launch_bt_apply<16>(q, nit, bt.nmax[c], d.A, d.S, d.Zc, d.U, st);
+        else launch_bt_apply<8>(q, nit, bt.nmax[c], d.A, d.S, d.Zc, d.U, st);
+    }
+    // wider blocks: U = Q Z, Q column-major (Zc), Z column-major (A), U row-major
     std::vector<GemmProblem<double, double, double>> probs;
     for (size_t b = 0; b < dims.size(); ++b) {
         const int n = dims[b];
+        if (bt_class(n) >= 0) continue;
         GemmProblem<double, double, double> g{};
         g.A = d.Zc + moff[b];
         g.B = d.A + moff[b];
