@@ -51,7 +51,7 @@ __device__ double block_sum(double v, double* red) {
 
 // ----------------------------------------------------------------------------
 // Householder stage for blocks too large for a cluster's shared memory
-// (n > 464): the blocked reduction of LAPACK's dsytrd / dlatrd (lower).
+// (n > 513): the blocked reduction of LAPACK's dsytrd / dlatrd (lower).
 // Panels of BHH_NB columns.  Column j of the panel that starts at k is first
 // brought up to date with the panel's earlier reflectors,
 //   a = A(j:, j) - V W(j, :)^T - W V(j, :)^T,
@@ -60,25 +60,25 @@ __device__ double block_sum(double v, double* red) {
 // with A the matrix as it was at the start of the panel: the trailing matrix
 // is only read per column (bhh_symv_kernel) and written once per panel,
 // A(k+p:, k+p:) -= V W^T + W V^T, by one GEMM of inner size 2p.
-// The reflectors stay, scaled to tau = 1, in the columns of A below the
-// diagonal (zeros above).  Up to 2165 states the eigenvectors are formed from
+// The reflectors stay, scaled to tau = 1, in the rows of A right of the
+// diagonal (zeros left of it).  Up to 2165 states the eigenvectors are formed from
 // them directly (bt_apply_kernel); beyond, Q = H_0 ... H_{n-3} is formed panel
 // by panel, from the last one, as
 // Q(k+1:, k+1:) += V (-T) (V^T Q(k+1:, k+1:)), where T is the upper
 // triangular factor of the panel's block reflector I - V T V^T (LAPACK
 // dlarft).  Every such block of a problem advances in the same launches.
 constexpr int BHH_NB = 32;  // panel width
-constexpr int BHH_COL_THREADS = 1024;
-constexpr int BHH_SYMV_THREADS = 256;
-constexpr int BHH_SYMV_ROWS = 32;  // trailing rows per symv CTA
+constexpr int BHH_COL_THREADS = 512, BHH_CS = 8;  // at most BHH_CS CTAs of a block per column step
+constexpr int BHH_SYMV_THREADS = 128;
+constexpr int BHH_SYMV_ROWS = 16;  // rows per symv CTA, four per warp
 
+struct BigBlk {
+    long moff, eoff, boff;  // matrix and vector offsets; scratch offset in S (doubles)
+    int n, pad;
+};
 struct BigArgs {
-    const int* big;    // the large blocks, largest first
-    const long* boff;  // per entry of `big`: scratch offset in S (doubles)
-    int nact;          // entries of `big` this launch covers (a prefix)
-    const int* dims;
-    const long* moff;
-    const long* eoff;
+    const BigBlk* blk;  // the large blocks, largest first
+    int nact;           // entries of `blk` this launch covers (a prefix)
     double* A;    // per block n x n row-major working copy of H
     double* Zc;   // per block Q, column-major
     double* S;    // scratch
@@ -89,151 +89,223 @@ struct BigArgs {
 };
 
 // Scratch of one large block, in doubles: V and W (BHH_NB columns of n each),
-// y (n), tau (n), then per panel its Gram matrix and -T (BHH_NB^2 each).
+// y (n), tau (n), then per panel its Gram matrix and -T (BHH_NB^2 each), and
+// the dots of the panel's columns with the reflector (2 BHH_NB).
 __host__ __device__ inline long bhh_panels(int n) { return n > 2 ? (n - 2 + BHH_NB - 1) / BHH_NB : 0; }
 __host__ __device__ inline long bhh_scratch_doubles(int n) {
-    return 2L * BHH_NB * n + 2L * n + 2 * bhh_panels(n) * BHH_NB * BHH_NB;
+    return 2L * BHH_NB * n + 2L * n + 2 * bhh_panels(n) * BHH_NB * BHH_NB + 2 * BHH_NB;
 }
+__host__ __device__ inline long bhh_dots_at(int n) { return bhh_scratch_doubles(n) - 2 * BHH_NB; }
 
-__global__ void __launch_bounds__(BHH_COL_THREADS) bhh_col_kernel(BigArgs g) {
+// Completes w of column fin (in this panel) and reflects column col = fin + 1,
+// a cluster of CTAs per block, each with a share of the rows.  Both need every
+// row's combination of the panel's earlier V and W columns, so one sweep reads
+// them for both (four lanes a row, each a quarter of the columns, all loads in
+// flight at once): the new column is formed but for the term in the w being
+// completed, which follows once the cluster knows w . v.  Sums and single
+// elements are pushed into the other CTAs ahead of the barrier; W is written
+// after the last barrier, which would wait for it.  What bounds it: the
+// latency of a chain of L2 reads, two barriers and two block sums.  7-site
+// ring (12 blocks to 1225 states), with the product kernel: 34 -> 20 us a
+// column against one CTA of 1024 threads per block reading V and W three times.
+__global__ void __launch_bounds__(BHH_COL_THREADS, 2) bhh_col_kernel(BigArgs g) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ double sh[];
     __shared__ double red[32];
-    __shared__ double dots[2 * BHH_NB];
-    __shared__ double sv[BHH_NB], sw[BHH_NB];
-    __shared__ double hh[2];
-    const int b = g.big[blockIdx.x];
-    const int n = g.dims[b];
-    double* A = g.A + g.moff[b];
-    double* V = g.S + g.boff[blockIdx.x];  // column t at V + t n
+    __shared__ double dw[BHH_NB], dv[BHH_NB], jw[BHH_NB], jv[BHH_NB];
+    __shared__ double slot_w[BHH_CS], slot_x[BHH_CS], s_wj, s_x[2];  // pushed by the other CTAs
+    const int CS = (int)cl.num_blocks(), c = (int)cl.block_rank();
+    cudaTriggerProgrammaticLaunchCompletion();
+    const BigBlk bl = g.blk[blockIdx.x / CS];
+    const int n = bl.n, last = n - 3;  // the last column with a reflector
+    double* A = g.A + bl.moff;
+    double* V = g.S + bl.boff;  // column t at V + t n
     double* W = V + (long)BHH_NB * n;
     const double* y = W + (long)BHH_NB * n;
     double* tau = W + (long)BHH_NB * n + n;
-    const long eo = g.eoff[b];
-    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5, nw = nt >> 5;
-    const int last = n - 3;  // the last column with a reflector
-    // ---- complete w of column fin
-    if (g.fin >= 0 && g.fin <= last) {
-        const int f = g.fin, cf = f - g.k;
-        const double* v = V + (long)cf * n;
-        double* w = W + (long)cf * n;
-        const double t = tau[f];
-        if (t == 0.0) {
-            for (int r = tid; r < n; r += nt) w[r] = 0.0;
-        } else {
-            // dots[2s] = W_s . v, dots[2s + 1] = V_s . v (v vanishes above row f + 1)
-            for (int q = wid; q < 2 * cf; q += nw) {
-                const double* x = ((q & 1) ? V : W) + (long)(q >> 1) * n;
-                double acc = 0.0;
-                for (int r = f + 1 + lane; r < n; r += 32) acc = fma(x[r], v[r], acc);
-                acc = warp_sum(acc);
-                if (lane == 0) dots[q] = acc;
-            }
-            __syncthreads();
-            double part = 0.0;
-            for (int r = tid; r < n; r += nt) {
-                double wr = 0.0;
-                if (r > f) {
-                    double acc = y[r];
-                    for (int s2 = 0; s2 < cf; ++s2)
-                        acc -= V[(long)s2 * n + r] * dots[2 * s2] + W[(long)s2 * n + r] * dots[2 * s2 + 1];
-                    wr = t * acc;
-                    part = fma(wr, v[r], part);
-                }
-                w[r] = wr;
-            }
-            const double K = 0.5 * t * block_sum(part, red);  // its barriers order the writes of w above
-            for (int r = f + 1 + tid; r < n; r += nt) w[r] -= K * v[r];
-        }
-        __syncthreads();
+    const double* dots = V + bhh_dots_at(n);
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const bool fin = g.fin >= 0 && g.fin <= last, col = g.col >= 0 && g.col <= last;
+    const int f = g.fin, j = g.col, cf = fin ? f - g.k : 0, cc = col ? j - g.k : 0;
+    const int share = (n + CS - 1) / CS, r0 = c * share, r1 = min(n, r0 + share);
+    double *xs = sh, *ws = sh + share, *vs = sh + 2 * share;
+    if (CS > 1) cl.barrier_arrive();  // waited for ahead of the first push
+    cudaGridDependencySynchronize();
+    double tf = 0.0;
+    if (fin) tf = tau[f];
+    if (tid < cf) {
+        dw[tid] = dots[2 * tid];
+        dv[tid] = dots[2 * tid + 1];
+        jw[tid] = col ? W[(long)tid * n + j] : 0.0;
+        jv[tid] = col ? V[(long)tid * n + j] : 0.0;
     }
-    // ---- reflect column col
-    if (g.col >= 0 && g.col <= last) {
-        const int j = g.col, cc = j - g.k;
-        for (int s2 = tid; s2 < cc; s2 += nt) {
-            sv[s2] = V[(long)s2 * n + j];
-            sw[s2] = W[(long)s2 * n + j];
-        }
-        __syncthreads();
-        double* a = V + (long)cc * n;         // the updated column, then the reflector, in place
-        const double* Arow = A + (long)j * n;  // row j holds column j (A symmetric)
-        double part = 0.0;
-        for (int r = tid; r < n; r += nt) {
-            double x = 0.0;
-            if (r >= j) {
-                x = Arow[r];
-                for (int s2 = 0; s2 < cc; ++s2) x -= V[(long)s2 * n + r] * sw[s2] + W[(long)s2 * n + r] * sv[s2];
-                if (r >= j + 2) part = fma(x, x, part);
+    if (CS > 1) cl.barrier_wait();
+    __syncthreads();
+    const double* vf = V + (long)cf * n;
+    const int sg = lane >> 3;
+    double part = 0.0;
+    for (int rb = r0 + 8 * wid; rb < r1; rb += 8 * (BHH_COL_THREADS / 32)) {
+        const int r = rb + (lane & 7);
+        double x = 0.0, acc = 0.0, v = 0.0;
+        if (r < r1) {
+            if (sg == 0 && col && r >= j) x = A[(long)j * n + r];  // row j holds column j (A symmetric)
+            if (sg == 0 && fin && r > f) {
+                acc = y[r];
+                v = vf[r];
             }
-            a[r] = x;
-        }
-        const double sigma = block_sum(part, red);
-        if (tid == 0) {
-            const double x0 = a[j + 1];
-            double alpha = x0, tj = 0.0, v0 = 0.0;
-            if (sigma != 0.0) {
-                const double mu = sqrt(x0 * x0 + sigma);
-                alpha = (x0 > 0.0) ? -mu : mu;  // v0 = x0 - alpha without cancellation
-                v0 = x0 - alpha;
-                tj = 2.0 / (sigma + v0 * v0);
+            double pv[BHH_NB / 4], pw[BHH_NB / 4];
+#pragma unroll
+            for (int q = 0; q < BHH_NB / 4; ++q) {
+                const int s = sg + 4 * q;
+                pv[q] = s < cf ? V[(long)s * n + r] : 0.0;
+                pw[q] = s < cf ? W[(long)s * n + r] : 0.0;
             }
-            hh[0] = tj;
-            hh[1] = v0;
-            g.tri[2 * eo + j] = a[j];
-            g.tri[2 * eo + n + j] = alpha;
+#pragma unroll
+            for (int q = 0; q < BHH_NB / 4; ++q) {
+                const int s = sg + 4 * q;
+                if (s < cf) {
+                    acc -= pv[q] * dw[s] + pw[q] * dv[s];
+                    x -= pv[q] * jw[s] + pw[q] * jv[s];
+                }
+            }
+        }
+#pragma unroll
+        for (int o = 8; o < 32; o <<= 1) {
+            acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            x += __shfl_xor_sync(0xffffffffu, x, o);
+        }
+        if (sg == 0 && r < r1) {
+            const double w = fin && r > f ? tf * acc : 0.0;
+            part = fma(w, v, part);
+            xs[r - r0] = col && r >= j ? x : 0.0;
+            ws[r - r0] = w;
+            vs[r - r0] = v;
+            if (fin && col && r == j)
+                for (int q = 0; q < CS; ++q) *cl.map_shared_rank(&s_wj, q) = w;
+        }
+    }
+    double K = 0.0, wj = 0.0, vj = 0.0;
+    if (fin) {
+        if (col) vj = vf[j];
+        part = block_sum(part, red);
+        if (tid < CS) cl.map_shared_rank(slot_w, tid)[c] = part;
+        if (CS > 1) cl.sync();
+        else __syncthreads();
+        for (int q = 0; q < CS; ++q) K += slot_w[q];
+        K *= 0.5 * tf;
+        if (col) wj = s_wj - K * vj;
+    } else {
+        __syncthreads();  // the sweep's rows are in place
+    }
+    double tj = 0.0, v0 = 0.0;
+    if (col) {
+        part = 0.0;
+        for (int r = r0 + tid; r < r1; r += BHH_COL_THREADS) {
+            double x = xs[r - r0];
+            if (fin && r >= j) {
+                const double v = vs[r - r0];
+                x -= v * wj + (ws[r - r0] - K * v) * vj;
+                xs[r - r0] = x;
+            }
+            if (r >= j + 2) part = fma(x, x, part);
+            if (r == j || r == j + 1)
+                for (int q = 0; q < CS; ++q) cl.map_shared_rank(s_x, q)[r - j] = x;
+        }
+        part = block_sum(part, red);
+        if (tid < CS) cl.map_shared_rank(slot_x, tid)[c] = part;
+        if (CS > 1) cl.sync();
+        else __syncthreads();
+        double sigma = 0.0;
+        for (int q = 0; q < CS; ++q) sigma += slot_x[q];
+        const double x0 = s_x[1];
+        double alpha = x0;
+        v0 = x0;
+        if (sigma != 0.0) {
+            const double t = fma(x0, x0, sigma), mu = t * rsqrt(t);
+            alpha = (x0 > 0.0) ? -mu : mu;  // v0 = x0 - alpha without cancellation
+            v0 = x0 - alpha;
+            tj = 2.0 * recip_pos(fma(v0, v0, sigma));
+        }
+        if (c == 0 && tid == 0) {
+            g.tri[2 * bl.eoff + j] = s_x[0];
+            g.tri[2 * bl.eoff + n + j] = alpha;
             tau[j] = tj;
         }
-        __syncthreads();
-        const double tj = hh[0], v0 = hh[1], st = sqrt(tj);
-        for (int r = tid; r < n; r += nt) {
-            const double vr = (tj != 0.0 && r > j) ? ((r == j + 1) ? v0 : a[r]) : 0.0;
-            a[r] = vr;
-            A[(long)r * n + j] = vr * st;  // column j of A: zeros down to the diagonal, then sqrt(tau) v
+    }
+    const double st = sqrt(tj);
+    for (int r = r0 + tid; r < r1; r += BHH_COL_THREADS) {
+        if (fin) W[(long)cf * n + r] = ws[r - r0] - K * vs[r - r0];
+        if (col) {
+            const double vr = (tj != 0.0 && r > j) ? ((r == j + 1) ? v0 : xs[r - r0]) : 0.0;
+            V[(long)cc * n + r] = vr;
+            A[(long)j * n + r] = vr * st;  // row j of A: zeros up to the diagonal, then sqrt(tau) v
         }
     }
 }
 
-// y(j+1:) = A(j+1:, j+1:) v for column j = col of every active block; one
-// warp per row, the CTAs of the active blocks in one flat grid.
+// y(j+1:) = A(j+1:, j+1:) v for column j = col of every active block, and the
+// dots W_s . v, V_s . v of the panel's earlier columns as further rows; grid
+// (rows, block), four rows per warp (each entry of v is loaded once for the
+// four, and eight row loads are in flight per lane).  What bounds it: reading
+// the trailing matrix, from L2 where the active blocks fit, else from HBM.
+// 64 models of 3 to 6 bath sites, whose large blocks exceed L2: 102 ms for all
+// columns, 4.4 TB/s, against 131 with one row and two loads per lane.
 __global__ void __launch_bounds__(BHH_SYMV_THREADS) bhh_symv_kernel(BigArgs g) {
-    extern __shared__ double svec[];
-    int q = blockIdx.x, bi = 0, m = 0;
-    for (; bi < g.nact; ++bi) {
-        m = g.dims[g.big[bi]] - g.col - 1;
-        const int cnt = (m + BHH_SYMV_ROWS - 1) / BHH_SYMV_ROWS;
-        if (q < cnt) break;
-        q -= cnt;
-    }
-    if (bi >= g.nact) return;
-    const int b = g.big[bi];
-    const int n = g.dims[b], j = g.col, cc = j - g.k;
-    const double* A = g.A + g.moff[b];
-    const double* v = g.S + g.boff[bi] + (long)cc * n + (j + 1);
-    double* y = g.S + g.boff[bi] + 2L * BHH_NB * n + (j + 1);
-    for (int c = threadIdx.x; c < m; c += blockDim.x) svec[c] = v[c];
-    __syncthreads();
+    cudaTriggerProgrammaticLaunchCompletion();
+    const BigBlk bl = g.blk[blockIdx.y];
+    const int n = bl.n, j = g.col, cc = j - g.k, m = n - j - 1, rows = m + 2 * cc;
+    double* V = g.S + bl.boff;
+    const double* v = V + (long)cc * n + (j + 1);
+    double* y = V + 2L * BHH_NB * n + (j + 1);
+    double* dots = V + bhh_dots_at(n);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int rr = wid; rr < BHH_SYMV_ROWS; rr += BHH_SYMV_THREADS / 32) {
-        const int r = q * BHH_SYMV_ROWS + rr;
-        if (r >= m) break;
-        const double* row = A + (long)(j + 1 + r) * n + (j + 1);
-        double s0 = 0.0, s1 = 0.0;
-        int c = lane;
-        for (; c + 32 < m; c += 64) {
-            s0 = fma(row[c], svec[c], s0);
-            s1 = fma(row[c + 32], svec[c + 32], s1);
+    const int rr = blockIdx.x * BHH_SYMV_ROWS + wid * 4;
+    if (rr >= rows) return;
+    const double* p[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int r = min(rr + u, rows - 1), d = r - m;
+        p[u] = r < m ? g.A + bl.moff + (long)(j + 1 + r) * n + (j + 1)
+                     : V + ((d & 1) ? 0L : (long)BHH_NB * n) + (long)(d >> 1) * n + (j + 1);
+    }
+    cudaGridDependencySynchronize();
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    int i = lane;
+    for (; i + 32 < m; i += 64) {
+        const double v0 = v[i], v1 = v[i + 32];
+        double a[4], e[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            a[u] = p[u][i];
+            e[u] = p[u][i + 32];
         }
-        if (c < m) s0 = fma(row[c], svec[c], s0);
-        const double sum = warp_sum(s0 + s1);
-        if (lane == 0) y[r] = sum;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s[u] = fma(e[u], v1, fma(a[u], v0, s[u]));
+    }
+    if (i < m) {
+        const double v0 = v[i];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s[u] = fma(p[u][i], v0, s[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const double t = warp_sum(s[u]);
+        const int r = rr + u;
+        if (lane == 0 && r < rows) {
+            if (r < m) y[r] = t;
+            else dots[r - m] = t;
+        }
     }
 }
 
 // the last 2 x 2 of the tridiagonal, and Q = I for the first nact blocks (those that form Q)
 __global__ void bhh_finish_kernel(BigArgs g) {
-    const int b = g.big[blockIdx.x];
-    const int n = g.dims[b];
-    const double* A = g.A + g.moff[b];
-    double* Z = g.Zc + g.moff[b];
-    const long eo = g.eoff[b];
+    const BigBlk bl = g.blk[blockIdx.x];
+    const int n = bl.n;
+    const double* A = g.A + bl.moff;
+    double* Z = g.Zc + bl.moff;
+    const long eo = bl.eoff;
     if (threadIdx.x == 0) {
         if (n >= 2) {
             g.tri[2 * eo + n - 2] = A[(long)(n - 2) * n + (n - 2)];
@@ -252,14 +324,14 @@ __global__ void bhh_finish_kernel(BigArgs g) {
 __global__ void bhh_tfactor_kernel(BigArgs g) {
     int q = blockIdx.x, bi = 0;
     for (; bi < g.nact; ++bi) {
-        const int np = (int)bhh_panels(g.dims[g.big[bi]]);
+        const int np = (int)bhh_panels(g.blk[bi].n);
         if (q < np) break;
         q -= np;
     }
     if (bi >= g.nact) return;
-    const int n = g.dims[g.big[bi]];
+    const int n = g.blk[bi].n;
     const int k = q * BHH_NB, p = min(BHH_NB, n - 2 - k);
-    double* base = g.S + g.boff[bi];
+    double* base = g.S + g.blk[bi].boff;
     const double* G = base + 2L * BHH_NB * n + 2L * n + (long)q * BHH_NB * BHH_NB;
     double* nT = base + 2L * BHH_NB * n + 2L * n + (bhh_panels(n) + q) * BHH_NB * BHH_NB;
     const int t = threadIdx.x;
@@ -285,27 +357,33 @@ __global__ void bhh_tfactor_kernel(BigArgs g) {
 
 // ----------------------------------------------------------------------------
 // Householder stage on a thread-block cluster (blocks whose matrix fits in
-// the shared memory of up to 8 CTAs: 464 states at 220 KB per CTA).
+// the shared memory of up to 16 CTAs, 513 states).
 //
 // The C CTAs of a cluster hold the block's symmetric matrix in distributed
 // shared memory, row r in CTA r mod C (cyclic, so the shrinking trailing
-// matrix stays spread over all CTAs).  Every CTA also keeps its own copy of
-// the current row k (the column below the diagonal), brought up to date
-// locally, so one cluster barrier per step suffices.  Step k:
-//   every CTA forms the Householder vector v, tau from its copy of row k,
-//   computes p = tau B v on its own rows and its share of v.p (into the
-//   buffers of this step's parity);
+// matrix stays spread over all CTAs).  Every CTA also holds the current row k
+// (the column below the diagonal), up to date, one element per thread.  Step k:
+//   every CTA forms the Householder vector v and tau from its copy of row k;
+//   one sweep over its own rows r > k applies the PREVIOUS step's update
+//   B -= v' w'^T + w' v'^T and forms p = tau B v with the result (up to eight
+//   rows per warp, whose sums over the lanes share five shuffle rounds), and the
+//   warp pushes p_r and the row's element in column k + 1 into every CTA's
+//   buffer of this step's parity;
 //   cluster barrier;
-//   every CTA gathers all of p and the v.p shares, forms
-//   w = p - (tau/2)(v.p) v, reads row k+1 from its owner (who leaves that
-//   row alone in this step: it leaves the trailing matrix) and updates it
-//   into its copy, and applies B -= v w^T + w v^T to its own rows r >= k+2.
-// A CTA one step ahead writes the other parity's buffers, and cannot get two
-// steps ahead before the others pass the barrier, so no reader is overrun.
+//   every CTA forms w = p - (tau/2)(v.p) v and from the pushed column its copy
+//   of row k + 1, less v_{k+1} w + w_{k+1} v.
+// So the matrix is read and written once per step, nothing is fetched from
+// another CTA after the barrier, and a step has one cluster barrier and three
+// CTA barriers.  A CTA one step ahead writes the other parity's buffers, and
+// cannot get two steps ahead before the others pass the barrier.  What bounds
+// it: those barriers and the push in large part, then shared-memory reads.
 // CTA 0 stores d_k, e_k and sqrt(tau) v (row k of V in global memory), from
-// which the eigenvectors are formed (bt_apply_kernel).
-constexpr int CL_THREADS = 512;
-constexpr int CL_MAX_DIM = CL_THREADS + 1;
+// which the eigenvectors are formed (bt_apply_kernel).  Anderson 1+5, the
+// 400-state block: 1.16 ms, against 2.04 with a fetch from the other CTAs after
+// the barrier and a sweep each for the update and the product.
+constexpr int CL_THREADS = 256, CL_NW = CL_THREADS / 32;
+constexpr int CL_MAX_DIM = 513;
+constexpr int CL_EL = (CL_MAX_DIM + CL_THREADS - 1) / CL_THREADS;  // elements of a row per thread
 
 struct ClusterArgs {
     const int* blocks;  // cluster -> block
@@ -319,119 +397,192 @@ struct ClusterArgs {
 
 __host__ __device__ inline size_t cluster_smem_doubles(int n, int C) {
     const int R = (n + C - 1) / C;
-    return (size_t)R * n + 3 * (size_t)n + 2 * (size_t)R + 2;
+    return (size_t)R * n + 7 * (size_t)n;
 }
 
 __global__ void __launch_bounds__(CL_THREADS) eigh_cluster_kernel(ClusterArgs g) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
-    extern __shared__ double sh[];
-    __shared__ double red[32];
+    extern __shared__ __align__(16) double sh[];
+    __shared__ double red[2][CL_NW], s_dot[2][CL_NW], s_x[2];
     const int C = (int)cl.num_blocks();
     const int c = (int)cl.block_rank();
     const int b = g.blocks[blockIdx.x / C];
     const int n = g.dims[b];
     const long mo = g.moff[b], eo = g.eoff[b];
-    const int R = (n + C - 1) / C;
-    const int nrows = (n - c + C - 1) / C;  // rows c, c + C, ...
-    double* slab = sh;                      // R x n rows
-    double* v = sh + (size_t)R * n;         // n
-    double* w = v + n;                      // n
-    double* cur = w + n;                    // n: row k, up to date (this CTA's copy)
-    double* pb = cur + n;                   // 2 R: p of the steps of either parity
-    double* dslot = pb + 2 * R;             // 2
-    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5, nw = nt >> 5;
+    const int nrows = (n - c + C - 1) / C;                // rows c, c + C, ...
+    double2* pb = reinterpret_cast<double2*>(sh);         // 2 n: (p_r, element of column k + 1) by parity
+    double* v = sh + 4 * n;                               // 2 n: v by parity
+    double* w = v + 2 * n;                                // n
+    double* slab = w + n;                                 // nrows x n
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const double* Hb = g.H + mo;
     double* V = g.V + mo;
 
-    for (long idx = tid; idx < (long)nrows * n; idx += nt) {
-        const int lr = (int)(idx / n), j = (int)(idx % n);
+    for (int idx = tid; idx < nrows * n; idx += CL_THREADS) {
+        const int lr = idx / n, j = idx % n;
         slab[idx] = Hb[(long)(c + C * lr) * n + j];
     }
-    for (int j = tid; j < n; j += nt) cur[j] = Hb[j];  // row 0
-    __syncthreads();
-    for (int k = 0; k + 2 < n; ++k) {
-        const int m = n - k - 1;
-        double* p = pb + (k & 1) * R;
-        double part = 0.0;
-        for (int i = tid; i < m; i += nt) {
-            const double x = cur[k + 1 + i];
-            v[i] = x;
-            if (i > 0) part += x * x;
+    double x[CL_EL];  // this thread's elements (columns tid + CL_THREADS e) of row k
+#pragma unroll
+    for (int e = 0; e < CL_EL; ++e) {
+        const int r = tid + CL_THREADS * e;
+        x[e] = r < n ? Hb[r] : 0.0;
+        if (r < n) {
+            w[r] = 0.0;
+            v[n + r] = 0.0;  // the step before the first
         }
-        const double sigma = block_sum(part, red);
-        const double x0 = v[0];
-        const double dk = cur[k];
+    }
+    cl.sync();  // every CTA of the cluster runs before the first push
+    for (int k = 0; k + 2 < n; ++k) {
+        const int par = k & 1;
+        double *vk = v + par * n, *vo = v + (par ^ 1) * n;
+        double part = 0.0;
+#pragma unroll
+        for (int e = 0; e < CL_EL; ++e) {
+            const int r = tid + CL_THREADS * e;
+            if (r < n && r >= k + 2) part = fma(x[e], x[e], part);
+            if (r == k + 1) s_x[par] = x[e];
+        }
+        part = warp_sum(part);
+        if (lane == 0) red[par][wid] = part;
+        __syncthreads();  // also: w of the previous step is complete
+        double sigma = 0.0;
+#pragma unroll
+        for (int q = 0; q < CL_NW; ++q) sigma += red[par][q];
+        const double x0 = s_x[par];
         double tau = 0.0, alpha = x0, v0 = x0;
         if (sigma != 0.0) {
-            const double mu = sqrt(x0 * x0 + sigma);
+            const double t = fma(x0, x0, sigma), mu = t * rsqrt(t);
             alpha = (x0 > 0.0) ? -mu : mu;  // v0 = x0 - alpha without cancellation
             v0 = x0 - alpha;
-            tau = 2.0 / (sigma + v0 * v0);
+            tau = 2.0 * recip_pos(fma(v0, v0, sigma));
+        }
+#pragma unroll
+        for (int e = 0; e < CL_EL; ++e) {
+            const int r = tid + CL_THREADS * e;
+            if (r < n) vk[r] = r > k + 1 ? x[e] : r == k + 1 ? v0 : 0.0;
         }
         __syncthreads();
-        if (tid == 0) v[0] = v0;
-        __syncthreads();
-        // p = tau B v on own rows r >= k+1 (one warp per row)
-        const int lr0 = (k + 1 - c + C - 1) / C;
-        double dpart = 0.0;
-        for (int lr = lr0 + wid; lr < nrows; lr += nw) {
-            const double* row = slab + (size_t)lr * n + (k + 1);
-            double sacc = 0.0;
-            for (int j = lane; j < m; j += 32) sacc = fma(row[j], v[j], sacc);
-            sacc = warp_sum(sacc) * tau;
-            if (lane == 0) {
-                p[lr] = sacc;
-                dpart += v[c + C * lr - (k + 1)] * sacc;
+        // ---- own rows r > k: previous update, then p = tau B v; up to eight rows a warp at once
+        const int m = n - k - 1;
+        const double *pn = vk + k + 1, *po = vo + k + 1, *qo = w + k + 1;
+        // NU rows base, base + CL_NW, ... of this warp
+        auto sweep = [&](auto nu_c, int base) {
+            constexpr int NU = decltype(nu_c)::value;
+            const int stride = CL_NW * n;
+            double* row = slab + base * n + (k + 1);
+            double va[NU], wa[NU], s[NU];
+#pragma unroll
+            for (int u = 0; u < NU; ++u) {
+                const int r = c + C * (base + CL_NW * u);
+                va[u] = vo[r];
+                wa[u] = w[r];
+                s[u] = 0.0;
+            }
+            for (int j = lane; j < m; j += 32) {
+                const double a = pn[j], p = po[j], q = qo[j];
+                double y[NU];
+#pragma unroll
+                for (int u = 0; u < NU; ++u) y[u] = row[u * stride + j];
+#pragma unroll
+                for (int u = 0; u < NU; ++u) {
+                    y[u] -= fma(va[u], q, wa[u] * p);
+                    s[u] = fma(y[u], a, s[u]);
+                    row[u * stride + j] = y[u];
+                }
+            }
+            // sums over the lanes, halving the rows a lane holds: lane l ends with row l NU / 32
+            int o = 16;
+#pragma unroll
+            for (int h = NU / 2; h > 0; h >>= 1, o >>= 1)
+#pragma unroll
+                for (int u = 0; u < h; ++u) {
+                    const bool up = lane & o;
+                    const double give = up ? s[u] : s[u + h], keep = up ? s[u + h] : s[u];
+                    s[u] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+            double sum = s[0];
+            for (; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            __syncwarp();  // the rows' first elements are written
+            constexpr int LU = 32 / NU;
+            const int lr = base + CL_NW * (lane / LU);
+            const double2 pa{sum * tau, slab[lr * n + k + 1]};
+            for (int q = lane % LU; q < C; q += LU) cl.map_shared_rank(pb, q)[par * n + c + C * lr] = pa;
+        };
+        for (int base = (k + 1 - c + C - 1) / C + wid; base < nrows;) {
+            const int left = (nrows - base + CL_NW - 1) / CL_NW;
+            if (left >= 8) {
+                sweep(std::integral_constant<int, 8>{}, base);
+                base += 8 * CL_NW;
+            } else if (left >= 4) {
+                sweep(std::integral_constant<int, 4>{}, base);
+                base += 4 * CL_NW;
+            } else if (left >= 2) {
+                sweep(std::integral_constant<int, 2>{}, base);
+                base += 2 * CL_NW;
+            } else {
+                sweep(std::integral_constant<int, 1>{}, base);
+                base += CL_NW;
             }
         }
-        const double dsum = block_sum(dpart, red);
-        if (tid == 0) dslot[k & 1] = dsum;
-        cl.sync();  // p and the v.p shares of this step are complete in every CTA
-        double dtot = 0.0;
-        for (int q = 0; q < C; ++q) dtot += cl.map_shared_rank(dslot, q)[k & 1];
-        const double K = 0.5 * tau * dtot;
-        for (int i = tid; i < m; i += nt) {
-            const int r = k + 1 + i;
-            w[i] = cl.map_shared_rank(pb, r % C)[(k & 1) * R + r / C] - K * v[i];
+        if (C > 1) cl.sync();  // p and the column k + 1 have arrived
+        else __syncthreads();
+        double dot = 0.0;
+        double2 pa[CL_EL];
+#pragma unroll
+        for (int e = 0; e < CL_EL; ++e) {
+            const int r = tid + CL_THREADS * e;
+            pa[e] = double2{0.0, 0.0};
+            if (r >= n || r <= k) continue;
+            pa[e] = pb[par * n + r];
+            dot = fma(vk[r], pa[e].x, dot);
         }
-        __syncthreads();
-        // row k+1, up to date through step k-1 in its owner's slab, updated into this CTA's copy
-        {
-            const double* nxt = cl.map_shared_rank(slab, (k + 1) % C) + (size_t)((k + 1) / C) * n;
-            const double v1 = v[0], w1 = w[0];
-            for (int i = tid; i < m; i += nt) cur[k + 1 + i] = nxt[k + 1 + i] - (v1 * w[i] + w1 * v[i]);
-        }
-        // own rows r >= k+2 (row k+1 is read by the other CTAs in this step)
-        const int lr2 = (k + 2 - c + C - 1) / C;
-        for (int lr = lr2 + wid; lr < nrows; lr += nw) {
-            double* row = slab + (size_t)lr * n + (k + 1);
-            const int i = c + C * lr - (k + 1);
-            const double vi = v[i], wi = w[i];
-            for (int j = lane; j < m; j += 32) row[j] -= vi * w[j] + wi * v[j];
-        }
-        if (c == 0) {
-            if (tid == 0) {
-                g.tri[2 * eo + k] = dk;
-                g.tri[2 * eo + n + k] = alpha;
-            }
+        const double p1 = pb[par * n + k + 1].x;
+        dot = warp_sum(dot);
+        if (lane == 0) s_dot[par][wid] = dot;
+        if (c == 0) {  // this step's outputs, while the others wait for the sum
             const double st = sqrt(tau);
-            for (int i = tid; i < m; i += nt) V[(size_t)k * n + k + 1 + i] = v[i] * st;
+#pragma unroll
+            for (int e = 0; e < CL_EL; ++e) {
+                const int r = tid + CL_THREADS * e;
+                if (r < n && r > k) V[(long)k * n + r] = vk[r] * st;
+                if (r == k) {
+                    g.tri[2 * eo + k] = x[e];
+                    g.tri[2 * eo + n + k] = alpha;
+                }
+            }
         }
-        __syncthreads();  // cur and v are reused by the next step
+        __syncthreads();
+        double dtot = 0.0;
+#pragma unroll
+        for (int q = 0; q < CL_NW; ++q) dtot += s_dot[par][q];
+        const double K = 0.5 * tau * dtot, w1 = p1 - K * v0;
+#pragma unroll
+        for (int e = 0; e < CL_EL; ++e) {
+            const int r = tid + CL_THREADS * e;
+            if (r >= n || r <= k) continue;
+            const double vr = vk[r], wr = pa[e].x - K * vr;
+            w[r] = wr;
+            x[e] = pa[e].y - fma(v0, wr, w1 * vr);
+        }
     }
-    cl.sync();
-    if (c == 0 && tid == 0) {
-        auto elem = [&](int r, int j) { return cl.map_shared_rank(slab, r % C)[(size_t)(r / C) * n + j]; };
-        // row n-2 is this CTA's copy (its owner skipped it in the last step); row n-1 its owner's
-        if (n >= 2) {
-            g.tri[2 * eo + n - 2] = cur[n - 2];
-            g.tri[2 * eo + n + n - 2] = cur[n - 1];
+    __syncthreads();
+    // the last 2 x 2: row n-2 is this CTA's copy; element (n-1, n-1) its owner's, which lacks the last update
+    if (c == 0 && n >= 2) {
+#pragma unroll
+        for (int e = 0; e < CL_EL; ++e) {
+            const int r = tid + CL_THREADS * e;
+            if (r == n - 2) g.tri[2 * eo + n - 2] = x[e];
+            if (r == n - 1) g.tri[2 * eo + n + n - 2] = x[e];
         }
-        g.tri[2 * eo + n - 1] = elem(n - 1, n - 1);
+    }
+    if (c == (n - 1) % C && tid == 0) {
+        double last = slab[(long)((n - 1) / C) * n + n - 1];
+        if (n >= 3) last -= 2.0 * v[((n - 3) & 1) * n + n - 1] * w[n - 1];
+        g.tri[2 * eo + n - 1] = last;
         g.tri[2 * eo + n + n - 1] = 0.0;
     }
-    cl.sync();  // no CTA reads another's shared memory after this point
 }
 
 // ----------------------------------------------------------------------------
@@ -448,7 +599,7 @@ __global__ void __launch_bounds__(CL_THREADS) eigh_cluster_kernel(ClusterArgs g)
 // per panel) from L2 for the narrow ones.  Anderson 1+5
 // (blocks to 400 states): 0.16 ms, against 0.74 ms of the clusters' time and
 // 0.09 ms of products; 7-site ring (blocks to 1225): 3.6 ms against 11.
-// The reflectors: element (r, k) of V at V[k ks + r rs], zero for r <= k.
+// Reflector k is row k of V, right of the diagonal.
 constexpr int BT_NB = 32, BT_THREADS = 256, BT_ROWS = 32;  // reflectors a panel, threads, rows of V a tile
 constexpr int BT_LDV = BT_NB + 4;                          // 4 mod 16 doubles: conflict-free fragment loads
 // Columns of Z per CTA and the largest n whose slab fits 227 KB beside the
@@ -472,25 +623,16 @@ __host__ __device__ inline int bt_panels(int n) { return n > 2 ? (n - 2 + BT_NB 
 
 struct BtItem {
     int block, at;    // block; its panel (T factors) or first column (application)
-    int n, by_col;    // size; reflector k is column k (1) or row k (0) of V
+    int n, pad;
     long moff, toff;  // matrix offset; offset of the block's T factors in T
 };
 
 // tile of BT_ROWS rows of the panel's V from row r0, zero outside it
-__device__ __forceinline__ void bt_load_v(double* dst, const double* V, int by_col, int n, int k0, int r0) {
+__device__ __forceinline__ void bt_load_v(double* dst, const double* V, int n, int k0, int r0) {
     for (int l = threadIdx.x; l < BT_ROWS * BT_NB; l += BT_THREADS) {
-        int r, k;
-        if (by_col) {
-            r = l / BT_NB;
-            k = l % BT_NB;
-        } else {
-            r = l % BT_ROWS;
-            k = l / BT_ROWS;
-        }
-        const int gr = r0 + r, gk = k0 + k;
+        const int r = l % BT_ROWS, k = l / BT_ROWS, gr = r0 + r, gk = k0 + k;
         const bool in = gr < n && gk < n - 2 && gr > gk;
-        const double* src = V + (in ? (by_col ? (long)gr * n + gk : (long)gk * n + gr) : 0L);
-        cp_elem(dst + r * BT_LDV + k, src, in);
+        cp_elem(dst + r * BT_LDV + k, V + (in ? (long)gk * n + gr : 0L), in);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
@@ -505,12 +647,12 @@ __global__ void __launch_bounds__(BT_THREADS) bt_tfactor_kernel(const BtItem* it
     // G = V^T V: warp -> rows 8 (warp % 4), columns 16 (warp / 4)
     const int gi = 8 * (warp % 4), gj = 16 * (warp / 4);
     double2 acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
-    bt_load_v(vt[0], V, it.by_col, n, k0, k0 + 1);
+    bt_load_v(vt[0], V, n, k0, k0 + 1);
     int buf = 0;
     for (int r0 = k0 + 1; r0 < n; r0 += BT_ROWS) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        if (r0 + BT_ROWS < n) bt_load_v(vt[buf ^ 1], V, it.by_col, n, k0, r0 + BT_ROWS);
+        if (r0 + BT_ROWS < n) bt_load_v(vt[buf ^ 1], V, n, k0, r0 + BT_ROWS);
         const double* v = vt[buf];
 #pragma unroll
         for (int r = 0; r < BT_ROWS; r += 4) {
@@ -573,13 +715,13 @@ __global__ void __launch_bounds__(BT_THREADS) bt_apply_kernel(const BtItem* item
 #pragma unroll
             for (int b = 0; b < NF; ++b) w[a][b] = double2{0.0, 0.0};
         __syncthreads();  // the tiles of V and W are free, the slab is up to date
-        bt_load_v(vt, V, it.by_col, n, k0, rb);
+        bt_load_v(vt, V, n, k0, rb);
         for (int t = 0; t < nt; ++t) {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();
             const double* v = vt + (t & 1) * BT_ROWS * BT_LDV;
             // the last tile of V stays in shared memory for the second sweep
-            if (t + 1 < nt) bt_load_v(vt + ((t + 1) & 1) * BT_ROWS * BT_LDV, V, it.by_col, n, k0, rb + (t + 1) * BT_ROWS);
+            if (t + 1 < nt) bt_load_v(vt + ((t + 1) & 1) * BT_ROWS * BT_LDV, V, n, k0, rb + (t + 1) * BT_ROWS);
 #pragma unroll
             for (int r = 0; r < BT_ROWS / 2; r += 4) {
                 const int rr = half * (BT_ROWS / 2) + r + l4, gr = min(rb + t * BT_ROWS + rr, n - 1);  // V is 0 beyond
@@ -644,7 +786,7 @@ __global__ void __launch_bounds__(BT_THREADS) bt_apply_kernel(const BtItem* item
             asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();
             const double* v = vt + (t & 1) * BT_ROWS * BT_LDV;
-            if (t > 0) bt_load_v(vt + ((t - 1) & 1) * BT_ROWS * BT_LDV, V, it.by_col, n, k0, rb + (t - 1) * BT_ROWS);
+            if (t > 0) bt_load_v(vt + ((t - 1) & 1) * BT_ROWS * BT_LDV, V, n, k0, rb + (t - 1) * BT_ROWS);
             const int gr = rb + t * BT_ROWS + strip + l8;
             if (mine) {
                 double2 z[HC];
@@ -1203,12 +1345,12 @@ static void tri_plan(const std::vector<int>& dims, std::vector<TriItem>& items, 
 
 constexpr int CL_NCLS = 5;
 constexpr int CL_SIZES[CL_NCLS] = {1, 2, 4, 8, 16};
-constexpr size_t CL_SMEM_MAX = 226 * 1024;  // dynamic shared memory per CTA (the static part is 256 bytes)
+constexpr size_t CL_SMEM_MAX = 226 * 1024;  // dynamic shared memory per CTA (the static part is small)
 
 // The cluster class of an n x n block, or -1 (the block then takes the
 // large-block path): the smallest cluster whose shared memory holds the
 // block.  16 CTAs (a non-portable cluster size) only where 8 do not suffice
-// (465 to 513 states): at 400 states the per-step cost is set by the cluster
+// (449 to 513 states): at 400 states the per-step cost is set by the cluster
 // barriers, and 16-CTA clusters were measured slower than 8-CTA ones there.
 static int cluster_class(int n) {
     if (n > CL_MAX_DIM) return -1;
@@ -1240,7 +1382,7 @@ static BtPlan bt_plan(const std::vector<int>& dims) {
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return dims[x] > dims[y]; });
     BtPlan p;
     auto add = [&](int b, int at) {
-        p.items.push_back(BtItem{b, at, dims[b], cluster_class(dims[b]) < 0 ? 1 : 0, moff[b], toff[b]});
+        p.items.push_back(BtItem{b, at, dims[b], 0, moff[b], toff[b]});
     };
     p.first[0] = 0;
     for (int b : order)
@@ -1317,7 +1459,7 @@ static std::vector<int> big_blocks(const std::vector<int>& dims) {
 static size_t big_desc_bytes(const std::vector<int>& dims) {
     const size_t nb = big_blocks(dims).size();
     if (nb == 0) return 0;
-    return 8 + nb * sizeof(long) + (size_t)BHH_NB * 4 * BHH_NB * sizeof(int);
+    return 8 + nb * sizeof(BigBlk) + (size_t)BHH_NB * 4 * BHH_NB * sizeof(int);
 }
 size_t eigh_item_bytes(const std::vector<int>& dims) {
     std::vector<TriItem> items;
@@ -1336,11 +1478,10 @@ size_t eigh_gemm_bytes(const std::vector<int>& dims, size_t* tiles_bytes) {
 }
 
 // The large-block Householder path (see bhh_col_kernel) on stream st.
-// big: the blocks, largest first; d_big / d_boff / d_kidx: their device list,
-// scratch offsets and the panel-update column table (uploaded by the caller).
+// big: the blocks, largest first; d_blk, d_kidx: their device list and the
+// panel-update column table (uploaded by the caller).
 static void launch_big(const EighDev& d, const std::vector<int>& dims, const std::vector<long>& moff,
-                       const std::vector<int>& big, const int* d_big, const long* d_boff, const int* d_kidx,
-                       cudaStream_t st) {
+                       const std::vector<int>& big, const BigBlk* d_blk, const int* d_kidx, cudaStream_t st) {
     const int nbig = (int)big.size();
     std::vector<long> boff(nbig);
     long o = 2 * BHH_NB;
@@ -1356,11 +1497,7 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
         return c;
     };
     BigArgs a{};
-    a.big = d_big;
-    a.boff = d_boff;
-    a.dims = d.dims;
-    a.moff = d.moff;
-    a.eoff = d.eoff;
+    a.blk = d_blk;
     a.A = d.A;
     a.Zc = d.Zc;
     a.S = d.S;
@@ -1380,8 +1517,43 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
         for (double& x : neg) x = -1.0;
         h2d(d.S, neg, sizeof(neg), st);
     }
-    PGX_CUDA(cudaFuncSetAttribute(bhh_symv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(sizeof(double) * nmax)));
+    // The column and product kernels alternate, each launched while the one
+    // before it drains (it waits for that one's results itself).
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.stream = st;
+    const size_t col_smem = 3 * sizeof(double) * (size_t)nmax;
+    PGX_CUDA(cudaFuncSetAttribute(bhh_col_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)std::min<size_t>(col_smem, 200 * 1024)));
+    auto col_step = [&]() {
+        // CTAs per block: more shorten a block's sweep, as long as all blocks
+        // are resident at once (two CTAs per SM) and their rows fit
+        int cs = BHH_CS;
+        while (cs > 1 && a.nact * cs > 2 * 148 && 2 * col_smem / cs <= 100 * 1024) cs /= 2;
+        cfg.gridDim = dim3((unsigned)(a.nact * cs));
+        cfg.blockDim = dim3(BHH_COL_THREADS);
+        cfg.dynamicSmemBytes = 3 * sizeof(double) * (size_t)ceil_div(nmax, cs);
+        attr[1].val.clusterDim.x = cs;
+        cfg.numAttrs = 2;
+        ProfRange r1("bhh_col_kernel", st, 0.0, 0.0);
+        PGX_CUDA(cudaLaunchKernelEx(&cfg, bhh_col_kernel, a));
+        check_launch("bhh_col_kernel");
+    };
+    auto symv_step = [&](int rows, double bytes) {
+        cfg.gridDim = dim3((unsigned)ceil_div(rows, BHH_SYMV_ROWS), (unsigned)a.nact);
+        cfg.blockDim = dim3(BHH_SYMV_THREADS);
+        cfg.dynamicSmemBytes = 0;
+        cfg.numAttrs = 1;
+        ProfRange r2("bhh_symv_kernel", st, 0.0, bytes);
+        PGX_CUDA(cudaLaunchKernelEx(&cfg, bhh_symv_kernel, a));
+        check_launch("bhh_symv_kernel");
+    };
     std::vector<GemmProblem<double, double, double>> probs;
     size_t tiles_cap = 0;
     const size_t probs_cap = eigh_gemm_bytes(dims, &tiles_cap);
@@ -1393,32 +1565,20 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
             a.fin = (j > k) ? j - 1 : -1;
             a.col = j;
             a.nact = nact(j > k ? j - 1 : j);
-            {
-                ProfRange r1("bhh_col_kernel", st, 0.0, 0.0);
-                bhh_col_kernel<<<(unsigned)a.nact, BHH_COL_THREADS, 0, st>>>(a);
-                check_launch("bhh_col_kernel");
-            }
+            col_step();
             a.fin = -1;
             a.nact = nact(j);
-            long ctas = 0;
             double bytes = 0.0;
             for (int i = 0; i < a.nact; ++i) {
-                const long m = dims[big[i]] - j - 1;
-                ctas += (m + BHH_SYMV_ROWS - 1) / BHH_SYMV_ROWS;
+                const double m = dims[big[i]] - j - 1;
                 bytes += 8.0 * m * m;
             }
-            ProfRange r2("bhh_symv_kernel", st, 0.0, bytes);
-            bhh_symv_kernel<<<(unsigned)ctas, BHH_SYMV_THREADS, sizeof(double) * nmax, st>>>(a);
-            check_launch("bhh_symv_kernel");
+            symv_step(nmax - j - 1 + 2 * (j - k), bytes);
         }
         a.fin = jend - 1;
         a.col = -1;
         a.nact = nact(jend - 1);
-        {
-            ProfRange r1("bhh_col_kernel", st, 0.0, 0.0);
-            bhh_col_kernel<<<(unsigned)a.nact, BHH_COL_THREADS, 0, st>>>(a);
-            check_launch("bhh_col_kernel");
-        }
+        col_step();
         // A(k+p:, k+p:) -= V W^T + W V^T, p = the block's columns in this panel
         probs.clear();
         for (int i = 0; i < nact(k); ++i) {
@@ -1465,18 +1625,18 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
         npan_total += np;
         for (long q = 0; q < np; ++q) {
             const int k = (int)q * BHH_NB, p = std::min(BHH_NB, n - 2 - k), m = n - k - 1;
-            const double* Vp = d.A + moff[big[i]] + (long)(k + 1) * n + k;
+            const double* Vp = d.A + moff[big[i]] + (long)k * n + (k + 1);  // V^T, p x m
             GemmProblem<double, double, double> g{};
-            g.A = Vp;  // V^T
+            g.A = Vp;
             g.B = Vp;
             g.C = d.S + boff[i] + 2L * BHH_NB * n + 2L * n + q * BHH_NB * BHH_NB;
             g.M = p;
             g.N = p;
             g.K = m;
-            g.sa_i = 1;
-            g.sa_k = n;
-            g.sb_k = n;
-            g.sb_j = 1;
+            g.sa_i = n;
+            g.sa_k = 1;
+            g.sb_k = 1;
+            g.sb_j = n;
             g.sc_i = BHH_NB;
             g.sc_j = 1;
             probs.push_back(g);
@@ -1491,15 +1651,15 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
         for (int i = 0; i < std::min(nwide, nact(k)); ++i) {
             const int n = dims[big[i]];
             const int p = std::min(BHH_NB, n - 2 - k), m = n - k - 1;
-            const double* Vp = d.A + moff[big[i]] + (long)(k + 1) * n + k;
+            const double* Vp = d.A + moff[big[i]] + (long)k * n + (k + 1);  // V^T, p x m
             double* Qs = d.Zc + moff[big[i]] + (long)(k + 1) * n + (k + 1);
             double* Y = d.S + boff[i];
             double* Y2 = Y + (long)BHH_NB * n;
             const double* nT = d.S + boff[i] + 2L * BHH_NB * n + 2L * n + (bhh_panels(n) + q) * BHH_NB * BHH_NB;
             GemmProblem<double, double, double> g{};
             g.A = Vp;  // Y = V^T Q
-            g.sa_i = 1;
-            g.sa_k = n;
+            g.sa_i = n;
+            g.sa_k = 1;
             g.B = Qs;
             g.sb_k = 1;
             g.sb_j = n;
@@ -1526,8 +1686,8 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
             pt.push_back(h);
             GemmProblem<double, double, double> u{};  // Q += V Y2
             u.A = Vp;
-            u.sa_i = n;
-            u.sa_k = 1;
+            u.sa_i = 1;
+            u.sa_k = n;
             u.B = Y2;
             u.sb_k = n;
             u.sb_j = 1;
@@ -1611,12 +1771,14 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
     const size_t lists_end = lists_at + lists.size() * sizeof(int);
     const size_t boff_at = (lists_end + 7) & ~size_t(7);
     size_t host_bytes = lists_end;
-    std::vector<long> boff;
+    std::vector<BigBlk> blk;
     std::vector<int> kidx;
     if (!big.empty()) {
+        std::vector<long> eoff(dims.size() + 1, 0);
+        for (size_t b = 0; b < dims.size(); ++b) eoff[b + 1] = eoff[b] + dims[b];
         long o = 2 * BHH_NB;
         for (int b : big) {
-            boff.push_back(o);
+            blk.push_back(BigBlk{moff[b], eoff[b], o, dims[b], 0});
             o += bhh_scratch_doubles(dims[b]);
         }
         for (int p = 1; p <= BHH_NB; ++p) {
@@ -1630,7 +1792,7 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
             kidx.insert(kidx.end(), ia.begin(), ia.end());
             kidx.insert(kidx.end(), ib.begin(), ib.end());
         }
-        host_bytes = boff_at + boff.size() * sizeof(long) + kidx.size() * sizeof(int);
+        host_bytes = boff_at + blk.size() * sizeof(BigBlk) + kidx.size() * sizeof(int);
         PGX_CHECK(host_bytes <= eigh_item_bytes(dims), PGX_ERR_ARG, "eigensolver descriptor layout overflow");
     }
     std::vector<char> host(host_bytes);
@@ -1639,15 +1801,15 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
         std::memcpy(host.data() + items.size() * sizeof(TriItem), bt.items.data(), bt.items.size() * sizeof(BtItem));
     std::memcpy(host.data() + lists_at, lists.data(), lists.size() * sizeof(int));
     if (!big.empty()) {
-        std::memcpy(host.data() + boff_at, boff.data(), boff.size() * sizeof(long));
-        std::memcpy(host.data() + boff_at + boff.size() * sizeof(long), kidx.data(), kidx.size() * sizeof(int));
+        std::memcpy(host.data() + boff_at, blk.data(), blk.size() * sizeof(BigBlk));
+        std::memcpy(host.data() + boff_at + blk.size() * sizeof(BigBlk), kidx.data(), kidx.size() * sizeof(int));
     }
     h2d(d.items, host.data(), host.size(), st);
     const BtItem* d_bt = reinterpret_cast<const BtItem*>(static_cast<const TriItem*>(d.items) + items.size());
     const int* d_lists = reinterpret_cast<const int*>(static_cast<const char*>(d.items) + lists_at);
-    const long* d_boff = reinterpret_cast<const long*>(static_cast<const char*>(d.items) + boff_at);
+    const BigBlk* d_blk = reinterpret_cast<const BigBlk*>(static_cast<const char*>(d.items) + boff_at);
     const int* d_kidx = reinterpret_cast<const int*>(static_cast<const char*>(d.items) + boff_at +
-                                                     boff.size() * sizeof(long));
+                                                     blk.size() * sizeof(BigBlk));
 
     // LAPACK operation counts: tridiagonalisation 4/3 n^3, forming Q 4/3 n^3;
     // minimum DRAM traffic: read H, write Q and the tridiagonal
@@ -1666,7 +1828,7 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
         PGX_CUDA(cudaEventRecord(d.fork, st));
         for (int i = 0; i < 4; ++i) PGX_CUDA(cudaStreamWaitEvent(d.aux[i], d.fork, 0));
     }
-    if (!big.empty()) launch_big(d, dims, moff, big, d_lists, d_boff, d_kidx, st);
+    if (!big.empty()) launch_big(d, dims, moff, big, d_blk, d_kidx, st);
     for (int q = 0; q < CL_NCLS; ++q) {
         if (hp.cls[q].empty()) continue;
         const cudaStream_t sq = (fork && q > 0) ? d.aux[q - 1] : st;
