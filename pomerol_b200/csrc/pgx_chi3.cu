@@ -114,6 +114,21 @@ __global__ void chi3_dress_ff_kernel(const Chi3Dev<T>* parts, const cd* Z1, int 
     }
 }
 
+// The columns N2u .. N2 - 1 of the swapped parts' rows of R: conjugates of the
+// columns src.
+template <typename T>
+__global__ void chi3_mirror_kernel(const Chi3Dev<T>* parts, const int* src, int N2, int N2u, cd* R) {
+    const Chi3Dev<T> p = parts[blockIdx.y];
+    if (!p.swapped) return;
+    const int nm = N2 - N2u;
+    const long n = (long)p.d3 * p.d2 * nm;
+    for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
+        cd* row = R + (p.offN + e / nm) * N2;
+        const int b = (int)(e % nm);
+        row[N2u + b] = conj(row[src[b]]);
+    }
+}
+
 // RF[(i, k), Om] = cF m_ik B_ki (w_k - w_i) / (Om - E_ik)
 template <typename T>
 __global__ void chi3_dress_fb_kernel(const Chi3Dev<T>* parts, const cd* ZO, int NO, cd* RF) {
@@ -255,14 +270,50 @@ void run_chi3_t(pgx_ctx* c, int channel, int nparts, const pgx_chi3_part* parts,
     const double sig = channel == PGX_PP ? 1.0 : -1.0, spp = channel == PGX_PP ? -1.0 : 1.0;
     // ---- duplets: distinct z1, sig z2 and Om = z1 - xi z2
     std::vector<cd> z1(nfreq), sz2(nfreq), om(nfreq);
+    // With real matrix elements chi3 at the conjugate duplet is the conjugate of
+    // chi3, so duplets are evaluated where z1 is not below the real axis (half
+    // of the z1 of a symmetric grid), and R's columns of a z2 below the axis are
+    // the conjugates of those above where both occur.  Anderson 1+5, 32 x 32
+    // duplets: 17.6 -> 10.6 ms.
+    const bool real = !is_cd<T>::value;
+    std::vector<char> flip(nfreq, 0);
     for (int q = 0; q < nfreq; ++q) {
         z1[q] = cd{z[4 * q], z[4 * q + 1]};
-        sz2[q] = cd{sig * z[4 * q + 2], sig * z[4 * q + 3]};
-        om[q] = cd{z[4 * q] - xi * z[4 * q + 2], z[4 * q + 1] - xi * z[4 * q + 3]};
+        cd z2{z[4 * q + 2], z[4 * q + 3]};
+        if (real && (z1[q].y < 0.0 || (z1[q].y == 0.0 && z2.y < 0.0))) {
+            flip[q] = 1;
+            z1[q] = conj(z1[q]);
+            z2 = conj(z2);
+        }
+        sz2[q] = cd{sig * z2.x, sig * z2.y};
+        om[q] = cd{z1[q].x - xi * z2.x, z1[q].y - xi * z2.y};
     }
     std::vector<cd> Z1, SZ2, ZO;
     std::vector<int> i1, i2, io;
     const int N1 = distinct_index(z1, Z1, i1), N2 = distinct_index(sz2, SZ2, i2), NO = distinct_index(om, ZO, io);
+    // z2 whose columns are computed first, then those mirrored from msrc
+    int N2u = N2;
+    std::vector<int> msrc;
+    if (real) {
+        std::map<std::pair<double, double>, int> at;
+        for (int b = 0; b < N2; ++b) at[{SZ2[b].x, SZ2[b].y}] = b;
+        std::vector<int> order, low, pos(N2);
+        for (int b = 0; b < N2; ++b) {
+            const auto it = at.find({SZ2[b].x, -SZ2[b].y});
+            if (SZ2[b].y < 0.0 && it != at.end()) low.push_back(b);
+            else order.push_back(b);
+        }
+        N2u = (int)order.size();
+        for (int i = 0; i < N2u; ++i) pos[order[i]] = i;
+        for (size_t i = 0; i < low.size(); ++i) {
+            pos[low[i]] = N2u + (int)i;
+            msrc.push_back(pos[at[{SZ2[low[i]].x, -SZ2[low[i]].y}]]);
+        }
+        std::vector<cd> v(N2);
+        for (int b = 0; b < N2; ++b) v[pos[b]] = SZ2[b];
+        SZ2 = std::move(v);
+        for (int& b : i2) b = pos[b];
+    }
     std::vector<DupletIdx> dq(nfreq);
     bool any_res = false;
     for (int q = 0; q < nfreq; ++q) {
@@ -317,8 +368,8 @@ void run_chi3_t(pgx_ctx* c, int channel, int nparts, const pgx_chi3_part* parts,
     const size_t b_outn = al(nOUTN * sizeof(cd)), b_outf = al(nOUTF * sizeof(cd)), b_res = al(N1 * sizeof(cd)),
                  b_z = al(std::max(N1, 1) * sizeof(cd)), b_z2 = al(std::max(N2, 1) * sizeof(cd)),
                  b_zo = al(std::max(NO, 1) * sizeof(cd)), b_dq = al(std::max(nfreq, 1) * sizeof(DupletIdx)),
-                 b_out = al(std::max(nfreq, 1) * sizeof(cd));
-    tab.reserve(b_outn + b_outf + b_res + 2 * b_z + 2 * b_z2 + b_zo + b_dq + b_out);
+                 b_out = al(std::max(nfreq, 1) * sizeof(cd)), b_src = al(std::max(N2, 1) * sizeof(int));
+    tab.reserve(b_outn + b_outf + b_res + 2 * b_z + 2 * b_z2 + b_zo + b_dq + b_out + b_src);
     char* tp = tab.as<char>();
     cd* OUTN = reinterpret_cast<cd*>(tp);
     cd* OUTF = reinterpret_cast<cd*>(tp + b_outn);
@@ -330,6 +381,7 @@ void run_chi3_t(pgx_ctx* c, int channel, int nparts, const pgx_chi3_part* parts,
     cd* dZO = reinterpret_cast<cd*>(reinterpret_cast<char*>(dnSZ2) + b_z2);
     DupletIdx* dDQ = reinterpret_cast<DupletIdx*>(reinterpret_cast<char*>(dZO) + b_zo);
     cd* dOut = reinterpret_cast<cd*>(reinterpret_cast<char*>(dDQ) + b_dq);
+    int* dSrc = reinterpret_cast<int*>(reinterpret_cast<char*>(dOut) + b_out);
     PGX_CUDA(cudaMemsetAsync(tp, 0, b_outn + b_outf + b_res, st));
     if (nfreq > 0) {
         h2d(dZ1, Z1.data(), N1 * sizeof(cd), st);
@@ -338,6 +390,7 @@ void run_chi3_t(pgx_ctx* c, int channel, int nparts, const pgx_chi3_part* parts,
         h2d(dnSZ2, nSZ2.data(), N2 * sizeof(cd), st);
         h2d(dZO, ZO.data(), NO * sizeof(cd), st);
         h2d(dDQ, dq.data(), nfreq * sizeof(DupletIdx), st);
+        h2d(dSrc, msrc.data(), msrc.size() * sizeof(int), st);
     }
     // ---- parts in groups whose frequency-dependent matrices fit the budget
     const double budget = 4.0e9;
@@ -481,7 +534,7 @@ void run_chi3_t(pgx_ctx* c, int channel, int nparts, const pgx_chi3_part* parts,
                     g.C = R + x.offN * N2;
                     g.sc_i = (long)x.d2 * N2;
                     g.sc_j = N2;
-                    g.nb = N2;
+                    g.nb = N2u;
                     g.bc = 1;
                     g.dzs = dnSZ2;
                 }
@@ -535,6 +588,15 @@ void run_chi3_t(pgx_ctx* c, int channel, int nparts, const pgx_chi3_part* parts,
             c->scratch[5].reserve(gemm_index_bytes(pb.size()));
             launch_gemm_batch(pb, c->scratch[4].p, c->scratch[4].bytes, c->scratch[5].p, c->scratch[5].bytes, st);
         }
+        if (N2u < N2) {
+            long most = 1;
+            for (auto& x : dv)
+                if (x.swapped) most = std::max(most, (long)x.d3 * x.d2 * (N2 - N2u));
+            ProfRange pr("chi3_mirror_kernel", st, 0.0, 0.0);
+            chi3_mirror_kernel<T><<<dim3(std::min(ceil_div(most, 256), 1024), (unsigned)dv.size()), 256, 0, st>>>(
+                dp, dSrc, N2, N2u, R);
+            check_launch("chi3_mirror_kernel");
+        }
         // (3) materialised dressed sides
         long maxff = 1, maxfb = 1;
         for (auto& x : dv) {
@@ -587,6 +649,8 @@ void run_chi3_t(pgx_ctx* c, int channel, int nparts, const pgx_chi3_part* parts,
         PGX_CUDA(cudaMemcpyAsync(out, dOut, nfreq * sizeof(cd), cudaMemcpyDeviceToHost, st));
     }
     PGX_CUDA(cudaStreamSynchronize(st));
+    for (int q = 0; q < nfreq; ++q)
+        if (flip[q]) out[2 * q + 1] = -out[2 * q + 1];
 }
 
 }  // namespace
