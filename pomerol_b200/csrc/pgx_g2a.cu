@@ -27,9 +27,10 @@
 // resonant delta test in FP64).  A(z1) and C(z3) are never stored: the GEMM
 // tile loads dress O1 and O3 with the frequency as they read them.
 
+#include <algorithm>
 #include <array>
+#include <iterator>
 #include <map>
-#include <set>
 #include <tuple>
 #include <unordered_map>
 
@@ -301,9 +302,10 @@ void launch_contract(int BM, int BN, unsigned n, cudaStream_t st, const DTerm* t
 // part, and the class's value is out[u] + conj(out[ncls + u]).  On a grid that
 // holds the conjugates of its frequencies this halves the z1' of every
 // permutation, and with them the stacked products, the contractions and the
-// workspace: Anderson 1+5, 16^3: 16.2 -> 12.0 ms;
-// the 8-site ring's largest chain, 16^3, split products: 325 -> 181 ms.  A complex Hamiltonian has the
-// triples themselves as classes, in order, without conjugates.
+// workspace: Anderson 1+5, 16^3: 11.9 -> 7.3
+// ms; the 8-site ring's largest chain, 16^3, split products: 288 -> 158 ms.  A
+// complex Hamiltonian has the triples themselves as classes, in order, without
+// conjugates.
 struct Points {
     int ncls = 0, npts = 0;
     std::vector<cd> val[3];
@@ -383,34 +385,58 @@ void build_points(Points& pt, int nfreq, const double* z, bool real) {
     }
 }
 
-// Per point, the four frequency sums the contractions use under one
-// permutation: z2', z1'+z2'+z3', z1'+z2', z2'+z3', where (z1', z2', z3') is the
-// permuted (z1, z2, -z3), z1' dressing O1 and z3' dressing O3.
-struct PermSums {
-    std::vector<cd> h;  // sum k of point e at h[k * npts + e]
-    int npts = 0;
-};
-
-void build_sums(PermSums& ps, const int perm[3], const Points& pt) {
-    const size_t n = (size_t)pt.npts;
-    ps.h.resize(4 * n);
-    for (size_t e = 0; e < n; ++e) {
-        const cd a = pt.at(perm[0], (int)e), b = pt.at(perm[1], (int)e), c = pt.at(perm[2], (int)e);
-        ps.h[e] = b;
-        ps.h[n + e] = a + b + c;
-        ps.h[2 * n + e] = a + b;
-        ps.h[3 * n + e] = b + c;
-    }
-    ps.npts = pt.npts;
-}
-
 // The points a permutation evaluates (one per class), their distinct z1' and
-// z3' in order of first appearance, and each point's index into them.
+// z3' in order of first appearance, and each point's index into them.  Per
+// point also the numbers of the four frequency sums the contractions use: z2',
+// z1'+z2'+z3', z1'+z2', z2'+z3', where (z1', z2', z3') is the permuted (z1, z2,
+// -z3), z1' dressing O1 and z3' dressing O3.  Sums equal up to rounding (2^-46
+// of the largest) have one number; the numbers ascend with the values.
 struct PermIndex {
     std::vector<int> pts;
     std::vector<cd> Z1, Z3;
     std::vector<int> j1, j3;
+    std::vector<int> sid[4];  // sum k of point e (of pts): number sid[k][e]
+    std::vector<cd> sval[4];  // its value
 };
+
+// Numbers of x + y over the pairs (i, j) that occur: `val` receives a value
+// per distinct pair, `id` each point's pair.  A pair is added once, so the
+// cost per point is a table lookup.
+void number_pairs(const std::vector<int>& pts, const std::vector<int>& xi, const std::vector<cd>& xv,
+                  const std::vector<int>& yi, const std::vector<cd>& yv, std::vector<int>& id, std::vector<cd>& val) {
+    const size_t ny = yv.size(), cells = xv.size() * ny;
+    std::vector<int> dense(cells <= (size_t(1) << 20) ? cells : 0, -1);
+    std::unordered_map<size_t, int> sparse;
+    for (int e : pts) {
+        const size_t cell = (size_t)xi[e] * ny + yi[e];
+        int& q = dense.empty() ? sparse.emplace(cell, -1).first->second : dense[cell];
+        if (q < 0) {
+            q = (int)val.size();
+            val.push_back(xv[xi[e]] + yv[yi[e]]);
+        }
+        id[e] = q;
+    }
+}
+
+// Merges the numbers of values equal up to rounding and orders them.
+void order_values(const std::vector<int>& pts, std::vector<int>& id, std::vector<cd>& val) {
+    double big = 0.0;
+    for (const cd& v : val) big = std::max(big, std::max(std::fabs(v.x), std::fabs(v.y)));
+    const double q = big > 0.0 ? std::ldexp(big, -46) : 1.0;
+    std::vector<std::tuple<long long, long long, int>> key;
+    for (size_t i = 0; i < val.size(); ++i)
+        key.emplace_back(std::llround(val[i].x / q), std::llround(val[i].y / q), (int)i);
+    std::sort(key.begin(), key.end());
+    std::vector<int> to(val.size());
+    std::vector<cd> out;
+    for (size_t i = 0; i < key.size(); ++i) {
+        if (i == 0 || std::get<0>(key[i]) != std::get<0>(key[i - 1]) || std::get<1>(key[i]) != std::get<1>(key[i - 1]))
+            out.push_back(val[std::get<2>(key[i])]);
+        to[std::get<2>(key[i])] = (int)out.size() - 1;
+    }
+    for (int e : pts) id[e] = to[id[e]];
+    val = std::move(out);
+}
 
 void index_perm(PermIndex& ix, const int perm[3], const Points& pt) {
     ix.pts.resize(pt.ncls);
@@ -436,66 +462,102 @@ void index_perm(PermIndex& ix, const int perm[3], const Points& pt) {
     };
     order(perm[0], ix.Z1, ix.j1);
     order(perm[2], ix.Z3, ix.j3);
+    order(perm[1], ix.sval[0], ix.sid[0]);
 }
 
-// The triples of one tile of a permutation's (z1', z3') plane: z1' indices
-// [o1, o1 + n1) and z3' indices [o3, o3 + n3) of its PermIndex, the triples
-// grouped by (z1', z3'), each group one warp's work in the contraction.
+// The numbers of the sums (after index_perm).
+void number_sums(PermIndex& ix) {
+    const std::vector<int> j2 = ix.sid[0];
+    const std::vector<cd> Z2 = ix.sval[0];
+    for (auto& v : ix.sid) v.resize(j2.size());
+    order_values(ix.pts, ix.sid[0], ix.sval[0]);
+    number_pairs(ix.pts, ix.j1, ix.Z1, j2, Z2, ix.sid[2], ix.sval[2]);
+    order_values(ix.pts, ix.sid[2], ix.sval[2]);
+    number_pairs(ix.pts, ix.sid[2], ix.sval[2], ix.j3, ix.Z3, ix.sid[1], ix.sval[1]);
+    order_values(ix.pts, ix.sid[1], ix.sval[1]);
+    number_pairs(ix.pts, j2, Z2, ix.j3, ix.Z3, ix.sid[3], ix.sval[3]);
+    order_values(ix.pts, ix.sid[3], ix.sval[3]);
+}
+
+// What the device needs of all plans of a call, gathered on the host and
+// uploaded at once; until then pointers are offsets into it.
+struct Blob {
+    std::vector<char> h;
+    template <typename T> T* put(const T* src, size_t n) {
+        const size_t at = (h.size() + 15) & ~size_t(15);
+        h.resize(at);
+        h.insert(h.end(), reinterpret_cast<const char*>(src), reinterpret_cast<const char*>(src + n));
+        return reinterpret_cast<T*>(at);
+    }
+    template <typename T> T* put(const std::vector<T>& v) { return put(v.data(), v.size()); }
+};
+template <typename T> void rebase(T*& p, char* base) {
+    p = reinterpret_cast<T*>(base + reinterpret_cast<size_t>(p));
+}
+
+// The points of one tile of a permutation's (z1', z3') plane: z1' indices
+// [o1, o1 + n1) and z3' indices [o3, o3 + n3) of its PermIndex, the points
+// grouped by (z1', z3'), and the contraction classes per frequency sum (term
+// unset).
 struct APlan {
     std::vector<cd> Z1, Z3;
-    std::vector<int> gt, goff, gi1, gi3;  // triple ids grouped by (i1, i3)
-    DevBuf buf;
+    std::vector<int> gt, goff, gi1, gi3;  // points grouped by (i1, i3)
     cd *dZ1 = nullptr, *dZ3 = nullptr;
-    int *dgt = nullptr, *dgoff = nullptr, *dgi1 = nullptr, *dgi3 = nullptr;
-    const PermSums* sums = nullptr;
-    // contraction classes per frequency sum (built on first use), device
-    // pointers in `cls` (term unset), storage in cbuf
-    bool have_cls[4] = {false, false, false, false};
+    int *dgi1 = nullptr, *dgi3 = nullptr;
     std::vector<CClass> cls[4];
-    DevBuf cbuf[4];
 };
 
 // Contraction classes of one plan for frequency sum k: the (z1, z3) groups
-// whose triples carry the same sums (compared after rounding to 2^-46 of the
-// largest |s|, so sums equal up to rounding share a class; the class uses its
-// first group's values), columns ordered by sum, split into chunks of at most
-// CG_BN_MAX columns.
-void build_classes(APlan& pl, int k, cudaStream_t st) {
-    if (pl.have_cls[k]) return;
-    const PermSums& ps = *pl.sums;
-    const cd* sv = ps.h.data() + (size_t)k * ps.npts;
-    double smax = 0.0;
-    for (int t : pl.gt) smax = std::max(smax, std::max(std::fabs(sv[t].x), std::fabs(sv[t].y)));
-    const double q = smax > 0.0 ? std::ldexp(smax, -46) : 1.0;
-    using Key = std::vector<std::pair<long long, long long>>;
+// whose points carry the same sums form a class, columns ordered by sum, split
+// into chunks of at most CG_BN_MAX columns.
+void build_classes(APlan& pl, int k, const PermIndex& ix, Blob& blob) {
+    const std::vector<int>& sid = ix.sid[k];
     struct HC {
-        std::vector<cd> s;
-        std::vector<int> rows, slots;
+        std::vector<int> s, rows, slots;  // sum numbers; groups; points, row by row
     };
-    std::map<Key, int> idx;
+    std::unordered_multimap<size_t, int> idx;  // hash of a list of sums -> class
     std::vector<HC> hc;
     const int ng = (int)pl.gi1.size();
-    std::vector<std::tuple<long long, long long, int>> el;
+    std::vector<std::pair<int, int>> el;
+    std::vector<int> ids, pts;
+    int ci = -1;
     for (int g = 0; g < ng; ++g) {
-        el.clear();
-        for (int u = pl.goff[g]; u < pl.goff[g + 1]; ++u) {
-            const int t = pl.gt[u];
-            el.emplace_back(std::llround(sv[t].x / q), std::llround(sv[t].y / q), t);
+        const int* t = pl.gt.data() + pl.goff[g];
+        const int n = pl.goff[g + 1] - pl.goff[g];
+        ids.resize(n);
+        bool ordered = true;
+        for (int i = 0; i < n; ++i) {
+            ids[i] = sid[t[i]];
+            ordered = ordered && (i == 0 || ids[i - 1] <= ids[i]);
         }
-        std::sort(el.begin(), el.end());
-        Key key;
-        key.reserve(el.size());
-        for (auto& e : el) key.emplace_back(std::get<0>(e), std::get<1>(e));
-        auto it = idx.find(key);
-        if (it == idx.end()) {
-            it = idx.emplace(std::move(key), (int)hc.size()).first;
-            hc.emplace_back();
-            for (auto& e : el) hc.back().s.push_back(sv[std::get<2>(e)]);
+        if (!ordered) {
+            el.clear();
+            for (int i = 0; i < n; ++i) el.emplace_back(ids[i], t[i]);
+            std::sort(el.begin(), el.end());
+            pts.resize(n);
+            for (int i = 0; i < n; ++i) {
+                ids[i] = el[i].first;
+                pts[i] = el[i].second;
+            }
+            t = pts.data();
         }
-        HC& c = hc[it->second];
-        c.rows.push_back(g);
-        for (auto& e : el) c.slots.push_back(std::get<2>(e));
+        if (ci < 0 || hc[ci].s != ids) {  // most often the class of the group before
+            size_t h = n;
+            for (int x : ids) h = (h ^ (size_t)x) * 0x9E3779B97F4A7C15ull;
+            ci = -1;
+            for (auto r = idx.equal_range(h); r.first != r.second && ci < 0; ++r.first)
+                if (hc[r.first->second].s == ids) ci = r.first->second;
+            if (ci < 0) {
+                ci = (int)hc.size();
+                idx.emplace(h, ci);
+                hc.emplace_back();
+                hc.back().s = ids;
+            }
+        }
+        hc[ci].rows.push_back(g);
+        hc[ci].slots.insert(hc[ci].slots.end(), t, t + n);
     }
+    std::sort(hc.begin(), hc.end(), [](const HC& x, const HC& y) { return x.s < y.s; });
     // Classes of few rows (such as the z1 + z3 classes of the T2 sub-terms
     // near the grid's corners) make 8- or 16-row tiles that leave the FP64 pipe
     // idle.  Consecutive ones, in the order of their sum lists, are merged while
@@ -504,25 +566,25 @@ void build_classes(APlan& pl, int k, cudaStream_t st) {
     // its tile computes those products and drops them.
     std::vector<HC> merged;
     {
-        using QK = std::pair<long long, long long>;
-        auto qk = [&](cd v) { return QK{std::llround(v.x / q), std::llround(v.y / q)}; };
+        std::vector<int> both;
+        auto unite = [&](std::vector<int>& u, const std::vector<int>& v) {
+            both.clear();
+            std::set_union(u.begin(), u.end(), v.begin(), v.end(), std::back_inserter(both));
+            return (int)both.size();
+        };
         // groups of consecutive small classes under a row cap (sums within CG_BN_MAX)
         auto split_run = [&](const std::vector<int>& run, int cap) {
             std::vector<std::vector<int>> out;
-            std::set<QK> uni;
+            std::vector<int> uni;
             int rows = 0;
             for (int ci : run) {
-                std::set<QK> u2 = uni;
-                for (const cd& v : hc[ci].s) u2.insert(qk(v));
                 const int r = (int)hc[ci].rows.size();
-                if (!out.empty() && !out.back().empty() && ((int)u2.size() > CG_BN_MAX || rows + r > cap)) {
+                if (out.empty() || unite(uni, hc[ci].s) > CG_BN_MAX || rows + r > cap) {
                     out.emplace_back();
-                    uni.clear();
-                    for (const cd& v : hc[ci].s) uni.insert(qk(v));
+                    uni = hc[ci].s;
                     rows = 0;
                 } else {
-                    if (out.empty()) out.emplace_back();
-                    uni = std::move(u2);
+                    uni = both;
                 }
                 out.back().push_back(ci);
                 rows += r;
@@ -534,14 +596,10 @@ void build_classes(APlan& pl, int k, cudaStream_t st) {
                 merged.push_back(std::move(hc[group[0]]));
                 return;
             }
-            std::map<QK, int> col;
-            std::map<QK, cd> uni;
-            for (int ci : group)
-                for (const cd& v : hc[ci].s) uni.emplace(qk(v), v);
             HC m;
-            for (auto& e : uni) {
-                col[e.first] = (int)m.s.size();
-                m.s.push_back(e.second);
+            for (int ci : group) {
+                unite(m.s, hc[ci].s);
+                m.s = both;
             }
             const int w = (int)m.s.size();
             for (int ci : group) {
@@ -551,7 +609,10 @@ void build_classes(APlan& pl, int k, cudaStream_t st) {
                     m.rows.push_back(c.rows[r]);
                     const size_t base = m.slots.size();
                     m.slots.resize(base + w, -1);
-                    for (int j = 0; j < nc; ++j) m.slots[base + col[qk(c.s[j])]] = c.slots[r * nc + j];
+                    for (int j = 0, col = 0; j < nc; ++j) {
+                        while (m.s[col] != c.s[j]) ++col;
+                        m.slots[base + col] = c.slots[r * nc + j];
+                    }
                 }
             }
             merged.push_back(std::move(m));
@@ -566,20 +627,17 @@ void build_classes(APlan& pl, int k, cudaStream_t st) {
                 total += (int)hc[ci].rows.size();
                 big = std::max(big, (int)hc[ci].rows.size());
             }
-            const int ng = (int)split_run(run, 64).size();
-            const int cap = std::max(big, (total + ng - 1) / ng);
+            const int ng2 = (int)split_run(run, 64).size();
+            const int cap = std::max(big, (total + ng2 - 1) / ng2);
             for (const auto& g : split_run(run, cap)) emit(g);
             run.clear();
         };
         std::vector<int> run;
-        for (auto& e : idx) {  // classes in the order of their sum lists
-            const int ci = e.second;
+        for (int ci = 0; ci < (int)hc.size(); ++ci) {
             const HC& c = hc[ci];
-            std::set<QK> own;
-            for (const cd& v : c.s) own.insert(qk(v));
             // large classes, and classes holding one sum twice (one column each
             // in a merged class would collide), stay as they are
-            if (c.rows.size() > 16 || own.size() != c.s.size()) {
+            if (c.rows.size() > 16 || std::adjacent_find(c.s.begin(), c.s.end()) != c.s.end()) {
                 flush_run(run);
                 emit({ci});
                 continue;
@@ -588,57 +646,49 @@ void build_classes(APlan& pl, int k, cudaStream_t st) {
         }
         flush_run(run);
     }
-    // column chunks, then one device buffer for every class of this sum
-    std::vector<HC> fin;
-    for (HC& c : merged) {
+    std::vector<cd> sums;
+    std::vector<int> part;
+    for (const HC& c : merged) {
         const int nc = (int)c.s.size(), nr = (int)c.rows.size();
         for (int j0 = 0; j0 < nc; j0 += CG_BN_MAX) {
             const int w = std::min(CG_BN_MAX, nc - j0);
-            HC f;
-            f.s.assign(c.s.begin() + j0, c.s.begin() + j0 + w);
-            f.rows = c.rows;
-            f.slots.resize((size_t)nr * w);
-            for (int r = 0; r < nr; ++r)
-                for (int j = 0; j < w; ++j) f.slots[(size_t)r * w + j] = c.slots[(size_t)r * nc + j0 + j];
-            fin.push_back(std::move(f));
+            sums.clear();
+            for (int j = 0; j < w; ++j) sums.push_back(ix.sval[k][c.s[j0 + j]]);
+            if (w < nc) {
+                part.clear();
+                for (int r = 0; r < nr; ++r)
+                    part.insert(part.end(), c.slots.begin() + (size_t)r * nc + j0, c.slots.begin() + (size_t)r * nc + j0 + w);
+            }
+            const std::vector<int>& slots = w < nc ? part : c.slots;
+            CClass f{};
+            f.term = -1;
+            f.nrows = nr;
+            f.ncols = w;
+            f.s = blob.put(sums);
+            f.rows = blob.put(c.rows);
+            f.slots = blob.put(slots);
+            pl.cls[k].push_back(f);
         }
     }
-    auto al = [](size_t b) { return (b + 15) & ~size_t(15); };
-    size_t bytes = 0;
-    for (const HC& f : fin) bytes += al(f.s.size() * sizeof(cd)) + al(f.rows.size() * sizeof(int)) + al(f.slots.size() * sizeof(int));
-    pl.cbuf[k].reserve(std::max<size_t>(bytes, 16));
-    std::vector<char> host(std::max<size_t>(bytes, 16));
-    char* dev = pl.cbuf[k].as<char>();
-    size_t o = 0;
-    for (const HC& f : fin) {
-        CClass c{};
-        c.term = -1;
-        c.nrows = (int)f.rows.size();
-        c.ncols = (int)f.s.size();
-        std::memcpy(host.data() + o, f.s.data(), f.s.size() * sizeof(cd));
-        c.s = reinterpret_cast<const cd*>(dev + o);
-        o += al(f.s.size() * sizeof(cd));
-        std::memcpy(host.data() + o, f.rows.data(), f.rows.size() * sizeof(int));
-        c.rows = reinterpret_cast<const int*>(dev + o);
-        o += al(f.rows.size() * sizeof(int));
-        std::memcpy(host.data() + o, f.slots.data(), f.slots.size() * sizeof(int));
-        c.slots = reinterpret_cast<const int*>(dev + o);
-        o += al(f.slots.size() * sizeof(int));
-        pl.cls[k].push_back(c);
-    }
-    if (bytes) h2d(dev, host.data(), bytes, st);
-    pl.have_cls[k] = true;
 }
 
-void build_aplan(APlan& pl, const std::vector<int>& tids, const PermIndex& ix, int o1, int n1, int o3, int n3,
-                 const PermSums& ps, cudaStream_t st) {
+void build_aplan(APlan& pl, const std::vector<int>& pts, const PermIndex& ix, int o1, int n1, int o3, int n3,
+                 Blob& blob) {
     pl.Z1.assign(ix.Z1.begin() + o1, ix.Z1.begin() + o1 + n1);
     pl.Z3.assign(ix.Z3.begin() + o3, ix.Z3.begin() + o3 + n3);
-    const size_t nt = tids.size();
-    pl.gt = tids;
-    std::stable_sort(pl.gt.begin(), pl.gt.end(), [&](int x, int y) {
-        return std::make_pair(ix.j1[x], ix.j3[x]) < std::make_pair(ix.j1[y], ix.j3[y]);
-    });
+    const size_t nt = pts.size();
+    // in the order of (j1, j3): by j3, then stably by j1
+    pl.gt = pts;
+    std::vector<int> start, to(nt);
+    auto sort_by = [&](const std::vector<int>& j, int o, int n) {
+        start.assign(n + 1, 0);
+        for (int t : pl.gt) ++start[j[t] - o + 1];
+        for (int i = 0; i < n; ++i) start[i + 1] += start[i];
+        for (int t : pl.gt) to[start[j[t] - o]++] = t;
+        pl.gt.swap(to);
+    };
+    sort_by(ix.j3, o3, n3);
+    sort_by(ix.j1, o1, n1);
     for (size_t q = 0; q < nt; ++q) {
         const int t = pl.gt[q];
         if (q == 0 || ix.j1[t] != ix.j1[pl.gt[q - 1]] || ix.j3[t] != ix.j3[pl.gt[q - 1]]) {
@@ -648,31 +698,51 @@ void build_aplan(APlan& pl, const std::vector<int>& tids, const PermIndex& ix, i
         }
     }
     pl.goff.push_back((int)nt);
-    pl.sums = &ps;
-    const size_t ng = pl.gi1.size();
-    pl.buf.reserve((size_t)(n1 + n3) * sizeof(cd) + (nt + 3 * ng + 1) * sizeof(int) + 256);
-    char* p = pl.buf.as<char>();
-    auto take = [&](size_t b) {
-        char* r = p;
-        p += (b + 15) & ~size_t(15);
-        return r;
-    };
-    pl.dZ1 = reinterpret_cast<cd*>(take((size_t)n1 * sizeof(cd)));
-    pl.dZ3 = reinterpret_cast<cd*>(take((size_t)n3 * sizeof(cd)));
-    pl.dgt = reinterpret_cast<int*>(take(nt * sizeof(int)));
-    pl.dgoff = reinterpret_cast<int*>(take((ng + 1) * sizeof(int)));
-    pl.dgi1 = reinterpret_cast<int*>(take(ng * sizeof(int)));
-    pl.dgi3 = reinterpret_cast<int*>(take(ng * sizeof(int)));
-    auto up = [&](void* d, const void* h, size_t b) {
-        if (b) h2d(d, h, b, st);
-    };
-    up(pl.dZ1, pl.Z1.data(), (size_t)n1 * sizeof(cd));
-    up(pl.dZ3, pl.Z3.data(), (size_t)n3 * sizeof(cd));
-    up(pl.dgt, pl.gt.data(), nt * sizeof(int));
-    up(pl.dgoff, pl.goff.data(), (ng + 1) * sizeof(int));
-    up(pl.dgi1, pl.gi1.data(), ng * sizeof(int));
-    up(pl.dgi3, pl.gi3.data(), ng * sizeof(int));
+    pl.dZ1 = blob.put(pl.Z1);
+    pl.dZ3 = blob.put(pl.Z3);
+    pl.dgi1 = blob.put(pl.gi1);
+    pl.dgi3 = blob.put(pl.gi3);
 }
+
+char* upload(const Blob& blob, DevBuf& buf, cudaStream_t st) {
+    buf.reserve(std::max<size_t>(blob.h.size(), 16));
+    if (!blob.h.empty()) h2d(buf.p, blob.h.data(), blob.h.size(), st);
+    return buf.as<char>();
+}
+
+// The plans of a call.  Their classes are built on first use, while the first
+// batch's products run.
+struct Plans {
+    std::vector<APlan> list;
+    std::vector<PermIndex> perm;
+    std::vector<int> perm_of;  // plan -> permutation
+    bool have_classes = false;
+    void upload_groups(const Blob& blob, DevBuf& buf, cudaStream_t st) {
+        char* base = upload(blob, buf, st);
+        for (APlan& pl : list) {
+            rebase(pl.dZ1, base);
+            rebase(pl.dZ3, base);
+            rebase(pl.dgi1, base);
+            rebase(pl.dgi3, base);
+        }
+    }
+    void classes(DevBuf& buf, cudaStream_t st) {
+        if (have_classes) return;
+        have_classes = true;
+        for (PermIndex& ix : perm) number_sums(ix);
+        Blob blob;
+        for (size_t i = 0; i < list.size(); ++i)
+            for (int k = 0; k < 4; ++k) build_classes(list[i], k, perm[perm_of[i]], blob);
+        char* base = upload(blob, buf, st);
+        for (APlan& pl : list)
+            for (auto& cls : pl.cls)
+                for (CClass& c : cls) {
+                    rebase(c.s, base);
+                    rebase(c.rows, base);
+                    rebase(c.slots, base);
+                }
+    }
+};
 
 // Workspace of one chain inside a batch (element offsets into one cd pool).
 struct ChainWs {
@@ -720,10 +790,10 @@ GemmProblem<TA, TB, cd> gp(const typename src_t<TA>::type* A, long sai, long sak
 
 template <typename T>
 static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector<int>& bplan,
-                      const std::vector<ChainWs>& wsl, const pgx_g2_part* parts, std::vector<APlan>& plans,
+                      const std::vector<ChainWs>& wsl, const pgx_g2_part* parts, Plans& plans,
                       const std::vector<std::array<int, 4>>& rs, cd* pool, const int* d_hot,
                       const std::vector<long>& hot_off, double pole_res, int split, const std::vector<int>& bdig,
-                      cd* d_out) {
+                      std::vector<cudaEvent_t>* gemm_ev, cd* d_out) {
     Problem& P = c->P;
     cudaStream_t st = c->stream;
     constexpr bool TC = is_cd<T>::value;
@@ -744,7 +814,7 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
     for (size_t j = 0; j < idx.size(); ++j) {
         const int q = idx[j];
         const pgx_g2_part& g = parts[q];
-        const APlan& pl = plans[bplan[j]];
+        const APlan& pl = plans.list[bplan[j]];
         const ChainWs& w = wsl[j];
         const int S1 = g.block[0], S2 = g.block[1], S3 = g.block[2], S4 = g.block[3];
         const int d1 = P.dims[S1], d2 = P.dims[S2], d3 = P.dims[S3], d4 = P.dims[S4];
@@ -820,6 +890,19 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
         }
         launch_on(rest, region, st);
     };
+    auto mark = [&]() {
+        if (!gemm_ev) return;
+        gemm_ev->push_back(c->prof.event());
+        PGX_CUDA(cudaEventRecord(gemm_ev->back(), st));
+    };
+    mark();
+    if (gemm_ev) {
+        auto count = [&](const auto& list) {
+            for (const auto& g : list) c->g2t.gemm_flops += 8.0 * g.nb * g.M * g.N * (double)g.K;
+        };
+        count(pc);
+        count(pd);
+    }
     if (split) {  // the split products share one workspace: one stream
         if constexpr (TC) {
             launch_on(pa, 0, st);
@@ -848,12 +931,14 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
         launch_on(pc, 2, s0);
         launch_on(pd, 3, s1);
     }
+    mark();
+    plans.classes(c->scratch[1], st);
     // ---- contractions per triple
     std::vector<DTerm> dt;
     for (size_t j = 0; j < idx.size(); ++j) {
         const int q = idx[j];
         const pgx_g2_part& g = parts[q];
-        const APlan& pl = plans[bplan[j]];
+        const APlan& pl = plans.list[bplan[j]];
         const ChainWs& w = wsl[j];
         const int S[4] = {g.block[0], g.block[1], g.block[2], g.block[3]};
         const int d1 = P.dims[S[0]], d2 = P.dims[S[1]], d3 = P.dims[S[2]], d4 = P.dims[S[3]];
@@ -944,8 +1029,7 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
         double macs[CG_NBM][CG_NBN] = {};
         for (size_t q = 0; q < dt.size(); ++q) {
             const DTerm& d = dt[q];
-            APlan& pl = plans[d.plan];
-            build_classes(pl, d.sidx, st);
+            const APlan& pl = plans.list[d.plan];
             for (const CClass& c0 : pl.cls[d.sidx]) {
                 int bm = 0, bn = 0;
                 while (bm < CG_NBM - 1 && CG_BMS[bm] < c0.nrows) ++bm;
@@ -1006,10 +1090,51 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
     // the next batch reuses the device descriptor buffers in stream order
 }
 
-void run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, const double* z, double pole_res,
-                     double anchor_tol, int split, double* out) {
+// Whether the sum over every state runs faster in this form, every state an
+// anchor, than part by part in full matrices (pgx_g2.cu).  That form has two
+// products per pair (z1', z3') that occurs and two per z1' and z3', this one
+// four per pair of the (z1', z3') plane (z1' taken up to conjugation for a real
+// Hamiltonian) and four per z1' and z3', about 15% slower each for the
+// dressing; but that form spends some 0.25 ms per part, worth
+// 5e9 operations, on its own launches and waits.  Plaquette (96 parts, 8^3):
+// 13.2 ms there, 2.0 here; 6-site ring (216 parts, blocks to 400) 9^3: 203,
+// 171; Anderson 1+5 (blocks to 400) 8^3: 163, 93; 7-site ring (blocks to 1225)
+// 4^3: 897, 1011.
+static bool anchored_faster(const Problem& P, int nparts, const pgx_g2_part* parts, int nfreq, const Points& pt) {
+    double all[3], up[3], closed[3];  // values that occur; those above the axis, and all, with their conjugates
+    for (int k = 0; k < 3; ++k) {
+        std::vector<char> direct(pt.val[k].size(), 0);
+        for (int t = 0; t < nfreq; ++t)
+            if (!pt.flip[t]) direct[pt.id[k][pt.cls[t]]] = 1;
+            else direct[pt.id[k][pt.ncls + pt.cls[t]]] = 1;
+        all[k] = (double)std::count(direct.begin(), direct.end(), 1);
+        closed[k] = (double)pt.val[k].size();
+        up[k] = 0.0;
+        for (const cd& v : pt.val[k]) up[k] += v.y >= 0.0;
+        if (pt.npts == pt.ncls) up[k] = all[k];
+    }
+    double extra = 0.0;
+    for (int q = 0; q < nparts; ++q) {
+        double d[4];
+        for (int k = 0; k < 4; ++k) d[k] = P.dims[parts[q].block[k]];
+        const int a = parts[q].perm[0], b = parts[q].perm[2];
+        const double m1 = d[0] * d[1] * d[3], m2 = d[0] * d[1] * d[2], m3 = d[0] * d[2] * d[3], m4 = d[1] * d[2] * d[3];
+        const double there = 8.0 * std::min((double)nfreq, all[a] * all[b]) * (m3 + m4) +
+                             4.0 * (all[a] * (m1 + m2) + all[b] * (m3 + m4));
+        const double here = 8.0 * up[a] * closed[b] * (m1 + m2 + m3 + m4) +
+                            8.0 * (up[a] * (m1 + m2) + closed[b] * (m3 + m4));
+        extra += 1.15 * here - there;
+    }
+    return extra <= 5e9 * nparts;
+}
+
+bool run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, const double* z, double pole_res,
+                     double anchor_tol, int split, bool only_if_faster, double* out) {
     Problem& P = c->P;
     cudaStream_t st = c->stream;
+    Points pt;
+    build_points(pt, nfreq, z, !P.is_complex);
+    if (only_if_faster && !anchored_faster(P, nparts, parts, nfreq, pt)) return false;
     // anchor states per block (weights above the threshold)
     const std::vector<double>& w = P.w_host;  // copied when the weights were computed
     PGX_CHECK((long)w.size() == P.esize, PGX_ERR_STATE, "pgx_weights first");
@@ -1047,7 +1172,7 @@ void run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq
     DevBuf& bh = c->scratch[11];
     bh.reserve(std::max<size_t>(hot.size(), 1) * sizeof(int));
     if (!hot.empty()) h2d(bh.p, hot.data(), hot.size() * sizeof(int), st);
-    // permutations of the parts, and the frequency sums of each
+    // permutations of the parts
     std::map<std::tuple<int, int, int>, int> perm_id;
     std::vector<std::array<int, 3>> perms;
     std::vector<int> part_perm(nparts);
@@ -1060,10 +1185,6 @@ void run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq
         }
         part_perm[q] = it->second;
     }
-    std::vector<PermSums> sums(perms.size());
-    Points pt;
-    build_points(pt, nfreq, z, !P.is_complex);
-    for (size_t p = 0; p < perms.size(); ++p) build_sums(sums[p], perms[p].data(), pt);
     // anchor counts per part, and the workspace of one chain for N1 x N3 frequencies
     std::vector<std::array<int, 4>> rs(nparts);
     for (int q = 0; q < nparts; ++q)
@@ -1114,10 +1235,12 @@ void run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq
         }
         return tile_budget;
     };
-    std::vector<APlan> plans;
+    Plans plans;
+    plans.perm.resize(perms.size());
+    Blob blob;
     std::vector<std::vector<int>> perm_plans(perms.size());
     for (size_t p = 0; p < perms.size(); ++p) {
-        PermIndex ix;
+        PermIndex& ix = plans.perm[p];
         index_perm(ix, perms[p].data(), pt);
         const long N1 = (long)ix.Z1.size(), N3 = (long)ix.Z3.size();
         auto fits = [&](long b) {
@@ -1145,27 +1268,32 @@ void run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq
                 if (tl.empty()) continue;
                 const int o1 = (int)(u * b1), o3 = (int)(v * b3);
                 const int n1 = (int)std::min(b1, N1 - o1), n3 = (int)std::min(b3, N3 - o3);
-                perm_plans[p].push_back((int)plans.size());
-                plans.emplace_back();
-                build_aplan(plans.back(), tl, ix, o1, n1, o3, n3, sums[p], st);
+                perm_plans[p].push_back((int)plans.list.size());
+                plans.list.emplace_back();
+                plans.perm_of.push_back((int)p);
+                build_aplan(plans.list.back(), tl, ix, o1, n1, o3, n3, blob);
             }
     }
+    plans.upload_groups(blob, c->scratch[10], st);
     DevBuf& pool_b = c->scratch[6];
     DevBuf& out_b = c->scratch[9];
     out_b.reserve(std::max(pt.npts, 1) * sizeof(cd));
     PGX_CUDA(cudaMemsetAsync(out_b.p, 0, std::max(pt.npts, 1) * sizeof(cd), st));
     std::vector<int> batch, bplan;
     std::vector<ChainWs> bws;
+    // the full sum reports the time and operations of its products
+    std::vector<cudaEvent_t> gemm_ev;
+    std::vector<cudaEvent_t>* ev = only_if_faster ? &gemm_ev : nullptr;
     long used = 0;
     auto flush = [&]() {
         if (batch.empty()) return;
         pool_b.reserve(std::max<long>(used, 1) * sizeof(cd));
         if (P.is_complex)
             run_batch<cd>(c, batch, bplan, bws, parts, plans, rs, pool_b.as<cd>(), bh.as<int>(), hot_off, pole_res,
-                          split, bdig, out_b.as<cd>());
+                          split, bdig, ev, out_b.as<cd>());
         else
             run_batch<double>(c, batch, bplan, bws, parts, plans, rs, pool_b.as<cd>(), bh.as<int>(), hot_off, pole_res,
-                              split, bdig, out_b.as<cd>());
+                              split, bdig, ev, out_b.as<cd>());
         batch.clear();
         bplan.clear();
         bws.clear();
@@ -1175,7 +1303,7 @@ void run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq
         for (int pid : perm_plans[p])
             for (int q = 0; q < nparts; ++q) {
                 if (part_perm[q] != (int)p || !active(q)) continue;
-                ChainWs x = chain_ws(q, (long)plans[pid].Z1.size(), (long)plans[pid].Z3.size());
+                ChainWs x = chain_ws(q, (long)plans.list[pid].Z1.size(), (long)plans.list[pid].Z3.size());
                 if (used > 0 && used + x.end > budget) flush();
                 for (long* f : {&x.Lc, &x.Lr, &x.Pr, &x.Pc, &x.Rho, &x.Qc, &x.Rr, &x.Rc, &x.V1a, &x.V1b, &x.V2a,
                                 &x.V2b, &x.end})
@@ -1196,6 +1324,15 @@ void run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq
         out[2 * (size_t)t] = v.x;
         out[2 * (size_t)t + 1] = v.y;
     }
+    if (only_if_faster) {
+        for (size_t i = 0; i + 1 < gemm_ev.size(); i += 2) {
+            float ms = 0.f;
+            PGX_CUDA(cudaEventElapsedTime(&ms, gemm_ev[i], gemm_ev[i + 1]));
+            c->g2t.gemm_ms += ms;
+        }
+        for (cudaEvent_t e : gemm_ev) c->prof.spare.push_back(e);
+    }
+    return true;
 }
 
 }  // namespace pgx

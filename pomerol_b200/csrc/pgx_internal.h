@@ -403,8 +403,9 @@ void run_susc(pgx_ctx* c, int opA, int opB, int nparts, const int32_t* outer, co
 void run_ensemble_average(pgx_ctx* c, int op, double* out);
 void run_g2(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, const double* z, double pole_res,
             double coef_tol, int flags, double* out);
-void run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, const double* z, double pole_res,
-                     double anchor_tol, int split_slices, double* out);
+// only_if_faster: returns false, nothing done, where the form of pgx_g2.cu is faster
+bool run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, const double* z, double pole_res,
+                     double anchor_tol, int split_slices, bool only_if_faster, double* out);
 void run_split_gemm_check(pgx_ctx* c, int M, int N, int K, int nb, int S, unsigned long long seed, double* err,
                           double* ms_split, double* ms_fp64);
 void run_chi3(pgx_ctx* c, int channel, int nparts, const pgx_chi3_part* parts, int nfreq, const double* z,

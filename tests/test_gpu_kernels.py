@@ -122,3 +122,127 @@ def test_pair_sums(dims, nz, is_complex):
     ref[0] += 1.3 * w0
     assert abs(zero - w0) <= 40 * EPS * w0
     assert np.all(np.abs(got - ref) <= 40 * EPS * (size + 1.3 * w0))
+
+
+# ---------------------------------------------------------------- G2 and chi3
+def small_model(kind):
+    from oracle import model as M
+    if kind == "complex":
+        e = M.CoulombS("A", 2.0, -1.2) + M.CoulombS("B", 2.5, -0.9) + M.CoulombS("C", 1.5, -0.8)
+        for a, b, t in (("A", "B", 0.7 * np.exp(0.4j)), ("B", "C", 0.5j), ("C", "A", -0.6)):
+            for s in (M.UP, M.DOWN):
+                e += M.HoppingS(a, b, t, 0, 0, s, s)
+        return M.make_model(e)
+    e = M.CoulombS("C", 2.0, -0.7)
+    for k, (ek, vk) in enumerate([(-0.7, 0.4), (0.2, 0.3), (0.9, 0.5)]):
+        e += M.Level(f"b{k}", ek)
+        e += M.Hopping("C", f"b{k}", vk)
+    return M.make_model(e)
+
+
+def freq_list(form, dim, beta, rng):
+    """Forms of frequency lists: cubes that hold all, some or none of their
+    conjugates, shuffled lists with repeats, general points off the axis."""
+    def cube(ns):
+        k = np.stack(np.meshgrid(*[np.asarray(n) for n in ns], indexing="ij"), -1).reshape(-1, dim)
+        return 1j * np.pi * (2 * k + 1) / beta
+    if form == "even":
+        return cube([range(-2, 2)] * dim)
+    if form == "odd":
+        return cube([range(-1, 2)] * dim)
+    if form == "above":
+        return cube([range(0, 3)] * dim)
+    if form == "ragged":
+        return cube([range(-3, 2), range(-1, 1), range(0, 4)][:dim])
+    if form == "repeats":
+        z = cube([range(-2, 2)] * dim)
+        z = np.concatenate([z, z[::3], z.conj()[::2], z[5:6], z[5:6].conj()])
+        return z[rng.permutation(len(z))]
+    if form == "one":
+        return cube([[1]] * dim)
+    z = rng.uniform(-2, 2, (40, dim)) + 1j * rng.uniform(0.2, 3, (40, dim)) * rng.choice([-1, 1], (40, dim))
+    z[::4] = z[1::4].conj()     # some conjugate pairs
+    z[2, 0] = 0.123 + 0.0j      # on the real axis, off every pole
+    z[3, :] = z[2, :].conj()
+    return z
+
+
+FORMS = ["even", "odd", "above", "ragged", "repeats", "one", "general"]
+
+
+# A sum over at most 3e5 quadruples of terms that the resolvents bound: errors
+# stay below 1e-12 of the largest value, the bound the other parity tests use.
+@pytest.mark.parametrize("kind", ["real", "complex"])
+@pytest.mark.parametrize("form", FORMS)
+def test_g2_over_forms_of_frequency_lists(form, kind):
+    from oracle import ed as EDm
+    from oracle import lehmann as L
+    from pomerol_b200.pgx import PGX_G2_ANCHORED, PGX_G2_EXACT
+    from tests.pgx_harness import GpuED
+    m, beta = small_model(kind), 7.0
+    lab = "A" if kind == "complex" else "C"
+    u, d = m.info.getIndex(lab, 0, 1), m.info.getIndex(lab, 0, 0)
+    g, ed = GpuED(m, beta), EDm.ED(m, beta)
+    z = freq_list(form, 3, beta, np.random.default_rng(5))
+    parts = g.g2_parts(g.c(u), g.c(d), g.cdag(u), g.cdag(d))
+    oparts = L.g2_parts(ed, ed.c(u), ed.c(d), ed.cdag(u), ed.cdag(d))
+    sel = np.unique(np.linspace(0, len(z) - 1, 24).astype(int))
+    ref = L.g2_exact(ed, oparts, [tuple(z[t]) for t in sel])
+    exact = g.eng.g2(parts, z, flags=PGX_G2_EXACT)
+    anchored = g.eng.g2(parts, z, coef_tol=0.0, flags=PGX_G2_ANCHORED)
+    scale = max(np.abs(ref).max(), np.abs(exact).max())
+    assert np.abs(exact[sel] - ref).max() < 1e-12 * scale
+    assert np.abs(anchored - exact).max() < 1e-12 * scale
+    # tiles of the (z1, z3) plane, and one part at a time
+    g.eng.set_g2_workspace(0, 1 << 15)
+    tiled = g.eng.g2(parts, z, coef_tol=0.0, flags=PGX_G2_ANCHORED)
+    assert np.abs(tiled - exact).max() < 1e-12 * scale
+
+
+def test_exact_g2_on_both_sides_of_its_rule():
+    """Scattered triples of one chain of 70 to 126 states: the plane of their
+    z1 and z3 holds far more pairs than occur, so the full-matrix form runs;
+    a small grid of the same chain goes to the batched form."""
+    from pomerol_b200.pgx import PGX_G2_ANCHORED, PGX_G2_EXACT
+    rng = np.random.default_rng(9)
+    dims = [70, 96, 126, 84]
+    e = engine([symmetric(rng, n) / 4 for n in dims])
+    e.eigh()
+    e.weights(2.0)
+    ops = []
+    for q in range(4):
+        left, right = q, (q + 1) % 4
+        tgt = np.full(dims[right], -1)
+        k = min(dims[left], dims[right])
+        tgt[:k] = rng.permutation(dims[left])[:k]
+        ops.append(e.op_define([(right, left, tgt, np.where(tgt >= 0, 1.0, 0.0))]))
+        e.op_rotate(ops[-1])
+    parts = [(tuple(ops), (0, 1, 2, 3), (0, 1, 2), 1)]
+    scattered = 1j * rng.uniform(0.5, 9, (150, 3)) * rng.choice([-1, 1], (150, 3))
+    k = 1j * np.pi * (2 * np.arange(-2, 2) + 1) / 2.0
+    grid = np.stack(np.meshgrid(k, k, k, indexing="ij"), -1).reshape(-1, 3)
+    for z in (scattered, grid):
+        a = e.g2(parts, z, flags=PGX_G2_EXACT)
+        t = e.g2_timing()
+        assert t["total_ms"] > 0 and t["gemm_ms"] > 0 and t["gemm_flops"] > 0
+        b = e.g2(parts, z, coef_tol=0.0, flags=PGX_G2_ANCHORED)
+        assert np.abs(a - b).max() < 1e-12 * np.abs(a).max()
+
+
+@pytest.mark.parametrize("kind", ["real", "complex"])
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("channel", [0, 1, 2])
+def test_chi3_over_forms_of_frequency_lists(channel, form, kind):
+    from oracle import chi3 as X3
+    from oracle import ed as EDm
+    from tests.pgx_harness import GpuED
+    m, beta = small_model(kind), 7.0
+    lab = "A" if kind == "complex" else "C"
+    u, d = m.info.getIndex(lab, 0, 1), m.info.getIndex(lab, 0, 0)
+    g, ed = GpuED(m, beta), EDm.ED(m, beta)
+    z = freq_list(form, 2, beta, np.random.default_rng(6))
+    got, _ = g.chi3(channel, (u, u, d, d), z)
+    parts = X3.chi3_parts(ed, channel, ed.cdag(u), ed.c(u), ed.cdag(d), ed.c(d))
+    sel = np.unique(np.linspace(0, len(z) - 1, 24).astype(int))
+    ref = X3.chi3_exact(ed, parts, channel, [tuple(z[t]) for t in sel])
+    assert np.abs(got[sel] - ref).max() < 1e-12 * max(1.0, np.abs(ref).max())
