@@ -90,31 +90,37 @@ struct CItem {
     int cls, row0, h0, h1;
 };
 
-constexpr int CG_NX = 8;
-// rows per thread: 4 in 64-row tiles (16 thread rows), BM / 8 below (8 thread rows)
-__host__ __device__ constexpr int cg_tm(int bm) { return bm >= 64 ? 4 : bm / 8; }
+constexpr int CG_THREADS = 128;
+// of its four warps, how many split the rows; the others split the k's of a tile
+__host__ __device__ constexpr int cg_wr(int bm) { return bm >= 32 ? 4 : bm == 16 ? 2 : 1; }
 
-// One CTA per work item: BM rows x BN columns, (BM / TM) x CG_NX threads,
-// each a TM x (BN / CG_NX) block of complex accumulators.  The next k-tile's
-// operand loads are issued into registers before the current tile's products.
+// One CTA per work item: BM rows x BN columns in 8 x 8 tiles of the FP64
+// tensor cores (mma_tile).  The next k-tile's operand loads are issued into
+// registers before the current tile's products.  What bounds it: for 64-row
+// classes the FP64 pipe, on the products and a tenth of them again to form the
+// operands; for the small ones the latency of the loads, which is why their
+// warps split the k's.  Anderson 1+5, 16^3: 2.2 ms of
+// launches one after another with scalar FMAs, 1.1 together so; a plaquette 8^3,
+// every state an anchor: 0.67 and 0.12 ms.
 template <int BM, int BN>
-__global__ void __launch_bounds__((BM / cg_tm(BM)) * CG_NX)
+__global__ void __launch_bounds__(CG_THREADS, 3)
     contract_gemm_kernel(const DTerm* __restrict__ terms, const CClass* __restrict__ classes,
                          const CItem* __restrict__ items, double beta, double tol2, cd* __restrict__ out) {
-    constexpr int CG_TM = cg_tm(BM);
-    constexpr int NY = BM / CG_TM, NT = NY * CG_NX, TN = BN / CG_NX;
-    // k-tile depth: 16, or 8 where two 16-deep buffers would pass 48 KB
-    constexpr int CG_BK = (BM * BN > 64 * 24) ? 8 : 16;
+    constexpr int NT = CG_THREADS;
+    constexpr int WR = cg_wr(BM), WK = 4 / WR, FM = BM / 8 / WR, FN = BN / 8;
+    static_assert(FM * 8 * WR == BM && FN * 8 == BN, "tile shape does not fit the warps");
+    // k-tile depth: two buffers within 48 KB
+    constexpr int CG_BK = BM >= 64 ? 8 : 16;
     constexpr int LA = (BM * CG_BK + NT - 1) / NT, LB = (BN * CG_BK + NT - 1) / NT;
-    __shared__ cd As[2][CG_BK][BM + 1];
-    __shared__ cd Bs[2][CG_BK][BN + 1];
+    __shared__ __align__(16) cd As[2][CG_BK][BM + 2];
+    __shared__ __align__(16) cd Bs[2][CG_BK][BN + 2];
     __shared__ cd s_s[BN];
     __shared__ long s_oa[BM], s_ob[BM];
     __shared__ DTerm s_term;  // the sub-term's descriptor, read once per CTA
     const CItem it = items[blockIdx.x];
     const CClass cc = classes[it.cls];
     const DTerm& d = s_term;
-    const int tid = threadIdx.x, tx = tid % CG_NX, ty = tid / CG_NX;
+    const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32, wr = warp % WR, wk = warp / WR;
     if (tid == 0) s_term = terms[cc.term];
     __syncthreads();
     const int nrows = min(BM, cc.nrows - it.row0);
@@ -130,11 +136,11 @@ __global__ void __launch_bounds__((BM / cg_tm(BM)) * CG_NX)
         s_oa[r] = oa;
         s_ob[r] = ob;
     }
-    cd acc[CG_TM][TN];
+    AccC acc[FM][FN];
 #pragma unroll
-    for (int a = 0; a < CG_TM; ++a)
+    for (int a = 0; a < FM; ++a)
 #pragma unroll
-        for (int b = 0; b < TN; ++b) acc[a][b] = cd{0.0, 0.0};
+        for (int b = 0; b < FN; ++b) acc_zero(acc[a][b]);
     __syncthreads();
 
     const int nk = d.nk;
@@ -218,41 +224,39 @@ __global__ void __launch_bounds__((BM / cg_tm(BM)) * CG_NX)
         const bool more = q + 1 < nsteps;
         if (more) fetch(q + 1);
 #pragma unroll
-        for (int kk = 0; kk < CG_BK; ++kk) {
-            cd a[CG_TM], b[TN];
+        for (int k4 = 0; k4 < CG_BK; k4 += 4 * WK) {
+            const int kk = k4 + 4 * wk + lane % 4;
+            cd a[FM], b[FN];
 #pragma unroll
-            for (int u = 0; u < CG_TM; ++u) a[u] = As[buf][kk][ty + NY * u];
+            for (int u = 0; u < FM; ++u) a[u] = As[buf][kk][8 * (wr * FM + u) + lane / 4];
 #pragma unroll
-            for (int u = 0; u < TN; ++u) b[u] = Bs[buf][kk][tx + CG_NX * u];
+            for (int u = 0; u < FN; ++u) b[u] = Bs[buf][kk][8 * u + lane / 4];
 #pragma unroll
-            for (int qa = 0; qa < CG_TM; ++qa)
+            for (int qa = 0; qa < FM; ++qa)
 #pragma unroll
-                for (int qb = 0; qb < TN; ++qb) {
-                    acc[qa][qb].x = fma(a[qa].x, b[qb].x, acc[qa][qb].x);
-                    acc[qa][qb].x = fma(-a[qa].y, b[qb].y, acc[qa][qb].x);
-                    acc[qa][qb].y = fma(a[qa].x, b[qb].y, acc[qa][qb].y);
-                    acc[qa][qb].y = fma(a[qa].y, b[qb].x, acc[qa][qb].y);
-                }
+                for (int qb = 0; qb < FN; ++qb) mma_tile(acc[qa][qb], a[qa], b[qb]);
         }
         if (more) finish(q + 1, buf ^ 1);
         __syncthreads();
         buf ^= 1;
     }
 #pragma unroll
-    for (int qa = 0; qa < CG_TM; ++qa) {
-        const int r = ty + NY * qa;
+    for (int qa = 0; qa < FM; ++qa) {
+        const int r = 8 * (wr * FM + qa) + lane / 4;
         if (r >= nrows) continue;
 #pragma unroll
-        for (int qb = 0; qb < TN; ++qb) {
-            const int j = tx + CG_NX * qb;
-            if (j >= cc.ncols) continue;
-            const int t = cc.slots[(long)(it.row0 + r) * cc.ncols + j];
-            const double x = acc[qa][qb].x, y = acc[qa][qb].y;
-            if (t >= 0 && (x != 0.0 || y != 0.0)) {
-                atomicAdd(&out[t].x, d.pref * x);
-                atomicAdd(&out[t].y, d.pref * y);
+        for (int qb = 0; qb < FN; ++qb)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int j = 8 * qb + 2 * (lane % 4) + u;
+                if (j >= cc.ncols) continue;
+                const int t = cc.slots[(long)(it.row0 + r) * cc.ncols + j];
+                const cd v = acc_at(acc[qa][qb], u);
+                if (t >= 0 && (v.x != 0.0 || v.y != 0.0)) {
+                    atomicAdd(&out[t].x, d.pref * v.x);
+                    atomicAdd(&out[t].y, d.pref * v.y);
+                }
             }
-        }
     }
 }
 
@@ -264,7 +268,7 @@ constexpr int CG_BNS[CG_NBN] = {8, 16, 24, 32};
 template <int BM, int BN>
 void launch_contract_t(unsigned n, cudaStream_t st, const DTerm* t, const CClass* c, const CItem* i, double beta,
                        double tol2, cd* out) {
-    contract_gemm_kernel<BM, BN><<<n, (BM / cg_tm(BM)) * CG_NX, 0, st>>>(t, c, i, beta, tol2, out);
+    contract_gemm_kernel<BM, BN><<<n, CG_THREADS, 0, st>>>(t, c, i, beta, tol2, out);
 }
 
 template <int BM>
@@ -1023,10 +1027,16 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
     if (!dt.empty()) {
         // classes of every sub-term, grouped by tile shape (BM 32 or 64 rows,
         // BN 8 / 16 / 24 / 32 columns); a work item is one row tile of a class
-        // over a range of anchors, about 2^22 complex multiply-adds
+        // over a range of anchors: as many multiply-adds as give each SM 32
+        // items, between 2^16 (less is lost in an item's start and its sums'
+        // atomics) and 2^22
         std::vector<CClass> cls[CG_NBM][CG_NBN];
         std::vector<CItem> its[CG_NBM][CG_NBN];
         double macs[CG_NBM][CG_NBN] = {};
+        double total = 0.0;
+        for (const DTerm& d : dt)
+            for (const CClass& c0 : plans.list[d.plan].cls[d.sidx]) total += (double)c0.nrows * c0.ncols * d.nh * d.nk;
+        const long item = std::min(1L << 22, std::max(1L << 16, (long)(total / (148 * 32))));
         for (size_t q = 0; q < dt.size(); ++q) {
             const DTerm& d = dt[q];
             const APlan& pl = plans.list[d.plan];
@@ -1039,7 +1049,7 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
                 c.term = (int)q;
                 const int ci = (int)cls[bm][bn].size();
                 cls[bm][bn].push_back(c);
-                const int hc = (int)std::max<long>(1, (1L << 22) / ((long)BM * BN * std::max(d.nk, 1)));
+                const int hc = (int)std::max<long>(1, item / ((long)BM * BN * std::max(d.nk, 1)));
                 for (int r0 = 0; r0 < c.nrows; r0 += BM)
                     for (int h0 = 0; h0 < d.nh; h0 += hc) its[bm][bn].push_back(CItem{ci, r0, h0, std::min(d.nh, h0 + hc)});
                 macs[bm][bn] += (double)c.nrows * c.ncols * d.nh * d.nk;
@@ -1075,16 +1085,35 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
             {"contract_gemm_kernel<64,8>", "contract_gemm_kernel<64,16>", "contract_gemm_kernel<64,24>",
              "contract_gemm_kernel<64,32>"}};
         const double tol2 = pole_res * pole_res;
+        // the shapes' launches are independent (their sums meet in atomics):
+        // dealt to the side streams, so that one's last wave overlaps the next
+        struct Shape {
+            int a, b;
+            const CClass* c;
+            const CItem* i;
+        };
+        std::vector<Shape> shapes;
         for (int a = 0; a < CG_NBM; ++a)
             for (int b = 0; b < CG_NBN; ++b) {
                 if (its[a][b].empty()) continue;
-                ProfRange pr(kName[a][b], st, 8.0 * macs[a][b], 0.0);
                 PGX_CHECK(its[a][b].size() < (1u << 31), PGX_ERR_ARG, "G2 contraction: too many work items");
                 const CClass* dc = reinterpret_cast<const CClass*>(put(cls[a][b].data(), cls[a][b].size() * sizeof(CClass)));
                 const CItem* di = reinterpret_cast<const CItem*>(put(its[a][b].data(), its[a][b].size() * sizeof(CItem)));
-                const unsigned n = (unsigned)its[a][b].size();
-                launch_contract(CG_BMS[a], CG_BNS[b], n, st, d_terms, dc, di, P.beta, tol2, d_out);
+                shapes.push_back(Shape{a, b, dc, di});
             }
+        std::sort(shapes.begin(), shapes.end(), [&](const Shape& x, const Shape& y) { return macs[x.a][x.b] > macs[y.a][y.b]; });
+        ensure_side_streams(c);
+        const int nside = (int)std::min<size_t>(4, shapes.size());
+        PGX_CUDA(cudaEventRecord(c->fork, st));
+        for (int i = 0; i < nside; ++i) PGX_CUDA(cudaStreamWaitEvent(c->aux[i], c->fork, 0));
+        SideJoin join(c, st, nside);
+        for (size_t i = 0; i < shapes.size(); ++i) {
+            const Shape& x = shapes[i];
+            cudaStream_t sx = c->aux[i % nside];
+            ProfRange pr(kName[x.a][x.b], sx, 8.0 * macs[x.a][x.b], 0.0);
+            launch_contract(CG_BMS[x.a], CG_BNS[x.b], (unsigned)its[x.a][x.b].size(), sx, d_terms, x.c, x.i, P.beta, tol2,
+                            d_out);
+        }
         check_launch("contract_gemm_kernel");
     }
     // the next batch reuses the device descriptor buffers in stream order
