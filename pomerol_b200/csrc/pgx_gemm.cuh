@@ -54,7 +54,13 @@ template <typename TA, typename TB, typename TC> struct GemmProblem {
     int nb;
     long ba, bb, bc;
     const cd* dzs;
+    // a second output of the same strides (nullable): GEMM_CONJ the conjugate
+    // of C; GEMM_CONJ_A conj(A) B and GEMM_CONJ_B A conj(B) (A and B complex),
+    // which share the four real products of A B
+    TC* C2;
+    int mirror;
 };
+constexpr int GEMM_CONJ = 1, GEMM_CONJ_A = 2, GEMM_CONJ_B = 3;
 
 // Bytes of the per-class tile index a launch_gemm_batch of nprobs problems needs.
 inline size_t gemm_index_bytes(size_t nprobs) { return (nprobs + 16) * sizeof(int); }
@@ -96,6 +102,22 @@ struct AccR {
 struct AccC {
     double2 re, im;
 };
+// All four real products apart, for A B together with conj(A) B or A conj(B).
+struct AccQ {
+    double2 rr, ii, ri, ir;
+};
+__device__ __forceinline__ void mma_tile(AccQ& c, cd a, cd b) {
+    mma_f64(c.rr, a.x, b.x);
+    mma_f64(c.ri, a.x, b.y);
+    mma_f64(c.ii, a.y, b.y);
+    mma_f64(c.ir, a.y, b.x);
+}
+__device__ __forceinline__ void acc_zero(AccQ& c) { c.rr = c.ii = c.ri = c.ir = double2{0.0, 0.0}; }
+__device__ __forceinline__ void acc_pair(const AccQ& c, int u, int mirror, cd& first, cd& second) {
+    const double rr = u ? c.rr.y : c.rr.x, ii = u ? c.ii.y : c.ii.x, ri = u ? c.ri.y : c.ri.x, ir = u ? c.ir.y : c.ir.x;
+    first = cd{rr - ii, ri + ir};
+    second = cd{rr + ii, mirror == GEMM_CONJ_A ? ri - ir : ir - ri};
+}
 __device__ __forceinline__ void mma_tile(AccR& c, double a, double b) { mma_f64(c.re, a, b); }
 __device__ __forceinline__ void mma_tile(AccC& c, cd a, double b) {
     mma_f64(c.re, a.x, b);
@@ -144,13 +166,18 @@ __host__ __device__ constexpr int gemm_wr(int bm) { return bm <= 16 ? 1 : bm <= 
 // on 4 x 4 register tiles, 17.6 ms so.  Dressed operands in a large product
 // leave the tensor path 60% busy (75% undressed): the rest is the barrier per
 // k-tile between the dressing and the products.
-template <typename TA, typename TB, typename TC, int BM, int BN>
+//
+// QUAD: problems with GEMM_CONJ_A or GEMM_CONJ_B, in tiles of half the outputs
+// (twice the accumulators each), so two complex products for the tensor work
+// of one: 18 to 21 TFLOP/s of both with two launches side by side on the 7-site
+// ring's G2, against 10.5 each one by one.
+template <typename TA, typename TB, typename TC, int BM, int BN, bool QUAD>
 __global__ void __launch_bounds__(GEMM_THREADS, 2)
     gemm_tiles_kernel(const GemmProblem<TA, TB, TC>* __restrict__ probs, const int* __restrict__ tile0, int nprobs) {
     using VA = typename val_t<TA>::type;  // operand values as they enter the product
     using VB = typename val_t<TB>::type;
     constexpr bool CX = is_cd<VA>::value || is_cd<VB>::value;
-    using Acc = typename std::conditional<CX, AccC, AccR>::type;
+    using Acc = typename std::conditional<QUAD, AccQ, typename std::conditional<CX, AccC, AccR>::type>::type;
     constexpr bool DA = is_dressed<TA>::value, DB = is_dressed<TB>::value;
     constexpr int BK = CX ? 8 : 16;
     constexpr int WR = gemm_wr(BM), WC = GEMM_THREADS / 32 / WR;
@@ -324,6 +351,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2)
         buf ^= 1;
     }
     TC* pC = p.C + item * p.bc;
+    TC* pC2 = p.C2 ? p.C2 + item * p.bc : nullptr;
 #pragma unroll
     for (int qa = 0; qa < FM; ++qa) {
         const int gi = i0 + wr * WM + 8 * qa + lane / 4;
@@ -333,7 +361,19 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2)
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const int gj = j0 + wc * WN + 8 * qb + 2 * (lane % 4) + u;
-                if (gj < N) store_c(pC[gi * p.sc_i + gj * p.sc_j], acc_at(acc[qa][qb], u), p.accumulate);
+                if (gj >= N) continue;
+                const long o = gi * p.sc_i + gj * p.sc_j;
+                if constexpr (QUAD) {
+                    cd first, second;
+                    acc_pair(acc[qa][qb], u, p.mirror, first, second);
+                    pC[o] = first;
+                    pC2[o] = second;
+                } else {
+                    const auto v = acc_at(acc[qa][qb], u);
+                    store_c(pC[o], v, p.accumulate);
+                    if constexpr (is_cd<TC>::value)
+                        if (pC2) pC2[o] = conj(tocd(v));
+                }
             }
     }
 }
@@ -354,9 +394,24 @@ template <typename TA, typename TB, typename TC> const char* gemm_name() {
 // Tile classes (BM x BN).  A problem takes the class that pads it least
 // (ties: the larger tile); the classes other than 64x64 are used only when
 // their short side covers the problem's M or N in one tile.
-constexpr int GEMM_NCLS = 9;
-constexpr int GEMM_CLS_M[GEMM_NCLS] = {64, 16, 128, 64, 64, 32, 48, 8, 128};
-constexpr int GEMM_CLS_N[GEMM_NCLS] = {64, 128, 16, 32, 48, 64, 64, 128, 8};
+// The classes from GEMM_NCLS on are those of QUAD problems: 32 x 64 and 64 x 32
+// (the dressed operand on the short side, where fewer elements are dressed),
+// and the narrow ones.
+constexpr int GEMM_NCLS = 9, GEMM_NCLS_ALL = 15;
+constexpr int GEMM_CLS_M[GEMM_NCLS_ALL] = {64, 16, 128, 64, 64, 32, 48, 8, 128, 32, 64, 16, 128, 8, 128};
+constexpr int GEMM_CLS_N[GEMM_NCLS_ALL] = {64, 128, 16, 32, 48, 64, 64, 128, 8, 64, 32, 128, 16, 128, 8};
+
+template <typename TA, typename TB, typename TC> inline int gemm_quad_class(const GemmProblem<TA, TB, TC>& p) {
+    int best = is_dressed<TB>::value ? 10 : 9;
+    auto area = [&](int c) {
+        return (long)ceil_div(p.M, GEMM_CLS_M[c]) * GEMM_CLS_M[c] * ((long)ceil_div(p.N, GEMM_CLS_N[c]) * GEMM_CLS_N[c]);
+    };
+    for (int c = GEMM_NCLS; c < GEMM_NCLS_ALL; ++c) {
+        if ((GEMM_CLS_M[c] <= 16 && p.M > GEMM_CLS_M[c]) || (GEMM_CLS_N[c] <= 16 && p.N > GEMM_CLS_N[c])) continue;
+        if (area(c) < area(best)) best = c;
+    }
+    return best;
+}
 
 template <typename P> inline int gemm_class(const P& p) {
     int best = 0;
@@ -394,6 +449,7 @@ inline bool gemm_class_valid(int c, int M, int N) {
 }
 
 template <typename TA, typename TB, typename TC> int gemm_class_for(const GemmProblem<TA, TB, TC>& p) {
+    if (p.mirror >= GEMM_CONJ_A) return gemm_quad_class(p);
     const int f = forced_gemm_class();
     if (f >= 0 && gemm_class_valid(f, p.M, p.N)) return f;
     const GemmTune* t = active_tune();
@@ -404,11 +460,11 @@ template <typename TA, typename TB, typename TC> int gemm_class_for(const GemmPr
     return gemm_class(p);
 }
 
-template <typename TA, typename TB, typename TC, int BM, int BN>
+template <typename TA, typename TB, typename TC, int BM, int BN, bool QUAD = false>
 void launch_gemm_class(const GemmProblem<TA, TB, TC>* dp, const int* d_index, size_t pb, size_t pe, int ntiles,
                        cudaStream_t st) {
     if (pe <= pb || ntiles <= 0) return;
-    gemm_tiles_kernel<TA, TB, TC, BM, BN><<<(unsigned)ntiles, GEMM_THREADS, 0, st>>>(dp + pb, d_index, (int)(pe - pb));
+    gemm_tiles_kernel<TA, TB, TC, BM, BN, QUAD><<<(unsigned)ntiles, GEMM_THREADS, 0, st>>>(dp + pb, d_index, (int)(pe - pb));
     check_launch("gemm_tiles_kernel");
 }
 
@@ -432,6 +488,7 @@ void record_gemm_batch(const std::vector<GemmProblem<TA, TB, TC>>& probs, cudaSt
             size_t bytes = 0;
             bool redirectable = true;
             for (const auto& g : probs) {
+                if (g.mirror >= GEMM_CONJ_A) continue;  // one class rule, not tuned
                 if (g.M <= 0 || g.N <= 0 || gemm_bucket(g.M) != mb || gemm_bucket(g.N) != nb) continue;
                 if (g.sc_i < 0 || g.sc_j < 0 || g.bc < 0) redirectable = false;  // not laid out in scratch
                 // the output's extent: last item's last element
@@ -439,6 +496,7 @@ void record_gemm_batch(const std::vector<GemmProblem<TA, TB, TC>>& probs, cudaSt
                 const long last = (items - 1) * g.bc + (long)(g.M - 1) * g.sc_i + (long)(g.N - 1) * g.sc_j;
                 grp.push_back(g);
                 grp.back().C = reinterpret_cast<TC*>(bytes);  // offset into the scratch, made a pointer below
+                grp.back().C2 = nullptr;
                 bytes += ((size_t)(last + 1) * sizeof(TC) + 255) & ~size_t(255);
             }
             if (grp.empty() || !redirectable) continue;
@@ -466,12 +524,12 @@ void launch_gemm_batch(const std::vector<GemmProblem<TA, TB, TC>>& probs, void* 
     std::vector<GemmProblem<TA, TB, TC>> sorted;
     sorted.reserve(probs.size());
     std::vector<int> index;  // per class: prefix over its problems, then the total
-    index.reserve(probs.size() + 2 * GEMM_NCLS);
-    size_t pstart[GEMM_NCLS + 1] = {}, istart[GEMM_NCLS] = {};
-    int ntiles[GEMM_NCLS] = {};
+    index.reserve(probs.size() + 2 * GEMM_NCLS_ALL);
+    size_t pstart[GEMM_NCLS_ALL + 1] = {}, istart[GEMM_NCLS_ALL] = {};
+    int ntiles[GEMM_NCLS_ALL] = {};
     std::vector<int> cls(probs.size());
     for (size_t q = 0; q < probs.size(); ++q) cls[q] = gemm_class_for(probs[q]);
-    for (int c = 0; c < GEMM_NCLS; ++c) {
+    for (int c = 0; c < GEMM_NCLS_ALL; ++c) {
         pstart[c] = sorted.size();
         istart[c] = index.size();
         long t = 0;
@@ -486,7 +544,7 @@ void launch_gemm_batch(const std::vector<GemmProblem<TA, TB, TC>>& probs, void* 
         index.push_back((int)t);
         ntiles[c] = (int)t;
     }
-    pstart[GEMM_NCLS] = sorted.size();
+    pstart[GEMM_NCLS_ALL] = sorted.size();
     if (sorted.empty()) return;
     PGX_CHECK(sorted.size() * sizeof(sorted[0]) <= probs_cap, PGX_ERR_ARG, "gemm problem list overflow");
     PGX_CHECK(index.size() * sizeof(int) <= index_cap, PGX_ERR_ARG, "gemm tile index overflow");
@@ -502,7 +560,7 @@ void launch_gemm_batch(const std::vector<GemmProblem<TA, TB, TC>>& probs, void* 
                            : (is_cd<VA>::value || is_cd<VB>::value) ? 4.0 : 2.0;
     double fl = 0.0, by = 0.0;
     for (const auto& q : sorted) {
-        const double nb = std::max(q.nb, 1);
+        const double nb = std::max(q.nb, 1) * (q.mirror >= GEMM_CONJ_A ? 2.0 : 1.0);
         fl += nb * mac * q.M * (double)q.N * q.K;
         by += nb * ((double)q.M * q.K * sizeof(typename src_t<TA>::type) +
                     (double)q.K * q.N * sizeof(typename src_t<TB>::type) +
@@ -518,6 +576,18 @@ void launch_gemm_batch(const std::vector<GemmProblem<TA, TB, TC>>& probs, void* 
     launch_gemm_class<TA, TB, TC, 48, 64>(dp, di + istart[6], pstart[6], pstart[7], ntiles[6], st);
     launch_gemm_class<TA, TB, TC, 8, 128>(dp, di + istart[7], pstart[7], pstart[8], ntiles[7], st);
     launch_gemm_class<TA, TB, TC, 128, 8>(dp, di + istart[8], pstart[8], pstart[9], ntiles[8], st);
+    // an unequal pair of operand types: a plain cd x cd product is never mirrored
+    if constexpr (is_cd<VA>::value && is_cd<VB>::value && is_dressed<TA>::value != is_dressed<TB>::value &&
+                  !std::is_same<TA, Dressed<cd>>::value && !std::is_same<TB, Dressed<cd>>::value) {
+        launch_gemm_class<TA, TB, TC, 32, 64, true>(dp, di + istart[9], pstart[9], pstart[10], ntiles[9], st);
+        launch_gemm_class<TA, TB, TC, 64, 32, true>(dp, di + istart[10], pstart[10], pstart[11], ntiles[10], st);
+        launch_gemm_class<TA, TB, TC, 16, 128, true>(dp, di + istart[11], pstart[11], pstart[12], ntiles[11], st);
+        launch_gemm_class<TA, TB, TC, 128, 16, true>(dp, di + istart[12], pstart[12], pstart[13], ntiles[12], st);
+        launch_gemm_class<TA, TB, TC, 8, 128, true>(dp, di + istart[13], pstart[13], pstart[14], ntiles[13], st);
+        launch_gemm_class<TA, TB, TC, 128, 8, true>(dp, di + istart[14], pstart[14], pstart[15], ntiles[14], st);
+    } else {
+        PGX_CHECK(pstart[GEMM_NCLS_ALL] == pstart[GEMM_NCLS], PGX_ERR_ARG, "mirrored product of these operand types");
+    }
 }
 
 // C = A B through the int8 split scheme (pgx_ozaki.cu): S slices, plain

@@ -18,6 +18,14 @@
 //   A' = [Re A, Im A] (M x 2K) and, per complex column j of B, two columns
 //   [Re B_j; -Im B_j] (the real part of C_j) and [Im B_j; Re B_j] (its imaginary
 //   part), so C' = A' B' holds Re C and Im C in adjacent columns.
+// Two forms need half of that.  Where one operand is real, its row (or column)
+// is the plain real one and the other's real and imaginary parts are two
+// columns (rows) of depth K.  Where the product with one operand conjugated is
+// wanted too (GEMM_CONJ_A, GEMM_CONJ_B), both operands are plain: rows 2i, 2i + 1
+// of A' are Re and Im of row i, columns 2j, 2j + 1 of B' those of column j, so
+// a 2 x 2 block of C' holds the four real products, from which two lanes of the
+// drain form both outputs.  8-site ring's largest chain, 16^3, five digits:
+// 118 -> 60 ms in the product kernel, 24 -> 14 ms in the digits.
 // Digits are stored K-contiguous per row (A) or per column (B):
 //   A row i: [digits of slice 0 | slice 1 | ... | slice S-1], each K2 = 2K
 //   rounded up to 128 bytes; B column j: [slice S-1 | ... | slice 0].
@@ -151,11 +159,67 @@ struct OzArgs2 {
     long ea_item;
     const int* fb;
     long fb_item;
-    int M, N, K2, S;
+    int M, N, K2, S;  // M: rows of A' (two per row of A where `quad`)
+    int quad;         // 0, or GEMM_CONJ_A / GEMM_CONJ_B: rows of A' are Re and Im in turn
     cd* C;
+    cd* C2;           // second output: of `quad`, else the conjugate of C (nullable)
     long c_item, sc_i, sc_j;
     int* err;
 };
+
+// Where a drain thread's row of C' goes.
+struct OzRow {
+    cd *c, *c2;
+    int e;
+    bool ok, odd;
+};
+__device__ __forceinline__ OzRow oz_row(const OzArgs2& p, int item, int i) {
+    OzRow r;
+    r.ok = i < p.M;
+    const int ia = !r.ok ? 0 : p.quad ? i >> 1 : i;
+    r.odd = p.quad && (i & 1);
+    r.e = r.ok ? p.ea[item * p.ea_item + ia] : 0;
+    const long o = item * p.c_item + ia * p.sc_i;
+    r.c = (r.odd ? p.C2 : p.C) + o;
+    r.c2 = !p.quad && p.C2 ? p.C2 + o : nullptr;
+    return r;
+}
+// Adds eight complex columns jc0 .. of one diagonal (sixteen accumulator
+// columns), scaled, to the row's output; by whole warps.
+__device__ __forceinline__ void oz_add_columns(const OzArgs2& p, const OzRow& r, const int* fbi, const uint32_t (&v)[16],
+                                               int s, double dw, int jc0) {
+    double x[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) x[e] = (double)(int)v[e];
+    if (p.quad) {  // even lanes hold (rr, ri), odd ones (ir, ii): exact in double
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const double o0 = (double)(int)__shfl_xor_sync(0xffffffffu, v[2 * e], 1);
+            const double o1 = (double)(int)__shfl_xor_sync(0xffffffffu, v[2 * e + 1], 1);
+            const double a = x[2 * e], b = x[2 * e + 1];
+            // even: rr - ii, ri + ir; odd: rr + ii, +-(ri - ir)
+            x[2 * e] = r.odd ? o0 + b : a - o1;
+            x[2 * e + 1] = r.odd ? (p.quad == GEMM_CONJ_A ? o1 - a : a - o1) : b + o0;
+        }
+    }
+    if (!r.ok) return;
+    // the eight earlier partial sums are read before any store, so their
+    // loads are in flight together
+    cd old[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) old[e] = (s > 0 && jc0 + e < p.N) ? r.c[(long)(jc0 + e) * p.sc_j] : cd{0.0, 0.0};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int jc = jc0 + e;
+        if (jc < p.N) {
+            const double sc = pow2i(r.e + fbi[jc]) * dw;
+            const cd add{x[2 * e] * sc, x[2 * e + 1] * sc};
+            const cd sum = s == 0 ? add : cd{old[e].x + add.x, old[e].y + add.y};
+            r.c[(long)jc * p.sc_j] = sum;
+            if (r.c2 && s == p.S - 1) r.c2[(long)jc * p.sc_j] = conj(sum);
+        }
+    }
+}
 
 __device__ __forceinline__ void tma_load3(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
     asm volatile(
@@ -306,10 +370,7 @@ __global__ void __launch_bounds__(384, 1) oz_gemm_tma_kernel(const __grid_consta
     // 128 accumulator columns of half w / 4, and adds them, scaled, to C
     const int lane_base = 32 * (warp & 3), col_base = 128 * ((warp >> 2) & 1);
     if (warp < 8) {
-        const int i = i0 + lane_base + lane;
-        const bool row_ok = i < p.M;
-        const int ei = row_ok ? p.ea[item * p.ea_item + i] : 0;
-        cd* crow = p.C + item * p.c_item + (long)(row_ok ? i : 0) * p.sc_i;
+        const OzRow row = oz_row(p, item, i0 + lane_base + lane);
         const int* fbi = p.fb + item * p.fb_item;
         for (int s = 0; s < p.S; ++s) {
             if (!mbar_wait(smem_u32(&accf[s & 1]), (uint32_t)((s >> 1) & 1))) {
@@ -324,24 +385,7 @@ __global__ void __launch_bounds__(384, 1) oz_gemm_tma_kernel(const __grid_consta
                 uint32_t v[16];
                 tmem_ld16(base + 16 * q, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                if (row_ok) {
-                    // the eight earlier partial sums are read before any store, so
-                    // their loads are in flight together
-                    const int jc0 = (j0 + col_base) / 2 + 8 * q;
-                    cd old[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        old[e] = (s > 0 && jc0 + e < p.N) ? crow[(long)(jc0 + e) * p.sc_j] : cd{0.0, 0.0};
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const int jc = jc0 + e;
-                        if (jc < p.N) {
-                            const double sc = pow2i(ei + fbi[jc]) * dw;
-                            const cd add{(double)(int)v[2 * e] * sc, (double)(int)v[2 * e + 1] * sc};
-                            crow[(long)jc * p.sc_j] = s == 0 ? add : cd{old[e].x + add.x, old[e].y + add.y};
-                        }
-                    }
-                }
+                oz_add_columns(p, row, fbi, v, s, dw, (j0 + col_base) / 2 + 8 * q);
             }
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
@@ -559,10 +603,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
     // the 128 accumulator columns of half w / 4, and adds them, scaled, to C
     const int lane_base = 32 * (warp & 3), col_base = 128 * ((warp >> 2) & 1);
     if (warp < 8) {
-        const int i = i0 + lane_base + lane;
-        const bool row_ok = i < p.M;
-        const int ei = row_ok ? p.ea[item * p.ea_item + i] : 0;
-        cd* crow = p.C + item * p.c_item + (long)(row_ok ? i : 0) * p.sc_i;
+        const OzRow row = oz_row(p, item, i0 + lane_base + lane);
         const int* fbi = p.fb + item * p.fb_item;
         for (int s = 0; s < p.S; ++s) {
             if (!mbar_wait(smem_u32(&accf[s & 1]), (uint32_t)((s >> 1) & 1))) {
@@ -577,24 +618,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
                 uint32_t v[16];
                 tmem_ld16(base + 16 * q, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                if (row_ok) {
-                    // the eight earlier partial sums are read before any store, so
-                    // their loads are in flight together
-                    const int jc0 = (j0 + col_base) / 2 + 8 * q;
-                    cd old[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        old[e] = (s > 0 && jc0 + e < p.N) ? crow[(long)(jc0 + e) * p.sc_j] : cd{0.0, 0.0};
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const int jc = jc0 + e;
-                        if (jc < p.N) {
-                            const double sc = pow2i(ei + fbi[jc]) * dw;
-                            const cd add{(double)(int)v[2 * e] * sc, (double)(int)v[2 * e + 1] * sc};
-                            crow[(long)jc * p.sc_j] = s == 0 ? add : cd{old[e].x + add.x, old[e].y + add.y};
-                        }
-                    }
-                }
+                oz_add_columns(p, row, fbi, v, s, dw, (j0 + col_base) / 2 + 8 * q);
             }
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
@@ -672,9 +696,8 @@ __device__ __forceinline__ cd oz_value(const OzSrc& q, int item, int r, int k) {
 // oz_prep_kernel: one CTA per OP_ROWS rows x OP_KC reduction indices: the
 // values scaled by 127 2^-e go through a shared tile, then each thread turns
 // four consecutive k of one row into digits and stores each digit plane's four
-// bytes as one 32-bit word (a warp writes 64 contiguous bytes per row); is_b
-// selects the B' layout (two rows per complex column, digits in reverse
-// order).  Source reads are coalesced either way: lanes run along k when the
+// bytes as one 32-bit word (a warp writes 64 contiguous bytes per row); the
+// layout says what the rows are, and is_b stores the digits in reverse order.  Source reads are coalesced either way: lanes run along k when the
 // source is k-contiguous (s_k == 1), along the rows otherwise.
 constexpr int OP_ROWS = 32, OP_KC = 64, OP_THREADS = 256, OP_KSPAN = 512;
 constexpr int OP_EXP_FLOOR = -1000;  // rows below 2^-1000 keep a representable scale
@@ -727,7 +750,13 @@ __global__ void __launch_bounds__(OP_THREADS) oz_rowmax_kernel(OzSrc q, int R, i
     }
 }
 
-__global__ void __launch_bounds__(OP_THREADS) oz_prep_kernel(OzSrc q, int R, int K, int K2, int S, int is_b,
+// Layouts of an operand's digits: one row [Re, Im] or two rows [Re; -Im], [Im;
+// Re] of depth 2 K per complex row or column, or two plain rows Re, Im, or one
+// real row, of depth K.
+enum { OZ_LONG = 0, OZ_TWICE = 1, OZ_PLAIN = 2, OZ_REAL = 3 };
+inline int oz_rows_of(int layout) { return layout == OZ_TWICE || layout == OZ_PLAIN ? 2 : 1; }
+
+__global__ void __launch_bounds__(OP_THREADS) oz_prep_kernel(OzSrc q, int R, int K, int K2, int S, int layout, int is_b,
                                                              int8_t* out, long out_item, const int* ex, long ex_item) {
     __shared__ cd tile[OP_ROWS * (OP_KC + 1)];
     __shared__ double s_scale[OP_ROWS];
@@ -787,15 +816,18 @@ __global__ void __launch_bounds__(OP_THREADS) oz_prep_kernel(OzSrc q, int R, int
         }
         if (r0 + rr >= R) continue;
         const int r = r0 + rr, k = k0 + 4 * g;
-        int8_t* o0 = out + item * out_item + (long)(is_b ? 2 * r : r) * row_bytes;
+        int8_t* o0 = out + item * out_item + (long)(layout == OZ_TWICE || layout == OZ_PLAIN ? 2 * r : r) * row_bytes;
 #pragma unroll
         for (int d = 0; d < 8; ++d) {
             if (d >= S) break;
             const long base = (long)(is_b ? S - 1 - d : d) * K2;
-            // the first K2/2 positions pair with Re of the other side, the rest with Im
-            if (!is_b) {  // A' = [Re A, Im A]
+            // [Re, Im] layouts: the first K2/2 positions pair with Re of the other side, the rest with Im
+            if (layout == OZ_LONG) {  // A' = [Re A, Im A]
                 *reinterpret_cast<uint32_t*>(o0 + base + k) = wr[d];
                 *reinterpret_cast<uint32_t*>(o0 + base + half + k) = wi[d];
+            } else if (layout >= OZ_PLAIN) {
+                *reinterpret_cast<uint32_t*>(o0 + base + k) = wr[d];
+                if (layout == OZ_PLAIN) *reinterpret_cast<uint32_t*>(o0 + row_bytes + base + k) = wi[d];
             } else {
                 // negated bytes: each byte is in [-127, 127], so per-byte negation never carries
                 uint32_t nwi = 0u;
@@ -814,7 +846,7 @@ __global__ void __launch_bounds__(OP_THREADS) oz_prep_kernel(OzSrc q, int R, int
 
 // Digits of one operand (rows R, reduction length K) for `items` items:
 // exponents into ex[item][R], digits into out[item].
-void oz_prepare(const OzSrc& q, int R, int K, int K2, int S, int is_b, int items, int8_t* out, long out_item, int* ex,
+void oz_prepare(const OzSrc& q, int R, int K, int K2, int S, int layout, int is_b, int items, int8_t* out, long out_item, int* ex,
                 double min_bytes, cudaStream_t st) {
     ProfRange pr("oz_prep_kernel", st, 0.0, min_bytes);
     // below every exponent (0x80808080 = -2139062144): each row's first atomicMax sets it
@@ -822,8 +854,8 @@ void oz_prepare(const OzSrc& q, int R, int K, int K2, int S, int is_b, int items
     dim3 g1((unsigned)ceil_div((long)R, (long)OP_ROWS), (unsigned)ceil_div((long)K, (long)OP_KSPAN), (unsigned)items);
     oz_rowmax_kernel<<<g1, OP_THREADS, 0, st>>>(q, R, K, ex, R);
     check_launch("oz_rowmax_kernel");
-    dim3 g2((unsigned)ceil_div((long)R, (long)OP_ROWS), (unsigned)(K2 / 2 / OP_KC), (unsigned)items);
-    oz_prep_kernel<<<g2, OP_THREADS, 0, st>>>(q, R, K, K2, S, is_b, out, out_item, ex, R);
+    dim3 g2((unsigned)ceil_div((long)R, (long)OP_ROWS), (unsigned)(K2 / OP_KC / (layout >= OZ_PLAIN ? 1 : 2)), (unsigned)items);
+    oz_prep_kernel<<<g2, OP_THREADS, 0, st>>>(q, R, K, K2, S, layout, is_b, out, out_item, ex, R);
     check_launch("oz_prep_kernel");
 }
 
@@ -866,18 +898,68 @@ bool oz_supported(int M, int N, int K) { return M > 0 && N > 0 && K > 0 && 2L * 
 template <typename TA, typename TB>
 void oz_zgemm(const GemmProblem<TA, TB, cd>& g, int S, OzWork& w, cudaStream_t st) {
     static_assert(!is_dressed<TA>::value || !is_dressed<TB>::value, "one dressed operand at most");
-    const int M = g.M, N = g.N, K = g.K, nb = std::max(g.nb, 1);
+    const int nb = std::max(g.nb, 1);
     PGX_CHECK(!g.accumulate && !g.a_kidx && !g.b_kidx && !g.kscale && !g.conj_a, PGX_ERR_ARG,
               "split product: strided operands with row / column gathers only");
     PGX_CHECK(S >= 1 && S <= 8, PGX_ERR_ARG, "split product: 1..8 slices");
-    const int K2 = (int)(ceil_div(2L * K, OZ_BK) * OZ_BK);
+    // The sides of the product: rows of A and columns of B, or, where B is real,
+    // the transposed product, so that a real operand is always on the row side.
+    using SA = typename src_t<TA>::type;
+    using SB = typename src_t<TB>::type;
+    constexpr bool REAL_A = !is_cd<typename val_t<TA>::type>::value, REAL_B = !is_cd<typename val_t<TB>::type>::value;
+    static_assert(!REAL_A || !REAL_B, "one real operand at most");
+    struct Side {
+        OzSrc q;
+        int n;
+        bool item;  // changes per item: dressed (per-item frequency) or strided over items
+        double bytes;
+    };
+    Side sa{}, sb{};
+    sa.q.X = g.A;
+    sa.q.cplx = is_cd<SA>::value;
+    sa.q.ridx = g.a_iidx;
+    sa.q.s_r = g.sa_i;
+    sa.q.s_k = g.sa_k;
+    sa.q.s_item = g.ba;
+    if (is_dressed<TA>::value) {  // dress(x, dEa[i], dEb[k], z)
+        sa.q.Er = g.dEa;
+        sa.q.Ek = g.dEb;
+        sa.q.rk_order = 1;
+        sa.q.zs = g.dzs;
+    }
+    sa.n = g.M;
+    sa.item = is_dressed<TA>::value || g.ba != 0;
+    sa.bytes = sizeof(SA);
+    sb.q.X = g.B;
+    sb.q.cplx = is_cd<SB>::value;
+    sb.q.ridx = g.b_jidx;
+    sb.q.s_r = g.sb_j;
+    sb.q.s_k = g.sb_k;
+    sb.q.s_item = g.bb;
+    if (is_dressed<TB>::value) {  // dress(x, dEa[k], dEb[j], z)
+        sb.q.Er = g.dEb;
+        sb.q.Ek = g.dEa;
+        sb.q.rk_order = 0;
+        sb.q.zs = g.dzs;
+    }
+    sb.n = g.N;
+    sb.item = is_dressed<TB>::value || g.bb != 0;
+    sb.bytes = sizeof(SB);
+    long sc_i = g.sc_i, sc_j = g.sc_j;
+    if (REAL_B) {
+        std::swap(sa, sb);
+        std::swap(sc_i, sc_j);
+    }
+    const int M = sa.n, N = sb.n, K = g.K;
+    const bool quad = g.C2 && g.mirror >= GEMM_CONJ_A, real = REAL_A || REAL_B;
+    const int la = quad ? OZ_PLAIN : real ? OZ_REAL : OZ_LONG, lb = quad || real ? OZ_PLAIN : OZ_TWICE;
+    const int K2 = (int)(ceil_div((quad || real ? 1L : 2L) * K, OZ_BK) * OZ_BK);
     const long row_bytes = (long)S * K2;
-    // an operand changes per item when it is dressed (per-item frequency) or strided over items
-    const bool a_item = is_dressed<TA>::value || g.ba != 0;
-    const bool b_item = is_dressed<TB>::value || g.bb != 0;
+    const bool a_item = sa.item, b_item = sb.item;
+    const int Mr = M * oz_rows_of(la);  // rows of A'
     // int32 accumulation: depth (S) K2 with |digit| <= 127 stays below 2^31
     PGX_CHECK((double)S * K2 * 127.0 * 127.0 < 2147483647.0, PGX_ERR_ARG, "split product too deep for int32");
-    const long a_bytes = (long)M * row_bytes, b_bytes = 2L * N * row_bytes;
+    const long a_bytes = (long)Mr * row_bytes, b_bytes = 2L * N * row_bytes;
     // items per chunk under about 4 GiB of digits
     const long per_item = (a_item ? a_bytes : 0) + (b_item ? b_bytes : 0);
     int chunk = nb;
@@ -901,51 +983,22 @@ void oz_zgemm(const GemmProblem<TA, TB, cd>& g, int S, OzWork& w, cudaStream_t s
         PGX_CUDA(cudaFuncSetAttribute(oz_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ2_SMEM));
         if (dev >= 0 && dev < 64) attr[dev] = true;
     }
-    using SA = typename src_t<TA>::type;
-    using SB = typename src_t<TB>::type;
     for (int b0 = 0; b0 < nb; b0 += chunk) {
         const int cn = std::min(chunk, nb - b0);
-        // A rows: A(i, k) = A[i sa_i + k sa_k]; dressed as dress(x, dEa[i], dEb[k], z)
-        if (a_item || b0 == 0) {
-            OzSrc q{};
-            q.X = g.A + (a_item ? b0 * g.ba : 0);
-            q.cplx = is_cd<SA>::value;
-            q.ridx = g.a_iidx;
-            q.s_r = g.sa_i;
-            q.s_k = g.sa_k;
-            q.s_item = g.ba;
-            if (is_dressed<TA>::value) {
-                q.Er = g.dEa;
-                q.Ek = g.dEb;
-                q.rk_order = 1;
-                q.zs = g.dzs + b0;
-            }
-            const int items = a_item ? cn : 1;
+        auto digits = [&](const Side& x, int layout, int is_b, DevBuf& out, long bytes, DevBuf& ex) {
+            if (!x.item && b0 != 0) return;
+            OzSrc src = x.q;
+            if (x.item) src.X = static_cast<const char*>(x.q.X) + (size_t)(b0 * x.q.s_item) * (size_t)x.bytes;
+            if (src.zs) src.zs += b0;
+            const int items = x.item ? cn : 1;
             // minimum traffic: the source values twice (maxima, digits), the digits once
-            oz_prepare(q, M, K, K2, S, 0, items, w.A.as<int8_t>(), a_bytes, w.ea.as<int>(),
-                       2.0 * items * M * K * (is_cd<SA>::value ? 16.0 : 8.0) + (double)items * a_bytes, st);
-        }
-        // B columns: B(k, j) = B[k sb_k + j sb_j]; dressed as dress(x, dEa[k], dEb[j], z)
-        if (b_item || b0 == 0) {
-            OzSrc q{};
-            q.X = g.B + (b_item ? b0 * g.bb : 0);
-            q.cplx = is_cd<SB>::value;
-            q.ridx = g.b_jidx;
-            q.s_r = g.sb_j;
-            q.s_k = g.sb_k;
-            q.s_item = g.bb;
-            if (is_dressed<TB>::value) {
-                q.Er = g.dEb;
-                q.Ek = g.dEa;
-                q.rk_order = 0;
-                q.zs = g.dzs + b0;
-            }
-            const int items = b_item ? cn : 1;
-            oz_prepare(q, N, K, K2, S, 1, items, w.B.as<int8_t>(), b_bytes, w.fb.as<int>(),
-                       2.0 * items * N * K * (is_cd<SB>::value ? 16.0 : 8.0) + (double)items * b_bytes, st);
-        }
+            oz_prepare(src, x.n, K, K2, S, layout, is_b, items, out.as<int8_t>(), bytes, ex.as<int>(),
+                       2.0 * items * x.n * K * x.bytes + (double)items * bytes, st);
+        };
+        digits(sa, la, 0, w.A, a_bytes, w.ea);
+        digits(sb, lb, 1, w.B, b_bytes, w.fb);
         const bool pair = w.cta_pair != 0;
-        const CUtensorMap tmA = digit_map(w.A.p, row_bytes, M, a_item ? cn : 1, pair ? OZ2_HALF : OZ_BM);
+        const CUtensorMap tmA = digit_map(w.A.p, row_bytes, Mr, a_item ? cn : 1, pair ? OZ2_HALF : OZ_BM);
         const CUtensorMap tmB = digit_map(w.B.p, row_bytes, 2L * N, b_item ? cn : 1, pair ? OZ2_HALF : OZ_BN);
         OzArgs2 a{};
         a.a_items = a_item;
@@ -954,23 +1007,26 @@ void oz_zgemm(const GemmProblem<TA, TB, cd>& g, int S, OzWork& w, cudaStream_t s
         a.ea_item = a_item ? M : 0;
         a.fb = w.fb.as<int>();
         a.fb_item = b_item ? N : 0;
-        a.M = M;
+        a.M = Mr;
+        a.quad = quad ? (g.mirror == GEMM_CONJ_A ? GEMM_CONJ_A : GEMM_CONJ_B) : 0;
         a.N = N;
         a.K2 = K2;
         a.S = S;
         a.C = g.C + (long)b0 * g.bc;
+        a.C2 = g.C2 ? g.C2 + (long)b0 * g.bc : nullptr;
         a.c_item = g.bc;
-        a.sc_i = g.sc_i;
-        a.sc_j = g.sc_j;
+        a.sc_i = sc_i;
+        a.sc_j = sc_j;
         a.err = w.err.as<int>();
         // algorithmic work, as int8 operations (2 per multiply-add): per complex
-        // multiply-add 4 real ones in each of the S(S+1)/2 digit products;
+        // multiply-add 4 real ones (2 with a real operand; with both outputs of
+        // `quad` 4 for two) in each of the S(S+1)/2 digit products;
         // minimum traffic: the digits of both operands once and C written once
-        const double fl = 2.0 * 4.0 * (S * (S + 1) / 2) * (double)M * N * K * cn;
+        const double fl = 2.0 * (real ? 2.0 : 4.0) * (S * (S + 1) / 2) * (double)M * N * K * cn;
         const double by = (double)(a_item ? cn : 1) * a_bytes + (double)(b_item ? cn : 1) * b_bytes +
-                          16.0 * (double)M * N * cn;
+                          16.0 * (double)M * N * cn * (g.C2 ? 2.0 : 1.0);
         if (pair) {  // 256 x 256 tiles, one per CTA pair
-            a.tiles_m = (int)ceil_div((long)M, 2L * OZ2_HALF);
+            a.tiles_m = (int)ceil_div((long)Mr, 2L * OZ2_HALF);
             a.tiles_n = (int)ceil_div(2L * N, 2L * OZ2_HALF);
             PGX_CHECK((long)a.tiles_m * a.tiles_n < (1L << 30), PGX_ERR_ARG, "split product: too many tiles");
             dim3 grid((unsigned)(2L * a.tiles_m * a.tiles_n), 1u, (unsigned)cn);
@@ -978,7 +1034,7 @@ void oz_zgemm(const GemmProblem<TA, TB, cd>& g, int S, OzWork& w, cudaStream_t s
             oz_gemm_pair_kernel<<<grid, 384, OZ2_SMEM, st>>>(tmA, tmB, a);
             check_launch("oz_gemm_pair_kernel");
         } else {
-            a.tiles_m = (int)ceil_div((long)M, OZ_BM);
+            a.tiles_m = (int)ceil_div((long)Mr, OZ_BM);
             a.tiles_n = (int)ceil_div(2L * N, OZ_BN);
             PGX_CHECK((long)a.tiles_m * a.tiles_n < (1L << 31), PGX_ERR_ARG, "split product: too many tiles");
             dim3 grid((unsigned)((long)a.tiles_m * a.tiles_n), 1u, (unsigned)cn);
