@@ -161,16 +161,15 @@ __host__ __device__ constexpr int gemm_wr(int bm) { return bm <= 16 ? 1 : bm <= 
 // through registers, both issued before the current k-tile's products.  The
 // leading dimensions (BM + 2 complex, BM + 4 real) put the 4 k x 4 (8) rows
 // that a fragment load touches together in different banks.  Complex x complex
-// 2048^3: 27.4 TFLOP/s (peak of the FP64 tensor path 37); the chi3 of Anderson
+// 2048^3: 31.8 TFLOP/s (peak of the FP64 tensor path 37); the chi3 of Anderson
 // 1+5 on 32 x 32 duplets, whose products these are: 23.3 ms with scalar FMAs
-// on 4 x 4 register tiles, 17.6 ms so.  Dressed operands in a large product
-// leave the tensor path 60% busy (75% undressed): the rest is the barrier per
-// k-tile between the dressing and the products.
+// on 4 x 4 register tiles, 17.6 ms when the products moved here.  Deeper
+// k-tiles (16 for mixed types, 32 for real ones) measured no faster.
 //
 // QUAD: problems with GEMM_CONJ_A or GEMM_CONJ_B, in tiles of half the outputs
 // (twice the accumulators each), so two complex products for the tensor work
-// of one: 18 to 21 TFLOP/s of both with two launches side by side on the 7-site
-// ring's G2, against 10.5 each one by one.
+// of one: 25 to 28 TFLOP/s of both in each of two launches side by side on the
+// 7-site ring's G2, against 10.5 each one by one.
 template <typename TA, typename TB, typename TC, int BM, int BN, bool QUAD>
 __global__ void __launch_bounds__(GEMM_THREADS, 2)
     gemm_tiles_kernel(const GemmProblem<TA, TB, TC>* __restrict__ probs, const int* __restrict__ tile0, int nprobs) {
@@ -216,111 +215,108 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2)
 #pragma unroll
         for (int b = 0; b < FN; ++b) acc_zero(acc[a][b]);
 
-    const bool a_i_fast = (p.sa_i == 1);
-    const bool b_j_fast = (p.sb_j == 1);
-    const bool a_reg = DA || p.conj_a, b_reg = DB || p.kscale != nullptr;
-    // position (row or column, k) inside the tile of element l of a k-tile
-    auto a_pos = [&](int l, int& ii, int& kk) {
-        if (a_i_fast) {
-            ii = l % BM;
-            kk = l / BM;
-        } else {
-            ii = l / BK;
-            kk = l % BK;
-        }
-    };
-    auto b_pos = [&](int l, int& jj, int& kk) {
-        if (b_j_fast) {
-            jj = l % BN;
-            kk = l / BN;
-        } else {
-            jj = l / BK;
-            kk = l % BK;
-        }
-    };
+    // Each thread copies the same elements of every k-tile (LA of A, LB of B);
+    // their places, source pointers and row energies are set up once, since
+    // recomputing them cost more issue slots than the products (18 instructions
+    // per tensor instruction for a real x dressed product, and the tensor path
+    // 44% busy).  Complex x complex 2048^3: 27.4 -> 31.8 TFLOP/s; the 7-site
+    // ring's G2 (7^3): 386 -> 291 ms; chi3 of Anderson 1+5: 10.6 -> 8.9 ms.
+    // k gathers, kscale and conj_a come with plain operands of one type only
+    constexpr bool GATHER = std::is_same<TA, TB>::value;
+    const bool a_reg = DA || (GATHER && p.conj_a), b_reg = DB || (GATHER && p.kscale != nullptr);
+    const int *a_kidx = GATHER ? p.a_kidx : nullptr, *b_kidx = GATHER ? p.b_kidx : nullptr;
+    const long sa_k = p.sa_k, sb_k = p.sb_k;
     using SA = typename src_t<TA>::type;
     using SB = typename src_t<TB>::type;
+    const SA* srcA[LA];  // next element (k gathered: element k = 0 of its row)
+    const SB* srcB[LB];
+    int atA[LA], atB[LB];  // place in the tile
+    int kA[LA], kB[LB];    // k inside the tile; beyond every K outside the problem
     SA ra[LA];
     SB rb[LB];
-    double ea[DA || DB ? (DA ? LA : LB) : 1], eb[DA || DB ? (DA ? LA : LB) : 1];
-    // issues the loads of the k-tile at k0 (buffer buf)
+    double eA[DA ? LA : 1], eB[DB ? LB : 1];  // energies of the rows of A, columns of B
+    double ek[DA || DB ? (DA ? LA : LB) : 1];
+#pragma unroll
+    for (int q = 0; q < LA; ++q) {
+        const int l = tid + q * GEMM_THREADS;
+        const bool fast = p.sa_i == 1;
+        const int ii = fast ? l % BM : l / BK, kk = fast ? l / BM : l % BK;
+        const bool in = (BM * BK % GEMM_THREADS == 0 || l < BM * BK) && i0 + ii < M;
+        const long iq = !in ? 0 : p.a_iidx ? p.a_iidx[i0 + ii] : i0 + ii;
+        atA[q] = kk * LDA + ii;
+        kA[q] = in ? kk : 1 << 30;
+        srcA[q] = pA + iq * p.sa_i + (a_kidx || !in ? 0 : kk * sa_k);
+        if constexpr (DA) eA[q] = in ? p.dEa[iq] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < LB; ++q) {
+        const int l = tid + q * GEMM_THREADS;
+        const bool fast = p.sb_j == 1;
+        const int jj = fast ? l % BN : l / BK, kk = fast ? l / BN : l % BK;
+        const bool in = (BN * BK % GEMM_THREADS == 0 || l < BN * BK) && j0 + jj < N;
+        const long jq = !in ? 0 : p.b_jidx ? p.b_jidx[j0 + jj] : j0 + jj;
+        atB[q] = kk * LDB + jj;
+        kB[q] = in ? kk : 1 << 30;
+        srcB[q] = pB + jq * p.sb_j + (b_kidx || !in ? 0 : kk * sb_k);
+        if constexpr (DB) eB[q] = in ? p.dEb[jq] : 0.0;
+    }
+    const long stepA = BK * sa_k, stepB = BK * sb_k;
+    // issues the loads of the k-tile at k0 (buffer buf), k-tiles in order
     auto load = [&](int k0, int buf) {
+        const int left = K - k0;
 #pragma unroll
         for (int q = 0; q < LA; ++q) {
-            const int l = tid + q * GEMM_THREADS;
-            if (BM * BK % GEMM_THREADS == 0 || l < BM * BK) {
-                int ii, kk;
-                a_pos(l, ii, kk);
-                const int gi = i0 + ii, gk = k0 + kk;
-                const bool in = gi < M && gk < K;
-                long kq = 0, iq = 0;
-                if (in) {
-                    kq = p.a_kidx ? p.a_kidx[gk] : gk;
-                    iq = p.a_iidx ? p.a_iidx[gi] : gi;
-                }
-                const SA* src = pA + iq * p.sa_i + kq * p.sa_k;
-                if constexpr (DA) {
-                    ra[q] = in ? *src : zero_of<SA>();
-                    ea[q] = in ? p.dEa[iq] : 0.0;
-                    eb[q] = in ? p.dEb[kq] : 0.0;
-                } else {
-                    if (a_reg) ra[q] = in ? maybe_conj(*src, 1) : zero_of<SA>();
-                    else cp_elem(&As[buf][kk][ii], src, in);
-                }
+            if (BM * BK % GEMM_THREADS != 0 && tid + q * GEMM_THREADS >= BM * BK) continue;
+            const bool in = kA[q] < left;
+            const SA* src = srcA[q];
+            if (a_kidx) src += in ? a_kidx[k0 + kA[q]] * sa_k : 0L;
+            else srcA[q] += stepA;
+            src = in ? src : pA;
+            if constexpr (DA) {
+                ra[q] = in ? *src : zero_of<SA>();
+                ek[q] = in ? p.dEb[a_kidx ? a_kidx[k0 + kA[q]] : k0 + kA[q]] : 0.0;
+            } else {
+                if (a_reg) ra[q] = in ? maybe_conj(*src, 1) : zero_of<SA>();
+                else cp_elem(&As[buf][0][0] + atA[q], src, in);
             }
         }
 #pragma unroll
         for (int q = 0; q < LB; ++q) {
-            const int l = tid + q * GEMM_THREADS;
-            if (BN * BK % GEMM_THREADS == 0 || l < BN * BK) {
-                int jj, kk;
-                b_pos(l, jj, kk);
-                const int gj = j0 + jj, gk = k0 + kk;
-                const bool in = gj < N && gk < K;
-                long kq = 0, jq = 0;
-                if (in) {
-                    kq = p.b_kidx ? p.b_kidx[gk] : gk;
-                    jq = p.b_jidx ? p.b_jidx[gj] : gj;
-                }
-                const SB* src = pB + kq * p.sb_k + jq * p.sb_j;
-                if constexpr (DB) {
-                    rb[q] = in ? *src : zero_of<SB>();
-                    ea[q] = in ? p.dEa[kq] : 0.0;
-                    eb[q] = in ? p.dEb[jq] : 0.0;
-                } else {
-                    if (b_reg) rb[q] = in ? scale_by(*src, p.kscale[gk]) : zero_of<SB>();
-                    else cp_elem(&Bs[buf][kk][jj], src, in);
-                }
+            if (BN * BK % GEMM_THREADS != 0 && tid + q * GEMM_THREADS >= BN * BK) continue;
+            const bool in = kB[q] < left;
+            const SB* src = srcB[q];
+            if (b_kidx) src += in ? b_kidx[k0 + kB[q]] * sb_k : 0L;
+            else srcB[q] += stepB;
+            src = in ? src : pB;
+            if constexpr (DB) {
+                rb[q] = in ? *src : zero_of<SB>();
+                ek[q] = in ? p.dEa[b_kidx ? b_kidx[k0 + kB[q]] : k0 + kB[q]] : 0.0;
+            } else {
+                if (b_reg) rb[q] = in ? scale_by(*src, p.kscale[k0 + kB[q]]) : zero_of<SB>();
+                else cp_elem(&Bs[buf][0][0] + atB[q], src, in);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     // stores the register operands of that k-tile (dressed), then waits for its copies
     auto store = [&](int k0, int buf) {
+        const int left = K - k0;
         if (a_reg) {
 #pragma unroll
             for (int q = 0; q < LA; ++q) {
-                const int l = tid + q * GEMM_THREADS;
-                if (BM * BK % GEMM_THREADS == 0 || l < BM * BK) {
-                    int ii, kk;
-                    a_pos(l, ii, kk);
-                    if constexpr (DA)
-                        As[buf][kk][ii] = i0 + ii < M && k0 + kk < K ? dress(ra[q], ea[q], eb[q], dz) : cd{0.0, 0.0};
-                    else As[buf][kk][ii] = ra[q];
-                }
+                if (BM * BK % GEMM_THREADS != 0 && tid + q * GEMM_THREADS >= BM * BK) continue;
+                VA* at = &As[buf][0][0] + atA[q];
+                if constexpr (DA) *at = kA[q] < left ? dress(ra[q], eA[q], ek[q], dz) : cd{0.0, 0.0};
+                else *at = ra[q];
             }
         }
         if (b_reg) {
 #pragma unroll
             for (int q = 0; q < LB; ++q) {
-                const int l = tid + q * GEMM_THREADS;
-                if (BN * BK % GEMM_THREADS == 0 || l < BN * BK) {
-                    int jj, kk;
-                    b_pos(l, jj, kk);
-                    if constexpr (DB)
-                        Bs[buf][kk][jj] = j0 + jj < N && k0 + kk < K ? dress(rb[q], ea[q], eb[q], dz) : cd{0.0, 0.0};
-                    else Bs[buf][kk][jj] = rb[q];
-                }
+                if (BN * BK % GEMM_THREADS != 0 && tid + q * GEMM_THREADS >= BN * BK) continue;
+                VB* at = &Bs[buf][0][0] + atB[q];
+                if constexpr (DB) *at = kB[q] < left ? dress(rb[q], ek[q], eB[q], dz) : cd{0.0, 0.0};
+                else *at = rb[q];
             }
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -528,7 +524,12 @@ void launch_gemm_batch(const std::vector<GemmProblem<TA, TB, TC>>& probs, void* 
     size_t pstart[GEMM_NCLS_ALL + 1] = {}, istart[GEMM_NCLS_ALL] = {};
     int ntiles[GEMM_NCLS_ALL] = {};
     std::vector<int> cls(probs.size());
-    for (size_t q = 0; q < probs.size(); ++q) cls[q] = gemm_class_for(probs[q]);
+    for (size_t q = 0; q < probs.size(); ++q) {
+        const auto& g = probs[q];
+        PGX_CHECK((std::is_same<TA, TB>::value || (!g.a_kidx && !g.b_kidx && !g.kscale && !g.conj_a)), PGX_ERR_ARG,
+                  "k gathers need operands of one plain type");
+        cls[q] = gemm_class_for(g);
+    }
     for (int c = 0; c < GEMM_NCLS_ALL; ++c) {
         pstart[c] = sorted.size();
         istart[c] = index.size();
