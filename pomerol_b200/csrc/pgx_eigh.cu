@@ -70,7 +70,6 @@ __device__ double block_sum(double v, double* red) {
 constexpr int BHH_NB = 32;  // panel width
 constexpr int BHH_COL_THREADS = 512, BHH_CS = 8;  // at most BHH_CS CTAs of a block per column step
 constexpr int BHH_SYMV_THREADS = 128;
-constexpr int BHH_SYMV_ROWS = 16;  // rows per symv CTA, four per warp
 
 struct BigBlk {
     long moff, eoff, boff;  // matrix and vector offsets; scratch offset in S (doubles)
@@ -246,12 +245,17 @@ __global__ void __launch_bounds__(BHH_COL_THREADS, 2) bhh_col_kernel(BigArgs g) 
 
 // y(j+1:) = A(j+1:, j+1:) v for column j = col of every active block, and the
 // dots W_s . v, V_s . v of the panel's earlier columns as further rows; grid
-// (rows, block), four rows per warp (each entry of v is loaded once for the
-// four, and eight row loads are in flight per lane).  What bounds it: reading
-// the trailing matrix, from L2 where the active blocks fit, else from HBM.
-// 64 models of 3 to 6 bath sites, whose large blocks exceed L2: 102 ms for all
-// columns, 4.4 TB/s, against 131 with one row and two loads per lane.
+// (rows, block), RW rows per warp and 8 / RW columns per lane at once, so eight
+// row loads are in flight per lane, and with several rows each entry of v is
+// loaded once for them.  What bounds it: reading the trailing matrix, from HBM
+// where the active blocks exceed L2 (64 models of 3 to 6 bath sites, all
+// columns: 90 ms, 5.0 TB/s, against 102 with a rest of up to 64 columns read
+// one load at a time), else the latency of L2 with the warps there are, hence
+// fewer rows per warp for fewer rows (blocks of 4 x 1225 and 8 x 735 states,
+// whole eigensolve: 24.8 ms, against 32.3 with four rows per warp throughout).
+template <int RW>
 __global__ void __launch_bounds__(BHH_SYMV_THREADS) bhh_symv_kernel(BigArgs g) {
+    constexpr int U = 8 / RW;
     cudaTriggerProgrammaticLaunchCompletion();
     const BigBlk bl = g.blk[blockIdx.y];
     const int n = bl.n, j = g.col, cc = j - g.k, m = n - j - 1, rows = m + 2 * cc;
@@ -260,36 +264,49 @@ __global__ void __launch_bounds__(BHH_SYMV_THREADS) bhh_symv_kernel(BigArgs g) {
     double* y = V + 2L * BHH_NB * n + (j + 1);
     double* dots = V + bhh_dots_at(n);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int rr = blockIdx.x * BHH_SYMV_ROWS + wid * 4;
+    const int rr = (blockIdx.x * (BHH_SYMV_THREADS / 32) + wid) * RW;
     if (rr >= rows) return;
-    const double* p[4];
+    const double* p[RW];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < RW; ++u) {
         const int r = min(rr + u, rows - 1), d = r - m;
         p[u] = r < m ? g.A + bl.moff + (long)(j + 1 + r) * n + (j + 1)
                      : V + ((d & 1) ? 0L : (long)BHH_NB * n) + (long)(d >> 1) * n + (j + 1);
     }
     cudaGridDependencySynchronize();
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    int i = lane;
-    for (; i + 32 < m; i += 64) {
-        const double v0 = v[i], v1 = v[i + 32];
-        double a[4], e[4];
+    double s[RW];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            a[u] = p[u][i];
-            e[u] = p[u][i + 32];
+    for (int u = 0; u < RW; ++u) s[u] = 0.0;
+    int i = lane;
+    for (; i + 32 * (U - 1) < m; i += 32 * U) {
+        double x[U], a[RW][U];
+#pragma unroll
+        for (int t = 0; t < U; ++t) {
+            x[t] = v[i + 32 * t];
+#pragma unroll
+            for (int u = 0; u < RW; ++u) a[u][t] = p[u][i + 32 * t];
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) s[u] = fma(e[u], v1, fma(a[u], v0, s[u]));
-    }
-    if (i < m) {
-        const double v0 = v[i];
+        for (int u = 0; u < RW; ++u)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) s[u] = fma(p[u][i], v0, s[u]);
+            for (int t = 0; t < U; ++t) s[u] = fma(a[u][t], x[t], s[u]);
+    }
+    {  // the rest: up to U columns per lane
+        double x[U], a[RW][U];
+#pragma unroll
+        for (int t = 0; t < U; ++t) {
+            const bool in = i + 32 * t < m;
+            x[t] = in ? v[i + 32 * t] : 0.0;
+#pragma unroll
+            for (int u = 0; u < RW; ++u) a[u][t] = in ? p[u][i + 32 * t] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < RW; ++u)
+#pragma unroll
+            for (int t = 0; t < U; ++t) s[u] = fma(a[u][t], x[t], s[u]);
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < RW; ++u) {
         const double t = warp_sum(s[u]);
         const int r = rr + u;
         if (lane == 0 && r < rows) {
@@ -1545,13 +1562,15 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
         PGX_CUDA(cudaLaunchKernelEx(&cfg, bhh_col_kernel, a));
         check_launch("bhh_col_kernel");
     };
-    auto symv_step = [&](int rows, double bytes) {
-        cfg.gridDim = dim3((unsigned)ceil_div(rows, BHH_SYMV_ROWS), (unsigned)a.nact);
+    auto symv_step = [&](int rows, long all_rows, double bytes) {
+        // rows per warp: 24 warps per SM where there are that many rows
+        const int rw = all_rows >= 4L * 148 * 24 ? 4 : all_rows >= 2L * 148 * 24 ? 2 : 1;
+        cfg.gridDim = dim3((unsigned)ceil_div(rows, rw * (BHH_SYMV_THREADS / 32)), (unsigned)a.nact);
         cfg.blockDim = dim3(BHH_SYMV_THREADS);
         cfg.dynamicSmemBytes = 0;
         cfg.numAttrs = 1;
         ProfRange r2("bhh_symv_kernel", st, 0.0, bytes);
-        PGX_CUDA(cudaLaunchKernelEx(&cfg, bhh_symv_kernel, a));
+        PGX_CUDA(cudaLaunchKernelEx(&cfg, rw == 4 ? bhh_symv_kernel<4> : rw == 2 ? bhh_symv_kernel<2> : bhh_symv_kernel<1>, a));
         check_launch("bhh_symv_kernel");
     };
     std::vector<GemmProblem<double, double, double>> probs;
@@ -1569,11 +1588,13 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
             a.fin = -1;
             a.nact = nact(j);
             double bytes = 0.0;
+            long all_rows = 0;
             for (int i = 0; i < a.nact; ++i) {
                 const double m = dims[big[i]] - j - 1;
                 bytes += 8.0 * m * m;
+                all_rows += dims[big[i]] - j - 1 + 2 * (j - k);
             }
-            symv_step(nmax - j - 1 + 2 * (j - k), bytes);
+            symv_step(nmax - j - 1 + 2 * (j - k), all_rows, bytes);
         }
         a.fin = jend - 1;
         a.col = -1;
