@@ -68,7 +68,7 @@ __device__ double block_sum(double v, double* red) {
 // triangular factor of the panel's block reflector I - V T V^T (LAPACK
 // dlarft).  Every such block of a problem advances in the same launches.
 constexpr int BHH_NB = 32;  // panel width
-constexpr int BHH_COL_THREADS = 512, BHH_CS = 8;  // at most BHH_CS CTAs of a block per column step
+constexpr int BHH_COL_THREADS = 512;
 constexpr int BHH_SYMV_THREADS = 128;
 
 struct BigBlk {
@@ -96,77 +96,104 @@ __host__ __device__ inline long bhh_scratch_doubles(int n) {
 }
 __host__ __device__ inline long bhh_dots_at(int n) { return bhh_scratch_doubles(n) - 2 * BHH_NB; }
 
-// Completes w of column fin (in this panel) and reflects column col = fin + 1,
-// a cluster of CTAs per block, each with a share of the rows.  Both need every
-// row's combination of the panel's earlier V and W columns, so one sweep reads
-// them for both (four lanes a row, each a quarter of the columns, all loads in
-// flight at once): the new column is formed but for the term in the w being
-// completed, which follows once the cluster knows w . v.  Sums and single
-// elements are pushed into the other CTAs ahead of the barrier; W is written
-// after the last barrier, which would wait for it.  What bounds it: the
-// latency of a chain of L2 reads, two barriers and two block sums.  7-site
-// ring (12 blocks to 1225 states), with the product kernel: 34 -> 20 us a
-// column against one CTA of 1024 threads per block reading V and W three times.
+// Completes w of column fin (in this panel) and brings column col = fin + 1 up
+// to date; grid (row groups, block).  The column stays raw in V: the product
+// kernel reflects it, and leaves tau and the reflector's leading entry v0 (in
+// y[fin]), which takes its place in V here.  Every CTA finds w . v for itself,
+//   w . v = tau (v . y - 2 sum_s (V_s . v)(W_s . v)),
+// so CTAs need nothing of one another.  Both vectors need every row's
+// combination of the panel's earlier V and W columns: one sweep reads them for
+// both (four lanes a row, each a quarter of the columns), the first eight rows
+// of a warp ahead of the block sum.  What bounds it: the latency of one round
+// of L2 reads, a block sum and the launch.  64 models of 3 to 6 bath sites: 26 ms
+// for all columns, against 42 on clusters that reduced the column's norm and
+// w . v between their CTAs; blocks of 4 x 1225 and 8 x 735 states, whole
+// eigensolve: 24.8 -> 22.9 ms.
 __global__ void __launch_bounds__(BHH_COL_THREADS, 2) bhh_col_kernel(BigArgs g) {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cl = cg::this_cluster();
-    extern __shared__ double sh[];
-    __shared__ double red[32];
     __shared__ double dw[BHH_NB], dv[BHH_NB], jw[BHH_NB], jv[BHH_NB];
-    __shared__ double slot_w[BHH_CS], slot_x[BHH_CS], s_wj, s_x[2];  // pushed by the other CTAs
-    const int CS = (int)cl.num_blocks(), c = (int)cl.block_rank();
+    __shared__ double red[BHH_COL_THREADS / 32], s_dd, s_dj;
     cudaTriggerProgrammaticLaunchCompletion();
-    const BigBlk bl = g.blk[blockIdx.x / CS];
+    const BigBlk bl = g.blk[blockIdx.y];
     const int n = bl.n, last = n - 3;  // the last column with a reflector
     double* A = g.A + bl.moff;
     double* V = g.S + bl.boff;  // column t at V + t n
     double* W = V + (long)BHH_NB * n;
     const double* y = W + (long)BHH_NB * n;
-    double* tau = W + (long)BHH_NB * n + n;
+    const double* tau = y + n;
     const double* dots = V + bhh_dots_at(n);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const bool fin = g.fin >= 0 && g.fin <= last, col = g.col >= 0 && g.col <= last;
+    if (!fin && !col) return;
     const int f = g.fin, j = g.col, cf = fin ? f - g.k : 0, cc = col ? j - g.k : 0;
-    const int share = (n + CS - 1) / CS, r0 = c * share, r1 = min(n, r0 + share);
-    double *xs = sh, *ws = sh + share, *vs = sh + 2 * share;
-    if (CS > 1) cl.barrier_arrive();  // waited for ahead of the first push
-    cudaGridDependencySynchronize();
-    double tf = 0.0;
-    if (fin) tf = tau[f];
-    if (tid < cf) {
-        dw[tid] = dots[2 * tid];
-        dv[tid] = dots[2 * tid + 1];
-        jw[tid] = col ? W[(long)tid * n + j] : 0.0;
-        jv[tid] = col ? V[(long)tid * n + j] : 0.0;
-    }
-    if (CS > 1) cl.barrier_wait();
-    __syncthreads();
-    const double* vf = V + (long)cf * n;
+    const int lo = fin ? f + 1 : j;  // the first row of v, w and the column
+    double* vf = V + (long)cf * n;
     const int sg = lane >> 3;
-    double part = 0.0;
-    for (int rb = r0 + 8 * wid; rb < r1; rb += 8 * (BHH_COL_THREADS / 32)) {
+    cudaGridDependencySynchronize();
+    double tf = 0.0, v0 = 0.0;
+    if (fin) {
+        tf = tau[f];
+        v0 = y[f];
+    }
+    double pv[BHH_NB / 4], pw[BHH_NB / 4], x = 0.0, acc = 0.0, v = 0.0;
+    auto load = [&](int r) {
+        x = acc = v = 0.0;
+        const bool in = r >= lo && r < n;
+        if (in && fin) v = r == lo ? v0 : vf[r];
+        if (in && sg == 0) {
+            if (col) x = A[(long)j * n + r];  // row j holds column j (A symmetric)
+            if (fin) acc = y[r];
+        }
+#pragma unroll
+        for (int q = 0; q < BHH_NB / 4; ++q) {
+            const int s = sg + 4 * q;
+            pv[q] = in && s < cf ? V[(long)s * n + r] : 0.0;
+            pw[q] = in && s < cf ? W[(long)s * n + r] : 0.0;
+        }
+    };
+    const int stride = 8 * (BHH_COL_THREADS / 32) * (int)gridDim.x;
+    int rb = (lo & ~7) + 8 * (blockIdx.x * (BHH_COL_THREADS / 32) + wid);
+    load(rb + (lane & 7));
+    double K = 0.0, wj = 0.0;
+    if (fin) {
+        double vy = 0.0;
+        for (int r = lo + 1 + tid; r < n; r += BHH_COL_THREADS) vy = fma(vf[r], y[r], vy);
+        if (tid < BHH_NB) {
+            double a = 0.0, b = 0.0, c = 0.0, d = 0.0;
+            if (tid < cf) {
+                a = dots[2 * tid];
+                b = dots[2 * tid + 1];
+                c = col ? W[(long)tid * n + j] : 0.0;
+                d = col ? V[(long)tid * n + j] : 0.0;
+            }
+            dw[tid] = a;
+            dv[tid] = b;
+            jw[tid] = c;
+            jv[tid] = d;
+            const double dd = warp_sum(a * b), dj = warp_sum(d * a + c * b);
+            if (tid == 0) {
+                s_dd = dd;
+                s_dj = dj;
+                vy = fma(v0, y[lo], vy);
+            }
+        }
+        vy = warp_sum(vy);
+        if (lane == 0) red[wid] = vy;
+        __syncthreads();
+        double t = 0.0;
+#pragma unroll
+        for (int q = 0; q < BHH_COL_THREADS / 32; ++q) t += red[q];
+        K = 0.5 * tf * (tf * (t - 2.0 * s_dd));
+        wj = tf * (y[lo] - s_dj) - K * v0;
+    }
+    const double st = sqrt(tf);
+    for (; rb < n; rb += stride) {
         const int r = rb + (lane & 7);
-        double x = 0.0, acc = 0.0, v = 0.0;
-        if (r < r1) {
-            if (sg == 0 && col && r >= j) x = A[(long)j * n + r];  // row j holds column j (A symmetric)
-            if (sg == 0 && fin && r > f) {
-                acc = y[r];
-                v = vf[r];
-            }
-            double pv[BHH_NB / 4], pw[BHH_NB / 4];
 #pragma unroll
-            for (int q = 0; q < BHH_NB / 4; ++q) {
-                const int s = sg + 4 * q;
-                pv[q] = s < cf ? V[(long)s * n + r] : 0.0;
-                pw[q] = s < cf ? W[(long)s * n + r] : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < BHH_NB / 4; ++q) {
-                const int s = sg + 4 * q;
-                if (s < cf) {
-                    acc -= pv[q] * dw[s] + pw[q] * dv[s];
-                    x -= pv[q] * jw[s] + pw[q] * jv[s];
-                }
+        for (int q = 0; q < BHH_NB / 4; ++q) {
+            const int s = sg + 4 * q;
+            if (s < cf) {
+                acc -= pv[q] * dw[s] + pw[q] * dv[s];
+                x -= pv[q] * jw[s] + pw[q] * jv[s];
             }
         }
 #pragma unroll
@@ -174,87 +201,48 @@ __global__ void __launch_bounds__(BHH_COL_THREADS, 2) bhh_col_kernel(BigArgs g) 
             acc += __shfl_xor_sync(0xffffffffu, acc, o);
             x += __shfl_xor_sync(0xffffffffu, x, o);
         }
-        if (sg == 0 && r < r1) {
-            const double w = fin && r > f ? tf * acc : 0.0;
-            part = fma(w, v, part);
-            xs[r - r0] = col && r >= j ? x : 0.0;
-            ws[r - r0] = w;
-            vs[r - r0] = v;
-            if (fin && col && r == j)
-                for (int q = 0; q < CS; ++q) *cl.map_shared_rank(&s_wj, q) = w;
-        }
-    }
-    double K = 0.0, wj = 0.0, vj = 0.0;
-    if (fin) {
-        if (col) vj = vf[j];
-        part = block_sum(part, red);
-        if (tid < CS) cl.map_shared_rank(slot_w, tid)[c] = part;
-        if (CS > 1) cl.sync();
-        else __syncthreads();
-        for (int q = 0; q < CS; ++q) K += slot_w[q];
-        K *= 0.5 * tf;
-        if (col) wj = s_wj - K * vj;
-    } else {
-        __syncthreads();  // the sweep's rows are in place
-    }
-    double tj = 0.0, v0 = 0.0;
-    if (col) {
-        part = 0.0;
-        for (int r = r0 + tid; r < r1; r += BHH_COL_THREADS) {
-            double x = xs[r - r0];
-            if (fin && r >= j) {
-                const double v = vs[r - r0];
-                x -= v * wj + (ws[r - r0] - K * v) * vj;
-                xs[r - r0] = x;
+        if (r >= lo && r < n) {
+            const double w = tf * acc - K * v;
+            if (fin && sg == 0) {
+                W[(long)cf * n + r] = w;
+                if (r == lo) vf[r] = v0;
             }
-            if (r >= j + 2) part = fma(x, x, part);
-            if (r == j || r == j + 1)
-                for (int q = 0; q < CS; ++q) cl.map_shared_rank(s_x, q)[r - j] = x;
+            if (fin && sg == 1) A[(long)f * n + r] = v * st;  // row f of A: sqrt(tau) v
+            if (col && sg == 2) {
+                x -= v * wj + w * v0;
+                if (r == j) g.tri[2 * bl.eoff + j] = x;
+                V[(long)cc * n + r] = x;
+            }
         }
-        part = block_sum(part, red);
-        if (tid < CS) cl.map_shared_rank(slot_x, tid)[c] = part;
-        if (CS > 1) cl.sync();
-        else __syncthreads();
-        double sigma = 0.0;
-        for (int q = 0; q < CS; ++q) sigma += slot_x[q];
-        const double x0 = s_x[1];
-        double alpha = x0;
-        v0 = x0;
-        if (sigma != 0.0) {
-            const double t = fma(x0, x0, sigma), mu = t * rsqrt(t);
-            alpha = (x0 > 0.0) ? -mu : mu;  // v0 = x0 - alpha without cancellation
-            v0 = x0 - alpha;
-            tj = 2.0 * recip_pos(fma(v0, v0, sigma));
-        }
-        if (c == 0 && tid == 0) {
-            g.tri[2 * bl.eoff + j] = s_x[0];
-            g.tri[2 * bl.eoff + n + j] = alpha;
-            tau[j] = tj;
-        }
+        if (rb + stride < n) load(r + stride);
     }
-    const double st = sqrt(tj);
-    for (int r = r0 + tid; r < r1; r += BHH_COL_THREADS) {
-        if (fin) W[(long)cf * n + r] = ws[r - r0] - K * vs[r - r0];
-        if (col) {
-            const double vr = (tj != 0.0 && r > j) ? ((r == j + 1) ? v0 : xs[r - r0]) : 0.0;
-            V[(long)cc * n + r] = vr;
-            A[(long)j * n + r] = vr * st;  // row j of A: zeros up to the diagonal, then sqrt(tau) v
-        }
-    }
+    if (fin)  // zeros up to the diagonal
+        for (int r = blockIdx.x * BHH_COL_THREADS + tid; r < lo; r += gridDim.x * BHH_COL_THREADS) A[(long)f * n + r] = 0.0;
 }
 
-// y(j+1:) = A(j+1:, j+1:) v for column j = col of every active block, and the
-// dots W_s . v, V_s . v of the panel's earlier columns as further rows; grid
-// (rows, block), RW rows per warp and 8 / RW columns per lane at once, so eight
-// row loads are in flight per lane, and with several rows each entry of v is
-// loaded once for them.  What bounds it: reading the trailing matrix, from HBM
-// where the active blocks exceed L2 (64 models of 3 to 6 bath sites, all
-// columns: 90 ms, 5.0 TB/s, against 102 with a rest of up to 64 columns read
-// one load at a time), else the latency of L2 with the warps there are, hence
-// fewer rows per warp for fewer rows (blocks of 4 x 1225 and 8 x 735 states,
-// whole eigensolve: 24.8 ms, against 32.3 with four rows per warp throughout).
+// A load that is issued where it stands: the compiler otherwise groups the row
+// loads with their products, three or four in flight instead of the eight.
+__device__ inline double ld_now(const double* p) {
+    double r;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(r) : "l"(p) : "memory");
+    return r;
+}
+
+// Reflects column j = col of every active block (raw in V): v, tau, e_j, then
+// y(j+1:) = A(j+1:, j+1:) v and the dots W_s . v, V_s . v of the panel's
+// earlier columns as further rows.  v is the raw column but for its leading
+// entry, which needs the column's norm: a warp sums the squares on its way
+// through the column and adds that entry's product at the end.  Grid (rows,
+// block), RW rows per warp and 8 / RW columns per lane at once, so eight row
+// loads are in flight per lane, and with several rows each entry of v is loaded
+// once for them.  What bounds it: reading the trailing matrix, from HBM where
+// the active blocks exceed L2 (64 models of 3 to 6 bath sites, all columns:
+// 95 ms, 4.7 TB/s, against 102 with two rows' loads at a time), else the latency
+// of L2 with the warps there are, hence fewer rows per warp for fewer rows
+// (blocks of 4 x 1225 and 8 x 735 states, whole eigensolve: 24.8 ms, against
+// 32.3 with four rows per warp throughout; 21.8 with the loads issued together).
 template <int RW>
-__global__ void __launch_bounds__(BHH_SYMV_THREADS) bhh_symv_kernel(BigArgs g) {
+__global__ void __launch_bounds__(BHH_SYMV_THREADS, RW == 4 ? 10 : 6) bhh_symv_kernel(BigArgs g) {
     constexpr int U = 8 / RW;
     cudaTriggerProgrammaticLaunchCompletion();
     const BigBlk bl = g.blk[blockIdx.y];
@@ -264,6 +252,7 @@ __global__ void __launch_bounds__(BHH_SYMV_THREADS) bhh_symv_kernel(BigArgs g) {
     double* y = V + 2L * BHH_NB * n + (j + 1);
     double* dots = V + bhh_dots_at(n);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (m < 2) return;  // no reflector
     const int rr = (blockIdx.x * (BHH_SYMV_THREADS / 32) + wid) * RW;
     if (rr >= rows) return;
     const double* p[RW];
@@ -274,7 +263,7 @@ __global__ void __launch_bounds__(BHH_SYMV_THREADS) bhh_symv_kernel(BigArgs g) {
                      : V + ((d & 1) ? 0L : (long)BHH_NB * n) + (long)(d >> 1) * n + (j + 1);
     }
     cudaGridDependencySynchronize();
-    double s[RW];
+    double s[RW], sigma = 0.0;
 #pragma unroll
     for (int u = 0; u < RW; ++u) s[u] = 0.0;
     int i = lane;
@@ -282,10 +271,13 @@ __global__ void __launch_bounds__(BHH_SYMV_THREADS) bhh_symv_kernel(BigArgs g) {
         double x[U], a[RW][U];
 #pragma unroll
         for (int t = 0; t < U; ++t) {
-            x[t] = v[i + 32 * t];
+            x[t] = ld_now(v + i + 32 * t);
 #pragma unroll
-            for (int u = 0; u < RW; ++u) a[u][t] = p[u][i + 32 * t];
+            for (int u = 0; u < RW; ++u) a[u][t] = ld_now(p[u] + i + 32 * t);
         }
+        if (i == 0) x[0] = 0.0;  // the leading entry follows
+#pragma unroll
+        for (int t = 0; t < U; ++t) sigma = fma(x[t], x[t], sigma);
 #pragma unroll
         for (int u = 0; u < RW; ++u)
 #pragma unroll
@@ -300,14 +292,34 @@ __global__ void __launch_bounds__(BHH_SYMV_THREADS) bhh_symv_kernel(BigArgs g) {
 #pragma unroll
             for (int u = 0; u < RW; ++u) a[u][t] = in ? p[u][i + 32 * t] : 0.0;
         }
+        if (i == 0) x[0] = 0.0;
+#pragma unroll
+        for (int t = 0; t < U; ++t) sigma = fma(x[t], x[t], sigma);
 #pragma unroll
         for (int u = 0; u < RW; ++u)
 #pragma unroll
             for (int t = 0; t < U; ++t) s[u] = fma(a[u][t], x[t], s[u]);
     }
+    const double x0 = v[0];
+    double a0[RW];
+#pragma unroll
+    for (int u = 0; u < RW; ++u) a0[u] = p[u][0];
+    sigma = warp_sum(sigma);
+    double alpha = x0, v0 = 0.0, tj = 0.0;
+    if (sigma != 0.0) {
+        const double t = fma(x0, x0, sigma), mu = t * rsqrt(t);
+        alpha = (x0 > 0.0) ? -mu : mu;  // v0 = x0 - alpha without cancellation
+        v0 = x0 - alpha;
+        tj = 2.0 * recip_pos(fma(v0, v0, sigma));
+    }
+    if (rr == 0 && lane == 0) {
+        g.tri[2 * bl.eoff + n + j] = alpha;
+        V[2L * BHH_NB * n + n + j] = tj;
+        V[2L * BHH_NB * n + j] = v0;
+    }
 #pragma unroll
     for (int u = 0; u < RW; ++u) {
-        const double t = warp_sum(s[u]);
+        const double t = fma(a0[u], v0, warp_sum(s[u]));
         const int r = rr + u;
         if (lane == 0 && r < rows) {
             if (r < m) y[r] = t;
@@ -1537,27 +1549,20 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
     // The column and product kernels alternate, each launched while the one
     // before it drains (it waits for that one's results itself).
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
+    cfg.numAttrs = 1;
     cfg.stream = st;
-    const size_t col_smem = 3 * sizeof(double) * (size_t)nmax;
-    PGX_CUDA(cudaFuncSetAttribute(bhh_col_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)std::min<size_t>(col_smem, 200 * 1024)));
     auto col_step = [&]() {
-        // CTAs per block: more shorten a block's sweep, as long as all blocks
-        // are resident at once (two CTAs per SM) and their rows fit
-        int cs = BHH_CS;
-        while (cs > 1 && a.nact * cs > 2 * 148 && 2 * col_smem / cs <= 100 * 1024) cs /= 2;
-        cfg.gridDim = dim3((unsigned)(a.nact * cs));
+        // CTAs per block: eight rows a warp, as long as all blocks are
+        // resident at once (two CTAs per SM)
+        const int lo = (a.fin >= 0 ? a.fin + 1 : a.col) & ~7;
+        int cs = std::max(1, (int)ceil_div(nmax - lo, BHH_COL_THREADS / 4));
+        while (cs > 1 && a.nact * cs > 2 * 148) cs = (cs + 1) / 2;
+        cfg.gridDim = dim3((unsigned)cs, (unsigned)a.nact);
         cfg.blockDim = dim3(BHH_COL_THREADS);
-        cfg.dynamicSmemBytes = 3 * sizeof(double) * (size_t)ceil_div(nmax, cs);
-        attr[1].val.clusterDim.x = cs;
-        cfg.numAttrs = 2;
         ProfRange r1("bhh_col_kernel", st, 0.0, 0.0);
         PGX_CUDA(cudaLaunchKernelEx(&cfg, bhh_col_kernel, a));
         check_launch("bhh_col_kernel");
@@ -1567,8 +1572,6 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
         const int rw = all_rows >= 4L * 148 * 24 ? 4 : all_rows >= 2L * 148 * 24 ? 2 : 1;
         cfg.gridDim = dim3((unsigned)ceil_div(rows, rw * (BHH_SYMV_THREADS / 32)), (unsigned)a.nact);
         cfg.blockDim = dim3(BHH_SYMV_THREADS);
-        cfg.dynamicSmemBytes = 0;
-        cfg.numAttrs = 1;
         ProfRange r2("bhh_symv_kernel", st, 0.0, bytes);
         PGX_CUDA(cudaLaunchKernelEx(&cfg, rw == 4 ? bhh_symv_kernel<4> : rw == 2 ? bhh_symv_kernel<2> : bhh_symv_kernel<1>, a));
         check_launch("bhh_symv_kernel");
