@@ -59,7 +59,7 @@ __device__ double block_sum(double v, double* red) {
 //   w = tau (A(j+1:, j+1:) v - V (W^T v) - W (V^T v)),  w -= (tau/2)(w.v) v,
 // with A the matrix as it was at the start of the panel: the trailing matrix
 // is only read per column (bhh_symv_kernel) and written once per panel,
-// A(k+p:, k+p:) -= V W^T + W V^T, by one GEMM of inner size 2p.
+// A(k+p:, k+p:) -= V W^T + W V^T (bhh_update_kernel).
 // The reflectors stay, scaled to tau = 1, in the rows of A right of the
 // diagonal (zeros left of it).  Up to 2165 states the eigenvectors are formed from
 // them directly (bt_apply_kernel); beyond, Q = H_0 ... H_{n-3} is formed panel
@@ -326,6 +326,96 @@ __global__ void __launch_bounds__(BHH_SYMV_THREADS, RW == 4 ? 10 : 6) bhh_symv_k
             else dots[r - m] = t;
         }
     }
+}
+
+// A(k+p:, k+p:) -= V W^T + W V^T after the panel's p columns: one 64 x 64 tile on
+// or below the diagonal per CTA on the FP64 tensor cores, both operands of the
+// tile whole in shared memory (up to 32 columns of V and W each), each of four
+// warps 32 x 32 of it; every element is also written in its mirrored place, as
+// the product kernel reads rows.  Grid (tiles of the largest block, block).
+// What bounds it: the FP64 pipe for full tiles, the latency of one round of
+// loads when few are left.  64 models of 3 to 6 bath sites, all panels: 10.4 ms,
+// against 34 with general products of inner size 2p, whose columns were gathered
+// and scaled and whose tiles covered both triangles; 7-site ring 1.0 against 2.5.
+constexpr int UPD_T = 64, UPD_LD = UPD_T + 4, UPD_THREADS = 128;
+constexpr size_t UPD_SMEM = 4UL * BHH_NB * UPD_LD * sizeof(double);
+__global__ void __launch_bounds__(UPD_THREADS, 3) bhh_update_kernel(BigArgs g) {
+    extern __shared__ double sh[];
+    const BigBlk bl = g.blk[blockIdx.y];
+    const int n = bl.n, p = min(BHH_NB, n - 2 - g.k), kp = g.k + p, m = n - kp;
+    int ti = (int)((sqrtf(8.0f * blockIdx.x + 1.0f) - 1.0f) * 0.5f);
+    while ((ti + 1) * (ti + 2) / 2 <= (int)blockIdx.x) ++ti;
+    while (ti * (ti + 1) / 2 > (int)blockIdx.x) --ti;
+    const int tj = blockIdx.x - ti * (ti + 1) / 2, i0 = ti * UPD_T, j0 = tj * UPD_T;
+    if (i0 >= m) return;
+    const double* V = g.S + bl.boff + kp;
+    const double* W = V + (long)BHH_NB * n;
+    double* A = g.A + bl.moff + (long)kp * n + kp;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    double *Vi = sh, *Wi = sh + BHH_NB * UPD_LD, *Vj = Vi, *Wj = Wi;
+    const int p4 = (p + 3) & ~3;
+    auto fill = [&](double* dst, const double* src, int at) {
+        for (int e = tid; e < p4 * UPD_T; e += UPD_THREADS) {
+            const int s = e / UPD_T, r = e % UPD_T;
+            const bool in = s < p && at + r < m;
+            cp_elem(dst + s * UPD_LD + r, in ? src + (long)s * n + at + r : src, in);
+        }
+    };
+    fill(Vi, V, i0);
+    fill(Wi, W, i0);
+    if (ti != tj) {
+        Vj = Wi + BHH_NB * UPD_LD;
+        Wj = Vj + BHH_NB * UPD_LD;
+        fill(Vj, V, j0);
+        fill(Wj, W, j0);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const int wr = 32 * (wid >> 1), wc = 32 * (wid & 1), fr = lane / 4, fk = lane % 4;
+    double2 acc[4][4], old[4][4];
+    auto mine = [&](int i, int j) { return i < m && j < m && j <= i; };
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+            const int i = i0 + wr + 8 * x + fr, j = j0 + wc + 8 * y + 2 * fk;
+            acc[x][y] = double2{0.0, 0.0};
+            old[x][y].x = mine(i, j) ? A[(long)i * n + j] : 0.0;
+            old[x][y].y = mine(i, j + 1) ? A[(long)i * n + j + 1] : 0.0;
+        }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (ti == tj && wc > wr) return;  // above the diagonal
+    for (int s0 = 0; s0 < p4; s0 += 4) {
+        const int at = (s0 + fk) * UPD_LD + fr;
+        double av[4], aw[4], bv[4], bw[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            av[x] = Vi[at + wr + 8 * x];
+            aw[x] = Wi[at + wr + 8 * x];
+            bv[x] = Vj[at + wc + 8 * x];
+            bw[x] = Wj[at + wc + 8 * x];
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+            for (int y = 0; y < 4; ++y) mma_f64(acc[x][y], av[x], bw[y]);
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+            for (int y = 0; y < 4; ++y) mma_f64(acc[x][y], aw[x], bv[y]);
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int i = i0 + wr + 8 * x + fr, j = j0 + wc + 8 * y + 2 * fk + u;
+                if (!mine(i, j)) continue;
+                const double r = u ? old[x][y].y - acc[x][y].y : old[x][y].x - acc[x][y].x;
+                A[(long)i * n + j] = r;
+                A[(long)j * n + i] = r;
+            }
 }
 
 // the last 2 x 2 of the tridiagonal, and Q = I for the first nact blocks (those that form Q)
@@ -1439,10 +1529,9 @@ static void launch_bt_apply(const BtItem* items, size_t n, int nmax, const doubl
 }
 
 // doubles of vector_kernel scratch (EighDev::S); the large-block path uses
-// the same buffer before the vector stage (a -1 scale vector, then one
-// scratch per large block)
+// the same buffer before the vector stage (one scratch per large block)
 size_t eigh_vec_scratch_doubles(const std::vector<int>& dims) {
-    size_t s = 0, big = 2 * BHH_NB;
+    size_t s = 0, big = 0;
     for (int n : dims) {
         // the vectors' scratch, later the T factors
         s += std::max(4 * (size_t)n * TRI_THREADS * ((n + TRI_THREADS - 1) / TRI_THREADS),
@@ -1483,12 +1572,11 @@ static std::vector<int> big_blocks(const std::vector<int>& dims) {
 }
 
 // descriptor bytes: bisection items, one int per block (Householder lists);
-// with large blocks also their scratch offsets and the column-index table of
-// the panel updates
+// with large blocks also their descriptors
 static size_t big_desc_bytes(const std::vector<int>& dims) {
     const size_t nb = big_blocks(dims).size();
     if (nb == 0) return 0;
-    return 8 + nb * sizeof(BigBlk) + (size_t)BHH_NB * 4 * BHH_NB * sizeof(int);
+    return 8 + nb * sizeof(BigBlk);
 }
 size_t eigh_item_bytes(const std::vector<int>& dims) {
     std::vector<TriItem> items;
@@ -1507,13 +1595,13 @@ size_t eigh_gemm_bytes(const std::vector<int>& dims, size_t* tiles_bytes) {
 }
 
 // The large-block Householder path (see bhh_col_kernel) on stream st.
-// big: the blocks, largest first; d_blk, d_kidx: their device list and the
-// panel-update column table (uploaded by the caller).
+// big: the blocks, largest first; d_blk: their device list (uploaded by the
+// caller).
 static void launch_big(const EighDev& d, const std::vector<int>& dims, const std::vector<long>& moff,
-                       const std::vector<int>& big, const BigBlk* d_blk, const int* d_kidx, cudaStream_t st) {
+                       const std::vector<int>& big, const BigBlk* d_blk, cudaStream_t st) {
     const int nbig = (int)big.size();
     std::vector<long> boff(nbig);
-    long o = 2 * BHH_NB;
+    long o = 0;
     for (int i = 0; i < nbig; ++i) {
         boff[i] = o;
         o += bhh_scratch_doubles(dims[big[i]]);
@@ -1541,11 +1629,6 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
     for (int b : big)
         PGX_CUDA(cudaMemcpyAsync(d.A + moff[b], d.H + moff[b], (size_t)dims[b] * dims[b] * sizeof(double),
                                  cudaMemcpyDeviceToDevice, st));
-    {
-        double neg[2 * BHH_NB];
-        for (double& x : neg) x = -1.0;
-        h2d(d.S, neg, sizeof(neg), st);
-    }
     // The column and product kernels alternate, each launched while the one
     // before it drains (it waits for that one's results itself).
     cudaLaunchConfig_t cfg = {};
@@ -1576,9 +1659,7 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
         PGX_CUDA(cudaLaunchKernelEx(&cfg, rw == 4 ? bhh_symv_kernel<4> : rw == 2 ? bhh_symv_kernel<2> : bhh_symv_kernel<1>, a));
         check_launch("bhh_symv_kernel");
     };
-    std::vector<GemmProblem<double, double, double>> probs;
-    size_t tiles_cap = 0;
-    const size_t probs_cap = eigh_gemm_bytes(dims, &tiles_cap);
+    PGX_CUDA(cudaFuncSetAttribute(bhh_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)UPD_SMEM));
     // ---- tridiagonalisation
     for (int k = 0; k < nmax - 2; k += BHH_NB) {
         a.k = k;
@@ -1603,33 +1684,17 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
         a.col = -1;
         a.nact = nact(jend - 1);
         col_step();
-        // A(k+p:, k+p:) -= V W^T + W V^T, p = the block's columns in this panel
-        probs.clear();
-        for (int i = 0; i < nact(k); ++i) {
-            const int n = dims[big[i]];
-            const int p = std::min(BHH_NB, n - 2 - k), kp = k + p, m = n - kp;
-            if (m <= 0) continue;
-            double* VW = d.S + boff[i] + kp;
-            GemmProblem<double, double, double> g{};
-            g.A = VW;
-            g.B = VW;
-            g.C = d.A + moff[big[i]] + (long)kp * n + kp;
-            g.M = m;
-            g.N = m;
-            g.K = 2 * p;
-            g.sa_i = 1;
-            g.sa_k = n;
-            g.sb_k = n;
-            g.sb_j = 1;
-            g.sc_i = n;
-            g.sc_j = 1;
-            g.a_kidx = d_kidx + (p - 1) * 4 * BHH_NB;
-            g.b_kidx = g.a_kidx + 2 * BHH_NB;
-            g.kscale = d.S;
-            g.accumulate = 1;
-            probs.push_back(g);
+        a.nact = nact(k);
+        const long nt = ceil_div(nmax - jend, UPD_T);  // of the largest block
+        double ufl = 0.0, uby = 0.0;
+        for (int i = 0; i < a.nact; ++i) {
+            const double p = std::min(BHH_NB, dims[big[i]] - 2 - k), m = dims[big[i]] - k - p;
+            ufl += 2.0 * p * m * m;
+            uby += 12.0 * m * m;
         }
-        launch_gemm_batch(probs, d.gemm_probs, probs_cap, d.gemm_tiles, tiles_cap, st);
+        ProfRange ru("bhh_update_kernel", st, ufl, uby);
+        bhh_update_kernel<<<dim3((unsigned)(nt * (nt + 1) / 2), (unsigned)a.nact), UPD_THREADS, UPD_SMEM, st>>>(a);
+        check_launch("bhh_update_kernel");
     }
     // blocks beyond the direct back-transformation, a prefix of the list
     int nwide = 0;
@@ -1639,7 +1704,9 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
     check_launch("bhh_finish_kernel");
     if (nwide == 0) return;
     // ---- Q: Gram matrices and -T of every panel, then the panels from the last
-    probs.clear();
+    std::vector<GemmProblem<double, double, double>> probs;
+    size_t tiles_cap = 0;
+    const size_t probs_cap = eigh_gemm_bytes(dims, &tiles_cap);
     long npan_total = 0;
     long npan_max = 0;
     for (int i = 0; i < nwide; ++i) {
@@ -1789,34 +1856,21 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
     }
     const BtPlan bt = bt_plan(dims);
     const size_t lists_at = items.size() * sizeof(TriItem) + bt.items.size() * sizeof(BtItem);
-    // large blocks: scratch offsets (doubles into S) and, per panel width p, the
-    // column gathers of the panel update [V_0..V_p-1 W_0..W_p-1] and [W.. V..]
+    // large blocks: scratch offsets (doubles into S)
     const std::vector<int>& big = hp.global;
     const size_t lists_end = lists_at + lists.size() * sizeof(int);
     const size_t boff_at = (lists_end + 7) & ~size_t(7);
     size_t host_bytes = lists_end;
     std::vector<BigBlk> blk;
-    std::vector<int> kidx;
     if (!big.empty()) {
         std::vector<long> eoff(dims.size() + 1, 0);
         for (size_t b = 0; b < dims.size(); ++b) eoff[b + 1] = eoff[b] + dims[b];
-        long o = 2 * BHH_NB;
+        long o = 0;
         for (int b : big) {
             blk.push_back(BigBlk{moff[b], eoff[b], o, dims[b], 0});
             o += bhh_scratch_doubles(dims[b]);
         }
-        for (int p = 1; p <= BHH_NB; ++p) {
-            std::vector<int> ia(2 * BHH_NB, 0), ib(2 * BHH_NB, 0);
-            for (int t = 0; t < p; ++t) {
-                ia[t] = t;
-                ia[p + t] = BHH_NB + t;
-                ib[t] = BHH_NB + t;
-                ib[p + t] = t;
-            }
-            kidx.insert(kidx.end(), ia.begin(), ia.end());
-            kidx.insert(kidx.end(), ib.begin(), ib.end());
-        }
-        host_bytes = boff_at + blk.size() * sizeof(BigBlk) + kidx.size() * sizeof(int);
+        host_bytes = boff_at + blk.size() * sizeof(BigBlk);
         PGX_CHECK(host_bytes <= eigh_item_bytes(dims), PGX_ERR_ARG, "eigensolver descriptor layout overflow");
     }
     std::vector<char> host(host_bytes);
@@ -1824,16 +1878,11 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
     if (!bt.items.empty())
         std::memcpy(host.data() + items.size() * sizeof(TriItem), bt.items.data(), bt.items.size() * sizeof(BtItem));
     std::memcpy(host.data() + lists_at, lists.data(), lists.size() * sizeof(int));
-    if (!big.empty()) {
-        std::memcpy(host.data() + boff_at, blk.data(), blk.size() * sizeof(BigBlk));
-        std::memcpy(host.data() + boff_at + blk.size() * sizeof(BigBlk), kidx.data(), kidx.size() * sizeof(int));
-    }
+    if (!big.empty()) std::memcpy(host.data() + boff_at, blk.data(), blk.size() * sizeof(BigBlk));
     h2d(d.items, host.data(), host.size(), st);
     const BtItem* d_bt = reinterpret_cast<const BtItem*>(static_cast<const TriItem*>(d.items) + items.size());
     const int* d_lists = reinterpret_cast<const int*>(static_cast<const char*>(d.items) + lists_at);
     const BigBlk* d_blk = reinterpret_cast<const BigBlk*>(static_cast<const char*>(d.items) + boff_at);
-    const int* d_kidx = reinterpret_cast<const int*>(static_cast<const char*>(d.items) + boff_at +
-                                                     blk.size() * sizeof(BigBlk));
 
     // LAPACK operation counts: tridiagonalisation 4/3 n^3, forming Q 4/3 n^3;
     // minimum DRAM traffic: read H, write Q and the tridiagonal
@@ -1852,7 +1901,7 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
         PGX_CUDA(cudaEventRecord(d.fork, st));
         for (int i = 0; i < 4; ++i) PGX_CUDA(cudaStreamWaitEvent(d.aux[i], d.fork, 0));
     }
-    if (!big.empty()) launch_big(d, dims, moff, big, d_blk, d_kidx, st);
+    if (!big.empty()) launch_big(d, dims, moff, big, d_blk, st);
     for (int q = 0; q < CL_NCLS; ++q) {
         if (hp.cls[q].empty()) continue;
         const cudaStream_t sq = (fork && q > 0) ? d.aux[q - 1] : st;
