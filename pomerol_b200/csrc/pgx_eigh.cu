@@ -15,7 +15,7 @@
 //      inside chains of close eigenvalues; eigenvalues are ranked so that the
 //      output is ascending.
 //   4. the reflectors applied to Z panel by panel (bt_apply_kernel); blocks
-//      beyond 2165 states form Q and U = Q Z by GEMMs.
+//      beyond 3073 states form Q and U = Q Z by GEMMs.
 // A non-finite eigenvector sets a device status word instead of trapping.
 
 #include <cooperative_groups.h>
@@ -61,7 +61,7 @@ __device__ double block_sum(double v, double* red) {
 // is only read per column (bhh_symv_kernel) and written once per panel,
 // A(k+p:, k+p:) -= V W^T + W V^T (bhh_update_kernel).
 // The reflectors stay, scaled to tau = 1, in the rows of A right of the
-// diagonal (zeros left of it).  Up to 2165 states the eigenvectors are formed from
+// diagonal (zeros left of it).  Up to 3073 states the eigenvectors are formed from
 // them directly (bt_apply_kernel); beyond, Q = H_0 ... H_{n-3} is formed panel
 // by panel, from the last one, as
 // Q(k+1:, k+1:) += V (-T) (V^T Q(k+1:, k+1:)), where T is the upper
@@ -716,23 +716,25 @@ __global__ void __launch_bounds__(CL_THREADS) eigh_cluster_kernel(ClusterArgs g)
 // in 2 n steps of a cluster, or three GEMM launches per panel, and a product
 // Q Z.  What bounds it: the FP64 pipe for the wide classes; reading V (twice
 // per panel) from L2 for the narrow ones.  Anderson 1+5
-// (blocks to 400 states): 0.16 ms, against 0.74 ms of the clusters' time and
-// 0.09 ms of products; 7-site ring (blocks to 1225): 3.6 ms against 11.
+// (blocks to 400 states): 0.13 ms, against 0.74 ms of the clusters' time and
+// 0.09 ms of products; 7-site ring (blocks to 1225): 2.2 ms against 11; one
+// block of 3070 states, whole eigensolve: 51 ms, of 3080, by GEMMs: 63.
 // Reflector k is row k of V, right of the diagonal.
 constexpr int BT_NB = 32, BT_THREADS = 256, BT_ROWS = 32;  // reflectors a panel, threads, rows of V a tile
 constexpr int BT_LDV = BT_NB + 4;                          // 4 mod 16 doubles: conflict-free fragment loads
+constexpr int BT_STAGES = 3;                               // tiles of V in flight or in use
 // Columns of Z per CTA and the largest n whose slab fits 227 KB beside the
-// tiles of V and W: 32 up to 679 states, 16 to 1273, 8 to 2165; larger blocks
+// tiles of V and W: 32 up to 697 states, 16 to 1489, 8 to 3073; larger blocks
 // form Q by GEMMs (launch_big).
 constexpr int BT_NCLS = 3;
 constexpr int BT_COLS[BT_NCLS] = {32, 16, 8};
 constexpr size_t BT_SMEM_MAX = 227 * 1024;
 __host__ __device__ constexpr size_t bt_smem_doubles(int n, int C) {
-    return (size_t)n * (C + 4) + 2 * BT_ROWS * BT_LDV + 2 * BT_NB * (C + 4);
+    return (size_t)(n + BT_ROWS - 1) * C + BT_STAGES * BT_ROWS * BT_LDV + 2 * BT_NB * (C + 4);
 }
 // the largest n of the last class
 constexpr int BT_MAX_DIM =
-    (int)((BT_SMEM_MAX / sizeof(double) - bt_smem_doubles(0, BT_COLS[BT_NCLS - 1])) / (BT_COLS[BT_NCLS - 1] + 4));
+    (int)((BT_SMEM_MAX / sizeof(double) - bt_smem_doubles(0, BT_COLS[BT_NCLS - 1])) / BT_COLS[BT_NCLS - 1]);
 static int bt_class(int n) {
     for (int q = 0; q < BT_NCLS; ++q)
         if (bt_smem_doubles(n, BT_COLS[q]) * sizeof(double) <= BT_SMEM_MAX) return q;
@@ -746,13 +748,23 @@ struct BtItem {
     long moff, toff;  // matrix offset; offset of the block's T factors in T
 };
 
-// tile of BT_ROWS rows of the panel's V from row r0, zero outside it
+// tile of BT_ROWS rows of the panel's V from row r0, zero outside it: lane =
+// row, warp = column mod 8
 __device__ __forceinline__ void bt_load_v(double* dst, const double* V, int n, int k0, int r0) {
-    for (int l = threadIdx.x; l < BT_ROWS * BT_NB; l += BT_THREADS) {
-        const int r = l % BT_ROWS, k = l / BT_ROWS, gr = r0 + r, gk = k0 + k;
-        const bool in = gr < n && gk < n - 2 && gr > gk;
-        cp_elem(dst + r * BT_LDV + k, V + (in ? (long)gk * n + gr : 0L), in);
+    static_assert(BT_ROWS == 32 && BT_THREADS == 256, "a warp loads 32 rows");
+    const int gr = r0 + (threadIdx.x & 31), gk = k0 + (threadIdx.x >> 5);
+    const double* src = V + (long)gk * n + gr;
+    dst += (threadIdx.x & 31) * BT_LDV + (threadIdx.x >> 5);
+    const int lim = gr < n ? min(gr, n - 2) : 0;  // columns of this row
+#pragma unroll
+    for (int u = 0; u < BT_NB / 8; ++u) {
+        const bool in = gk + 8 * u < lim;
+        cp_elem(dst + 8 * u, in ? src : V, in);
+        src += 8L * n;
     }
+}
+__device__ __forceinline__ void bt_load_v_group(double* dst, const double* V, int n, int k0, int r0) {
+    bt_load_v(dst, V, n, k0, r0);
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
@@ -766,12 +778,12 @@ __global__ void __launch_bounds__(BT_THREADS) bt_tfactor_kernel(const BtItem* it
     // G = V^T V: warp -> rows 8 (warp % 4), columns 16 (warp / 4)
     const int gi = 8 * (warp % 4), gj = 16 * (warp / 4);
     double2 acc[2] = {{0.0, 0.0}, {0.0, 0.0}};
-    bt_load_v(vt[0], V, n, k0, k0 + 1);
+    bt_load_v_group(vt[0], V, n, k0, k0 + 1);
     int buf = 0;
     for (int r0 = k0 + 1; r0 < n; r0 += BT_ROWS) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        if (r0 + BT_ROWS < n) bt_load_v(vt[buf ^ 1], V, n, k0, r0 + BT_ROWS);
+        if (r0 + BT_ROWS < n) bt_load_v_group(vt[buf ^ 1], V, n, k0, r0 + BT_ROWS);
         const double* v = vt[buf];
 #pragma unroll
         for (int r = 0; r < BT_ROWS; r += 4) {
@@ -805,64 +817,103 @@ __global__ void __launch_bounds__(BT_THREADS) bt_tfactor_kernel(const BtItem* it
 }
 
 // Warps: MG groups of 8 MF rows of W, NG of 8 NF columns and two halves of the
-// rows of Z for W = V^T Z; one 8-row strip at a time for Z += V W.
+// rows of Z for W = V^T Z; one 8-row strip at a time for Z += V W.  The tiles of
+// V of all panels, each panel's forward and then backward, form one sequence
+// that runs BT_STAGES - 1 tiles ahead of the products, through the panels' ends:
+// a tile's products take 256 cycles, a third of the latency of L2.  Addresses
+// advance by constants from tile to tile, since two warps a scheduler leave few
+// issue slots (rows beyond the last get a tile's rows of zeros instead of a
+// bound).  Columns of the slab are swizzled by row, so that fragments and pairs
+// are read without bank conflicts.  7-site ring 3.6 -> 2.2 ms, 64 models of 3 to
+// 6 bath sites 54 -> 33 against one tile ahead with addresses found per tile
+// (tiles further ahead alone: 3.1 and 47).
 template <int C>
 __global__ void __launch_bounds__(BT_THREADS) bt_apply_kernel(const BtItem* items, const double* Vall, const double* T,
                                                                const double* Zall, double* Uall) {
-    constexpr int LDZ = C + 4, NF = C >= 16 ? 2 : 1, NG = C / (8 * NF), MG = 4 / NG, MF = 4 / MG;
+    constexpr int LDW = C + 4, NF = C >= 16 ? 2 : 1, NG = C / (8 * NF), MG = 4 / NG, MF = 4 / MG;
+    constexpr int TILE = BT_ROWS * BT_LDV;
     extern __shared__ __align__(16) double sh[];
     const BtItem it = items[blockIdx.x];
-    const int n = it.n, c0 = it.at, nc = min(C, n - c0);
+    const int n = it.n, c0 = it.at, nc = min(C, n - c0), np = bt_panels(n);
     const double* V = Vall + it.moff;
     const double* Z = Zall + it.moff;  // column-major
-    double* vt = sh;                            // 2 tiles of V
-    double* W = vt + 2 * BT_ROWS * BT_LDV;      // 2 partial W; the first then holds -T W
-    double* zs = W + 2 * BT_NB * LDZ;           // n x C slab of Z
+    double* vt = sh;                         // BT_STAGES tiles of V
+    double* W = vt + BT_STAGES * TILE;       // 2 partial W; the first then holds -T W
+    double* zs = W + 2 * BT_NB * LDW;        // n x C slab of Z
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int l4 = lane % 4, l8 = lane / 4;
+    auto at = [&](int r, int c) { return r * C + (c ^ (C >= 16 ? (r & 1) << 3 | (r & 2) << 1 : (r & 2) << 1)); };
+    auto tiles = [&](int q) { return (n - q * BT_NB - 1 + BT_ROWS - 1) / BT_ROWS; };
+    int lq = np - 1, ls = 0, lnt = np > 0 ? tiles(lq) : 0, lstage = 0;  // the next tile to load: panel, step in it
+    auto issue = [&]() {
+        if (lq >= 0) {
+            const int t = ls < lnt ? ls : 2 * lnt - 1 - ls;
+            bt_load_v(vt + lstage * TILE, V, n, lq * BT_NB, lq * BT_NB + 1 + t * BT_ROWS);
+            lstage = lstage + 1 == BT_STAGES ? 0 : lstage + 1;
+            if (++ls == 2 * lnt) {
+                ls = 0;
+                if (--lq >= 0) lnt = tiles(lq);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int u = 0; u < BT_STAGES - 1; ++u) issue();
     for (long l = tid; l < (long)n * C; l += BT_THREADS) {
         const int c = (int)(l / n), r = (int)(l % n);
-        zs[(long)r * LDZ + c] = c < nc ? Z[(long)(c0 + c) * n + r] : 0.0;
+        zs[at(r, c)] = c < nc ? Z[(long)(c0 + c) * n + r] : 0.0;
     }
+    for (int l = tid; l < (BT_ROWS - 1) * C; l += BT_THREADS) zs[n * C + l] = 0.0;  // rows of the last tile beyond n
     const int half = warp / 4, wm = (warp % 4) / NG * 8 * MF, wn = (warp % 4) % NG * 8 * NF;
-    for (int q = bt_panels(n) - 1; q >= 0; --q) {
-        const int k0 = q * BT_NB, rb = k0 + 1, nt = (n - rb + BT_ROWS - 1) / BT_ROWS;
+    int stage = 0;
+    // the next tile of the sequence; the one before it is free for every warp
+    auto next = [&]() {
+        asm volatile("cp.async.wait_group %0;" ::"n"(BT_STAGES - 2) : "memory");
+        __syncthreads();
+        issue();
+        const double* v = vt + stage * TILE;
+        stage = stage + 1 == BT_STAGES ? 0 : stage + 1;
+        return v;
+    };
+    for (int q = np - 1; q >= 0; --q) {
+        const int rb = q * BT_NB + 1, nt = tiles(q);
         // ---- W = V^T Z
         double2 w[MF][NF];
+        double ta[BT_NB / 4][MF];
+        const double* nT = T + it.toff + (long)q * BT_NB * BT_NB;
 #pragma unroll
-        for (int a = 0; a < MF; ++a)
+        for (int a = 0; a < MF; ++a) {
 #pragma unroll
             for (int b = 0; b < NF; ++b) w[a][b] = double2{0.0, 0.0};
-        __syncthreads();  // the tiles of V and W are free, the slab is up to date
-        bt_load_v(vt, V, n, k0, rb);
+#pragma unroll
+            for (int k = 0; k < BT_NB / 4; ++k) ta[k][a] = half == 0 ? nT[(wm + 8 * a + l8) * BT_NB + 4 * k + l4] : 0.0;
+        }
+        const double* zb[NF];  // rows 4 apart have the same swizzle
+#pragma unroll
+        for (int u = 0; u < NF; ++u) zb[u] = zs + at(rb + half * (BT_ROWS / 2) + l4, wn + 8 * u + l8);
         for (int t = 0; t < nt; ++t) {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            __syncthreads();
-            const double* v = vt + (t & 1) * BT_ROWS * BT_LDV;
-            // the last tile of V stays in shared memory for the second sweep
-            if (t + 1 < nt) bt_load_v(vt + ((t + 1) & 1) * BT_ROWS * BT_LDV, V, n, k0, rb + (t + 1) * BT_ROWS);
+            const double* v = next() + (half * (BT_ROWS / 2) + l4) * BT_LDV + wm + l8;
 #pragma unroll
             for (int r = 0; r < BT_ROWS / 2; r += 4) {
-                const int rr = half * (BT_ROWS / 2) + r + l4, gr = min(rb + t * BT_ROWS + rr, n - 1);  // V is 0 beyond
                 double a[MF], b[NF];
 #pragma unroll
-                for (int u = 0; u < MF; ++u) a[u] = v[rr * BT_LDV + wm + 8 * u + l8];
+                for (int u = 0; u < MF; ++u) a[u] = v[r * BT_LDV + 8 * u];
 #pragma unroll
-                for (int u = 0; u < NF; ++u) b[u] = zs[(long)gr * LDZ + wn + 8 * u + l8];
+                for (int u = 0; u < NF; ++u) b[u] = zb[u][r * C];
 #pragma unroll
                 for (int x = 0; x < MF; ++x)
 #pragma unroll
                     for (int y = 0; y < NF; ++y) mma_f64(w[x][y], a[x], b[y]);
             }
+#pragma unroll
+            for (int u = 0; u < NF; ++u) zb[u] += BT_ROWS * C;
         }
 #pragma unroll
         for (int x = 0; x < MF; ++x)
 #pragma unroll
             for (int y = 0; y < NF; ++y)
-                *reinterpret_cast<double2*>(&W[half * BT_NB * LDZ + (wm + 8 * x + l8) * LDZ + wn + 8 * y + 2 * l4]) = w[x][y];
+                *reinterpret_cast<double2*>(&W[half * BT_NB * LDW + (wm + 8 * x + l8) * LDW + wn + 8 * y + 2 * l4]) = w[x][y];
         __syncthreads();
         // ---- W <- -T (W_0 + W_1), by the first four warps
-        const double* nT = T + it.toff + (long)q * BT_NB * BT_NB;
 #pragma unroll
         for (int x = 0; x < MF; ++x)
 #pragma unroll
@@ -870,18 +921,16 @@ __global__ void __launch_bounds__(BT_THREADS) bt_apply_kernel(const BtItem* item
         if (half == 0) {
 #pragma unroll
             for (int k = 0; k < BT_NB; k += 4) {
-                double a[MF], b[NF];
-#pragma unroll
-                for (int u = 0; u < MF; ++u) a[u] = nT[(wm + 8 * u + l8) * BT_NB + k + l4];
+                double b[NF];
 #pragma unroll
                 for (int u = 0; u < NF; ++u) {
-                    const int o = (k + l4) * LDZ + wn + 8 * u + l8;
-                    b[u] = W[o] + W[BT_NB * LDZ + o];
+                    const int o = (k + l4) * LDW + wn + 8 * u + l8;
+                    b[u] = W[o] + W[BT_NB * LDW + o];
                 }
 #pragma unroll
                 for (int x = 0; x < MF; ++x)
 #pragma unroll
-                    for (int y = 0; y < NF; ++y) mma_f64(w[x][y], a[x], b[y]);
+                    for (int y = 0; y < NF; ++y) mma_f64(w[x][y], ta[k / 4][x], b[y]);
             }
         }
         __syncthreads();
@@ -890,7 +939,7 @@ __global__ void __launch_bounds__(BT_THREADS) bt_apply_kernel(const BtItem* item
             for (int x = 0; x < MF; ++x)
 #pragma unroll
                 for (int y = 0; y < NF; ++y)
-                    *reinterpret_cast<double2*>(&W[(wm + 8 * x + l8) * LDZ + wn + 8 * y + 2 * l4]) = w[x][y];
+                    *reinterpret_cast<double2*>(&W[(wm + 8 * x + l8) * LDW + wn + 8 * y + 2 * l4]) = w[x][y];
         __syncthreads();
         // ---- Z += V W, tiles of V in reverse, strips of 8 rows: four warps a tile, C / 2 columns each
         constexpr int HC = C >= 16 ? C / 16 : 1;  // 8-column tiles a warp takes
@@ -900,27 +949,27 @@ __global__ void __launch_bounds__(BT_THREADS) bt_apply_kernel(const BtItem* item
 #pragma unroll
         for (int k = 0; k < BT_NB / 4; ++k)
 #pragma unroll
-            for (int y = 0; y < HC; ++y) wb[k][y] = W[(4 * k + l4) * LDZ + hc + 8 * y + l8];
+            for (int y = 0; y < HC; ++y) wb[k][y] = W[(4 * k + l4) * LDW + hc + 8 * y + l8];
+        double* zp[HC];
+#pragma unroll
+        for (int y = 0; y < HC; ++y) zp[y] = zs + at(rb + (nt - 1) * BT_ROWS + strip + l8, hc + 8 * y + 2 * l4);
         for (int t = nt - 1; t >= 0; --t) {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            __syncthreads();
-            const double* v = vt + (t & 1) * BT_ROWS * BT_LDV;
-            if (t > 0) bt_load_v(vt + ((t - 1) & 1) * BT_ROWS * BT_LDV, V, n, k0, rb + (t - 1) * BT_ROWS);
-            const int gr = rb + t * BT_ROWS + strip + l8;
+            const double* v = next() + (strip + l8) * BT_LDV + l4;
             if (mine) {
                 double2 z[HC];
 #pragma unroll
-                for (int y = 0; y < HC; ++y)
-                    z[y] = gr < n ? *reinterpret_cast<double2*>(&zs[(long)gr * LDZ + hc + 8 * y + 2 * l4]) : double2{0.0, 0.0};
+                for (int y = 0; y < HC; ++y) z[y] = *reinterpret_cast<double2*>(zp[y]);
 #pragma unroll
                 for (int k = 0; k < BT_NB / 4; ++k) {
-                    const double a = v[(strip + l8) * BT_LDV + 4 * k + l4];
+                    const double a = v[4 * k];
 #pragma unroll
                     for (int y = 0; y < HC; ++y) mma_f64(z[y], a, wb[k][y]);
                 }
-                if (gr < n)
 #pragma unroll
-                    for (int y = 0; y < HC; ++y) *reinterpret_cast<double2*>(&zs[(long)gr * LDZ + hc + 8 * y + 2 * l4]) = z[y];
+                for (int y = 0; y < HC; ++y) {
+                    *reinterpret_cast<double2*>(zp[y]) = z[y];
+                    zp[y] -= BT_ROWS * C;
+                }
             }
         }
     }
@@ -928,7 +977,7 @@ __global__ void __launch_bounds__(BT_THREADS) bt_apply_kernel(const BtItem* item
     double* U = Uall + it.moff;
     for (long l = tid; l < (long)n * C; l += BT_THREADS) {
         const int r = (int)(l / C), c = (int)(l % C);
-        if (c < nc) U[(long)r * n + c0 + c] = zs[(long)r * LDZ + c];
+        if (c < nc) U[(long)r * n + c0 + c] = zs[at(r, c)];
     }
 }
 
