@@ -85,14 +85,23 @@ struct BigArgs {
     int k;        // first column of the current panel
     int fin;      // column whose w is completed (-1: none)
     int col;      // column to reflect (-1: none)
+    int slots;    // the product before this column was left in slots (bhh_symv_tri_kernel)
+    int ntri;     // tiles of the largest block there
 };
 
 // Scratch of one large block, in doubles: V and W (BHH_NB columns of n each),
-// y (n), tau (n), then per panel its Gram matrix and -T (BHH_NB^2 each), and
-// the dots of the panel's columns with the reflector (2 BHH_NB).
+// y (n), tau (n), then per panel its Gram matrix and -T (BHH_NB^2 each), the
+// slots of y and the tiles' parts of v . y (bhh_symv_tri_kernel), and the dots of
+// the panel's columns with the reflector (2 BHH_NB).
+constexpr int TRI_T = 128;  // rows and columns of a tile there
+__host__ __device__ inline long bhh_slots(int m) { return (m + TRI_T - 1) / TRI_T; }
 __host__ __device__ inline long bhh_panels(int n) { return n > 2 ? (n - 2 + BHH_NB - 1) / BHH_NB : 0; }
 __host__ __device__ inline long bhh_scratch_doubles(int n) {
-    return 2L * BHH_NB * n + 2L * n + 2 * bhh_panels(n) * BHH_NB * BHH_NB + 2 * BHH_NB;
+    return 2L * BHH_NB * n + 2L * n + 2 * bhh_panels(n) * BHH_NB * BHH_NB + bhh_slots(n) * n +
+           bhh_slots(n) * (bhh_slots(n) + 1) / 2 + 2 * BHH_NB;
+}
+__host__ __device__ inline long bhh_slots_at(int n) {
+    return 2L * BHH_NB * n + 2L * n + 2 * bhh_panels(n) * BHH_NB * BHH_NB;
 }
 __host__ __device__ inline long bhh_dots_at(int n) { return bhh_scratch_doubles(n) - 2 * BHH_NB; }
 
@@ -109,9 +118,10 @@ __host__ __device__ inline long bhh_dots_at(int n) { return bhh_scratch_doubles(
 // for all columns, against 42 on clusters that reduced the column's norm and
 // w . v between their CTAs; blocks of 4 x 1225 and 8 x 735 states, whole
 // eigensolve: 24.8 -> 22.9 ms.
-__global__ void __launch_bounds__(BHH_COL_THREADS, 2) bhh_col_kernel(BigArgs g) {
+template <bool SLOTS>
+__global__ void __launch_bounds__(BHH_COL_THREADS, SLOTS ? 1 : 2) bhh_col_kernel(BigArgs g) {
     __shared__ double dw[BHH_NB], dv[BHH_NB], jw[BHH_NB], jv[BHH_NB];
-    __shared__ double red[BHH_COL_THREADS / 32], s_dd, s_dj;
+    __shared__ double red[BHH_COL_THREADS / 32], s_dd, s_yj;
     cudaTriggerProgrammaticLaunchCompletion();
     const BigBlk bl = g.blk[blockIdx.y];
     const int n = bl.n, last = n - 3;  // the last column with a reflector
@@ -121,11 +131,14 @@ __global__ void __launch_bounds__(BHH_COL_THREADS, 2) bhh_col_kernel(BigArgs g) 
     const double* y = W + (long)BHH_NB * n;
     const double* tau = y + n;
     const double* dots = V + bhh_dots_at(n);
+    const double* slot = V + bhh_slots_at(n);  // slot t of y at slot + t n
+    const double* parts = slot + bhh_slots(n) * n;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const bool fin = g.fin >= 0 && g.fin <= last, col = g.col >= 0 && g.col <= last;
     if (!fin && !col) return;
     const int f = g.fin, j = g.col, cf = fin ? f - g.k : 0, cc = col ? j - g.k : 0;
     const int lo = fin ? f + 1 : j;  // the first row of v, w and the column
+    const int ns = SLOTS && fin ? (int)bhh_slots(n - lo) : 0;
     double* vf = V + (long)cf * n;
     const int sg = lane >> 3;
     cudaGridDependencySynchronize();
@@ -141,8 +154,10 @@ __global__ void __launch_bounds__(BHH_COL_THREADS, 2) bhh_col_kernel(BigArgs g) 
         if (in && fin) v = r == lo ? v0 : vf[r];
         if (in && sg == 0) {
             if (col) x = A[(long)j * n + r];  // row j holds column j (A symmetric)
-            if (fin) acc = y[r];
+            if (fin && !SLOTS) acc = y[r];
         }
+        if constexpr (SLOTS)
+            for (int t = sg; t < ns; t += 4) acc += in ? slot[(long)t * n + r] : 0.0;
 #pragma unroll
         for (int q = 0; q < BHH_NB / 4; ++q) {
             const int s = sg + 4 * q;
@@ -156,7 +171,10 @@ __global__ void __launch_bounds__(BHH_COL_THREADS, 2) bhh_col_kernel(BigArgs g) 
     double K = 0.0, wj = 0.0;
     if (fin) {
         double vy = 0.0;
-        for (int r = lo + 1 + tid; r < n; r += BHH_COL_THREADS) vy = fma(vf[r], y[r], vy);
+        if constexpr (SLOTS)
+            for (int t = tid; t < ns * (ns + 1) / 2; t += BHH_COL_THREADS) vy += parts[t];
+        else
+            for (int r = lo + 1 + tid; r < n; r += BHH_COL_THREADS) vy = fma(vf[r], y[r], vy);
         if (tid < BHH_NB) {
             double a = 0.0, b = 0.0, c = 0.0, d = 0.0;
             if (tid < cf) {
@@ -169,11 +187,14 @@ __global__ void __launch_bounds__(BHH_COL_THREADS, 2) bhh_col_kernel(BigArgs g) 
             dv[tid] = b;
             jw[tid] = c;
             jv[tid] = d;
+            double yl = !SLOTS && tid == 0 ? y[lo] : 0.0;
+            for (int t = tid; t < ns; t += 32) yl += slot[(long)t * n + lo];
             const double dd = warp_sum(a * b), dj = warp_sum(d * a + c * b);
+            yl = warp_sum(yl);
             if (tid == 0) {
                 s_dd = dd;
-                s_dj = dj;
-                vy = fma(v0, y[lo], vy);
+                s_yj = yl - dj;
+                if (!SLOTS) vy = fma(v0, yl, vy);
             }
         }
         vy = warp_sum(vy);
@@ -183,7 +204,7 @@ __global__ void __launch_bounds__(BHH_COL_THREADS, 2) bhh_col_kernel(BigArgs g) 
 #pragma unroll
         for (int q = 0; q < BHH_COL_THREADS / 32; ++q) t += red[q];
         K = 0.5 * tf * (tf * (t - 2.0 * s_dd));
-        wj = tf * (y[lo] - s_dj) - K * v0;
+        wj = tf * s_yj - K * v0;
     }
     const double st = sqrt(tf);
     for (; rb < n; rb += stride) {
@@ -235,10 +256,8 @@ __device__ inline double ld_now(const double* p) {
 // through the column and adds that entry's product at the end.  Grid (rows,
 // block), RW rows per warp and 8 / RW columns per lane at once, so eight row
 // loads are in flight per lane, and with several rows each entry of v is loaded
-// once for them.  What bounds it: reading the trailing matrix, from HBM where
-// the active blocks exceed L2 (64 models of 3 to 6 bath sites, all columns:
-// 95 ms, 4.7 TB/s, against 102 with two rows' loads at a time), else the latency
-// of L2 with the warps there are, hence fewer rows per warp for fewer rows
+// once for them.  What bounds it: the latency of L2 with the warps there are,
+// hence fewer rows per warp for fewer rows
 // (blocks of 4 x 1225 and 8 x 735 states, whole eigensolve: 24.8 ms, against
 // 32.3 with four rows per warp throughout; 21.8 with the loads issued together).
 template <int RW>
@@ -325,6 +344,137 @@ __global__ void __launch_bounds__(BHH_SYMV_THREADS, RW == 4 ? 10 : 6) bhh_symv_k
             if (r < m) y[r] = t;
             else dots[r - m] = t;
         }
+    }
+}
+
+// The same products and dots where the active blocks exceed L2: only tiles on or
+// below the diagonal are read, each for both of its products, A_ij v_j and
+// A_ij^T v_i.  CTA (tile, block): a warp 16 rows, a lane 4 columns of the tile, 16
+// loads in flight; the products of rows of tile row R go to slot tj of y,
+// those of its columns to slot ti, so every row finds its parts in slots 0 ..
+// and nothing is added up in memory; the tile's part of v . y goes beside them.
+// CTAs past the tiles take the dots, a row per warp.  Every CTA sums the
+// column's squares itself.  What bounds it: reading the triangle from HBM, at
+// half the copy rate, as a CTA's column sums and exchanges stand between its
+// loads.  64 models of 3 to 6 bath sites: the 783 columns that take this path
+// 67 ms, 3.7 TB/s with the diagonal tiles, the column kernel's sums of slots 5
+// more; whole step 275 -> 266 ms.  Strips of 2 or 4 tiles per CTA: 70 to 77.
+constexpr int SYT_THREADS = 256;
+// The matrices' bytes above which one triangle is read: below, they come from L2,
+// where twice the bytes cost less than the sums (7-site ring, 80 MB at first:
+// whole solve 24.4 ms, against 29.7 with one triangle).
+constexpr double SYT_BYTES = 100e6;
+__global__ void __launch_bounds__(SYT_THREADS, 3) bhh_symv_tri_kernel(BigArgs g) {
+    __shared__ double red[SYT_THREADS / 32], vi[TRI_T], cols[SYT_THREADS / 32][TRI_T];
+    cudaTriggerProgrammaticLaunchCompletion();
+    const BigBlk bl = g.blk[blockIdx.y];
+    const int n = bl.n, j = g.col, cc = j - g.k, m = n - j - 1;
+    if (m < 2) return;  // no reflector
+    const int nt = (int)bhh_slots(m), tile = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const bool dot = tile >= g.ntri;
+    if (!dot && tile >= nt * (nt + 1) / 2) return;
+    if (dot && (tile - g.ntri) * (SYT_THREADS / 32) >= 2 * cc) return;
+    double* V = g.S + bl.boff;
+    const double* v = V + (long)cc * n + (j + 1);
+    cudaGridDependencySynchronize();
+    double sigma = 0.0;
+    for (int i = 1 + tid; i < m; i += SYT_THREADS) sigma = fma(v[i], v[i], sigma);
+    sigma = warp_sum(sigma);
+    if (lane == 0) red[wid] = sigma;
+    __syncthreads();
+    sigma = 0.0;
+#pragma unroll
+    for (int q = 0; q < SYT_THREADS / 32; ++q) sigma += red[q];
+    const double x0 = v[0];
+    double alpha = x0, v0 = 0.0, tj = 0.0;
+    if (sigma != 0.0) {
+        const double t = fma(x0, x0, sigma), mu = t * rsqrt(t);
+        alpha = (x0 > 0.0) ? -mu : mu;  // v0 = x0 - alpha without cancellation
+        v0 = x0 - alpha;
+        tj = 2.0 * recip_pos(fma(v0, v0, sigma));
+    }
+    if (tile == 0 && tid == 0) {
+        g.tri[2 * bl.eoff + n + j] = alpha;
+        V[2L * BHH_NB * n + n + j] = tj;
+        V[2L * BHH_NB * n + j] = v0;
+    }
+    if (dot) {
+        const int d = (tile - g.ntri) * (SYT_THREADS / 32) + wid;
+        if (d >= 2 * cc) return;
+        const double* p = V + ((d & 1) ? 0L : (long)BHH_NB * n) + (long)(d >> 1) * n + (j + 1);
+        double t = 0.0;
+        for (int i = lane; i < m; i += 32) t = fma(p[i], i == 0 ? v0 : v[i], t);
+        t = warp_sum(t);
+        if (lane == 0) V[bhh_dots_at(n) + d] = t;
+        return;
+    }
+    int ti = (int)((sqrtf(8.0f * tile + 1.0f) - 1.0f) * 0.5f);
+    while ((ti + 1) * (ti + 2) / 2 <= tile) ++ti;
+    while (ti * (ti + 1) / 2 > tile) --ti;
+    const int ct = tile - ti * (ti + 1) / 2, i0 = ti * TRI_T, j0 = ct * TRI_T;
+    if (tid < TRI_T) vi[tid] = i0 + tid == 0 ? v0 : i0 + tid < m ? v[i0 + tid] : 0.0;
+    double vj[4], c[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int jj = j0 + lane + 32 * q;
+        vj[q] = jj == 0 ? v0 : jj < m ? v[jj] : 0.0;
+    }
+    __syncthreads();
+    const double* A = g.A + bl.moff + (long)(j + 1) * n + (j + 1);
+    double s[16];
+#pragma unroll
+    for (int rb = 0; rb < 16; rb += 4) {
+        double a[4][4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            // clamped: v is 0 beyond
+            const double* row = A + (long)min(i0 + 16 * wid + rb + u, m - 1) * n;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                a[u][q] = ld_now(row + min(j0 + lane + 32 * q, m - 1));
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const double w = vi[16 * wid + rb + u];
+            s[rb + u] = 0.0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                s[rb + u] = fma(a[u][q], vj[q], s[rb + u]);
+                c[q] = fma(a[u][q], w, c[q]);
+            }
+        }
+    }
+    // the 16 row sums: halving the rows a lane holds at each exchange, lane -> row lane / 2
+#pragma unroll
+    for (int h = 8; h >= 1; h >>= 1) {
+        const bool up = lane & (2 * h);
+#pragma unroll
+        for (int u = 0; u < h; ++u) {
+            const double keep = up ? s[u + h] : s[u], give = up ? s[u] : s[u + h];
+            s[u] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * h);
+        }
+    }
+    const double ys = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);
+    double* slot = V + bhh_slots_at(n);
+    const int row = 16 * wid + (lane >> 1);
+    if (!(lane & 1) && i0 + row < m) slot[(long)ct * n + j + 1 + i0 + row] = ys;
+    const double part = warp_sum(lane & 1 ? 0.0 : ys * vi[row]);
+    if (ct != ti)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cols[wid][lane + 32 * q] = c[q];
+    if (lane == 0) red[wid] = part;
+    __syncthreads();
+    if (ct != ti && tid < TRI_T) {
+        double t = 0.0;
+#pragma unroll
+        for (int q = 0; q < SYT_THREADS / 32; ++q) t += cols[q][tid];
+        slot[(long)ti * n + j + 1 + j0 + tid] = t;
+    }
+    if (tid == 0) {
+        double t = 0.0;
+#pragma unroll
+        for (int q = 0; q < SYT_THREADS / 32; ++q) t += red[q];
+        (slot + bhh_slots(n) * n)[tile] = ct == ti ? t : 2.0 * t;
     }
 }
 
@@ -1668,6 +1818,7 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
     a.Zc = d.Zc;
     a.S = d.S;
     a.tri = d.tri;
+    a.slots = 0;
     double fl = 0.0, by = 0.0;
     for (int b : big) {
         const double n = dims[b];
@@ -1692,14 +1843,22 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
         // resident at once (two CTAs per SM)
         const int lo = (a.fin >= 0 ? a.fin + 1 : a.col) & ~7;
         int cs = std::max(1, (int)ceil_div(nmax - lo, BHH_COL_THREADS / 4));
-        while (cs > 1 && a.nact * cs > 2 * 148) cs = (cs + 1) / 2;
+        while (cs > 1 && a.nact * cs > (a.slots ? 1 : 2) * 148) cs = (cs + 1) / 2;
         cfg.gridDim = dim3((unsigned)cs, (unsigned)a.nact);
         cfg.blockDim = dim3(BHH_COL_THREADS);
         ProfRange r1("bhh_col_kernel", st, 0.0, 0.0);
-        PGX_CUDA(cudaLaunchKernelEx(&cfg, bhh_col_kernel, a));
+        PGX_CUDA(cudaLaunchKernelEx(&cfg, a.slots ? bhh_col_kernel<true> : bhh_col_kernel<false>, a));
         check_launch("bhh_col_kernel");
     };
     auto symv_step = [&](int rows, long all_rows, double bytes) {
+        if (a.slots) {
+            cfg.gridDim = dim3((unsigned)(a.ntri + ceil_div(2 * (a.col - a.k), SYT_THREADS / 32)), (unsigned)a.nact);
+            cfg.blockDim = dim3(SYT_THREADS);
+            ProfRange r2("bhh_symv_tri_kernel", st, 0.0, 0.5 * bytes);
+            PGX_CUDA(cudaLaunchKernelEx(&cfg, bhh_symv_tri_kernel, a));
+            check_launch("bhh_symv_tri_kernel");
+            return;
+        }
         // rows per warp: 24 warps per SM where there are that many rows
         const int rw = all_rows >= 4L * 148 * 24 ? 4 : all_rows >= 2L * 148 * 24 ? 2 : 1;
         cfg.gridDim = dim3((unsigned)ceil_div(rows, rw * (BHH_SYMV_THREADS / 32)), (unsigned)a.nact);
@@ -1727,6 +1886,8 @@ static void launch_big(const EighDev& d, const std::vector<int>& dims, const std
                 bytes += 8.0 * m * m;
                 all_rows += dims[big[i]] - j - 1 + 2 * (j - k);
             }
+            a.slots = bytes > SYT_BYTES;
+            a.ntri = (int)(bhh_slots(nmax - j - 1) * (bhh_slots(nmax - j - 1) + 1) / 2);
             symv_step(nmax - j - 1 + 2 * (j - k), all_rows, bytes);
         }
         a.fin = jend - 1;

@@ -34,7 +34,8 @@ def symmetric(rng, n, kind="dense"):
 # 1e-4 ||H|| are left as inverse iteration gives them, orthogonal to eps / 1e-4.
 @pytest.mark.parametrize("kind", ["dense", "pieces"])
 @pytest.mark.parametrize("dims", [[1, 2, 3, 4, 31, 32, 33, 34, 35, 66, 67, 127], [463, 464, 465, 513, 514, 679, 680],
-                                  [1273, 1274, 600], [697, 698, 1489, 1490], [3073, 3074], [3] * 400, [7, 5] * 150])
+                                  [1273, 1274, 600], [697, 698, 1489, 1490], [3073, 3074], [1025] + [900] * 16,
+                                  [3] * 400, [7, 5] * 150])
 def test_eigensolve_at_the_edges_of_its_paths(dims, kind):
     rng = np.random.default_rng(sum(dims))
     H = [symmetric(rng, n, kind) for n in dims]
