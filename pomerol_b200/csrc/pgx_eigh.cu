@@ -37,18 +37,6 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Sum over the CTA; result valid in every thread.  `red` holds >= 32 doubles.
-__device__ double block_sum(double v, double* red) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    v = warp_sum(v);
-    __syncthreads();
-    if (lane == 0) red[wid] = v;
-    __syncthreads();
-    double r = (lane < nw) ? red[lane] : 0.0;
-    r = warp_sum(r);
-    return r;
-}
-
 // ----------------------------------------------------------------------------
 // Householder stage for blocks too large for a cluster's shared memory
 // (n > 513): the blocked reduction of LAPACK's dsytrd / dlatrd (lower).

@@ -31,6 +31,7 @@
 #include <array>
 #include <iterator>
 #include <map>
+#include <limits>
 #include <tuple>
 #include <unordered_map>
 
@@ -394,20 +395,24 @@ void build_points(Points& pt, int nfreq, const double* z, bool real) {
 // point also the numbers of the four frequency sums the contractions use: z2',
 // z1'+z2'+z3', z1'+z2', z2'+z3', where (z1', z2', z3') is the permuted (z1, z2,
 // -z3), z1' dressing O1 and z3' dressing O3.  Sums equal up to rounding (2^-46
-// of the largest) have one number; the numbers ascend with the values.
+// of what they were added up from) have one number; finite numbers ascend with
+// the values.
 struct PermIndex {
     std::vector<int> pts;
     std::vector<cd> Z1, Z3;
     std::vector<int> j1, j3;
     std::vector<int> sid[4];  // sum k of point e (of pts): number sid[k][e]
     std::vector<cd> sval[4];  // its value
+    std::vector<double> size[4];  // the largest part of what it was added up from
 };
+inline double largest_part(cd v) { return std::max(std::fabs(v.x), std::fabs(v.y)); }
 
 // Numbers of x + y over the pairs (i, j) that occur: `val` receives a value
 // per distinct pair, `id` each point's pair.  A pair is added once, so the
 // cost per point is a table lookup.
 void number_pairs(const std::vector<int>& pts, const std::vector<int>& xi, const std::vector<cd>& xv,
-                  const std::vector<int>& yi, const std::vector<cd>& yv, std::vector<int>& id, std::vector<cd>& val) {
+                  const std::vector<int>& yi, const std::vector<cd>& yv, const std::vector<double>* xs,
+                  std::vector<int>& id, std::vector<cd>& val, std::vector<double>& size) {
     const size_t ny = yv.size(), cells = xv.size() * ny;
     std::vector<int> dense(cells <= (size_t(1) << 20) ? cells : 0, -1);
     std::unordered_map<size_t, int> sparse;
@@ -417,29 +422,42 @@ void number_pairs(const std::vector<int>& pts, const std::vector<int>& xi, const
         if (q < 0) {
             q = (int)val.size();
             val.push_back(xv[xi[e]] + yv[yi[e]]);
+            size.push_back(std::max(xs ? (*xs)[xi[e]] : largest_part(xv[xi[e]]), largest_part(yv[yi[e]])));
         }
         id[e] = q;
     }
 }
 
-// Merges the numbers of values equal up to rounding and orders them.
-void order_values(const std::vector<int>& pts, std::vector<int>& id, std::vector<cd>& val) {
+// Merges the numbers of values equal up to rounding and orders them.  Values in
+// one cell of 2^-46 of the largest are candidates; they are one number where
+// they differ by no more than 2^-46 of their own size, so a far value in the
+// list does not join others.
+void order_values(const std::vector<int>& pts, std::vector<int>& id, std::vector<cd>& val, std::vector<double>& size) {
     double big = 0.0;
-    for (const cd& v : val) big = std::max(big, std::max(std::fabs(v.x), std::fabs(v.y)));
+    for (const cd& v : val)
+        if (std::isfinite(v.x) && std::isfinite(v.y)) big = std::max(big, largest_part(v));
     const double q = big > 0.0 ? std::ldexp(big, -46) : 1.0;
+    auto cell = [&](double x) { return std::isfinite(x) ? std::llround(x / q) : std::numeric_limits<long long>::max(); };
     std::vector<std::tuple<long long, long long, int>> key;
-    for (size_t i = 0; i < val.size(); ++i)
-        key.emplace_back(std::llround(val[i].x / q), std::llround(val[i].y / q), (int)i);
+    for (size_t i = 0; i < val.size(); ++i) key.emplace_back(cell(val[i].x), cell(val[i].y), (int)i);
     std::sort(key.begin(), key.end());
     std::vector<int> to(val.size());
     std::vector<cd> out;
+    std::vector<double> osize;
     for (size_t i = 0; i < key.size(); ++i) {
-        if (i == 0 || std::get<0>(key[i]) != std::get<0>(key[i - 1]) || std::get<1>(key[i]) != std::get<1>(key[i - 1]))
-            out.push_back(val[std::get<2>(key[i])]);
-        to[std::get<2>(key[i])] = (int)out.size() - 1;
+        const int e = std::get<2>(key[i]);
+        bool same = i > 0 && std::get<0>(key[i]) == std::get<0>(key[i - 1]) && std::get<1>(key[i]) == std::get<1>(key[i - 1]);
+        if (same) same = largest_part(cd{val[e].x - out.back().x, val[e].y - out.back().y}) <=
+                         std::ldexp(std::max(size[e], osize.back()), -46);
+        if (!same) {
+            out.push_back(val[e]);
+            osize.push_back(size[e]);
+        }
+        to[e] = (int)out.size() - 1;
     }
     for (int e : pts) id[e] = to[id[e]];
     val = std::move(out);
+    size = std::move(osize);
 }
 
 void index_perm(PermIndex& ix, const int perm[3], const Points& pt) {
@@ -474,13 +492,15 @@ void number_sums(PermIndex& ix) {
     const std::vector<int> j2 = ix.sid[0];
     const std::vector<cd> Z2 = ix.sval[0];
     for (auto& v : ix.sid) v.resize(j2.size());
-    order_values(ix.pts, ix.sid[0], ix.sval[0]);
-    number_pairs(ix.pts, ix.j1, ix.Z1, j2, Z2, ix.sid[2], ix.sval[2]);
-    order_values(ix.pts, ix.sid[2], ix.sval[2]);
-    number_pairs(ix.pts, ix.sid[2], ix.sval[2], ix.j3, ix.Z3, ix.sid[1], ix.sval[1]);
-    order_values(ix.pts, ix.sid[1], ix.sval[1]);
-    number_pairs(ix.pts, j2, Z2, ix.j3, ix.Z3, ix.sid[3], ix.sval[3]);
-    order_values(ix.pts, ix.sid[3], ix.sval[3]);
+    for (const cd& v : Z2) ix.size[0].push_back(largest_part(v));
+    auto order = [&](int k) { order_values(ix.pts, ix.sid[k], ix.sval[k], ix.size[k]); };
+    order(0);
+    number_pairs(ix.pts, ix.j1, ix.Z1, j2, Z2, nullptr, ix.sid[2], ix.sval[2], ix.size[2]);
+    order(2);
+    number_pairs(ix.pts, ix.sid[2], ix.sval[2], ix.j3, ix.Z3, &ix.size[2], ix.sid[1], ix.sval[1], ix.size[1]);
+    order(1);
+    number_pairs(ix.pts, j2, Z2, ix.j3, ix.Z3, nullptr, ix.sid[3], ix.sval[3], ix.size[3]);
+    order(3);
 }
 
 // What the device needs of all plans of a call, gathered on the host and

@@ -161,6 +161,11 @@ def freq_list(form, dim, beta, rng):
         return z[rng.permutation(len(z))]
     if form == "one":
         return cube([[1]] * dim)
+    if form == "far":           # values far beyond the others do not blur them
+        z = cube([range(-2, 2)] * dim)
+        z[::5, 0] = 1e14j
+        z[1::7, -1] = -3e13j
+        return z
     z = rng.uniform(-2, 2, (40, dim)) + 1j * rng.uniform(0.2, 3, (40, dim)) * rng.choice([-1, 1], (40, dim))
     z[::4] = z[1::4].conj()     # some conjugate pairs
     z[2, 0] = 0.123 + 0.0j      # on the real axis, off every pole
@@ -168,7 +173,7 @@ def freq_list(form, dim, beta, rng):
     return z
 
 
-FORMS = ["even", "odd", "above", "ragged", "repeats", "one", "general"]
+FORMS = ["even", "odd", "above", "ragged", "repeats", "one", "far", "general"]
 
 
 # A sum over at most 3e5 quadruples of terms that the resolvents bound: errors
@@ -198,6 +203,28 @@ def test_g2_over_forms_of_frequency_lists(form, kind):
     g.eng.set_g2_workspace(0, 1 << 15)
     tiled = g.eng.g2(parts, z, coef_tol=0.0, flags=PGX_G2_ANCHORED)
     assert np.abs(tiled - exact).max() < 1e-12 * scale
+
+
+# Six balanced digits hold an operand to 254^-6 = 4e-15 of its row's or column's
+# largest entry; products along a chain of four operators bring that to no more
+# than 1e-9 of the largest value, the bound the other split tests use.
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("kind", ["real", "complex"])
+@pytest.mark.parametrize("form", ["even", "odd", "ragged", "far", "general"])
+def test_split_g2_over_forms_of_frequency_lists(form, kind, pair):
+    from pomerol_b200.pgx import PGX_G2_ANCHORED, PGX_G2_SPLIT_I8
+    from tests.pgx_harness import GpuED
+    m, beta = small_model(kind), 7.0
+    lab = "A" if kind == "complex" else "C"
+    u, d = m.info.getIndex(lab, 0, 1), m.info.getIndex(lab, 0, 0)
+    g = GpuED(m, beta)
+    z = freq_list(form, 3, beta, np.random.default_rng(5))
+    parts = g.g2_parts(g.c(u), g.c(d), g.cdag(u), g.cdag(d))
+    fp64 = g.eng.g2(parts, z, coef_tol=0.0, flags=PGX_G2_ANCHORED)
+    g.eng.set_split_cta_pair(pair)
+    g.eng.set_g2_split_threshold(0.0)
+    split = g.eng.g2(parts, z, coef_tol=0.0, flags=PGX_G2_ANCHORED | PGX_G2_SPLIT_I8)
+    assert np.abs(split - fp64).max() < 1e-9 * np.abs(fp64).max()
 
 
 def test_exact_g2_on_both_sides_of_its_rule():
