@@ -6,8 +6,8 @@
 //      Computations", 4th ed., 8.3.1):
 //      eigh_cluster_kernel, one thread-block cluster of 1-16 CTAs per block
 //      with the matrix in distributed shared memory (blocks up to 513 states);
-//      larger blocks: a blocked reduction (panels of 32 columns, trailing
-//      updates by GEMMs) over the whole GPU.
+//      larger blocks: a blocked reduction (panels of 32 columns, one trailing
+//      update per panel) over the whole GPU.
 //   2. bisect_kernel: multisection with Sturm counts on the unreduced pieces
 //      of T (8.4.1).
 //   3. vector_kernel, one thread per eigenvalue: inverse iteration with a
@@ -245,9 +245,9 @@ __device__ inline double ld_now(const double* p) {
 // block), RW rows per warp and 8 / RW columns per lane at once, so eight row
 // loads are in flight per lane, and with several rows each entry of v is loaded
 // once for them.  What bounds it: the latency of L2 with the warps there are,
-// hence fewer rows per warp for fewer rows
-// (blocks of 4 x 1225 and 8 x 735 states, whole eigensolve: 24.8 ms, against
-// 32.3 with four rows per warp throughout; 21.8 with the loads issued together).
+// hence fewer rows per warp for fewer rows (blocks of 4 x 1225 and 8 x 735
+// states, whole eigensolve: 24.8 ms, against 32.3 with four rows per warp
+// throughout; with the loads issued together 21.8, against 22.9 without).
 template <int RW>
 __global__ void __launch_bounds__(BHH_SYMV_THREADS, RW == 4 ? 10 : 6) bhh_symv_kernel(BigArgs g) {
     constexpr int U = 8 / RW;

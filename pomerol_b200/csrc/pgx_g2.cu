@@ -17,7 +17,10 @@
 // Per chain: dressed operators per distinct z1 / z3, four batched GEMMs per
 // distinct frequency, two batched GEMMs per distinct (z1, z3) pair (the
 // dominant FP64 work), and four contractions over the triples of each pair.
-// Everything stays FP64; the delta test is made per element in FP64.
+// Everything stays FP64; the delta test is made per element in FP64.  Exact
+// sums whose work is less in the batched form, every state an anchor, are sent
+// there (anchored_faster in pgx_g2a.cu): small blocks, for which this form's
+// launches per part cost more than its products.
 
 #include <chrono>
 #include <cstring>

@@ -23,7 +23,7 @@
 // (Z = z1+z2+z3, D = s - (E_b - E_a) with s = z1+z2 for T3 and z2+z3 for T4).
 // Stages, each one launch for a batch of chains: anchored products per
 // frequency (gather GEMMs); products per (z1, z3) stacked into GEMMs over all
-// anchors; contractions per triple (warp per (sub-term, (z1, z3) group),
+// anchors; contractions of classes of triples as products (contract_gemm_kernel,
 // resonant delta test in FP64).  A(z1) and C(z3) are never stored: the GEMM
 // tile loads dress O1 and O3 with the frequency as they read them.
 

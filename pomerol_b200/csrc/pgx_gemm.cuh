@@ -495,6 +495,37 @@ void launch_gemm_class(const GemmProblem<TA, TB, TC>* dp, const int* d_index, si
     check_launch("gemm_tiles_kernel");
 }
 
+// Classes of a few tiles join the 64 x 64 class, so that they need no launch of
+// their own: the launches follow one another, each taking the latency of its
+// longest k loop, about the same for every tile shape while the chip is nearly
+// empty.  A class joins when its products are fewer tiles than a quarter of the
+// SMs, and no more than twice as many of 64 x 64.  Two rotations of Anderson
+// 1+5, nine launches of 8 to 34 us each before: 174 -> 78 us; the gradient of a
+// Kanamori impurity, whole call: 3.75 -> 3.54 ms.  Classes that a caller's
+// measurement chose are left alone.
+template <typename TA, typename TB, typename TC>
+void gemm_join_small(const std::vector<GemmProblem<TA, TB, TC>>& probs, std::vector<int>& cls) {
+    if (forced_gemm_class() >= 0 || active_tune()) return;
+    long own[GEMM_NCLS] = {}, square[GEMM_NCLS] = {};
+    for (size_t q = 0; q < probs.size(); ++q) {
+        const auto& g = probs[q];
+        const int c = cls[q];
+        if (c >= GEMM_NCLS || g.M <= 0 || g.N <= 0) continue;
+        const long nb = std::max(g.nb, 1);
+        own[c] += nb * ceil_div(g.M, GEMM_CLS_M[c]) * ceil_div(g.N, GEMM_CLS_N[c]);
+        square[c] += nb * ceil_div(g.M, GEMM_CLS_M[0]) * ceil_div(g.N, GEMM_CLS_N[0]);
+    }
+    bool join[GEMM_NCLS] = {};
+    int n = own[0] > 0;
+    for (int c = 1; c < GEMM_NCLS; ++c) {
+        join[c] = own[c] > 0 && own[c] <= 37 && square[c] <= 74;
+        n += join[c];
+    }
+    if (n < 2) return;  // no launch fewer
+    for (int& c : cls)
+        if (c < GEMM_NCLS && join[c]) c = 0;
+}
+
 // Host helper: upload the problems (grouped by tile class) and, per class, the
 // prefix sums of their tile counts into scratch buffers, and launch one kernel
 // per tile class.  The index needs gemm_index_bytes(probs.size()) bytes.
@@ -561,6 +592,7 @@ void launch_gemm_batch(const std::vector<GemmProblem<TA, TB, TC>>& probs, void* 
                   "k gathers need operands of one plain type");
         cls[q] = gemm_class_for(g);
     }
+    gemm_join_small(probs, cls);
     for (int c = 0; c < GEMM_NCLS_ALL; ++c) {
         pstart[c] = sorted.size();
         istart[c] = index.size();

@@ -86,6 +86,34 @@ def pair_setup(rng, dims, is_complex):
     return e, E, w, op, e.op_adjoint(op), ref
 
 
+# Parts of every tile shape in one batch: few tiles of each, which share a
+# launch, and many.  Products of K terms of at most one in modulus, K eps each.
+@pytest.mark.parametrize("is_complex", [False, True])
+@pytest.mark.parametrize("copies", [1, 40])
+def test_rotation_of_parts_of_many_sizes(copies, is_complex):
+    rng = np.random.default_rng(copies)
+    dims = [1, 9, 130, 17, 200, 33, 70, 3, 90] * copies
+    H = []
+    for n in dims:
+        a = rng.standard_normal((n, n)) + (1j * rng.standard_normal((n, n)) if is_complex else 0)
+        H.append((a + a.conj().T) / 2)
+    e = engine(H, is_complex)
+    e.eigh()
+    _, U = e.eigensystem()
+    acts = []
+    for q in range(0, len(dims) - 1):
+        tgt = np.full(dims[q], -1)
+        k = min(dims[q], dims[q + 1])
+        tgt[rng.permutation(dims[q])[:k]] = rng.permutation(dims[q + 1])[:k]
+        acts.append((q, q + 1, tgt, np.where(tgt >= 0, rng.choice([-1.0, 0.5], dims[q]), 0.0)))
+    op = e.op_define(acts)
+    e.op_rotate(op)
+    for p, (q, r, tgt, cf) in enumerate(acts):
+        C = np.zeros((dims[r], dims[q]))
+        C[tgt[tgt >= 0], np.nonzero(tgt >= 0)[0]] = cf[tgt >= 0]
+        assert np.abs(e.op_read(op, p) - U[r].conj().T @ C @ U[q]).max() < 4 * (max(dims) + 4) * EPS
+
+
 # The sums' error is a few eps of the sum of the terms' moduli: ten or so
 # rounded operations per term, and up to a thousand additions per partial sum.
 @pytest.mark.parametrize("is_complex", [False, True])
