@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(EVAL_THREADS) pair_eval_kernel(const cd* __res
     int have = 0;
     bool fit = true;
     for (int t = 0; t < ch.cnt; t += EVAL_THREADS) {
-        // append this round's non-zero terms in order
+        // append the non-zero terms of this turn in order
         cd r{0.0, 0.0};
         double p = 0.0;
         if (t + tid < ch.cnt) {
