@@ -25,12 +25,12 @@
 // and (3) one split-K GEMM L R over all parts at once, whose result is the
 // (z1, z2) or (z1, Om) table.  A final kernel gathers the requested duplets.
 
-#include <map>
 #include <utility>
 
 #include "pgx_common.cuh"
 #include "pgx_gemm.cuh"
 #include "pgx_internal.h"
+#include "pgx_numbers.h"
 
 namespace pgx {
 
@@ -196,22 +196,6 @@ __global__ void chi3_gather_kernel(const DupletIdx* q, int n, const cd* OUTN, in
     out[t] = v;
 }
 
-// distinct values of a complex list (exact bits), in order of first appearance
-int distinct_index(const std::vector<cd>& v, std::vector<cd>& uniq, std::vector<int>& idx) {
-    std::map<std::pair<double, double>, int> seen;
-    idx.resize(v.size());
-    for (size_t q = 0; q < v.size(); ++q) {
-        auto key = std::make_pair(v[q].x, v[q].y);
-        auto it = seen.find(key);
-        if (it == seen.end()) {
-            it = seen.emplace(key, (int)uniq.size()).first;
-            uniq.push_back(v[q]);
-        }
-        idx[q] = it->second;
-    }
-    return (int)uniq.size();
-}
-
 // C (M x N) += A (M x K) B (K x N), row-major, split over K into partial
 // products that a reduction adds up
 void split_k_gemm(const cd* A, const cd* B, int M, int N, long K, cd* C, DevBuf& partial, DevBuf& probs,
@@ -294,26 +278,7 @@ void run_chi3_t(pgx_ctx* c, int channel, int nparts, const pgx_chi3_part* parts,
     // z2 whose columns are computed first, then those mirrored from msrc
     int N2u = N2;
     std::vector<int> msrc;
-    if (real) {
-        std::map<std::pair<double, double>, int> at;
-        for (int b = 0; b < N2; ++b) at[{SZ2[b].x, SZ2[b].y}] = b;
-        std::vector<int> order, low, pos(N2);
-        for (int b = 0; b < N2; ++b) {
-            const auto it = at.find({SZ2[b].x, -SZ2[b].y});
-            if (SZ2[b].y < 0.0 && it != at.end()) low.push_back(b);
-            else order.push_back(b);
-        }
-        N2u = (int)order.size();
-        for (int i = 0; i < N2u; ++i) pos[order[i]] = i;
-        for (size_t i = 0; i < low.size(); ++i) {
-            pos[low[i]] = N2u + (int)i;
-            msrc.push_back(pos[at[{SZ2[low[i]].x, -SZ2[low[i]].y}]]);
-        }
-        std::vector<cd> v(N2);
-        for (int b = 0; b < N2; ++b) v[pos[b]] = SZ2[b];
-        SZ2 = std::move(v);
-        for (int& b : i2) b = pos[b];
-    }
+    if (real) N2u = conjugates_last(SZ2, i2, msrc);
     std::vector<DupletIdx> dq(nfreq);
     bool any_res = false;
     for (int q = 0; q < nfreq; ++q) {

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "pgx_common.cuh"
+#include "pgx_numbers.h"
 
 namespace pgx {
 
@@ -53,25 +54,14 @@ struct Points {
     cd at(int axis, int e) const { return val[axis][id[axis][e]]; }
 };
 
-struct CdKey {
-    unsigned long long x, y;
-    bool operator==(const CdKey& o) const { return x == o.x && y == o.y; }
-};
-struct CdHash {
-    size_t operator()(const CdKey& k) const { return (k.x * 0x9E3779B97F4A7C15ull) ^ (k.y * 0xC2B2AE3D27D4EB4Full >> 7); }
-};
-
 inline void build_points(Points& pt, int nfreq, const double* z, bool real) {
     std::vector<int> tid[3];
     auto& cj = pt.cj;
     for (int k = 0; k < 3; ++k) {
-        std::unordered_map<CdKey, int, CdHash> seen;
+        CdMap seen;
         auto number = [&](cd v) {
-            v = cd{v.x + 0.0, v.y + 0.0};  // -0 and 0 are one value
-            CdKey key;
-            std::memcpy(&key, &v, sizeof(key));
-            const auto it = seen.emplace(key, (int)pt.val[k].size());
-            if (it.second) pt.val[k].push_back(v);
+            const auto it = seen.emplace(cd_key(v), (int)pt.val[k].size());
+            if (it.second) pt.val[k].push_back(cd{v.x + 0.0, v.y + 0.0});
             return it.first->second;
         };
         const double s = k == 2 ? -1.0 : 1.0;
@@ -96,7 +86,7 @@ inline void build_points(Points& pt, int nfreq, const double* z, bool real) {
         for (int t = 0; t < nfreq; ++t) pt.cls[t] = t;
         return;
     }
-    std::unordered_map<CdKey, int, CdHash> seen;
+    CdMap seen;
     seen.reserve(nfreq);
     std::vector<int> rep;  // class -> its first triple
     for (int t = 0; t < nfreq; ++t) {

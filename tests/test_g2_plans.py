@@ -1,5 +1,6 @@
 """The frequency plans of G2 and chi3: undefined and infinite frequencies among
-ordinary ones.  tests/cpp/plan_g2.cpp checks the plan itself without a GPU."""
+ordinary ones.  tests/cpp/plan_g2.cpp and plan_chi3.cpp check the
+plans themselves without a GPU."""
 import subprocess
 from pathlib import Path
 
@@ -13,11 +14,12 @@ NAN, INF = float("nan"), float("inf")
 ODD = [complex(NAN, NAN), complex(NAN, 1.0), complex(0.0, NAN), complex(0.0, INF), complex(-INF, 1.0)]
 
 
-def test_plan_of_undefined_frequencies(tmp_path):
-    exe = tmp_path / "plan_g2"
+@pytest.mark.parametrize("program", ["plan_g2", "plan_chi3"])
+def test_plan_of_undefined_frequencies(program, tmp_path):
+    exe = tmp_path / program
     r = subprocess.run(["g++", "-O1", "-std=c++17", "-Wall", "-D_GLIBCXX_ASSERTIONS", "-I",
                         str(ROOT / "pomerol_b200" / "csrc"), "-I", "/usr/local/cuda/include",
-                        str(ROOT / "tests" / "cpp" / "plan_g2.cpp"), "-o", str(exe)], capture_output=True, text=True)
+                        str(ROOT / "tests" / "cpp" / f"{program}.cpp"), "-o", str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
@@ -62,3 +64,17 @@ def test_g2_beside_undefined_frequencies(place, form, kind):
     g.eng.set_g2_workspace(0, 1 << 15)  # tiles of the (z1, z3) plane
     got = g.eng.g2(parts, y, coef_tol=0.0, flags=PGX_G2_ANCHORED)
     assert np.abs(got[keep] - ref[keep]).max() < 1e-9 * np.abs(ref).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["real", "complex"])
+@pytest.mark.parametrize("form", ["even", "odd", "general"])
+@pytest.mark.parametrize("channel", [0, 1, 2])
+def test_chi3_beside_undefined_frequencies(channel, form, kind):
+    g, u, d = solved(kind)
+    z = freq_list(form, 2, 7.0, np.random.default_rng(6))
+    for place in (0, 1):
+        y, keep = with_odd_values(z, place, np.random.default_rng(place))
+        ref, _ = g.chi3(channel, (u, u, d, d), z)
+        got, _ = g.chi3(channel, (u, u, d, d), y)
+        assert np.abs(got[keep] - ref[keep]).max() < 1e-12 * np.abs(ref).max()
