@@ -38,6 +38,9 @@ extern "C" {
                                     base-254 digits (six by default) with power-of-two
                                     row/column scales (Ozaki scheme), int32-exact partial
                                     products summed in FP64 */
+#define PGX_G2_FULL_MATRICES 8   /* without PGX_G2_ANCHORED: the sum over every quadruple part by
+                                    part in full matrices, also where it takes less work with
+                                    all parts together (the same sum; the default chooses) */
 
 typedef struct pgx_ctx pgx_ctx;
 
@@ -232,7 +235,8 @@ typedef struct pgx_g2_part {
 int pgx_g2(pgx_ctx* ctx, int32_t nparts, const pgx_g2_part* parts, int32_t nfreq, const double* z,
            double pole_res, double coef_tol, int32_t flags, double* out);
 
-/* Device workspace limits of pgx_g2's anchored form (0 keeps a default).
+/* Device workspace limits of pgx_g2's anchored form, and of exact sums where
+ * they take it with every state an anchor (0 keeps a default).
  * batch_bytes: parts are evaluated together while their workspaces fit in it
  * (default 3 GiB).  chain_bytes: the most one part may take (default half the
  * free device memory, at most 48 GiB); a part that needs more at the call's

@@ -20,7 +20,8 @@
 // Everything stays FP64; the delta test is made per element in FP64.  Exact
 // sums whose work is less in the batched form, every state an anchor, are sent
 // there (anchored_faster in pgx_g2a.cu): small blocks, for which this form's
-// launches per part cost more than its products.
+// launches per part cost more than its products.  PGX_G2_FULL_MATRICES keeps a
+// call here.
 
 #include <chrono>
 #include <cstring>
@@ -30,6 +31,7 @@
 #include "pgx_common.cuh"
 #include "pgx_gemm.cuh"
 #include "pgx_internal.h"
+#include "pgx_numbers.h"
 
 namespace pgx {
 
@@ -324,13 +326,7 @@ struct Plan {
     int *dpi1, *dpi3, *dptr, *dslot;
 };
 
-struct Key {
-    double a, b;
-    bool operator<(const Key& o) const { return std::tie(a, b) < std::tie(o.a, o.b); }
-};
-
 void build_plan(Plan& pl, const int perm[3], int nfreq, const double* z) {
-    std::map<Key, int> m1, m3;
     std::map<std::pair<int, int>, int> mp;
     std::vector<int> tp(nfreq);
     std::vector<cd> zz1(nfreq), zz2(nfreq), zz3(nfreq);
@@ -340,14 +336,15 @@ void build_plan(Plan& pl, const int perm[3], int nfreq, const double* z) {
         zz1[t] = a;
         zz2[t] = b;
         zz3[t] = c3;
-        auto i1 = m1.emplace(Key{a.x, a.y}, (int)pl.Z1.size());
-        if (i1.second) pl.Z1.push_back(a);
-        auto i3 = m3.emplace(Key{c3.x, c3.y}, (int)pl.Z3.size());
-        if (i3.second) pl.Z3.push_back(c3);
-        auto ip = mp.emplace(std::make_pair(i1.first->second, i3.first->second), (int)pl.pi1.size());
+    }
+    std::vector<int> i1, i3;
+    distinct_index(zz1, pl.Z1, i1);
+    distinct_index(zz3, pl.Z3, i3);
+    for (int t = 0; t < nfreq; ++t) {
+        auto ip = mp.emplace(std::make_pair(i1[t], i3[t]), (int)pl.pi1.size());
         if (ip.second) {
-            pl.pi1.push_back(i1.first->second);
-            pl.pi3.push_back(i3.first->second);
+            pl.pi1.push_back(i1[t]);
+            pl.pi3.push_back(i3[t]);
         }
         tp[t] = ip.first->second;
     }
@@ -592,7 +589,8 @@ void run_g2(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, const d
     PGX_CUDA(cudaEventRecord(ea, st));
     // the same sum with every state an anchor (weights are positive or zero)
     c->g2t = G2Timing{};
-    if (nfreq > 0 && nparts > 0 && run_g2_anchored(c, nparts, parts, nfreq, z, pole_res, -1.0, 0, true, out)) {
+    if (!(flags & PGX_G2_FULL_MATRICES) && nfreq > 0 && nparts > 0 &&
+        run_g2_anchored(c, nparts, parts, nfreq, z, pole_res, -1.0, 0, true, out)) {
         PGX_CUDA(cudaEventRecord(eb, st));
         PGX_CUDA(cudaEventSynchronize(eb));
         float tot = 0.f;
