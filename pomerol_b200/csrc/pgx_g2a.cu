@@ -724,7 +724,7 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
              "contract_gemm_kernel<32,32>"},
             {"contract_gemm_kernel<64,8>", "contract_gemm_kernel<64,16>", "contract_gemm_kernel<64,24>",
              "contract_gemm_kernel<64,32>"}};
-        const double tol2 = pole_res * pole_res;
+        const double tol2 = pole_res < 0.0 ? -1.0 : pole_res * pole_res;  // none is within a negative resolution
         // the shapes' launches are independent (their sums meet in atomics):
         // dealt to the side streams, so that one's last wave overlaps the next
         struct Shape {

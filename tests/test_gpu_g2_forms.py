@@ -125,6 +125,25 @@ def test_rule_of_the_exact_sum():
 
 
 @pytest.mark.parametrize("kind", ["real", "complex"])
+def test_negative_pole_resolution(kind):
+    """|D| <= pole_res holds nowhere then, also for bosonic sums nearer to a pole
+    than its modulus."""
+    from pomerol_b200.pgx import PGX_G2_ANCHORED, PGX_G2_EXACT, PGX_G2_FULL_MATRICES
+    g, u, d = solved(kind)
+    ed = EDm.ED(small_model(kind), 7.0)
+    rng = np.random.default_rng(8)
+    z = 1j * rng.uniform(0.4, 3, (12, 3)) * rng.choice([-1, 1], (12, 3))
+    z[::2, 1] = -z[::2, 0] + 0.2j
+    z[1::2, 2] = z[1::2, 1] - 0.15j
+    parts = g.g2_parts(g.c(u), g.c(d), g.cdag(u), g.cdag(d))
+    oparts = L.g2_parts(ed, ed.c(u), ed.c(d), ed.cdag(u), ed.cdag(d))
+    ref = L.g2_exact(ed, oparts, [tuple(t) for t in z], res=-0.5)
+    for flags in (PGX_G2_EXACT, PGX_G2_FULL_MATRICES, PGX_G2_ANCHORED):
+        v = g.eng.g2(parts, z, pole_res=-0.5, coef_tol=0.0, flags=flags)
+        assert np.abs(v - ref).max() < 1e-12 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("kind", ["real", "complex"])
 @pytest.mark.parametrize("place", [0, 1, 2])
 def test_full_matrices_beside_undefined_frequencies(place, kind):
     from pomerol_b200.pgx import PGX_G2_FULL_MATRICES
