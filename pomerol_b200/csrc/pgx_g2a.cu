@@ -21,6 +21,10 @@
 //   T4a   s  sum_4 [O2[h,:] C(z3)]_4 [X4 A(z1)[:,h]]_4 (delta ? -beta w2 : w2/D)
 //   T4b   s  sum_2 [O2 C(z3)[:,h]]_2 [X4[h,:] A(z1)]_2 (delta ? 0 : -w4/D)
 // (Z = z1+z2+z3, D = s - (E_b - E_a) with s = z1+z2 for T3 and z2+z3 for T4).
+// Where every state of both blocks is an anchor, T3a and T3b are one term with
+// (w3 - w1)/D, and T4a and T4b one with (w2 - w4)/D: of nearly equal levels the
+// weights cancel before the division by a small D, not between two sums whose
+// rounding it has enlarged.
 // Stages, each one launch for a batch of chains: anchored products per
 // frequency (gather GEMMs); products per (z1, z3) stacked into GEMMs over all
 // anchors; contractions of classes of triples as products (contract_gemm_kernel,
@@ -50,6 +54,7 @@ struct DTerm {
     const void* VB;
     long b1, b3, bh, bk;
     const double *Ek, *Eh, *wh;
+    const double* wk;     // weights of the k states where they enter too (T3, T4 over every state), else null
     const int* hot;       // anchor states (inner indices) of the anchor block
     const int* gi1;       // per group: index of z1 in the plan
     const int* gi3;       // per group: index of z3 in the plan
@@ -57,7 +62,7 @@ struct DTerm {
     int va_cplx, vb_cplx; // operand element types
     int va_hstate, vb_hstate;  // h stride applies to the anchor's state index instead of its position
     int use_delta;
-    double sgn, cdelta, cnum, pref;
+    double sgn, cdelta, cnum, cwk, pref;
     // host side only: the plan and the frequency sum (0: z2, 1: z1+z2+z3,
     // 2: z1+z2, 3: z2+z3) of the sub-term
     int plan, sidx;
@@ -74,7 +79,7 @@ __device__ __forceinline__ cd load_v(const void* p, int cplx, long idx) {
 //   out[t(g, j)] += pref * sum_{h, k} AB[g, (h, k)] K[(h, k), j]
 // with AB[g, (h, k)] = VA(g, h, k) VB(g, h, k) (the two anchored operand
 // arrays, multiplied as the tile is loaded) and the Lehmann kernel
-//   K[(h, k), j] = delta ? cdelta beta w_h : cnum w_h / (s_j - sgn (E_k - E_h)),
+//   K[(h, k), j] = delta ? cdelta beta w_h : (cnum w_h + cwk w_k) / (s_j - sgn (E_k - E_h)),
 // delta = |s_j - sgn (E_k - E_h)| <= PoleResolution (FP64, the reference's
 // rule for resonant terms).  K is formed once per tile element and used by
 // every row of the tile; the rows of a T1 class are all (z1, z3) groups, those
@@ -147,7 +152,7 @@ __global__ void __launch_bounds__(CG_THREADS, 3)
     // them and stores the tiles after the products, so the loads' latency is
     // covered by the inner loop instead of stalling ahead of it.
     cd rx[LA], ry[LA];
-    double rek[LB];
+    double rek[LB], rwk[LB];
     double r_eh = 0.0, r_w = 0.0;
     auto fetch = [&](long q) {
         const int h = it.h0 + (int)(q / ktiles), k0 = (int)(q % ktiles) * CG_BK;
@@ -172,12 +177,16 @@ __global__ void __launch_bounds__(CG_THREADS, 3)
 #pragma unroll
         for (int u = 0; u < LB; ++u) {
             const int l = tid + u * NT;
-            double ek = 0.0;
+            double ek = 0.0, wk = 0.0;
             if (l < BN * CG_BK) {
                 const int k = k0 + l / BN;
-                if (k < nk) ek = d.Ek[k];
+                if (k < nk) {
+                    ek = d.Ek[k];
+                    if (d.wk) wk = d.wk[k];
+                }
             }
             rek[u] = ek;
+            rwk[u] = d.cwk * wk;
         }
     };
     auto finish = [&](long q, int buf) {
@@ -201,7 +210,7 @@ __global__ void __launch_bounds__(CG_THREADS, 3)
                     if (d.use_delta && m2 <= tol2) {
                         v = cd{cdl, 0.0};
                     } else {
-                        const double rr = cw * recip_pos(m2);
+                        const double rr = (cw + rwk[u]) * recip_pos(m2);
                         v = cd{dx * rr, -sv.y * rr};
                     }
                 }
@@ -470,15 +479,18 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
                 push(list, digs, anchor_block, prob);
             }
         };
+        // T3a and T3b, T4a and T4b as one term each (split products keep them
+        // apart: their digits follow the weights of one block)
+        const bool all13 = !split && r1 == d1 && r3 == d3, all24 = !split && r2 == d2 && r4 == d4;
         // anchored products, one item per z1 (or z3)
         // outputs that the contractions read along k are stored k-contiguous
         if (r2) push(pa, pa_d, S2, gp<T, DT>(X4, d1, 1, O1, d2, 1, pool + w.Lc, 1, d4, r2, d1, nullptr, H2, A1, N1,
                                        (long)r2 * d4, d4));                               // Lc = X4 A1[:,H2]: [(i1,h)][k]
-        if (r4) push(pa, pa_d, S4, gp<T, DT>(X4, d1, 1, O1, d2, 1, pool + w.Lr, d2, r4, d2, d1, H4, nullptr, A1, N1,
+        if (r4 && !all24) push(pa, pa_d, S4, gp<T, DT>(X4, d1, 1, O1, d2, 1, pool + w.Lr, d2, r4, d2, d1, H4, nullptr, A1, N1,
                                        (long)r4 * d2));                                   // Lr = X4[H4,:] A1
         if (r1) push(pb, pb_d, S1, gp<DT, T>(O1, d2, 1, O2, d3, 1, pool + w.Pr, d3, r1, d3, d2, H1, nullptr, A1, N1,
                                        (long)r1 * d3));                                   // Pr = A1[H1,:] O2
-        if (r3) push(pb, pb_d, S3, gp<DT, T>(O1, d2, 1, O2, d3, 1, pool + w.Pc, 1, d1, r3, d2, nullptr, H3, A1, N1,
+        if (r3 && !all13) push(pb, pb_d, S3, gp<DT, T>(O1, d2, 1, O2, d3, 1, pool + w.Pc, 1, d1, r3, d2, nullptr, H3, A1, N1,
                                        (long)d1 * r3, d1));                               // Pc = A1 O2[:,H3]: [i1][h][k]
         if (r3) over_items(pb, pb_d, S3, gp<DT, T>(O3, d4, 1, X4, d1, 1, pool + w.Rho, d1, r3, d1, d4, H3, nullptr, C3, N3,
                                              (long)r3 * d1), GEMM_CONJ);                   // rho = C3[H3,:] X4
@@ -587,6 +599,7 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
         const int S[4] = {g.block[0], g.block[1], g.block[2], g.block[3]};
         const int d1 = P.dims[S[0]], d2 = P.dims[S[1]], d3 = P.dims[S[2]], d4 = P.dims[S[3]];
         const int r1 = rs[q][0], r2 = rs[q][1], r3 = rs[q][2], r4 = rs[q][3];
+        const bool all13 = !split && r1 == d1 && r3 == d3, all24 = !split && r2 == d2 && r4 == d4;
         const long N1 = (long)pl.Z1.size(), N3 = (long)pl.Z3.size();
         const Operator &o2 = P.ops[g.op[1]], &o4 = P.ops[g.op[3]];
         const T* O2 = o2.mat.as<T>() + o2.parts[o2.by_left[S[1]]].off;
@@ -628,6 +641,10 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
             DTerm e = base(1, r2, d4, 3, +1.0, 3, 1, -1.0, 1.0, sign);
             e.VA = pool + w.Rr; e.va_cplx = 1; e.a3 = (long)r2 * d4; e.ah = d4; e.ak = 1;
             e.VB = pool + w.Lc; e.vb_cplx = 1; e.bk = 1; e.b1 = (long)r2 * d4; e.bh = d4;
+            if (all24) {
+                e.wk = W[3];
+                e.cwk = -1.0;
+            }
             dt.push_back(e);
         }
         if (r3) {  // T1b: va = O2[k,h] (state h), vb = V1b[i1][(i3,h)][k]
@@ -639,7 +656,7 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
             DTerm e = base(2, r3, d1, 0, -1.0, 2, 1, 0.0, 1.0, sign);
             e.VA = pool + w.Pc; e.va_cplx = 1; e.a1 = (long)d1 * r3; e.ak = 1; e.ah = d1;
             e.VB = pool + w.Rho; e.vb_cplx = 1; e.b3 = (long)r3 * d1; e.bh = d1; e.bk = 1;
-            dt.push_back(e);
+            if (!all13) dt.push_back(e);
         }
         if (r1) {  // T2a: va = X4[k,h] (state h), vb = V2a[i3][(i1,h)][k]
             DTerm d = base(0, r1, d4, 3, +1.0, 1, 0, 0.0, 1.0, sign);
@@ -650,6 +667,10 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
             DTerm e = base(0, r1, d3, 2, +1.0, 2, 1, 1.0, -1.0, sign);
             e.VA = pool + w.Pr; e.va_cplx = 1; e.a1 = (long)r1 * d3; e.ah = d3; e.ak = 1;
             e.VB = pool + w.Qc; e.vb_cplx = 1; e.b3 = (long)d3 * r1; e.bk = 1; e.bh = d3;
+            if (all13) {
+                e.wk = W[2];
+                e.cwk = 1.0;
+            }
             dt.push_back(e);
         }
         if (r4) {  // T2b: va = X4[h,k] (state h), vb = V2b[i1][(i3,h)][k]
@@ -661,7 +682,7 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
             DTerm e = base(3, r4, d2, 1, -1.0, 3, 1, 0.0, -1.0, sign);
             e.VA = pool + w.Rc; e.va_cplx = 1; e.ak = 1; e.a3 = (long)r4 * d2; e.ah = d2;
             e.VB = pool + w.Lr; e.vb_cplx = 1; e.b1 = (long)r4 * d2; e.bh = d2; e.bk = 1;
-            dt.push_back(e);
+            if (!all24) dt.push_back(e);
         }
     }
     if (!dt.empty()) {
@@ -763,7 +784,7 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
 // anchor, than part by part in full matrices (pgx_g2.cu).  That form has two
 // products per pair (z1', z3') that occurs and two per z1' and z3', this one
 // four per pair of the (z1', z3') plane (z1' taken up to conjugation for a real
-// Hamiltonian) and four per z1' and z3', about 15% slower each for the
+// Hamiltonian), two per z1' and four per z3', about 15% slower each for the
 // dressing; but that form spends some 0.25 ms per part, worth
 // 5e9 operations, on its own launches and waits.  Plaquette (96 parts, 8^3):
 // 13.2 ms there, 2.0 here; 6-site ring (216 parts, blocks to 400) 9^3: 203,
@@ -791,7 +812,7 @@ static bool anchored_faster(const Problem& P, int nparts, const pgx_g2_part* par
         const double there = 8.0 * std::min((double)nfreq, all[a] * all[b]) * (m3 + m4) +
                              4.0 * (all[a] * (m1 + m2) + all[b] * (m3 + m4));
         const double z3 = pt.npts > pt.ncls ? 0.5 * closed[b] : closed[b];  // conjugate z3 share their products
-        const double here = 8.0 * up[a] * z3 * (m1 + m2 + m3 + m4) + 8.0 * (up[a] * (m1 + m2) + z3 * (m3 + m4));
+        const double here = 8.0 * up[a] * z3 * (m1 + m2 + m3 + m4) + 4.0 * up[a] * (m1 + m2) + 8.0 * z3 * (m3 + m4);
         extra += 1.15 * here - there;
     }
     return extra <= 5e9 * nparts;

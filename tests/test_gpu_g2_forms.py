@@ -124,6 +124,34 @@ def test_rule_of_the_exact_sum():
             assert np.abs(v - full).max() < 1e-12 * np.abs(full).max()
 
 
+# Nearly equal levels at zero bosonic transfer: (w3 - w1)/D is of the order of
+# beta w however small D is, and both forms take it from the same weights and
+# energies, so they differ by the rounding of the products around it only.  A
+# form that divides w3 and w1 by D apart enlarges that rounding by 1 / (beta D).
+@pytest.mark.parametrize("kind", ["real", "complex"])
+@pytest.mark.parametrize("split", [1e-7, 1e-6, 1e-5])
+def test_nearly_equal_levels(split, kind):
+    from pomerol_b200.pgx import PGX_G2_EXACT, PGX_G2_FULL_MATRICES
+    from tests.pgx_harness import GpuED
+    if kind == "real":
+        e = M.plaquette()
+    else:
+        e = M.CoulombS("A", 2.0, -1.2) + M.CoulombS("B", 2.5, -0.9) + M.CoulombS("C", 1.5, -0.8)
+        for a, b, t in (("A", "B", 0.7 * np.exp(0.4j)), ("B", "C", 0.5j), ("C", "A", -0.6)):
+            for s in (M.UP, M.DOWN):
+                e += M.HoppingS(a, b, t, 0, 0, s, s)
+    e += M.Level1("A", split, 0, M.DOWN)
+    m = M.make_model(e)
+    g = GpuED(m, 10.0)
+    u, d = m.info.getIndex("A", 0, 1), m.info.getIndex("A", 0, 0)
+    fz = L.fermionic(np.array([(a, b, x) for a in range(-2, 2) for b in range(-2, 2) for x in range(-2, 2)]), 10.0)
+    parts = g.g2_parts(g.c(u), g.c(d), g.cdag(u), g.cdag(d))
+    full = g.eng.g2(parts, fz, flags=PGX_G2_FULL_MATRICES)
+    exact, b = batched(g.eng, parts, fz, flags=PGX_G2_EXACT)
+    assert b
+    assert np.abs(exact - full).max() < 1e-13 * np.abs(full).max()
+
+
 @pytest.mark.parametrize("kind", ["real", "complex"])
 def test_negative_pole_resolution(kind):
     """|D| <= pole_res holds nowhere then, also for bosonic sums nearer to a pole
