@@ -8,7 +8,7 @@
 #include <cmath>
 #include <cstring>
 #include <iterator>
-#include <limits>
+#include <map>
 #include <tuple>
 #include <unordered_map>
 #include <utility>
@@ -118,9 +118,9 @@ inline void build_points(Points& pt, int nfreq, const double* z, bool real) {
 // z3' in order of first appearance, and each point's index into them.  Per
 // point also the numbers of the four frequency sums the contractions use: z2',
 // z1'+z2'+z3', z1'+z2', z2'+z3', where (z1', z2', z3') is the permuted (z1, z2,
-// -z3), z1' dressing O1 and z3' dressing O3.  Sums equal up to rounding (2^-46
-// of what they were added up from) have one number; finite numbers ascend with
-// the values.
+// -z3), z1' dressing O1 and z3' dressing O3.  Sums equal up to rounding have one
+// number; the values of z2' are the caller's and keep theirs.  Numbers ascend
+// with order_values's order.
 struct PermIndex {
     std::vector<int> pts;
     std::vector<cd> Z1, Z3;
@@ -153,32 +153,60 @@ inline void number_pairs(const std::vector<int>& pts, const std::vector<int>& xi
     }
 }
 
-// Merges the numbers of values equal up to rounding and orders them.  Values in
-// one cell of 2^-46 of the largest are candidates; they are one number where
-// they differ by no more than 2^-46 of their own size, so a far value in the
-// list does not join others.
-inline void order_values(const std::vector<int>& pts, std::vector<int>& id, std::vector<cd>& val, std::vector<double>& size) {
-    double big = 0.0;
-    for (const cd& v : val)
-        if (std::isfinite(v.x) && std::isfinite(v.y)) big = std::max(big, largest_part(v));
-    const double q = big > 0.0 ? std::ldexp(big, -46) : 1.0;
-    auto cell = [&](double x) { return std::isfinite(x) ? std::llround(x / q) : std::numeric_limits<long long>::max(); };
-    std::vector<std::tuple<long long, long long, int>> key;
-    for (size_t i = 0; i < val.size(); ++i) key.emplace_back(cell(val[i].x), cell(val[i].y), (int)i);
+// Orders the numbers by value and merges those of sums equal up to rounding: of
+// values no further apart than `ulps` units in the last place of what the
+// larger-sized one was added up from, that one takes the number of the
+// smaller-sized, which is the more accurate.  So no sum moves by more than its
+// own rounding, whatever else the list holds.  Undefined and infinite values
+// are merged with none.  The order is that of x + c y: two values close in both
+// parts are close in it, and others seldom are (on the axis it is that of y).
+inline void order_values(const std::vector<int>& pts, std::vector<int>& id, std::vector<cd>& val,
+                         std::vector<double>& size, int ulps) {
+    const int n = (int)val.size();
+    std::vector<std::pair<double, int>> key;  // finite values in order
+    std::vector<int> rep(n), to(n), run;
+    double most = 0.0;
+    for (int i = 0; i < n; ++i) {
+        rep[i] = i;
+        const double k = val[i].x + 0.6180339887498949 * val[i].y;
+        if (!std::isfinite(k)) continue;
+        key.emplace_back(k, i);
+        most = std::max(most, size[i]);
+    }
     std::sort(key.begin(), key.end());
-    std::vector<int> to(val.size());
+    const double unit = ulps * std::ldexp(1.0, -52), reach = 2.0 * unit * most;
+    for (size_t a = 0, b; ulps > 0 && a < key.size(); a = b) {
+        for (b = a + 1; b < key.size() && key[b].first - key[b - 1].first <= reach; ++b) {}
+        if (b - a < 2) continue;  // merges are within runs of such neighbours
+        run.clear();
+        for (size_t q = a; q < b; ++q) run.push_back((int)q);
+        std::sort(run.begin(), run.end(),
+                  [&](int p, int q) { return std::tie(size[key[p].second], p) < std::tie(size[key[q].second], q); });
+        std::multimap<double, int> stand;  // values that keep their number
+        for (int q : run) {
+            const int i = key[q].second;
+            const double tol = unit * size[i], at = key[q].first;
+            auto it = stand.lower_bound(at - 2.0 * tol);
+            for (; it != stand.end() && it->first <= at + 2.0 * tol; ++it) {
+                const cd v = val[it->second];
+                if (std::fabs(v.x - val[i].x) <= tol && std::fabs(v.y - val[i].y) <= tol) break;
+            }
+            if (it != stand.end() && it->first <= at + 2.0 * tol) rep[i] = it->second;
+            else stand.emplace(at, i);
+        }
+    }
     std::vector<cd> out;
     std::vector<double> osize;
-    for (size_t i = 0; i < key.size(); ++i) {
-        const int e = std::get<2>(key[i]);
-        bool same = i > 0 && std::get<0>(key[i]) == std::get<0>(key[i - 1]) && std::get<1>(key[i]) == std::get<1>(key[i - 1]);
-        if (same) same = largest_part(cd{val[e].x - out.back().x, val[e].y - out.back().y}) <=
-                         std::ldexp(std::max(size[e], osize.back()), -46);
-        if (!same) {
-            out.push_back(val[e]);
-            osize.push_back(size[e]);
-        }
-        to[e] = (int)out.size() - 1;
+    auto keep = [&](int i) {
+        to[i] = (int)out.size();
+        out.push_back(val[i]);
+        osize.push_back(size[i]);
+    };
+    for (const auto& k : key)
+        if (rep[k.second] == k.second) keep(k.second);
+    for (int i = 0; i < n; ++i) {
+        if (!std::isfinite(val[i].x + 0.6180339887498949 * val[i].y)) keep(i);
+        else to[i] = to[rep[i]];
     }
     for (int e : pts) id[e] = to[id[e]];
     val = std::move(out);
@@ -226,7 +254,10 @@ inline void number_sums(PermIndex& ix) {
     const std::vector<cd> Z2 = ix.sval[0];
     for (auto& v : ix.sid) v.resize(j2.size());
     for (const cd& v : Z2) ix.size[0].push_back(largest_part(v));
-    auto order = [&](int k) { order_values(ix.pts, ix.sid[k], ix.sval[k], ix.size[k]); };
+    // An odd multiple of pi / beta, a product and a quotient, is off by up to one
+    // unit, a sum of two by three, of three by five and a half.  Eight units apart
+    // join all but the rarest of equal sums (apart they cost a column each).
+    auto order = [&](int k) { order_values(ix.pts, ix.sid[k], ix.sval[k], ix.size[k], k == 0 ? 0 : 8); };
     order(0);
     number_pairs(ix.pts, ix.j1, ix.Z1, j2, Z2, nullptr, ix.sid[2], ix.sval[2], ix.size[2]);
     order(2);

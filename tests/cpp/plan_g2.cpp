@@ -87,7 +87,7 @@ static void check(const std::vector<double>& z, bool real, int tiles1, int tiles
                                 double size = std::max(std::fabs(b.x), std::fabs(b.y));
                                 if (k == 1 || k == 2) size = std::max(size, std::max(std::fabs(a.x), std::fabs(a.y)));
                                 if (k == 1 || k == 3) size = std::max(size, std::max(std::fabs(d.x), std::fabs(d.y)));
-                                const double tol = std::ldexp(size, -45);
+                                const double tol = k == 0 ? 0.0 : std::ldexp(size, -48);  // two merges of eight units
                                 EXPECT(std::fabs(s.x - sum.x) <= tol && std::fabs(s.y - sum.y) <= tol);
                             }
                     }
@@ -126,6 +126,58 @@ int main() {
                     for (bool real : {true, false})
                         for (int tiles : {1, 3}) check(y, real, tiles, tiles == 1 ? 1 : 2);
                 }
+    }
+    // neighbours of one frequency a few units apart; large opposite addends with
+    // small sums; magnitudes far apart: no sum moves by more than its own rounding
+    for (int form = 0; form < 4; ++form) {
+        std::vector<double> z;
+        auto value = [&](int k, int i) {
+            if (form == 0) return cd{0.0, (2 * i + 1) * (1.0 + (k == 1 ? i * 3e-16 : 0.0)) * (k == 1 ? 1.0 : 3.0)};
+            if (form == 1) return cd{0.25 * i, k == 0 ? 1e14 + i : k == 1 ? -1e14 + 3 * i : 1.0 + i};
+            if (form == 2) return cd{0.0, (k == 2 ? 1e-3 : 1.0) * std::ldexp(2 * i + 1.0, 12 * (i % 4))};
+            return cd{0.1 * i, 0.05};  // a line above the real axis
+        };
+        for (int a = 0; a < 6; ++a)
+            for (int b = 0; b < 6; ++b)
+                for (int c = 0; c < 6; ++c)
+                    for (const cd& v : {value(0, a), value(1, b), value(2, c)}) {
+                        z.push_back(v.x);
+                        z.push_back(v.y);
+                    }
+        for (bool real : {true, false}) check(z, real, 1, 1);
+    }
+    // on Matsubara grids every equal sum has one number
+    for (double beta : {1.0, 7.0, 10.0, 33.3, 1e3}) {
+        const double pi = 3.14159265358979323846;
+        for (int reach : {8, 40, 600}) {
+            std::vector<double> z;
+            std::vector<int> step;
+            for (int i = 0; i < 16; ++i) step.push_back(reach <= 8 ? i - 8 : (i - 8) * reach / 8 + i % 3);
+            for (int a : step)
+                for (int b : step)
+                    for (int c : step)
+                        for (int n : {a, b, c}) {
+                            z.push_back(0.0);
+                            z.push_back(pi * (2 * n + 1) / beta);
+                        }
+            std::set<int> pairs, differences, all;
+            for (int a : step)
+                for (int b : step) {
+                    pairs.insert(a + b + 1);
+                    differences.insert(b - a);
+                    for (int c : step) all.insert(a + b - c);
+                }
+            Points pt;
+            build_points(pt, (int)z.size() / 6, z.data(), false);
+            const int perm[3] = {0, 1, 2};
+            PermIndex ix;
+            index_perm(ix, perm, pt);
+            number_sums(ix);
+            EXPECT(ix.sval[0].size() == step.size());
+            EXPECT(ix.sval[1].size() == all.size());
+            EXPECT(ix.sval[2].size() == pairs.size());
+            EXPECT(ix.sval[3].size() == differences.size());
+        }
     }
     std::printf("%d failures\n", bad);
     return bad != 0;

@@ -153,6 +153,26 @@ def test_nearly_equal_levels(split, kind):
 
 
 @pytest.mark.parametrize("kind", ["real", "complex"])
+def test_neighbouring_frequencies_keep_their_own_values(kind):
+    """z2 a few units apart, 1e-9 from a pole, where 40 units are 1e-6 of the sum or more:
+    each triple's value is that of a call of its own.  A difference z - E is the
+    same number in both calls, so the values agree to rounding."""
+    from pomerol_b200.pgx import PGX_G2_ANCHORED, PGX_G2_EXACT
+    g, u, d = solved(kind)
+    parts = g.g2_parts(g.c(u), g.c(d), g.cdag(u), g.cdag(d))
+    ops, b, _, _ = next(p for p in parts if p[2] == (0, 1, 2) and min(len(g.E[x]) for x in p[1]) > 2)
+    left = [l for _, l in g.eng.op_info(ops[1])].index(b[1])
+    i, j = np.unravel_index(np.abs(g.eng.op_read(ops[1], left)).argmax(), (len(g.E[b[1]]), len(g.E[b[2]])))
+    pole = g.E[b[2]][j] - g.E[b[1]][i]
+    z = np.array([(0.7j, pole + 1e-9 + k * 40 * np.spacing(abs(pole)), 0.3 - 1.1j) for k in range(8)])
+    for flags in (PGX_G2_EXACT, PGX_G2_ANCHORED):
+        v = g.eng.g2(parts, z, coef_tol=0.0, flags=flags)
+        one = np.array([g.eng.g2(parts, t[None], coef_tol=0.0, flags=flags)[0] for t in z])
+        assert np.abs(np.diff(one)).max() > 1e-7 * np.abs(one).max()  # the pole is felt
+        assert np.all(np.abs(v - one) < 1e-9 * np.abs(one))
+
+
+@pytest.mark.parametrize("kind", ["real", "complex"])
 def test_negative_pole_resolution(kind):
     """|D| <= pole_res holds nowhere then, also for bosonic sums nearer to a pole
     than its modulus."""
