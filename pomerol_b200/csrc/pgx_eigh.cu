@@ -1491,8 +1491,6 @@ __global__ void __launch_bounds__(TRI_THREADS) vector_kernel(TriArgs g) {
     }
 }
 
-// Modified Gram-Schmidt, applied twice, of each chain member against the
-// earlier members closer than CHAIN_TOL ||T||; one thread per chain head.
 // The CTA's warp orthogonalises each chain whose head lies in its range:
 // modified Gram-Schmidt (two passes) of every member against its close
 // predecessors, the dot products and updates spread over the lanes (a chain
@@ -1656,7 +1654,7 @@ constexpr size_t CL_SMEM_MAX = 226 * 1024;  // dynamic shared memory per CTA (th
 // The cluster class of an n x n block, or -1 (the block then takes the
 // large-block path): the smallest cluster whose shared memory holds the
 // block.  16 CTAs (a non-portable cluster size) only where 8 do not suffice
-// (449 to 513 states): at 400 states the per-step cost is set by the cluster
+// (453 to 513 states): at 400 states the per-step cost is set by the cluster
 // barriers, and 16-CTA clusters were measured slower than 8-CTA ones there.
 static int cluster_class(int n) {
     if (n > CL_MAX_DIM) return -1;
@@ -1730,7 +1728,7 @@ size_t eigh_vec_scratch_doubles(const std::vector<int>& dims) {
 
 
 // Householder stage plan: the block list of each cluster size (largest
-// blocks first) and the blocks left to the single-CTA global-memory kernel.
+// blocks first) and the blocks left to the large-block path.
 struct HhPlan {
     std::vector<int> cls[CL_NCLS];
     std::vector<int> global;
@@ -2093,7 +2091,7 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
         }
     };
     // the launches are independent: with side streams, cluster class q > 0 runs
-    // on aux[q - 1] while the main stream runs the global-memory kernel and class 0
+    // on aux[q - 1] while the main stream runs the large blocks and class 0
     const bool fork = d.aux[0] && d.aux[1] && d.aux[2] && d.aux[3] && d.fork;
     if (fork) {
         PGX_CUDA(cudaEventRecord(d.fork, st));
