@@ -1663,6 +1663,10 @@ static int cluster_class(int n) {
     return -1;
 }
 
+// Whether a block may take the large-block path: beyond the clusters, or of a
+// size that needs 16 CTAs, which not every device can schedule.
+static bool maybe_big(int n) { return cluster_class(n) < 0 || CL_SIZES[cluster_class(n)] > 8; }
+
 // Back-transformation plan: the T factors' items (one per panel), then the
 // column slabs of each class, largest blocks first.  first[q] is where list q
 // starts (0: T factors, 1 + c: class c), first[BT_NCLS + 1] the total; nmax[c]
@@ -1721,7 +1725,7 @@ size_t eigh_vec_scratch_doubles(const std::vector<int>& dims) {
         // the vectors' scratch, later the T factors
         s += std::max(4 * (size_t)n * TRI_THREADS * ((n + TRI_THREADS - 1) / TRI_THREADS),
                       (size_t)bt_panels(n) * BT_NB * BT_NB);
-        if (cluster_class(n) < 0) big += (size_t)bhh_scratch_doubles(n);
+        if (maybe_big(n)) big += (size_t)bhh_scratch_doubles(n);
     }
     return std::max<size_t>(std::max(s, big), 1);
 }
@@ -1747,11 +1751,11 @@ static HhPlan hh_plan(const std::vector<int>& dims) {
     return h;
 }
 
-// the large blocks (beyond the cluster path), largest first
+// the blocks that may take the large-block path, largest first
 static std::vector<int> big_blocks(const std::vector<int>& dims) {
     std::vector<int> big;
     for (size_t b = 0; b < dims.size(); ++b)
-        if (cluster_class(dims[b]) < 0) big.push_back((int)b);
+        if (maybe_big(dims[b])) big.push_back((int)b);
     std::stable_sort(big.begin(), big.end(), [&](int x, int y) { return dims[x] > dims[y]; });
     return big;
 }
@@ -2005,7 +2009,8 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
     tri_plan(dims, items, &n_vec);
     const size_t n_bis = items.size() - n_vec;
     HhPlan hp = hh_plan(dims);
-    // a cluster size the device cannot schedule falls back to the global-memory kernel
+    // blocks of a 16-CTA cluster take the large-block path where the device
+    // cannot schedule one (a partition of a GPU, say)
     ClusterArgs ca;
     ca.dims = d.dims;
     ca.moff = d.moff;
@@ -2033,13 +2038,9 @@ void launch_eigh_raw(const EighDev& d, const std::vector<int>& dims, const std::
         int nclusters = 0;
         if (cudaOccupancyMaxActiveClusters(&nclusters, eigh_cluster_kernel, &cfg) != cudaSuccess || nclusters < 1) {
             cudaGetLastError();
-            // 16-CTA clusters not schedulable: their blocks go to 8-CTA clusters where they fit
-            bool moved = q == 4;
-            for (int b : hp.cls[q])
-                moved = moved && cluster_smem_doubles(dims[b], 8) * sizeof(double) <= CL_SMEM_MAX;
-            PGX_CHECK(moved, PGX_ERR_CUDA, "the eigensolver's thread-block clusters cannot be scheduled on this device");
-            hp.cls[3].insert(hp.cls[3].end(), hp.cls[q].begin(), hp.cls[q].end());
-            std::stable_sort(hp.cls[3].begin(), hp.cls[3].end(), [&](int x, int y) { return dims[x] > dims[y]; });
+            PGX_CHECK(CL_SIZES[q] > 8, PGX_ERR_CUDA,
+                      "the eigensolver's thread-block clusters cannot be scheduled on this device");
+            hp.global.insert(hp.global.end(), hp.cls[q].begin(), hp.cls[q].end());  // smaller than those there
             hp.cls[q].clear();
             cl_smem[q] = 0;
         }
