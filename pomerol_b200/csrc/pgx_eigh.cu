@@ -79,7 +79,7 @@ struct BigArgs {
 
 // Scratch of one large block, in doubles: V and W (BHH_NB columns of n each),
 // y (n), tau (n), then per panel its Gram matrix and -T (BHH_NB^2 each), the
-// slots of y and the tiles' parts of v . y (bhh_symv_tri_kernel), and the dots of
+// slots of y and the tiles' parts of v . (tau y) (bhh_symv_tri_kernel), and the dots of
 // the panel's columns with the reflector (2 BHH_NB).
 constexpr int TRI_T = 128;  // rows and columns of a tile there
 __host__ __device__ inline long bhh_slots(int m) { return (m + TRI_T - 1) / TRI_T; }
@@ -97,8 +97,9 @@ __host__ __device__ inline long bhh_dots_at(int n) { return bhh_scratch_doubles(
 // to date; grid (row groups, block).  The column stays raw in V: the product
 // kernel reflects it, and leaves tau and the reflector's leading entry v0 (in
 // y[fin]), which takes its place in V here.  Every CTA finds w . v for itself,
-//   w . v = tau (v . y - 2 sum_s (V_s . v)(W_s . v)),
-// so CTAs need nothing of one another.  Both vectors need every row's
+//   w . v = v . (tau y) - 2 sum_s (V_s . v) (tau (W_s . v)),
+// so CTAs need nothing of one another; tau enters each product first, as without
+// it they grow with the cube of the matrix's scale.  Both vectors need every row's
 // combination of the panel's earlier V and W columns: one sweep reads them for
 // both (four lanes a row, each a quarter of the columns), the first eight rows
 // of a warp ahead of the block sum.  What bounds it: the latency of one round
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(BHH_COL_THREADS, SLOTS ? 1 : 2) bhh_col_kernel
         if constexpr (SLOTS)
             for (int t = tid; t < ns * (ns + 1) / 2; t += BHH_COL_THREADS) vy += parts[t];
         else
-            for (int r = lo + 1 + tid; r < n; r += BHH_COL_THREADS) vy = fma(vf[r], y[r], vy);
+            for (int r = lo + 1 + tid; r < n; r += BHH_COL_THREADS) vy = fma(vf[r], tf * y[r], vy);
         if (tid < BHH_NB) {
             double a = 0.0, b = 0.0, c = 0.0, d = 0.0;
             if (tid < cf) {
@@ -177,12 +178,12 @@ __global__ void __launch_bounds__(BHH_COL_THREADS, SLOTS ? 1 : 2) bhh_col_kernel
             jv[tid] = d;
             double yl = !SLOTS && tid == 0 ? y[lo] : 0.0;
             for (int t = tid; t < ns; t += 32) yl += slot[(long)t * n + lo];
-            const double dd = warp_sum(a * b), dj = warp_sum(d * a + c * b);
+            const double dd = warp_sum(a * tf * b), dj = warp_sum(d * a + c * b);
             yl = warp_sum(yl);
             if (tid == 0) {
                 s_dd = dd;
                 s_yj = yl - dj;
-                if (!SLOTS) vy = fma(v0, yl, vy);
+                if (!SLOTS) vy = fma(v0, tf * yl, vy);
             }
         }
         vy = warp_sum(vy);
@@ -191,7 +192,7 @@ __global__ void __launch_bounds__(BHH_COL_THREADS, SLOTS ? 1 : 2) bhh_col_kernel
         double t = 0.0;
 #pragma unroll
         for (int q = 0; q < BHH_COL_THREADS / 32; ++q) t += red[q];
-        K = 0.5 * tf * (tf * (t - 2.0 * s_dd));
+        K = 0.5 * tf * (t - 2.0 * s_dd);
         wj = tf * s_yj - K * v0;
     }
     const double st = sqrt(tf);
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(BHH_SYMV_THREADS, RW == 4 ? 10 : 6) bhh_symv_k
 // A_ij^T v_i.  CTA (tile, block): a warp 16 rows, a lane 4 columns of the tile, 16
 // loads in flight; the products of rows of tile row R go to slot tj of y,
 // those of its columns to slot ti, so every row finds its parts in slots 0 ..
-// and nothing is added up in memory; the tile's part of v . y goes beside them.
+// and nothing is added up in memory; the tile's part of v . (tau y) goes beside them.
 // CTAs past the tiles take the dots, a row per warp.  Every CTA sums the
 // column's squares itself.  What bounds it: reading the triangle from HBM, at
 // half the copy rate, as a CTA's column sums and exchanges stand between its
@@ -446,7 +447,7 @@ __global__ void __launch_bounds__(SYT_THREADS, 3) bhh_symv_tri_kernel(BigArgs g)
     double* slot = V + bhh_slots_at(n);
     const int row = 16 * wid + (lane >> 1);
     if (!(lane & 1) && i0 + row < m) slot[(long)ct * n + j + 1 + i0 + row] = ys;
-    const double part = warp_sum(lane & 1 ? 0.0 : ys * vi[row]);
+    const double part = warp_sum(lane & 1 ? 0.0 : tj * ys * vi[row]);
     if (ct != ti)
 #pragma unroll
         for (int q = 0; q < 4; ++q) cols[wid][lane + 32 * q] = c[q];

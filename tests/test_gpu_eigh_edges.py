@@ -44,6 +44,19 @@ def test_eigenvalues_at_every_lane_count(n, count):
         assert np.abs(w - ref).max() < 10 * (n + 10) * EPS * np.abs(ref).max()
 
 
+# The reduction's products grow with the square of the matrix, which stays in
+# range between 1e-135 and 1e150; its third power does not.
+@pytest.mark.parametrize("scale", [1e-130, 1e-105, 1e120, 1e150])
+@pytest.mark.parametrize("dims", [[600, 520, 200, 40], [1130] * 10])
+def test_matrices_of_any_scale(dims, scale):
+    rng = np.random.default_rng(sum(dims))
+    H = [symmetric(rng, n) for n in dims]
+    e = engine([h * scale for h in H])
+    e.eigh()
+    E, U = e.eigensystem()
+    check(H, [w / scale for w in E], U)
+
+
 # above 513 states, and above 100 MB of matrices (one triangle read) down to below it
 @pytest.mark.parametrize("dims", [[600, 520, 40], [1130] * 10])
 def test_captured_large_blocks(dims):
