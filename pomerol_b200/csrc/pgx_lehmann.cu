@@ -307,10 +307,14 @@ __global__ void __launch_bounds__(EVAL_THREADS) pair_eval_kernel(const cd* __res
 #pragma unroll
     for (int u = 0; u < EVAL_ZPT; ++u) {
         // R (-P - iy): real part -R_re P + y R_im, imaginary part -R_im P - y R_re
-        cd v{ox[u] - acc[u][1], oy[u] - zy[u] * acc[u][0]};
-        if constexpr (CX) {
-            v.x = fma(zy[u], acc[u][2], v.x);
-            v.y -= acc[u][3];
+        cd v{ox[u], oy[u]};
+        if (axis) {  // else no shared sums, and an infinite y would make them undefined
+            v.x -= acc[u][1];
+            v.y -= zy[u] * acc[u][0];
+            if constexpr (CX) {
+                v.x = fma(zy[u], acc[u][2], v.x);
+                v.y -= acc[u][3];
+            }
         }
         sR[tid] = v;
         __syncthreads();
