@@ -90,7 +90,7 @@ struct CItem {
     int cls, row0, h0, h1;
 };
 
-constexpr int CG_THREADS = 128;
+constexpr int CG_THREADS = 128, CG_BK_MAX = 16;  // the latter: k's of a tile
 // of its four warps, how many split the rows; the others split the k's of a tile
 __host__ __device__ constexpr int cg_wr(int bm) { return bm >= 32 ? 4 : bm == 16 ? 2 : 1; }
 
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(CG_THREADS, 3)
     constexpr int WR = cg_wr(BM), WK = 4 / WR, FM = BM / 8 / WR, FN = BN / 8;
     static_assert(FM * 8 * WR == BM && FN * 8 == BN, "tile shape does not fit the warps");
     // k-tile depth: two buffers within 48 KB
-    constexpr int CG_BK = BM >= 64 ? 8 : 16;
+    constexpr int CG_BK = BM >= 64 ? CG_BK_MAX / 2 : CG_BK_MAX;
     constexpr int LA = (BM * CG_BK + NT - 1) / NT, LB = (BN * CG_BK + NT - 1) / NT;
     __shared__ __align__(16) cd As[2][CG_BK][BM + 2];
     __shared__ __align__(16) cd Bs[2][CG_BK][BN + 2];
@@ -686,10 +686,11 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
         }
     }
     if (!dt.empty()) {
-        // classes of every sub-term, grouped by tile shape (BM 32 or 64 rows,
-        // BN 8 / 16 / 24 / 32 columns); a work item is one row tile of a class
+        // classes of every sub-term, grouped by tile shape (BM 8, 16, 24, 32 or
+        // 64 rows, BN 8 / 16 / 24 / 32 columns); a work item is one row tile of a class
         // over a range of anchors: as many multiply-adds as give each SM 32
-        // items, between 2^16 (less is lost in an item's start and its sums'
+        // items (one triple of a chain of 300, 2, 310 and 1 states: 60 us in the
+        // kernel, 228 with anchors counted by their true k's), between 2^16 (less is lost in an item's start and its sums'
         // atomics) and 2^22
         std::vector<CClass> cls[CG_NBM][CG_NBN];
         std::vector<CItem> its[CG_NBM][CG_NBN];
@@ -710,7 +711,9 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
                 c.term = (int)q;
                 const int ci = (int)cls[bm][bn].size();
                 cls[bm][bn].push_back(c);
-                const int hc = (int)std::max<long>(1, item / ((long)BM * BN * std::max(d.nk, 1)));
+                // k's of a whole tile: where there are few of them, an item's
+                // steps are one after another for every anchor
+                const int hc = (int)std::max<long>(1, item / ((long)BM * BN * (ceil_div(d.nk, CG_BK_MAX) * CG_BK_MAX)));
                 for (int r0 = 0; r0 < c.nrows; r0 += BM)
                     for (int h0 = 0; h0 < d.nh; h0 += hc) its[bm][bn].push_back(CItem{ci, r0, h0, std::min(d.nh, h0 + hc)});
                 macs[bm][bn] += (double)c.nrows * c.ncols * d.nh * d.nk;
@@ -785,11 +788,14 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
 // products per pair (z1', z3') that occurs and two per z1' and z3', this one
 // four per pair of the (z1', z3') plane (z1' taken up to conjugation for a real
 // Hamiltonian), two per z1' and four per z3', about 15% slower each for the
-// dressing; but that form spends some 0.25 ms per part, worth
-// 5e9 operations, on its own launches and waits.  Plaquette (96 parts, 8^3):
-// 13.2 ms there, 2.0 here; 6-site ring (216 parts, blocks to 400) 9^3: 203,
-// 171; Anderson 1+5 (blocks to 400) 8^3: 163, 93; 7-site ring (blocks to 1225)
-// 4^3: 897, 1011.
+// dressing, on tiles of eight rows and columns at least; but that form spends
+// some 0.25 ms per part, worth 5e9 operations, on its own launches and waits, and
+// this one 0.15 ms per call and 2 us per (z1', z3') that occurs, worth 3e9 and
+// 4e7.  Wall times there and here: plaquette (96 parts) 8^3 12.7 and 0.88 ms, one
+// triple 9.5 and 0.48; 6-site ring (216 parts, blocks to 400) 9^3 192 and 64;
+// Anderson 1+5 (blocks to 400) 8^3 153 and 38; 7-site ring (blocks to 1225) 4^3
+// 781 and 393; one chain of 300, 2, 310 and 1 states at 25 scattered triples 0.37
+// and 0.73, of 1, 7, 2 and 9 states at 60 scattered ones 0.22 and 0.27.
 static bool anchored_faster(const Problem& P, int nparts, const pgx_g2_part* parts, int nfreq, const Points& pt) {
     double all[3], up[3], closed[3];  // values that occur; those above the axis, and all, with their conjugates
     for (int k = 0; k < 3; ++k) {
@@ -804,18 +810,22 @@ static bool anchored_faster(const Problem& P, int nparts, const pgx_g2_part* par
         if (pt.npts == pt.ncls) up[k] = all[k];
     }
     double extra = 0.0;
+    double groups[9] = {};  // pairs of a permutation's plan
     for (int q = 0; q < nparts; ++q) {
         double d[4];
-        for (int k = 0; k < 4; ++k) d[k] = P.dims[parts[q].block[k]];
+        for (int k = 0; k < 4; ++k) d[k] = std::max(8, P.dims[parts[q].block[k]]);
         const int a = parts[q].perm[0], b = parts[q].perm[2];
         const double m1 = d[0] * d[1] * d[3], m2 = d[0] * d[1] * d[2], m3 = d[0] * d[2] * d[3], m4 = d[1] * d[2] * d[3];
-        const double there = 8.0 * std::min((double)nfreq, all[a] * all[b]) * (m3 + m4) +
-                             4.0 * (all[a] * (m1 + m2) + all[b] * (m3 + m4));
+        const double pairs = std::min((double)nfreq, all[a] * all[b]);
+        const double there = 8.0 * pairs * (m3 + m4) + 4.0 * (all[a] * (m1 + m2) + all[b] * (m3 + m4));
         const double z3 = pt.npts > pt.ncls ? 0.5 * closed[b] : closed[b];  // conjugate z3 share their products
         const double here = 8.0 * up[a] * z3 * (m1 + m2 + m3 + m4) + 4.0 * up[a] * (m1 + m2) + 8.0 * z3 * (m3 + m4);
         extra += 1.15 * here - there;
+        auto& n = groups[a * 3 + b];
+        n = std::max(n, pairs);
     }
-    return extra <= 5e9 * nparts;
+    for (double n : groups) extra += 4e7 * n;
+    return extra <= 5e9 * nparts - 3e9;
 }
 
 bool run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, const double* z, double pole_res,

@@ -191,6 +191,32 @@ def test_negative_pole_resolution(kind):
         assert np.abs(v - ref).max() < 1e-12 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("dims,n", [([300, 2, 310, 1], 25), ([1, 7, 2, 9], 60)])
+def test_scattered_triples_of_one_chain_stay_in_full_matrices(dims, n):
+    """Few states in some blocks, so the batched form's products are mostly the
+    padding of their tiles, or few operations in all, so that its planning counts:
+    it took 1.3 to 1.9 times as long here."""
+    from pomerol_b200.pgx import PGX_G2_ANCHORED, PGX_G2_EXACT
+    rng = np.random.default_rng(5)
+    e = engine([symmetric(rng, k) / 4 for k in dims])
+    e.eigh()
+    e.weights(3.0)
+    ops = []
+    for q in range(4):
+        left, right = q, (q + 1) % 4
+        tgt = np.full(dims[right], -1)
+        k = min(dims[left], dims[right])
+        tgt[:k] = rng.permutation(dims[left])[:k]
+        ops.append(e.op_define([(right, left, tgt, np.where(tgt >= 0, 1.0, 0.0))]))
+        e.op_rotate(ops[-1])
+    parts = [(tuple(ops), (0, 1, 2, 3), (0, 1, 2), 1)]
+    z = rng.uniform(-2, 2, (n, 3)) + 1j * rng.uniform(0.2, 2, (n, 3))
+    v, b = batched(e, parts, z, flags=PGX_G2_EXACT)
+    assert not b
+    anchored = e.g2(parts, z, coef_tol=0.0, flags=PGX_G2_ANCHORED)
+    assert np.abs(v - anchored).max() < 1e-12 * np.abs(v).max()
+
+
 @pytest.mark.parametrize("kind", ["real", "complex"])
 @pytest.mark.parametrize("place", [0, 1, 2])
 def test_full_matrices_beside_undefined_frequencies(place, kind):
