@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(EVAL_THREADS) pair_eval_kernel(const cd* __res
                                                                   const cd* __restrict__ z, int nz, int zl, double sign,
                                                                   cd* out) {
     constexpr int NS = CX ? 4 : 2, NQ = 4 + 4 * NS;
+    static_assert(EVAL_CAP >= EVAL_THREADS * EVAL_ZPT, "the partial sums take the terms' place");
     __shared__ __align__(16) cd sR[EVAL_CAP];
     __shared__ double sP[EVAL_CAP];
     __shared__ __align__(16) double sQ[EVAL_CAP / 4][NQ];
@@ -316,15 +317,20 @@ __global__ void __launch_bounds__(EVAL_THREADS) pair_eval_kernel(const cd* __res
                 v.y -= acc[u][3];
             }
         }
-        sR[tid] = v;
-        __syncthreads();
-        const int k = z0 + u * zl;
-        if (slice == 0 && k < nz) {
-            for (int s = 1; s < nslice; ++s) v = v + sR[tid + s * zl];
-            atomicAdd(&out[zo + k].x, sign * v.x);
-            atomicAdd(&out[zo + k].y, sign * v.y);
+        // the slices of a frequency: lanes zl apart, then the warps
+        for (int o = zl; o < 32; o <<= 1) {
+            v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+            v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
         }
-        __syncthreads();
+        if (lane < zl) sR[(wid * EVAL_ZPT + u) * 32 + lane] = v;
+    }
+    __syncthreads();
+    const int k = blockIdx.y * zl * EVAL_ZPT + tid;
+    if (tid < zl * EVAL_ZPT && k < nz) {
+        cd v{0.0, 0.0};
+        for (int w2 = 0; w2 < EVAL_THREADS / 32; ++w2) v = v + sR[(w2 * EVAL_ZPT + slice) * 32 + zi];
+        atomicAdd(&out[zo + k].x, sign * v.x);
+        atomicAdd(&out[zo + k].y, sign * v.y);
     }
 }
 
@@ -587,17 +593,35 @@ static void run_pair(pgx_ctx* c, int op1, int op2, int nparts, const int32_t* ou
     }
     DevBuf& bR = c->scratch[0];
     DevBuf& bP = c->scratch[1];
-    DevBuf& bparts = c->scratch[2];
-    DevBuf& bz = c->scratch[3];
+    DevBuf& bin = c->scratch[2];
     DevBuf& bout = c->scratch[4];
     bR.reserve(std::max<long>(nterms, 1) * sizeof(cd));
     bP.reserve(std::max<long>(nterms, 1) * sizeof(double));
-    bparts.reserve(std::max<size_t>(pp.size(), 1) * sizeof(PairPart));
-    bz.reserve(std::max(nz, 1) * sizeof(cd));
     bout.reserve((std::max(nz, 1) + 1) * sizeof(cd));
-    if (!pp.empty())
-        h2d(bparts.p, pp.data(), pp.size() * sizeof(PairPart), st);
-    if (nz > 0) h2d(bz.p, z, nz * sizeof(cd), st);
+    std::vector<EvalChunk> chunks;
+    if (nz > 0 && nterms > 0) {
+        const int len = eval_chunk(nterms, nz);
+        for (long t = 0; t < nterms; t += len) chunks.push_back(EvalChunk{t, (int)std::min<long>(len, nterms - t), 0});
+        PGX_CHECK(chunks.size() < (1u << 31), PGX_ERR_ARG, "too many Lehmann terms for one call");
+    }
+    // Frequencies, chunks and parts in one upload, as each costs a small call
+    // about 5 us; many frequencies in one of their own, as the copy costs more.
+    const bool apart = nz > 512;
+    const size_t z_b = apart ? 0 : nz * sizeof(cd), ch_b = chunks.size() * sizeof(EvalChunk), pp_b = pp.size() * sizeof(PairPart);
+    static_assert(sizeof(EvalChunk) % 8 == 0 && alignof(PairPart) <= 8, "laid out one after another");
+    std::vector<char> in(z_b + ch_b + pp_b);
+    if (z_b) std::memcpy(in.data(), z, z_b);
+    if (ch_b) std::memcpy(in.data() + z_b, chunks.data(), ch_b);
+    if (pp_b) std::memcpy(in.data() + z_b + ch_b, pp.data(), pp_b);
+    bin.reserve(std::max<size_t>(in.size(), 1));
+    h2d(bin.p, in.data(), in.size(), st);
+    if (apart) {
+        c->scratch[3].reserve(nz * sizeof(cd));
+        h2d(c->scratch[3].p, z, nz * sizeof(cd), st);
+    }
+    const cd* d_z = (apart ? c->scratch[3] : bin).as<cd>();
+    const EvalChunk* d_chunks = reinterpret_cast<const EvalChunk*>(bin.as<char>() + z_b);
+    const PairPart* d_parts = reinterpret_cast<const PairPart*>(bin.as<char>() + z_b + ch_b);
     PGX_CUDA(cudaMemsetAsync(bout.p, 0, (nz + 1) * sizeof(cd), st));
     cd* d_out = bout.as<cd>();
     double* d_zero = reinterpret_cast<double*>(d_out + nz);
@@ -606,25 +630,18 @@ static void run_pair(pgx_ctx* c, int op1, int op2, int nparts, const int32_t* ou
         for (auto& x : pp) maxn = std::max(maxn, (long)x.d_o * x.d_i);
         dim3 g1(std::min(ceil_div(maxn, 256), 512), (unsigned)pp.size());
         if (P.is_complex)
-            pair_terms_kernel<cd><<<g1, 256, 0, st>>>(bparts.as<PairPart>(), (int)pp.size(), A.mat.as<cd>(),
-                                                      B.mat.as<cd>(), P.d_E, P.d_w, coef_tol, pole_res, mode,
-                                                      bR.as<cd>(), bP.as<double>(), d_zero);
+            pair_terms_kernel<cd><<<g1, 256, 0, st>>>(d_parts, (int)pp.size(), A.mat.as<cd>(), B.mat.as<cd>(), P.d_E,
+                                                      P.d_w, coef_tol, pole_res, mode, bR.as<cd>(), bP.as<double>(),
+                                                      d_zero);
         else
-            pair_terms_kernel<double><<<g1, 256, 0, st>>>(bparts.as<PairPart>(), (int)pp.size(), A.mat.as<double>(),
+            pair_terms_kernel<double><<<g1, 256, 0, st>>>(d_parts, (int)pp.size(), A.mat.as<double>(),
                                                           B.mat.as<double>(), P.d_E, P.d_w, coef_tol, pole_res, mode,
                                                           bR.as<cd>(), bP.as<double>(), d_zero);
         check_launch("pair_terms_kernel");
         if (nz > 0) {
-            const int len = eval_chunk(nterms, nz);
-            std::vector<EvalChunk> chunks;
-            for (long t = 0; t < nterms; t += len) chunks.push_back(EvalChunk{t, (int)std::min<long>(len, nterms - t), 0});
-            PGX_CHECK(chunks.size() < (1u << 31), PGX_ERR_ARG, "too many Lehmann terms for one call");
-            DevBuf& bch = c->scratch[5];
-            bch.reserve(chunks.size() * sizeof(EvalChunk));
-            h2d(bch.p, chunks.data(), chunks.size() * sizeof(EvalChunk), st);
             ProfRange pr("pair_eval_kernel", st, 12.0 * (double)nterms * nz, 24.0 * nterms);
-            launch_pair_eval(P.is_complex, (unsigned)chunks.size(), bR.as<cd>(), bP.as<double>(), bch.as<EvalChunk>(),
-                             bz.as<cd>(), nz, sign, d_out, st);
+            launch_pair_eval(P.is_complex, (unsigned)chunks.size(), bR.as<cd>(), bP.as<double>(), d_chunks, d_z, nz, sign,
+                             d_out, st);
         }
     }
     std::vector<cd> h(nz + 1);
