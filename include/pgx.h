@@ -101,8 +101,10 @@ int pgx_get_hamiltonian(pgx_ctx* ctx, double* H);
  * assumes the perturbation of H stays symmetric), and, when dE is non-NULL,
  * dL/dE_s for every state.  op1 and op2 are operators defined by their Fock
  * action or adjoints of such operators.  Real Hamiltonians only; derivative
- * terms between eigenvalues closer than 1e-10 max|E| are dropped (exact for
- * G, which does not depend on the basis of a degenerate subspace). */
+ * terms between eigenvalues closer than 1e-10 max|E| are dropped.  G does not
+ * depend on the basis of a degenerate subspace, but the mixing of its levels
+ * at first order is left out with them: where a block has exact degeneracies,
+ * lift them (a plaquette's gradients are 1 to 2% off without). */
 int pgx_gf_vjp(pgx_ctx* ctx, int32_t op1, int32_t op2, int32_t nparts, const int32_t* outer, const int32_t* inner,
                int32_t nz, const double* z, const double* lambda, double* dterm, double* dE);
 
@@ -417,7 +419,7 @@ long long pgx_launch_count(void);
 int pgx_g2_last_timing(pgx_ctx* ctx, double* total_ms, double* gemm_ms, double* gemm_flops);
 
 /* Numerics check of the device reciprocal used in the Lehmann kernels
- * (Newton-Raphson from a single-precision seed): out[i] = 1/x[i] for x[i] > 0,
+ * (one third-order step from the hardware's approximation): out[i] = 1/x[i] for x[i] > 0,
  * host arrays, computed on the current device. */
 int pgx_recip_check(const double* x, int32_t n, double* out);
 

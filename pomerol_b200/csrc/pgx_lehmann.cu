@@ -158,7 +158,9 @@ __global__ void pair_terms_kernel(const PairPart* parts, int nparts, const T* m1
 // used at every frequency of the tile: 4 + 2 * 3 + 3 (reciprocal) + 2 = 15
 // FP64 operations for four terms of a real residue, against 7 per term with a
 // reciprocal each.  Off the axis, or where D could leave the double range,
-// each term keeps its own reciprocal.  64 models of 3 to 6 bath sites, G on
+// each term keeps its own reciprocal.  On one eigensystem a plaquette's G is 2.2e-16
+// of its norm off long double sums, 3.5e-16 with a division per term.  64 models of
+// 3 to 6 bath sites, G on
 // 1024 and chi on 32 frequencies: 56 ms, against 201 ms with an IEEE division
 // per term and one frequency per thread; a plaquette's G on 256 and chi on 16
 // frequencies, whose few terms now also spread over the GPU: 0.11 ms a pair of

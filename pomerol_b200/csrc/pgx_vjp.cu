@@ -20,9 +20,10 @@
 // derivative results for forward and reverse mode algorithmic
 // differentiation", 2008, sec. 3.1)
 //   Hbar = U (diag(Ebar) + F o (U^T Ubar)) U^T,  F_ij = 1 / (E_j - E_i), i != j,
-// symmetrised; F is set to zero between eigenvalues closer than 1e-10 max|E|
-// (G does not depend on the basis inside a degenerate subspace, so those
-// terms cancel).  Finally dL/dc_t = sum over columns j of the terms' Fock
+// symmetrised; F is set to zero between eigenvalues closer than 1e-10 max|E|.
+// (G does not depend on the basis inside a degenerate subspace, but its levels
+// mix at first order there, which this leaves out: on a plaquette with exact
+// degeneracies the gradient is 1 to 2% off central differences.)  Finally dL/dc_t = sum over columns j of the terms' Fock
 // action sign * Hbar_sym[o][j], the transpose of the Hamiltonian assembly.
 
 #include <cfloat>
