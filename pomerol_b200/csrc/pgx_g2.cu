@@ -29,9 +29,9 @@
 #include <tuple>
 
 #include "pgx_common.cuh"
+#include "pgx_g2plan.h"
 #include "pgx_gemm.cuh"
 #include "pgx_internal.h"
-#include "pgx_numbers.h"
 
 namespace pgx {
 
@@ -326,27 +326,23 @@ struct Plan {
     int *dpi1, *dpi3, *dptr, *dslot;
 };
 
-void build_plan(Plan& pl, const int perm[3], int nfreq, const double* z) {
-    std::map<std::pair<int, int>, int> mp;
-    std::vector<int> tp(nfreq);
-    std::vector<cd> zz1(nfreq), zz2(nfreq), zz3(nfreq);
+void build_plan(Plan& pl, const int perm[3], int nfreq, const Values& v) {
+    const std::vector<int>&i1 = v.id[perm[0]], &i2 = v.id[perm[1]], &i3 = v.id[perm[2]];
+    const std::vector<cd>&v1 = v.val[perm[0]], &v2 = v.val[perm[1]], &v3 = v.val[perm[2]];
+    const size_t n3 = v.occur[perm[2]], cells = v.occur[perm[0]] * n3;
+    pl.Z1.assign(v1.begin(), v1.begin() + v.occur[perm[0]]);
+    pl.Z3.assign(v3.begin(), v3.begin() + n3);
+    std::vector<int> dense(cells <= (size_t(1) << 20) ? cells : 0, -1), tp(nfreq);
+    std::unordered_map<size_t, int> sparse;
     for (int t = 0; t < nfreq; ++t) {
-        const cd F[3] = {cd{z[6 * t], z[6 * t + 1]}, cd{z[6 * t + 2], z[6 * t + 3]}, cd{-z[6 * t + 4], -z[6 * t + 5]}};
-        const cd a = F[perm[0]], b = F[perm[1]], c3 = F[perm[2]];
-        zz1[t] = a;
-        zz2[t] = b;
-        zz3[t] = c3;
-    }
-    std::vector<int> i1, i3;
-    distinct_index(zz1, pl.Z1, i1);
-    distinct_index(zz3, pl.Z3, i3);
-    for (int t = 0; t < nfreq; ++t) {
-        auto ip = mp.emplace(std::make_pair(i1[t], i3[t]), (int)pl.pi1.size());
-        if (ip.second) {
+        const size_t cell = (size_t)i1[t] * n3 + i3[t];
+        int& q = dense.empty() ? sparse.emplace(cell, -1).first->second : dense[cell];
+        if (q < 0) {
+            q = (int)pl.pi1.size();
             pl.pi1.push_back(i1[t]);
             pl.pi3.push_back(i3[t]);
         }
-        tp[t] = ip.first->second;
+        tp[t] = q;
     }
     const int np = (int)pl.pi1.size();
     pl.ptr.assign(np + 1, 0);
@@ -361,10 +357,11 @@ void build_plan(Plan& pl, const int perm[3], int nfreq, const double* z) {
     for (int t = 0; t < nfreq; ++t) {
         const int k = fill[tp[t]]++;
         pl.slot[k] = t;
-        pl.s1[k] = zz2[t];
-        pl.s2[k] = zz1[t] + zz2[t] + zz3[t];
-        pl.s3[k] = zz1[t] + zz2[t];
-        pl.s4[k] = zz2[t] + zz3[t];
+        const cd a = v1[i1[t]], b = v2[i2[t]], d = v3[i3[t]];
+        pl.s1[k] = b;
+        pl.s2[k] = a + b + d;
+        pl.s3[k] = a + b;
+        pl.s4[k] = b + d;
     }
 }
 
@@ -569,7 +566,9 @@ void run_g2(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, const d
         PGX_CUDA(cudaEventRecord(a0, st));
         const int split = (flags & PGX_G2_SPLIT_I8) ? c->g2_split_slices : 0;
         if (split && c->oz.err.p) PGX_CUDA(cudaMemsetAsync(c->oz.err.p, 0, sizeof(int), st));
-        run_g2_anchored(c, nparts, parts, nfreq, z, pole_res, coef_tol, split, false, out);
+        Values values;
+        number_values(values, nfreq, z, !P.is_complex);
+        run_g2_anchored(c, nparts, parts, nfreq, std::move(values), pole_res, coef_tol, split, false, out);
         if (split && c->oz.err.p) {
             int e = 0;
             PGX_CUDA(cudaMemcpy(&e, c->oz.err.p, sizeof(int), cudaMemcpyDeviceToHost));
@@ -589,8 +588,10 @@ void run_g2(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, const d
     PGX_CUDA(cudaEventRecord(ea, st));
     // the same sum with every state an anchor (weights are positive or zero)
     c->g2t = G2Timing{};
-    if (!(flags & PGX_G2_FULL_MATRICES) && nfreq > 0 && nparts > 0 &&
-        run_g2_anchored(c, nparts, parts, nfreq, z, pole_res, -1.0, 0, true, out)) {
+    Values values;
+    number_values(values, nfreq, z, !P.is_complex);
+    if (!(flags & PGX_G2_FULL_MATRICES) && nfreq > 0 && nparts > 0 && anchored_faster(P, nparts, parts, nfreq, values)) {
+        run_g2_anchored(c, nparts, parts, nfreq, std::move(values), pole_res, -1.0, 0, true, out);
         PGX_CUDA(cudaEventRecord(eb, st));
         PGX_CUDA(cudaEventSynchronize(eb));
         float tot = 0.f;
@@ -614,7 +615,7 @@ void run_g2(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, const d
     }
     for (auto& kv : perm_id) {
         const int perm[3] = {std::get<0>(kv.first), std::get<1>(kv.first), std::get<2>(kv.first)};
-        build_plan(plans[kv.second], perm, nfreq, z);
+        build_plan(plans[kv.second], perm, nfreq, values);
         upload_plan(plans[kv.second], st);
     }
     // workspace: the largest part decides

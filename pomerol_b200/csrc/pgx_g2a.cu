@@ -789,25 +789,27 @@ static void run_batch(pgx_ctx* c, const std::vector<int>& idx, const std::vector
 // four per pair of the (z1', z3') plane (z1' taken up to conjugation for a real
 // Hamiltonian), two per z1' and four per z3', about 15% slower each for the
 // dressing, on tiles of eight rows and columns at least; but that form spends
-// some 0.25 ms per part, worth 5e9 operations, on its own launches and waits, and
-// this one 0.15 ms per call and 2 us per (z1', z3') that occurs, worth 3e9 and
-// 4e7.  Wall times there and here: plaquette (96 parts) 8^3 12.7 and 0.88 ms, one
-// triple 9.5 and 0.48; 6-site ring (216 parts, blocks to 400) 9^3 192 and 64;
-// Anderson 1+5 (blocks to 400) 8^3 153 and 38; 7-site ring (blocks to 1225) 4^3
-// 781 and 393; one chain of 300, 2, 310 and 1 states at 25 scattered triples 0.37
-// and 0.73, of 1, 7, 2 and 9 states at 60 scattered ones 0.22 and 0.27.
-static bool anchored_faster(const Problem& P, int nparts, const pgx_g2_part* parts, int nfreq, const Points& pt) {
+// some 0.12 ms per part, worth 3e9 operations, on its own launches and waits, and
+// 30 ns per triple of a permutation's plan, this one 0.08 ms per call and 1 us
+// per (z1', z3') that occurs.  Over 410 lists (cubes to 32^3, parts of them,
+// scattered ones; one, six or all parts of models of 1 to 5 sites) the choice
+// is 2% off the better one in the mean; the worst are 1.8 times the full matrices'
+// time (one chain, 1024 triples of one z1) and 2.3 times this form's (one chain of
+// 100 states, 16^3).  Wall times there and here: plaquette (96 parts) 8^3 12.5 and
+// 0.87 ms, one triple 9.3 and 0.46; 6-site ring (216 parts, blocks to 400) 9^3 190
+// and 64; Anderson 1+5 (blocks to 400) 8^3 153 and 38; 7-site ring (blocks to
+// 1225) 4^3 779 and 393; an atom's 64^3 grid 93 and 77, a tenth of it 14 and 76;
+// one chain of 300, 2, 310 and 1 states at 25 scattered triples 0.38 and 0.73, of
+// 1, 7, 2 and 9 states at 60 scattered ones 0.22 and 0.27.
+bool anchored_faster(const Problem& P, int nparts, const pgx_g2_part* parts, int nfreq, const Values& v) {
+    const bool real = !P.is_complex;
     double all[3], up[3], closed[3];  // values that occur; those above the axis, and all, with their conjugates
     for (int k = 0; k < 3; ++k) {
-        std::vector<char> direct(pt.val[k].size(), 0);
-        for (int t = 0; t < nfreq; ++t)
-            if (!pt.flip[t]) direct[pt.id[k][pt.cls[t]]] = 1;
-            else direct[pt.id[k][pt.ncls + pt.cls[t]]] = 1;
-        all[k] = (double)std::count(direct.begin(), direct.end(), 1);
-        closed[k] = (double)pt.val[k].size();
+        all[k] = v.occur[k];
+        closed[k] = (double)v.val[k].size();
         up[k] = 0.0;
-        for (const cd& v : pt.val[k]) up[k] += v.y >= 0.0;
-        if (pt.npts == pt.ncls) up[k] = all[k];
+        for (const cd& x : v.val[k]) up[k] += x.y >= 0.0;
+        if (!real) up[k] = all[k];
     }
     double extra = 0.0;
     double groups[9] = {};  // pairs of a permutation's plan
@@ -818,23 +820,23 @@ static bool anchored_faster(const Problem& P, int nparts, const pgx_g2_part* par
         const double m1 = d[0] * d[1] * d[3], m2 = d[0] * d[1] * d[2], m3 = d[0] * d[2] * d[3], m4 = d[1] * d[2] * d[3];
         const double pairs = std::min((double)nfreq, all[a] * all[b]);
         const double there = 8.0 * pairs * (m3 + m4) + 4.0 * (all[a] * (m1 + m2) + all[b] * (m3 + m4));
-        const double z3 = pt.npts > pt.ncls ? 0.5 * closed[b] : closed[b];  // conjugate z3 share their products
+        const double z3 = real ? 0.5 * closed[b] : closed[b];  // conjugate z3 share their products
         const double here = 8.0 * up[a] * z3 * (m1 + m2 + m3 + m4) + 4.0 * up[a] * (m1 + m2) + 8.0 * z3 * (m3 + m4);
         extra += 1.15 * here - there;
         auto& n = groups[a * 3 + b];
         n = std::max(n, pairs);
     }
-    for (double n : groups) extra += 4e7 * n;
-    return extra <= 5e9 * nparts - 3e9;
+    for (double n : groups)
+        if (n > 0.0) extra += 2.5e7 * n - 7.5e5 * nfreq;
+    return extra <= 3e9 * nparts - 2e9;
 }
 
-bool run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, const double* z, double pole_res,
-                     double anchor_tol, int split, bool only_if_faster, double* out) {
+void run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, Values values, double pole_res,
+                     double anchor_tol, int split, bool exact, double* out) {
     Problem& P = c->P;
     cudaStream_t st = c->stream;
     Points pt;
-    build_points(pt, nfreq, z, !P.is_complex);
-    if (only_if_faster && !anchored_faster(P, nparts, parts, nfreq, pt)) return false;
+    build_points(pt, std::move(values), nfreq, !P.is_complex);
     // anchor states per block (weights above the threshold)
     const std::vector<double>& w = P.w_host;  // copied when the weights were computed
     PGX_CHECK((long)w.size() == P.esize, PGX_ERR_STATE, "pgx_weights first");
@@ -983,7 +985,7 @@ bool run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq
     std::vector<ChainWs> bws;
     // the full sum reports the time and operations of its products
     std::vector<cudaEvent_t> gemm_ev;
-    std::vector<cudaEvent_t>* ev = only_if_faster ? &gemm_ev : nullptr;
+    std::vector<cudaEvent_t>* ev = exact ? &gemm_ev : nullptr;
     long used = 0;
     auto flush = [&]() {
         if (batch.empty()) return;
@@ -1024,7 +1026,7 @@ bool run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq
         out[2 * (size_t)t] = v.x;
         out[2 * (size_t)t + 1] = v.y;
     }
-    if (only_if_faster) {
+    if (exact) {
         for (size_t i = 0; i + 1 < gemm_ev.size(); i += 2) {
             float ms = 0.f;
             PGX_CUDA(cudaEventElapsedTime(&ms, gemm_ev[i], gemm_ev[i + 1]));
@@ -1032,7 +1034,6 @@ bool run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq
         }
         for (cudaEvent_t e : gemm_ev) c->prof.spare.push_back(e);
     }
-    return true;
 }
 
 }  // namespace pgx

@@ -30,6 +30,15 @@ struct CClass {
 };
 constexpr int CG_BN_MAX = 32;  // columns of a class; one with more is split into column chunks
 
+// The values of z1, z2 and -z3 in a call, numbered per axis, those that occur
+// first; for a real Hamiltonian their conjugates after them.
+struct Values {
+    std::vector<cd> val[3];
+    std::vector<int> cj[3];  // value -> its conjugate
+    std::vector<int> id[3];  // triple -> value
+    int occur[3] = {0, 0, 0};
+};
+
 // The evaluation points of a call.  Values of z1, z2 and -z3 are numbered per
 // axis (`val`), and a point is three numbers (`id`).  For a real Hamiltonian
 // every matrix element and energy is real, so a part's sum at the conjugate
@@ -54,29 +63,40 @@ struct Points {
     cd at(int axis, int e) const { return val[axis][id[axis][e]]; }
 };
 
-inline void build_points(Points& pt, int nfreq, const double* z, bool real) {
-    std::vector<int> tid[3];
-    auto& cj = pt.cj;
+inline void number_values(Values& v, int nfreq, const double* z, bool real) {
     for (int k = 0; k < 3; ++k) {
         CdMap seen;
-        auto number = [&](cd v) {
-            const auto it = seen.emplace(cd_key(v), (int)pt.val[k].size());
-            if (it.second) pt.val[k].push_back(cd{v.x + 0.0, v.y + 0.0});
+        auto& val = v.val[k];
+        auto& tid = v.id[k];
+        auto& cj = v.cj[k];
+        auto number = [&](cd x) {
+            const auto it = seen.emplace(cd_key(x), (int)val.size());
+            if (it.second) val.push_back(cd{x.x + 0.0, x.y + 0.0});
             return it.first->second;
         };
         const double s = k == 2 ? -1.0 : 1.0;
-        tid[k].resize(nfreq);
+        tid.resize(nfreq);
         for (int t = 0; t < nfreq; ++t) {
             const double* p = z + 6 * (size_t)t + 2 * k;
-            tid[k][t] = t > 0 && p[0] == p[-6] && p[1] == p[-5] ? tid[k][t - 1] : number(cd{s * p[0], s * p[1]});
+            tid[t] = t > 0 && p[0] == p[-6] && p[1] == p[-5] ? tid[t - 1] : number(cd{s * p[0], s * p[1]});
         }
+        v.occur[k] = (int)val.size();
         if (real)
-            for (size_t i = 0; i < pt.val[k].size(); ++i) {
-                const int j = number(conj(pt.val[k][i]));
-                cj[k].resize(std::max(cj[k].size(), std::max(i, (size_t)j) + 1));
-                cj[k][i] = j;
-                cj[k][j] = (int)i;
+            for (size_t i = 0; i < val.size(); ++i) {
+                const int j = number(conj(val[i]));
+                cj.resize(std::max(cj.size(), std::max(i, (size_t)j) + 1));
+                cj[i] = j;
+                cj[j] = (int)i;
             }
+    }
+}
+
+inline void build_points(Points& pt, Values v, int nfreq, bool real) {
+    std::vector<int>* tid = v.id;
+    auto& cj = pt.cj;
+    for (int k = 0; k < 3; ++k) {
+        pt.val[k] = std::move(v.val[k]);
+        pt.cj[k] = std::move(v.cj[k]);
     }
     pt.cls.resize(nfreq);
     pt.flip.assign(nfreq, 0);
@@ -112,6 +132,11 @@ inline void build_points(Points& pt, int nfreq, const double* z, bool real) {
             pt.id[k][pt.ncls + u] = cj[k][tid[k][rep[u]]];
         }
     }
+}
+inline void build_points(Points& pt, int nfreq, const double* z, bool real) {
+    Values v;
+    number_values(v, nfreq, z, real);
+    build_points(pt, std::move(v), nfreq, real);
 }
 
 // The points a permutation evaluates (one per class), their distinct z1' and

@@ -403,9 +403,12 @@ void run_susc(pgx_ctx* c, int opA, int opB, int nparts, const int32_t* outer, co
 void run_ensemble_average(pgx_ctx* c, int op, double* out);
 void run_g2(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, const double* z, double pole_res,
             double coef_tol, int flags, double* out);
-// only_if_faster: returns false, nothing done, where the form of pgx_g2.cu is faster
-bool run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, const double* z, double pole_res,
-                     double anchor_tol, int split_slices, bool only_if_faster, double* out);
+struct Values;  // the numbered frequencies of a call (pgx_g2plan.h)
+// exact: the sum over every state, whose products' time and operations are reported
+void run_g2_anchored(pgx_ctx* c, int nparts, const pgx_g2_part* parts, int nfreq, Values values, double pole_res,
+                     double anchor_tol, int split_slices, bool exact, double* out);
+// whether the exact sum is faster there than in the form of pgx_g2.cu
+bool anchored_faster(const Problem& P, int nparts, const pgx_g2_part* parts, int nfreq, const Values& v);
 void run_split_gemm_check(pgx_ctx* c, int M, int N, int K, int nb, int S, unsigned long long seed, double* err,
                           double* ms_split, double* ms_fp64);
 void run_chi3(pgx_ctx* c, int channel, int nparts, const pgx_chi3_part* parts, int nfreq, const double* z,
