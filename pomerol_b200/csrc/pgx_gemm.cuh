@@ -580,11 +580,10 @@ void launch_gemm_batch(const std::vector<GemmProblem<TA, TB, TC>>& probs, void* 
     if (probs.empty()) return;
     if (active_recorder()) record_gemm_batch(probs, st);
     std::vector<GemmProblem<TA, TB, TC>> sorted;
-    sorted.reserve(probs.size());
     std::vector<int> index;  // per class: prefix over its problems, then the total
-    index.reserve(probs.size() + 2 * GEMM_NCLS_ALL);
-    size_t pstart[GEMM_NCLS_ALL + 1] = {}, istart[GEMM_NCLS_ALL] = {};
+    size_t pstart[GEMM_NCLS_ALL + 1] = {}, istart[GEMM_NCLS_ALL] = {}, at[GEMM_NCLS_ALL];
     int ntiles[GEMM_NCLS_ALL] = {};
+    long tiles[GEMM_NCLS_ALL] = {};
     std::vector<int> cls(probs.size());
     for (size_t q = 0; q < probs.size(); ++q) {
         const auto& g = probs[q];
@@ -593,22 +592,29 @@ void launch_gemm_batch(const std::vector<GemmProblem<TA, TB, TC>>& probs, void* 
         cls[q] = gemm_class_for(g);
     }
     gemm_join_small(probs, cls);
-    for (int c = 0; c < GEMM_NCLS_ALL; ++c) {
-        pstart[c] = sorted.size();
-        istart[c] = index.size();
-        long t = 0;
-        for (size_t q = 0; q < probs.size(); ++q) {
-            const auto& g = probs[q];
-            if (g.M <= 0 || g.N <= 0 || cls[q] != c) continue;
-            sorted.push_back(g);
-            index.push_back((int)t);
-            t += (long)std::max(g.nb, 1) * ceil_div(g.M, GEMM_CLS_M[c]) * ceil_div(g.N, GEMM_CLS_N[c]);
-        }
-        PGX_CHECK(t < (1L << 31), PGX_ERR_ARG, "gemm batch too large");
-        index.push_back((int)t);
-        ntiles[c] = (int)t;
+    for (size_t q = 0; q < probs.size(); ++q) {
+        if (probs[q].M <= 0 || probs[q].N <= 0) cls[q] = -1;
+        else ++pstart[cls[q] + 1];
     }
-    pstart[GEMM_NCLS_ALL] = sorted.size();
+    for (int c = 0; c < GEMM_NCLS_ALL; ++c) {
+        pstart[c + 1] += pstart[c];
+        at[c] = pstart[c];
+        istart[c] = pstart[c] + c;
+    }
+    sorted.resize(pstart[GEMM_NCLS_ALL]);
+    index.resize(sorted.size() + GEMM_NCLS_ALL);
+    for (size_t q = 0; q < probs.size(); ++q) {
+        const int c = cls[q];
+        if (c < 0) continue;
+        const auto& g = probs[q];
+        sorted[at[c]] = g;
+        index[at[c]++ + c] = (int)tiles[c];
+        tiles[c] += (long)std::max(g.nb, 1) * ceil_div(g.M, GEMM_CLS_M[c]) * ceil_div(g.N, GEMM_CLS_N[c]);
+    }
+    for (int c = 0; c < GEMM_NCLS_ALL; ++c) {
+        PGX_CHECK(tiles[c] < (1L << 31), PGX_ERR_ARG, "gemm batch too large");
+        index[pstart[c + 1] + c] = ntiles[c] = (int)tiles[c];
+    }
     if (sorted.empty()) return;
     PGX_CHECK(sorted.size() * sizeof(sorted[0]) <= probs_cap, PGX_ERR_ARG, "gemm problem list overflow");
     PGX_CHECK(index.size() * sizeof(int) <= index_cap, PGX_ERR_ARG, "gemm tile index overflow");
